@@ -824,6 +824,9 @@ int x2_scene_load(x2_ctx* ctx, const x2_scene_desc* d, x2_scene** out) {
             r.hi = V3{x.bound_hi[0], x.bound_hi[1], x.bound_hi[2]};
             r.majorant = nullptr;
             r.majorantMax = 0.0f;
+            r.diagonal = 1;
+            for (int i = 0; i < 12; ++i)
+                if (i % 4 != 3 && i % 4 != i / 4 && x.world_to_grid[i] != 0.0f) r.diagonal = 0;
             if (!(x.gain[0] == x.gain[1] && x.gain[1] == x.gain[2])) s->greyVolumes = false;
             for (const auto& t : kBox)
                 for (int k = 0; k < 3; ++k)
@@ -845,6 +848,9 @@ int x2_scene_load(x2_ctx* ctx, const x2_scene_desc* d, x2_scene** out) {
             r.values = s->gridValues[g];
             for (int a = 0; a < 3; ++a) r.lo[a] = x.lo[a], r.dims[a] = x.dims[a];
             r.channels = x.channels;
+            r.diagonal = 1;
+            for (int i = 0; i < 12; ++i)
+                if (i % 4 != 3 && i % 4 != i / 4 && x.world_to_index[i] != 0.0) r.diagonal = 0;
         }
         // Each volume's majorant grid for the tracking estimator.
         std::vector<std::vector<float>> majorant(d->volume_count);

@@ -99,12 +99,14 @@ struct VolumeRec {
     V3 lo, hi;              // its bounds (world)
     const float* majorant;  // the largest extinction any lookup can read in each cell (the tracking estimator's)
     float majorantMax;
+    uint32_t diagonal;      // worldToGrid scales and moves each axis only (its other entries are zero)
 };
 struct GridRec {
     double worldToIndex[16];
     const float* values;
     int lo[3], dims[3];
     uint32_t channels;
+    uint32_t diagonal;  // worldToIndex scales and moves each axis only (its other entries are zero)
 };
 
 struct SceneView {

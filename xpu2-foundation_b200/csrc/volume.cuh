@@ -45,15 +45,27 @@ __device__ __forceinline__ V3 vtimes(V3 a, V3 b) { return V3{a.x * b.x, a.y * b.
 __device__ __forceinline__ V3 vscaled(V3 a, float s) { return V3{a.x * s, a.y * s, a.z * s}; }
 __device__ __forceinline__ V3 vplus(V3 a, V3 b) { return V3{a.x + b.x, a.y + b.y, a.z + b.z}; }
 __device__ __forceinline__ V3 cmax0(V3 a) { return V3{fmaxf(a.x, 0.0f), fmaxf(a.y, 0.0f), fmaxf(a.z, 0.0f)}; }
-__device__ __forceinline__ V3 expNeg(V3 a, float s) { return V3{mf::exp(-a.x * s), mf::exp(-a.y * s), mf::exp(-a.z * s)}; }
+// Grey extinction (three equal channels) takes one exponential: equal arguments have equal results.
+__device__ __forceinline__ V3 expNeg(V3 a, float s) {
+    const float x = mf::exp(-a.x * s);
+    if (a.y == a.x && a.z == a.x) return V3{x, x, x};
+    return V3{x, mf::exp(-a.y * s), mf::exp(-a.z * s)};
+}
 __device__ __forceinline__ float vlum(V3 a) { return 0.299f * a.x + 0.587f * a.y + 0.114f * a.z; }
 __device__ __forceinline__ bool vblack(V3 a) { return a.x == 0.0f && a.y == 0.0f && a.z == 0.0f; }
 __device__ __forceinline__ bool vIsZero(float x) { return fabsf(x) < kVolumeEpsilon; }
 __device__ __forceinline__ bool vfinite(float x) { return x - x == 0.0f; }
 
 // ---- dense grids (volume_grid.h:42-134): OpenVDB's world-to-index in doubles, point / box / quadratic sampling ----
+// A diagonal map (GridRec::diagonal) leaves out the products with its zeros: they add signed zeros to finite sums.
 __device__ __forceinline__ void gridIndex(const GridRec& g, V3 p, double out[3]) {
     const double* m = g.worldToIndex;
+    if (g.diagonal) {
+        out[0] = double(p.x) * m[0] + m[12];
+        out[1] = double(p.y) * m[5] + m[13];
+        out[2] = double(p.z) * m[10] + m[14];
+        return;
+    }
     for (int c = 0; c < 3; ++c) out[c] = double(p.x) * m[0 * 4 + c] + double(p.y) * m[1 * 4 + c] + double(p.z) * m[2 * 4 + c] + m[3 * 4 + c];
 }
 __device__ __forceinline__ float voxel(const GridRec& g, int i, int j, int k, int c) {
@@ -75,9 +87,19 @@ static __device__ __noinline__ float sampleGrid(const GridRec& g, V3 p, uint32_t
     const double u = ip[0] - i0, v = ip[1] - j0, w = ip[2] - k0;
     if (mode == kInterpBox) {
         float d[2][2][2];
-        for (int i = 0; i < 2; ++i)
-            for (int j = 0; j < 2; ++j)
-                for (int k = 0; k < 2; ++k) d[i][j][k] = voxel(g, i0 + i, j0 + j, k0 + k, c);
+        const int x = i0 - g.lo[0], y = j0 - g.lo[1], z = k0 - g.lo[2];
+        if (x >= 0 && y >= 0 && z >= 0 && x < g.dims[0] - 1 && y < g.dims[1] - 1 && z < g.dims[2] - 1) {
+            // All eight voxels inside the grid: one base address, no bounds check a voxel.
+            const size_t sx = g.channels, sy = sx * size_t(g.dims[0]), sz = sy * size_t(g.dims[1]);
+            const float* q = g.values + sz * size_t(z) + sy * size_t(y) + sx * size_t(x) + c;
+            for (int i = 0; i < 2; ++i)
+                for (int j = 0; j < 2; ++j)
+                    for (int k = 0; k < 2; ++k) d[i][j][k] = __ldg(q + i * sx + j * sy + k * sz);
+        } else {
+            for (int i = 0; i < 2; ++i)
+                for (int j = 0; j < 2; ++j)
+                    for (int k = 0; k < 2; ++k) d[i][j][k] = voxel(g, i0 + i, j0 + j, k0 + k, c);
+        }
         return boxLerp(boxLerp(boxLerp(d[0][0][0], d[0][0][1], w), boxLerp(d[0][1][0], d[0][1][1], w), v),
                        boxLerp(boxLerp(d[1][0][0], d[1][0][1], w), boxLerp(d[1][1][0], d[1][1][1], w), v), u);
     }
@@ -102,14 +124,25 @@ struct VolumeLocal {
 __device__ __forceinline__ V3 affine34(const float* m, V3 p) {
     return V3{m[0] * p.x + m[1] * p.y + m[2] * p.z + m[3], m[4] * p.x + m[5] * p.y + m[6] * p.z + m[7], m[8] * p.x + m[9] * p.y + m[10] * p.z + m[11]};
 }
-__device__ __forceinline__ VolumeLocal localAt(const SceneView& s, const VolumeRec& v, V3 p, uint32_t interpolation) {
-    const V3 gp = affine34(v.worldToGrid, p);
+__device__ __forceinline__ V3 gridSpace(const VolumeRec& v, V3 p) {
+    if (v.diagonal) return V3{v.worldToGrid[0] * p.x + v.worldToGrid[3], v.worldToGrid[5] * p.y + v.worldToGrid[7], v.worldToGrid[10] * p.z + v.worldToGrid[11]};
+    return affine34(v.worldToGrid, p);
+}
+// A three-channel grid's nearest voxel: one index for the three channels.
+static __device__ __noinline__ V3 samplePoint3(const GridRec& g, V3 p) {
+    double ip[3];
+    gridIndex(g, p, ip);
+    const int i = int(round(ip[0])), j = int(round(ip[1])), k = int(round(ip[2]));
+    return V3{voxel(g, i, j, k, 0), voxel(g, i, j, k, 1), voxel(g, i, j, k, 2)};
+}
+// emission: whether the caller reads the emission. Only a camera ray's march does (one step in eleven or so); the replays,
+// the shadow marches and the deeper rays leave the emission grid's index and three loads out.
+__device__ __forceinline__ VolumeLocal localAt(const SceneView& s, const VolumeRec& v, V3 p, uint32_t interpolation, bool emission) {
+    const V3 gp = gridSpace(v, p);
     const float density = v.densityGrid < s.gridCount && s.grids[v.densityGrid].channels == 1 ? sampleGrid(s.grids[v.densityGrid], gp, interpolation, 0) : 0.0f;
     V3 temperature{0, 0, 0};
-    if (v.emissionGrid != kNoGrid && v.emissionGrid < s.gridCount && s.grids[v.emissionGrid].channels == 3) {
-        const GridRec& e = s.grids[v.emissionGrid];
-        temperature = V3{sampleGrid(e, gp, kInterpPoint, 0), sampleGrid(e, gp, kInterpPoint, 1), sampleGrid(e, gp, kInterpPoint, 2)};
-    }
+    if (emission && v.emissionGrid != kNoGrid && v.emissionGrid < s.gridCount && s.grids[v.emissionGrid].channels == 3)
+        temperature = samplePoint3(s.grids[v.emissionGrid], gp);
     return VolumeLocal{cmax0(vscaled(v.gain, density)), cmax0(v.colorMult), cmax0(vtimes(temperature, v.incandescence)),
                        fminf(fmaxf(v.g, -1.0f), 1.0f)};
 }
@@ -128,7 +161,7 @@ static __device__ __noinline__ VolumeCoefficients evalShadersAt(const SceneView&
     uint32_t first = kMaxVolumes, chosen = kMaxVolumes;
     auto local = [&](uint32_t v) {
         const VolumeRec& vr = s.volumes[v];
-        return localAt(s, vr, p, interpolationOverride != kNoGrid ? interpolationOverride : vr.interpolation);
+        return localAt(s, vr, p, interpolationOverride != kNoGrid ? interpolationOverride : vr.interpolation, emissions != nullptr);
     };
     for (uint32_t v = 0; v < s.config.volume_count; ++v) {
         if (!(regions >> v & 1)) continue;
