@@ -113,6 +113,7 @@ struct x2_ctx {
     cudaStream_t stream = nullptr;
     int smCount = 0;
     int renderBlocksPerSm = 0;
+    x2::SideStreams side;  // for kernels of one iteration that run side by side
 };
 
 // An adaptive frame's device state (adaptive.h AdaptiveArgs) and its host-side layout.
@@ -532,12 +533,29 @@ int x2_open(int device, x2_ctx** out) {
         delete ctx;
         return X2_ECUDA;
     }
+    auto freeContext = [ctx] {
+        for (int j = 0; j < 2; ++j) {
+            if (ctx->side.stream[j]) cudaStreamDestroy(ctx->side.stream[j]);
+            if (ctx->side.join[j]) cudaEventDestroy(ctx->side.join[j]);
+        }
+        if (ctx->side.fork) cudaEventDestroy(ctx->side.fork);
+        cudaStreamDestroy(ctx->stream);
+        delete ctx;
+    };
+    bool side = cudaEventCreateWithFlags(&ctx->side.fork, cudaEventDisableTiming) == cudaSuccess;
+    for (int j = 0; j < 2; ++j)
+        side = side && cudaStreamCreateWithFlags(&ctx->side.stream[j], cudaStreamNonBlocking) == cudaSuccess &&
+               cudaEventCreateWithFlags(&ctx->side.join[j], cudaEventDisableTiming) == cudaSuccess;
+    if (!side) {
+        setError("stream creation failed");
+        freeContext();
+        return X2_ECUDA;
+    }
     uint32_t dirs[17][32];
     sobolDirections(dirs);
     if (uploadSobol(dirs) != cudaSuccess || uploadSobolWavefront(dirs) != cudaSuccess || uploadSobolAdjoint(dirs) != cudaSuccess) {
         setError("sobol table upload failed");
-        cudaStreamDestroy(ctx->stream);
-        delete ctx;
+        freeContext();
         return X2_ECUDA;
     }
     cudaDeviceGetAttribute(&ctx->smCount, cudaDevAttrMultiProcessorCount, device);
@@ -551,6 +569,11 @@ int x2_close(x2_ctx* ctx) {
     if (!ctx) return X2_OK;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    for (int j = 0; j < 2; ++j) {
+        cudaStreamDestroy(ctx->side.stream[j]);
+        cudaEventDestroy(ctx->side.join[j]);
+    }
+    cudaEventDestroy(ctx->side.fork);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
     return X2_OK;
@@ -1400,8 +1423,7 @@ int x2_launch_wavefront(x2_scene* s, const x2_chunk* chunks, uint32_t count) {
     cudaMemsetAsync(sl.counters, 0, sizeof(Counters), st);
     cudaMemsetAsync(s->outStatus, X2_SKIP, items, st);
     const WaveArgs a = launchArgs(s, sl, paths, records, items, count);
-    const int gridLogic = int((paths + kWaveBlock - 1) / kWaveBlock);
-    const int gridWork = s->ctx->smCount * int(s->blocksPerSm);
+    const WaveGrids grids = waveGrids(paths, records, s->ctx->smCount, s->blocksPerSm);
     const WaveKernels wk = waveKernels(s->traceBlocks, s->shadeBlocks, s->volumeCount != 0, s->triUV != nullptr, s->shortStack != 0,
                                        a.scene.stats != nullptr, s->shadeSplit != 0,
                                        s->wave.lightJob != nullptr ? s->lightSplit : 0u, s->triOverlap != 0 && s->shortStack != 0 && s->traceBlocks < 9);
@@ -1417,13 +1439,13 @@ int x2_launch_wavefront(x2_scene* s, const x2_chunk* chunks, uint32_t count) {
         for (;;) {
             wfResetQueues<<<1, 32, 0, st>>>(a);
             cudaEventRecord(ev[0], st);
-            wk.logic<<<gridLogic, kWaveBlock, 0, st>>>(a);
+            wk.logic<<<grids.logic, kWaveBlock, 0, st>>>(a);
             cudaEventRecord(ev[1], st);
-            wk.extend<<<gridWork, kWaveBlock, 0, st>>>(a);
+            wk.extend<<<grids.work, kWaveBlock, 0, st>>>(a);
             cudaEventRecord(ev[2], st);
-            launchShade(wk, a, gridWork, st);
+            launchShade(wk, a, grids.work, st);
             cudaEventRecord(ev[3], st);
-            wk.shadow<<<gridWork, kWaveBlock, 0, st>>>(a);
+            wk.shadow<<<grids.shadow, kWaveBlock, 0, st>>>(a);
             cudaEventRecord(ev[4], st);
             cudaMemcpyAsync(s->hostLast, s->waveCounters, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
             wfResetQueues<<<1, 32, 0, st>>>(a);
@@ -1488,11 +1510,7 @@ int x2_launch_wavefront(x2_scene* s, const x2_chunk* chunks, uint32_t count) {
     const uint32_t bound = uint32_t(std::min<uint64_t>(maxIter, 0xffffffffu));
     if (err == cudaSuccess && check(cudaStreamBeginCaptureToGraph(st, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                                                   cudaStreamCaptureModeThreadLocal))) {
-        wfResetQueues<<<1, 32, 0, st>>>(a);
-        wk.logic<<<gridLogic, kWaveBlock, 0, st>>>(a);
-        wk.extend<<<gridWork, kWaveBlock, 0, st>>>(a);
-        launchShade(wk, a, gridWork, st);
-        wk.shadow<<<gridWork, kWaveBlock, 0, st>>>(a);
+        launchIteration(wk, a, grids, st, false, &s->ctx->side);
         wfDrainCheck<<<1, 32, 0, st>>>(a, loop, s->drainWords, bound, s->drainWords + 2);
         check(cudaGetLastError());
         cudaGraph_t body = nullptr;
@@ -1795,7 +1813,7 @@ int x2_adjoint(x2_scene* s, uint32_t first, uint32_t count, const float* d_dloss
     }
     // Logic in a grid of a few blocks a SM (each block's partials go to a gradient row once a launch).
     const int gridLogic = std::min(int((paths + kWaveBlock - 1) / kWaveBlock), s->ctx->smCount * 8);
-    const int gridWork = s->ctx->smCount * int(s->blocksPerSm);
+    const WaveGrids grids = waveGrids(paths, records, s->ctx->smCount, s->blocksPerSm);
     const WaveKernels wk = waveKernels(s->traceBlocks, s->shadeBlocks, false, s->triUV != nullptr);
     const uint64_t maxIter = items * (uint64_t(s->config.max_depth) + 2) / paths + uint64_t(s->config.max_depth) + 64;
     constexpr int kIter = 8;
@@ -1809,10 +1827,10 @@ int x2_adjoint(x2_scene* s, uint32_t first, uint32_t count, const float* d_dloss
         for (int it = 0; it < kIter; ++it) {
             wfResetQueues<<<1, 32, 0, st>>>(a);
             wfLogicAdjoint<<<gridLogic, kWaveBlock, shared, st>>>(a);
-            wk.extend<<<gridWork, kWaveBlock, 0, st>>>(a);
-            if (a.shadeQ) wfSortShade<<<gridWork, kWaveBlock, 0, st>>>(a);
-            wfShadeAdjoint<<<gridWork, kWaveBlock, shared, st>>>(a);
-            wk.shadow<<<gridWork, kWaveBlock, 0, st>>>(a);
+            wk.extend<<<grids.work, kWaveBlock, 0, st>>>(a);
+            if (a.shadeQ) wfSortShade<<<grids.work, kWaveBlock, 0, st>>>(a);
+            wfShadeAdjoint<<<grids.work, kWaveBlock, shared, st>>>(a);
+            wk.shadow<<<grids.shadow, kWaveBlock, 0, st>>>(a);
         }
         wfResetQueues<<<1, 32, 0, st>>>(a);
         if (cudaStreamEndCapture(st, &graph) != cudaSuccess || cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) {
@@ -2155,8 +2173,7 @@ int renderAdaptive(x2_scene* s, uint32_t minSamples, uint32_t maxSamples, float 
     a.chunkMask = ad.chunkMasks;
     a.pixelBase = ad.base;
     a.liveChunks = ad.words;
-    const int gridLogic = int((paths + kWaveBlock - 1) / kWaveBlock);
-    const int gridWork = s->ctx->smCount * int(s->blocksPerSm);
+    const WaveGrids grids = waveGrids(paths, records, s->ctx->smCount, s->blocksPerSm);
     const WaveKernels wk = waveKernels(s->traceBlocks, s->shadeBlocks, s->volumeCount != 0, s->triUV != nullptr, s->shortStack != 0,
                                        a.scene.stats != nullptr, s->shadeSplit != 0,
                                        s->wave.lightJob != nullptr ? s->lightSplit : 0u, s->triOverlap != 0 && s->shortStack != 0 && s->traceBlocks < 9);
@@ -2208,11 +2225,7 @@ int renderAdaptive(x2_scene* s, uint32_t minSamples, uint32_t maxSamples, float 
         cudaGraphConditionalHandle loop;
         cudaGraph_t body = g.whileNode(&loop);
         if (!body || !g.begin(body, false)) break;
-        wfResetQueues<<<1, 32, 0, st>>>(a);
-        wk.logic<<<gridLogic, kWaveBlock, 0, st>>>(a);
-        wk.extend<<<gridWork, kWaveBlock, 0, st>>>(a);
-        launchShade(wk, a, gridWork, st);
-        wk.shadow<<<gridWork, kWaveBlock, 0, st>>>(a);
+        launchIteration(wk, a, grids, st, false, &s->ctx->side);
         wfDrainCheck<<<1, 32, 0, st>>>(a, loop, ad.words + 2, maxIter, ad.words + 4);
         g.check(cudaGetLastError());
         if (!g.end(false)) break;
@@ -2592,8 +2605,7 @@ int x2_render_batch(x2_ctx* ctx, const x2_request* req, uint32_t n, x2_completio
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     Counters hc{};
     int rc = X2_OK;
-    const int gridLogic = int((paths + kWaveBlock - 1) / kWaveBlock);
-    const int gridWork = ctx->smCount * int(s0->blocksPerSm);
+    const WaveGrids grids = waveGrids(paths, records, ctx->smCount, s0->blocksPerSm);
     bool anyVolumes = false, anyTextures = false;
     for (const SceneView& v : views) {
         anyVolumes = anyVolumes || v.config.volume_count != 0;
@@ -2673,10 +2685,7 @@ int x2_render_batch(x2_ctx* ctx, const x2_request* req, uint32_t n, x2_completio
         }
         for (int it = 0; it < kIter; ++it) {
             wfResetQueues<<<1, 32, 0, st>>>(a);
-            wk.logic<<<gridLogic, kWaveBlock, 0, st>>>(a);
-            wk.extend<<<gridWork, kWaveBlock, 0, st>>>(a);
-            launchShade(wk, a, gridWork, st, true);
-            wk.shadow<<<gridWork, kWaveBlock, 0, st>>>(a);
+            launchIteration(wk, a, grids, st, true, &ctx->side);
         }
         wfResetQueues<<<1, 32, 0, st>>>(a);
         if (cudaStreamEndCapture(st, &graph) != cudaSuccess || cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) {

@@ -17,6 +17,8 @@
 #include "credits.cuh"
 #include "wavefront.h"
 
+#include <algorithm>
+
 namespace x2 {
 
 enum : uint32_t { kEmpty = 0, kTrace = 1, kDone = 2, kError = 3 };
@@ -349,6 +351,10 @@ struct QueueSegments {
 template <bool kAny, bool kStats, bool kBatch, int kShort, bool kOverlap = false>
 __device__ __forceinline__ void persistentTrace(const WaveArgs& a, uint32_t n, const uint32_t* __restrict__ queue, uint32_t* next,
                                                 uint2* shortStacks, const QueueSegments seg = QueueSegments{nullptr, 0, 0}) {
+    // A block that no 128 entries of the queue fall to leaves at once: the grid is sized for the launch's largest queue
+    // (thousands of blocks), and a warp that found its queue empty only through the fetch counter cost one atomic on
+    // that one word (box 256x256 at one sample: the iterations' extend and shadow kernels 0.48 ms of 0.94).
+    if (blockIdx.x * blockDim.x >= n) return;
     const WaveState& w = a.w;
     Bvh8 bvh = a.scene.bvh;  // a batch: the lane's ray's scene, set at each fetch
     uint32_t* overflow = a.scene.overflow;
@@ -671,6 +677,7 @@ __device__ __forceinline__ void lightsBody(const WaveArgs& a) {
     const WaveState& w = a.w;
     const SceneView& s = a.scene;
     const uint32_t n = a.shadeCount[kQueue];
+    if (blockIdx.x * blockDim.x >= n) return;
     const uint32_t R = a.recordsPerPath;
     unsigned long long nee = 0;
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -711,6 +718,7 @@ template <bool kBatch, bool kVolumes, bool kAdjoint = false, bool kTextures = tr
 __device__ __forceinline__ void shadeBody(const WaveArgs& a) {
     const WaveState& w = a.w;
     const uint32_t n = kQueue < 0 ? *a.extendCount : a.shadeCount[kQueue];
+    if (blockIdx.x * blockDim.x >= n) return;
     extern __shared__ float partial[];  // the adjoint's block partials
     const Layout at{a.adj.materials, a.adj.lights};
     if (kAdjoint) partialsBegin(partial, at);
@@ -900,15 +908,45 @@ __global__ void __launch_bounds__(kWaveBlock, kMinBlocks) wfLightsQueue(WaveArgs
     lightsBody<kQueue>(a);
 }
 
-void launchShade(const WaveKernels& k, const WaveArgs& a, int grid, cudaStream_t st, bool batch) {
+// With side streams the three queues' kernels (and the two light kernels behind theirs) run side by side: they share
+// nothing but counters. A small queue's kernels are latency, not work (five in a row on a 65,536-sample box pass), and a
+// large queue's fill the tails of one another.
+void launchShade(const WaveKernels& k, const WaveArgs& a, int grid, cudaStream_t st, bool batch, const SideStreams* side) {
     if (a.shadeQ) (batch ? wfSortShadeBatch : wfSortShade)<<<grid, kWaveBlock, 0, st>>>(a);
     if (a.shadeQ && k.shadeBy[0]) {
-        for (int q = 0; q < 3; ++q) k.shadeBy[q]<<<grid, kWaveBlock, 0, st>>>(a);
+        cudaStream_t on[3] = {st, side ? side->stream[0] : st, side ? side->stream[1] : st};
+        if (side) {
+            cudaEventRecord(side->fork, st);
+            for (int j = 0; j < 2; ++j) cudaStreamWaitEvent(side->stream[j], side->fork, 0);
+        }
+        for (int q = 0; q < 3; ++q) k.shadeBy[q]<<<grid, kWaveBlock, 0, on[q]>>>(a);
         if (k.lightsBy[0])
-            for (int q = 0; q < 2; ++q) k.lightsBy[q]<<<grid, kWaveBlock, 0, st>>>(a);
+            for (int q = 0; q < 2; ++q) k.lightsBy[q]<<<grid, kWaveBlock, 0, on[q]>>>(a);
+        if (side)
+            for (int j = 0; j < 2; ++j) {
+                cudaEventRecord(side->join[j], side->stream[j]);
+                cudaStreamWaitEvent(st, side->join[j], 0);
+            }
     } else {
         k.shade<<<grid, kWaveBlock, 0, st>>>(a);
     }
+}
+
+void launchIteration(const WaveKernels& k, const WaveArgs& a, const WaveGrids& g, cudaStream_t st, bool batch, const SideStreams* side) {
+    k.logic<<<g.logic, kWaveBlock, 0, st>>>(a);
+    k.extend<<<g.work, kWaveBlock, 0, st>>>(a);
+    launchShade(k, a, g.work, st, batch, side);
+    k.shadow<<<g.shadow, kWaveBlock, 0, st>>>(a);
+}
+
+WaveGrids waveGrids(uint32_t paths, uint32_t records, int smCount, uint32_t blocksPerSm) {
+    auto blocks = [](uint64_t n) { return (n + kWaveBlock - 1) / kWaveBlock; };
+    const uint64_t most = uint64_t(smCount) * blocksPerSm;
+    WaveGrids g;
+    g.logic = int(blocks(paths));
+    g.work = int(std::min<uint64_t>(most, blocks(paths)));
+    g.shadow = int(std::min<uint64_t>(most, blocks(uint64_t(paths) * records)));
+    return g;
 }
 
 WaveKernels waveKernels(uint32_t traceBlocks, uint32_t shadeBlocks, bool volumes, bool textures, bool shortStack, bool counting,
@@ -964,23 +1002,25 @@ WaveKernels waveKernelsBatch(bool volumes, bool textures, bool shadeSplit) {
     return k;
 }
 
-// Queue counters for the next iteration: the extend and shadow counts start at zero; the previous counts are kept
-// for the host (the graph's last extend count tells whether paths remain).
+// Queue counters for the next iteration: the extend and shadow counts start at zero; the previous extend count is kept
+// for the host (it tells whether paths remain).
+__device__ __forceinline__ void resetQueues(const WaveArgs& a) {
+    *a.lastExtend = *a.extendCount;
+    *a.extendCount = 0;
+    *a.shadowCount = 0;
+    *a.extendNext = 0;
+    if (a.shadowSlots)
+        for (uint32_t k = 0; k < a.recordsPerPath; ++k) a.shadowSlots[k] = 0;
+    if (a.extendSlots)
+        for (uint32_t o = 0; o < kOctants; ++o) a.extendSlots[o] = 0;
+    *a.shadowNext = 0;
+    if (a.shadeQ) a.shadeCount[0] = a.shadeCount[1] = a.shadeCount[2] = 0;
+}
 __global__ void wfResetQueues(WaveArgs a) {
-    if (threadIdx.x == 0) {
-        *a.lastExtend = *a.extendCount;
-        *a.extendCount = 0;
-        *a.shadowCount = 0;
-        *a.extendNext = 0;
-        if (a.shadowSlots)
-            for (uint32_t k = 0; k < a.recordsPerPath; ++k) a.shadowSlots[k] = 0;
-        if (a.extendSlots)
-            for (uint32_t o = 0; o < kOctants; ++o) a.extendSlots[o] = 0;
-        *a.shadowNext = 0;
-        if (a.shadeQ) a.shadeCount[0] = a.shadeCount[1] = a.shadeCount[2] = 0;
-    }
+    if (threadIdx.x == 0) resetQueues(a);
 }
 
+// The drain's test and, in the same launch, the next iteration's reset (the first iteration's queues start cleared).
 __global__ void wfDrainCheck(WaveArgs a, cudaGraphConditionalHandle loop, uint32_t* iterations, uint32_t maxIterations,
                              uint32_t* overrun) {
     if (threadIdx.x != 0) return;
@@ -989,6 +1029,7 @@ __global__ void wfDrainCheck(WaveArgs a, cudaGraphConditionalHandle loop, uint32
     const bool more = *a.extendCount != 0;
     if (more && n >= maxIterations) *overrun = 1;
     cudaGraphSetConditional(loop, more && n < maxIterations ? 1u : 0u);
+    resetQueues(a);
 }
 
 // The film: each (chunk, position)'s samples summed in sample order, then added to the pixel (async_gpu.cu:320-364's

@@ -137,9 +137,24 @@ struct WaveKernels {
 // overlap: the traversal kernels that overlap a lane's node visits and triangle tests (walkStepOverlap; short stack).
 WaveKernels waveKernels(uint32_t traceBlocks, uint32_t shadeBlocks, bool volumes, bool textures, bool shortStack = kDefaultShortStack != 0,
                         bool counting = false, bool shadeSplit = false, uint32_t lightSplit = 0, bool overlap = false);
+// Two streams beside a context's own, with the events that fork work onto them and join it again (within one capture or
+// launch sequence).
+struct SideStreams {
+    cudaStream_t stream[2] = {nullptr, nullptr};
+    cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr};
+};
+// An iteration's grids: logic a thread a slot; extend, sort, shade and lights (work) and shadow at most blocksPerSm
+// blocks a SM and at most the blocks their largest possible queue fills.
+struct WaveGrids {
+    int logic, work, shadow;
+};
+WaveGrids waveGrids(uint32_t paths, uint32_t records, int smCount, uint32_t blocksPerSm);
 // The iteration's shade step: the per-lobe sort (when the queues are on) and the shade kernel or kernels (batch: the
-// batch form's sort).
-void launchShade(const WaveKernels& k, const WaveArgs& a, int grid, cudaStream_t st, bool batch = false);
+// batch form's sort; side: the queues' kernels side by side, null for one after the other).
+void launchShade(const WaveKernels& k, const WaveArgs& a, int grid, cudaStream_t st, bool batch = false, const SideStreams* side = nullptr);
+// An iteration's logic, extend, shade and shadow.
+void launchIteration(const WaveKernels& k, const WaveArgs& a, const WaveGrids& g, cudaStream_t st, bool batch = false,
+                     const SideStreams* side = nullptr);
 WaveKernels waveKernelsBatch(bool volumes, bool textures, bool shadeSplit = kDefaultShadeSplit != 0);
 __global__ void wfSortShade(WaveArgs a);
 __global__ void wfSortShadeBatch(WaveArgs a);
@@ -150,7 +165,7 @@ __global__ void wfShadeAdjoint(WaveArgs a);
 __global__ void wfGradRows(const float* rows, uint32_t rowCount, uint32_t params, double* grads);
 __global__ void wfResetQueues(WaveArgs a);
 // The drain loop's test, last in the body of a conditional while node: go on while the iteration extended a ray, at
-// most maxIterations times (then *overrun is set and the loop ends). iterations[0] counts this loop's iterations,
+// most maxIterations times (then *overrun is set and the loop ends); the queues are reset for the next iteration. iterations[0] counts this loop's iterations,
 // iterations[1] a running total.
 __global__ void wfDrainCheck(WaveArgs a, cudaGraphConditionalHandle loop, uint32_t* iterations, uint32_t maxIterations,
                              uint32_t* overrun);
