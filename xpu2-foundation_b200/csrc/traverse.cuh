@@ -1,8 +1,8 @@
 // Closest-hit and any-hit traversal of the compressed 8-wide BVH (bvh.cuh) for one ray a thread.
 //
 // A node is five 16-byte read-only loads. Its eight children are tested with one FMA a slab (Ylitie et al. 2017:
-// the ray is expressed in the node's quantised frame once, t = q * (2^e / d) + (p - o) / d), widened by a bound on
-// its rounding so the quantised boxes stay conservative (visitNode). Hit children enter a 32-bit mask: internal
+// the ray is expressed in the node's quantised frame once, t = q * (2^e / d) + (p - o) / d, two slabs an instruction),
+// widened by a bound on the roundings so the quantised boxes stay conservative (visitNode). Hit children enter a 32-bit mask: internal
 // children on bits 24..31 in near-to-far order for the ray's octant (the build places each child in the slot of
 // the octant it lies toward), leaf triangles on bits 0..23. The stack holds (child base, mask | imask) pairs and
 // lives in registers/local memory; an overflow is counted, never silent.
@@ -120,55 +120,76 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
     return r;
 }
 
-// Byte j of w with 2^23 added, as an exact float: 0x4B0000bb is 2^23 + bb (one byte permute, no conversion).
-__device__ __forceinline__ float qbyte23(uint32_t w, int j) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u | uint32_t(j))); }
+// Byte j of w with 2^15 added, as an exact float: 0x4700bb00 is 2^15 + bb (one byte permute, no conversion).
+__device__ __forceinline__ float qbyte15(uint32_t w, int j) { return __uint_as_float(__byte_perm(w, 0x47000000u, 0x7604u | uint32_t(j << 4))); }
+
+// Two floats side by side, and two FMAs in one instruction (sm_100a's packed single-precision FMA).
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void fma2(unsigned long long a, unsigned long long b, unsigned long long c, float& x, float& y) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(r));
+}
 
 // One node: the hit mask (bits 24..31 internal children in traversal order, 0..23 leaf triangles), its child and
 // triangle bases and its internal-child mask.
 //
-// Conservative by construction: the quantised child boxes contain the exact ones (the build rounds outward). The slab
-// distance q * s + a (s = 2^e * (1/d), a = (p - o) * (1/d)) is computed as one FMA of the byte with 2^23 added,
-// (2^23 + q) * s + c with c = (a -+ w) - 2^23 s, which saves the byte's conversion: against q * s + a exactly, it errs
-// by the four roundings of a and s (under 2^-22 (|a| + 255 |s|)), by c's rounding at the magnitude of 2^23 s (at most
-// |s| / 2 + 2^-24 (|a| + w)) and by the FMA's (under 2^-24 (|a| + 257 |s| + w)). Every slab is widened by
-// w = |s| / 2 + 2^-19 (|a| + 256 |s|) each way, which covers them; 2^23 s stays finite for the scene extents the
-// loader admits.
+// The traversals are bound by instruction issue (with the ALU pipe behind it), so the test is written for few
+// instructions: a child's near and far slab distances of an axis are one packed FMA, (2^15 + q) s + c with
+// s = 2^e * (1/d), a = (p - o) * (1/d) and c = a - 2^15 s -+ w, the byte placed in the float's mantissa by one permute.
+//
+// Conservative by construction: the quantised child boxes contain the exact ones (the build rounds outward), and every
+// slab is widened by w = 2^-20 L |1/d| + 2^-7 |s| each way, L the L1 distance from the ray's origin to the scene's
+// farthest corner (r.eps is 2^-18 L). Against q s + a exactly the computed distance errs by the four roundings of a and
+// s (under 2^-22 (|a| + 255 |s|)), c's two (each under 2^-24 |a| + 2^-9 |s|) and the FMA's (2^-24 (|a| + 256 |s|)): the
+// |s| part is under 2^-7 |s|, the |a| part under 2^-21.1 |a|, and |a| <= L |1/d|. The rest of the L term, over 2^-22 L of
+// distance along the axis, is for the triangle test, whose sheared vertices carry roundings of up to 2^-22 of their
+// distance from the origin: a hit it finds just outside a triangle's box is still reached. (With 2^23 in place of 2^15
+// c's rounding alone was half a quantum, and a shadow ray of the 12.3M-triangle field visited 20.4 nodes.)
 __device__ __forceinline__ uint32_t visitNode(const Node8* __restrict__ nodes, uint32_t index, const RayQ& r, float tmin, float tmax,
                                               uint32_t& childBase, uint32_t& triBase, uint32_t& imask) {
     const uint4* p = reinterpret_cast<const uint4*>(nodes + index);
     const uint4 n0 = __ldg(p), n1 = __ldg(p + 1), n2 = __ldg(p + 2), n3 = __ldg(p + 3), n4 = __ldg(p + 4);
     const float px = __uint_as_float(n0.x), py = __uint_as_float(n0.y), pz = __uint_as_float(n0.z);
-    const uint32_t ex = n0.w & 0xffu, ey = (n0.w >> 8) & 0xffu, ez = (n0.w >> 16) & 0xffu;
     imask = n0.w >> 24;
     childBase = n1.x;
     triBase = n1.y;
-    const float sx = __uint_as_float(ex << 23) * r.ix, sy = __uint_as_float(ey << 23) * r.iy, sz = __uint_as_float(ez << 23) * r.iz;
-    const float ax = (px - r.ox) * r.ix, ay = (py - r.oy) * r.iy, az = (pz - r.oz) * r.iz;
-    const float wx = 0.5f * fabsf(sx) + (fabsf(ax) + 256.0f * fabsf(sx)) * 0x1p-19f,
-                wy = 0.5f * fabsf(sy) + (fabsf(ay) + 256.0f * fabsf(sy)) * 0x1p-19f,
-                wz = 0.5f * fabsf(sz) + (fabsf(az) + 256.0f * fabsf(sz)) * 0x1p-19f;
-    const float axn = __fmaf_rn(-8388608.0f, sx, ax - wx), axf = __fmaf_rn(-8388608.0f, sx, ax + wx);
-    const float ayn = __fmaf_rn(-8388608.0f, sy, ay - wy), ayf = __fmaf_rn(-8388608.0f, sy, ay + wy);
-    const float azn = __fmaf_rn(-8388608.0f, sz, az - wz), azf = __fmaf_rn(-8388608.0f, sz, az + wz);
+    const float sx = __uint_as_float((n0.w << 23) & 0x7f800000u) * r.ix, sy = __uint_as_float((n0.w << 15) & 0x7f800000u) * r.iy,
+                sz = __uint_as_float((n0.w << 7) & 0x7f800000u) * r.iz;
+    const float slack = 0.25f * r.eps;
+    auto offsets = [&](float plane, float o, float inv, float s) {
+        const float c = __fmaf_rn(-32768.0f, s, (plane - o) * inv), w = __fmaf_rn(fabsf(inv), slack, fabsf(s) * 0x1p-7f);
+        return pack2(c - w, c + w);
+    };
+    const unsigned long long cx = offsets(px, r.ox, r.ix, sx), cy = offsets(py, r.oy, r.iy, sy), cz = offsets(pz, r.oz, r.iz, sz);
+    const unsigned long long sxx = pack2(sx, sx), syy = pack2(sy, sy), szz = pack2(sz, sz);
     // The near and far planes' quantised words for the ray's direction signs, chosen once a node.
     const bool fx = r.ix >= 0.0f, fy = r.iy >= 0.0f, fz = r.iz >= 0.0f;
     const uint32_t nx0 = fx ? n2.x : n3.z, nx1 = fx ? n2.y : n3.w, fx0 = fx ? n3.z : n2.x, fx1 = fx ? n3.w : n2.y;
     const uint32_t ny0 = fy ? n2.z : n4.x, ny1 = fy ? n2.w : n4.y, fy0 = fy ? n4.x : n2.z, fy1 = fy ? n4.y : n2.w;
     const uint32_t nz0 = fz ? n3.x : n4.z, nz1 = fz ? n3.y : n4.w, fz0 = fz ? n4.z : n3.x, fz1 = fz ? n4.w : n3.y;
     // Child metadata with internal slots' bit positions (24 + slot: bits 3 and 4 both set, which no triangle offset
-    // has) permuted to the ray's near-to-far order; an empty slot's byte is 0 and sets nothing.
+    // has) permuted to the ray's near-to-far order; an empty slot's byte is 0 and sets nothing. A slot's bits are the
+    // byte's top three, shifted by its low five: four slots' top bits at once, and a funnel shift that reads only the
+    // low five bits of its amount.
     const uint32_t m0 = n1.z ^ ((((n1.z & (n1.z << 1)) & 0x10101010u) >> 4) * r.oct7);
     const uint32_t m1 = n1.w ^ ((((n1.w & (n1.w << 1)) & 0x10101010u) >> 4) * r.oct7);
+    const uint32_t b0 = (n1.z >> 5) & 0x07070707u, b1 = (n1.w >> 5) & 0x07070707u;
     uint32_t hits = 0;
 #pragma unroll
     for (int s = 0; s < 8; ++s) {
         const int j = s & 3;
-        const float nx = __fmaf_rn(qbyte23(s < 4 ? nx0 : nx1, j), sx, axn), fxx = __fmaf_rn(qbyte23(s < 4 ? fx0 : fx1, j), sx, axf);
-        const float ny = __fmaf_rn(qbyte23(s < 4 ? ny0 : ny1, j), sy, ayn), fyy = __fmaf_rn(qbyte23(s < 4 ? fy0 : fy1, j), sy, ayf);
-        const float nz = __fmaf_rn(qbyte23(s < 4 ? nz0 : nz1, j), sz, azn), fzz = __fmaf_rn(qbyte23(s < 4 ? fz0 : fz1, j), sz, azf);
-        const float entry = max3f(nx, ny, fmaxf(nz, tmin)), exit = min3f(fxx, fyy, fminf(fzz, tmax));
-        const uint32_t meta = ((s < 4 ? m0 : m1) >> (8 * j)) & 0xffu;
-        if (entry <= exit) hits |= (meta >> 5) << (meta & 31u);
+        float nx, ny, nz, ex, ey, ez;
+        fma2(pack2(qbyte15(s < 4 ? nx0 : nx1, j), qbyte15(s < 4 ? fx0 : fx1, j)), sxx, cx, nx, ex);
+        fma2(pack2(qbyte15(s < 4 ? ny0 : ny1, j), qbyte15(s < 4 ? fy0 : fy1, j)), syy, cy, ny, ey);
+        fma2(pack2(qbyte15(s < 4 ? nz0 : nz1, j), qbyte15(s < 4 ? fz0 : fz1, j)), szz, cz, nz, ez);
+        const float entry = max3f(nx, ny, fmaxf(nz, tmin)), exit = min3f(ex, ey, fminf(ez, tmax));
+        const uint32_t bits = __funnelshift_l(0u, __byte_perm(s < 4 ? b0 : b1, 0u, 0x4440u | uint32_t(j)), (s < 4 ? m0 : m1) >> (8 * j));
+        if (entry <= exit) hits |= bits;
     }
     return hits;
 }
