@@ -148,3 +148,40 @@ def test_volume_golden(medium):
     ok = (np.abs(rgba - g["rgba"]) <= RTOL * np.abs(g["rgba"]) + ATOL).all(axis=1)
     print(f"volume golden: {ok.mean() * 100:.3f}% of {len(ok)} samples within {RTOL}")
     assert ok.mean() >= 0.99
+
+
+@pytest.mark.parametrize("estimator,overlap,volumes", [(0, 0, 1), (0, 1, 2), (0, 2, 2), (1, 0, 1), (1, 1, 2)])
+@pytest.mark.parametrize("width,height,spp", [(1, 1, 1), (50, 37, 3)])
+def test_volume_kernels_equal_the_march_inside_shade(ctx, estimator, overlap, volumes, width, height, spp):
+    """The volumes in kernels of their own and the lookups of axis-aligned grid maps against the plain form's march and
+    the general lookups (the same maps with an off-diagonal entry too small to change a sum): every film alike."""
+    films = []
+    for general in (False, True):
+        s = x2.SyntheticScene(33)
+        d, cfg = s.desc, x2.Config.from_buffer_copy(s.config)
+        cfg.width, cfg.height, cfg.spp = width, height, spp
+        cfg.volume_estimator, cfg.volume_overlap_mode, cfg.volume_count = estimator, overlap, volumes
+        records = (x2.Volume * volumes)()
+        for v in range(volumes):
+            records[v] = d.volumes[0]
+            for a in range(3):
+                records[v].bound_lo[a] += 0.4 * v  # a second box overlaps the first and sticks out of the grid
+            if v:
+                records[v].interpolation = 0
+            if general:
+                records[v].world_to_grid[1] = 1e-38
+        if general:
+            for g in range(d.grid_count):
+                d.grids[g].world_to_index[1] = 1e-300
+        d.volumes, d.volume_count = records, volumes
+        scene = x2.Scene(ctx, d, cfg)
+        for render in (scene.render_frame, scene.render_frame_wavefront):
+            scene.frame_begin(spp)
+            render(0, spp)
+            scene.wait()
+            scene.audit()
+            films.append(scene.film()[0])
+        scene.free()
+    assert np.abs(films[0][:, :3]).sum() > 0 or width * height == 1
+    for film in films[1:]:
+        assert np.allclose(film, films[0], rtol=1e-12, atol=1e-12)  # the FP64 film's own summation order

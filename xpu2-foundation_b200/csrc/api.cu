@@ -89,8 +89,9 @@ int waitEvent(cudaEvent_t e, int timeoutMs) {
 constexpr int kSlots = 2;  // launches in flight, as GpuLane keeps (async_gpu.h:1425)
 constexpr uint32_t kQueueLog = 4096;
 // extend count, last extend count, shadow count, extend fetch, shadow fetch, 3 shade queue counts, then the shadow
-// queue's record segments (x2::kRecordSegments), then the extend queue's octant bins (x2::kOctants)
-constexpr int kWaveCounters = 8 + int(x2::kRecordSegments) + int(x2::kOctants);
+// queue's record segments (x2::kRecordSegments), then the extend queue's octant bins (x2::kOctants), then the rays that
+// scatter in a volume
+constexpr int kWaveCounters = 8 + int(x2::kRecordSegments) + int(x2::kOctants) + 1;
 
 struct Slot {
     bool busy = false;
@@ -249,6 +250,8 @@ struct x2_scene {
     // the adaptive frame's state (x2_render_adaptive, x2_adaptive_step)
     AdaptiveState* adaptiveState = nullptr;
     // the adjoint's wavefront state (x2_adjoint): vertex records, scales, counts, dL/dI shares, record auxiliaries
+    x2::VolumeWave vol{};                 // a volume scene's wavefront state (its volumes in kernels of their own)
+    uint32_t volPaths = 0, volRecords = 0, volTasks = 0;  // the paths, records and samples its buffers hold
     uint4* avert = nullptr;
     float4* ascale = nullptr;
     uint32_t* avcount = nullptr;
@@ -358,17 +361,6 @@ void freeWave(x2_scene* s) {
     s->wavePaths = s->waveRecords = s->waveCap = 0;
 }
 
-// The paths in flight when the caller reserved none: kDefaultPaths, or fewer (a power of two, at least 2^18) when the
-// path state (slot, light job, queues and `records` shadow records a path) would pass kWaveBudgetBytes, as a scene with
-// many lights would.
-constexpr double kWaveBudgetBytes = 12e9;
-static uint32_t defaultPaths(uint32_t records) {
-    const double perPath = 128.0 + 16.0 * kLightJobWords + 4.0 * (kOctants + 3 + 1) + 53.0 * records;
-    uint32_t paths = kDefaultPaths;
-    while (paths > (1u << 18) && double(paths) * perPath > kWaveBudgetBytes) paths >>= 1;
-    return paths;
-}
-
 // Path slots for `paths` paths with `records` shadow records each.
 // Buffers that already hold at least `paths` paths are kept (a launch indexes them by its own path count), so launches
 // of varying sizes (an adaptive frame's passes) allocate once.
@@ -404,6 +396,64 @@ int ensureWave(x2_scene* s, uint32_t paths, uint32_t records) {
     s->wavePaths = s->waveCap = paths;
     s->waveRecords = records;
     return X2_OK;
+}
+
+void freeVolumeWave(x2_scene* s) {
+    x2::VolumeWave& v = s->vol;
+    void* ptrs[] = {v.head, v.pass, v.light, v.parts, v.crossings, v.checkpoints, v.branch, v.queue};
+    for (void* p : ptrs) cudaFree(p);
+    v = x2::VolumeWave{};
+    s->volPaths = s->volRecords = s->volTasks = 0;
+}
+
+// A ray's scattering samples at most, and the bytes a path slot's volume state takes.
+uint64_t volumeTasks(const x2_config& c) {
+    return uint64_t(c.light_count) * c.light_samples * std::max(c.volume_illumination_samples, 1u);
+}
+double volumeBytes(const x2_config& c, uint32_t records) {
+    return sizeof(x2::VolumeHead) + 32.0 + 4.0 + sizeof(x2::Crossing) * double(x2::kMaxCrossings) +
+           sizeof(x2::MarchCheckpoint) * double(x2::kVolumeCheckpoints) + 32.0 * double(volumeTasks(c)) + 8.0 * records;
+}
+
+// Whether a launch of `paths` slots runs its volumes in kernels of their own, and their buffers: a volume scene with single
+// scattering whose volume state fits kVolumeBudgetBytes (a caller may reserve any number of paths) and the device. Else
+// the march runs inside shade.
+constexpr double kVolumeBudgetBytes = 16e9;
+bool volumesApart(x2_scene* s, uint32_t paths, uint32_t records) {
+    const x2_config& c = s->config;
+    if (!s->volumeCount || c.max_volume_depth > 1 || c.volume_illumination_samples > 4096) return false;
+    const uint64_t tasks = volumeTasks(c);
+    if (tasks * paths > 0x7fffffffull || volumeBytes(c, records) * paths > kVolumeBudgetBytes) return false;
+    if (paths <= s->volPaths && records == s->volRecords && tasks == s->volTasks) return true;
+    freeVolumeWave(s);
+    x2::VolumeWave& v = s->vol;
+    const size_t P = paths;
+    if (cudaMalloc(&v.head, sizeof(x2::VolumeHead) * P) != cudaSuccess || cudaMalloc(&v.pass, sizeof(float4) * P) != cudaSuccess ||
+        cudaMalloc(&v.light, sizeof(float4) * P) != cudaSuccess ||
+        cudaMalloc(&v.parts, sizeof(float4) * 2 * P * std::max<uint64_t>(tasks, 1)) != cudaSuccess ||
+        cudaMalloc(&v.crossings, sizeof(x2::Crossing) * x2::kMaxCrossings * P) != cudaSuccess ||
+        cudaMalloc(&v.checkpoints, sizeof(x2::MarchCheckpoint) * x2::kVolumeCheckpoints * P) != cudaSuccess ||
+        cudaMalloc(&v.branch, sizeof(uint2) * records * P) != cudaSuccess || cudaMalloc(&v.queue, sizeof(uint32_t) * P) != cudaSuccess) {
+        cudaGetLastError();  // not enough memory: the form that needs none
+        freeVolumeWave(s);
+        return false;
+    }
+    v.tasks = uint32_t(tasks);
+    s->volPaths = paths;
+    s->volRecords = records;
+    s->volTasks = uint32_t(tasks);
+    return true;
+}
+
+// The paths in flight when the caller reserved none: kDefaultPaths, or fewer (a power of two, at least 2^18) when the
+// path state (slot, light job, queues, `records` shadow records a path, and a volume scene's volume state) would pass
+// kWaveBudgetBytes, as a scene with many lights would.
+constexpr double kWaveBudgetBytes = 12e9;
+static uint32_t defaultPaths(uint32_t records, double volumeState = 0.0) {
+    const double perPath = volumeState + 128.0 + 16.0 * kLightJobWords + 4.0 * (kOctants + 3 + 1) + 53.0 * records;
+    uint32_t paths = kDefaultPaths;
+    while (paths > (1u << 18) && double(paths) * perPath > kWaveBudgetBytes) paths >>= 1;
+    return paths;
 }
 
 int ensureItems(x2_scene* s, uint64_t items) {
@@ -958,6 +1008,7 @@ int x2_scene_free(x2_scene* s) {
     for (float* g : s->gridValues) cudaFree(g);
     for (float* m : s->majorants) cudaFree(m);
     freeWave(s);
+    freeVolumeWave(s);
     cudaFree(s->out);
     cudaFree(s->outStatus);
     cudaFree(s->extendQ);
@@ -1343,6 +1394,10 @@ namespace {
 // A single scene's wavefront launch of `count` chunks (sl.chunks) and `items` items over `paths` path slots.
 WaveArgs launchArgs(x2_scene* s, Slot& sl, uint32_t paths, uint32_t records, unsigned long long items, uint32_t count) {
     WaveArgs a;
+    if (volumesApart(s, paths, records)) {
+        a.vol = s->vol;
+        a.vol.count = s->waveCounters + kWaveCounters - 1;
+    }
     a.scene = viewOf(s);
     a.w = s->wave;
     a.paths = paths;
@@ -1356,7 +1411,7 @@ WaveArgs launchArgs(x2_scene* s, Slot& sl, uint32_t paths, uint32_t records, uns
     a.lastExtend = s->waveCounters + 1;
     a.shadowQ = s->shadowQ;
     a.shadowCount = s->waveCounters + 2;
-    a.shadowSlots = s->shadowOrder && a.recordsPerPath <= x2::kRecordSegments ? s->waveCounters + 8 : nullptr;
+    a.shadowSlots = s->shadowOrder && !a.vol.head && a.recordsPerPath <= x2::kRecordSegments ? s->waveCounters + 8 : nullptr;
     a.extendSlots = s->extendBins ? s->waveCounters + 8 + x2::kRecordSegments : nullptr;
     a.extendNext = s->waveCounters + 3;
     a.shadowNext = s->waveCounters + 4;
@@ -1410,7 +1465,7 @@ int x2_launch_wavefront(x2_scene* s, const x2_chunk* chunks, uint32_t count) {
         return X2_EINVAL;
     }
     const uint32_t records = s->config.light_count * s->config.light_samples + 1;
-    uint32_t paths = s->reservePaths ? s->reservePaths : defaultPaths(records);
+    uint32_t paths = s->reservePaths ? s->reservePaths : defaultPaths(records, s->volumeCount ? volumeBytes(s->config, records) : 0.0);
     if (paths > items) paths = uint32_t(items < 1024 ? 1024 : items);
     if (int rc = ensureWave(s, paths, records)) return rc;
     if (int rc = ensureItems(s, items)) return rc;
@@ -1426,7 +1481,8 @@ int x2_launch_wavefront(x2_scene* s, const x2_chunk* chunks, uint32_t count) {
     const WaveGrids grids = waveGrids(paths, records, s->ctx->smCount, s->blocksPerSm);
     const WaveKernels wk = waveKernels(s->traceBlocks, s->shadeBlocks, s->volumeCount != 0, s->triUV != nullptr, s->shortStack != 0,
                                        a.scene.stats != nullptr, s->shadeSplit != 0,
-                                       s->wave.lightJob != nullptr ? s->lightSplit : 0u, s->triOverlap != 0 && s->shortStack != 0 && s->traceBlocks < 9);
+                                       s->wave.lightJob != nullptr ? s->lightSplit : 0u, s->triOverlap != 0 && s->shortStack != 0 && s->traceBlocks < 9,
+                                       a.vol.head != nullptr);
     const uint64_t maxIter = items * (uint64_t(s->config.max_depth) + 2) / paths + uint64_t(s->config.max_depth) + 64;
     if (s->waveTiming) {
         // Diagnostic form: no graph; events around every kernel, the iteration's times added once it is done.
@@ -1446,6 +1502,7 @@ int x2_launch_wavefront(x2_scene* s, const x2_chunk* chunks, uint32_t count) {
             launchShade(wk, a, grids.work, st);
             cudaEventRecord(ev[3], st);
             wk.shadow<<<grids.shadow, kWaveBlock, 0, st>>>(a);
+            if (wk.volumeShadow) wk.volumeShadow<<<grids.shadow, kWaveBlock, 0, st>>>(a);
             cudaEventRecord(ev[4], st);
             cudaMemcpyAsync(s->hostLast, s->waveCounters, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
             wfResetQueues<<<1, 32, 0, st>>>(a);
@@ -1723,7 +1780,7 @@ int x2_adjoint(x2_scene* s, uint32_t first, uint32_t count, const float* d_dloss
         return X2_EINVAL;
     }
     const uint32_t records = s->config.light_count * s->config.light_samples + 1;
-    uint32_t paths = s->reservePaths ? s->reservePaths : defaultPaths(records);
+    uint32_t paths = s->reservePaths ? s->reservePaths : defaultPaths(records, s->volumeCount ? volumeBytes(s->config, records) : 0.0);
     if (paths > items) paths = uint32_t(items < 1024 ? 1024 : items);
     const uint32_t verts = s->config.max_depth + 1;
     if (int rc = ensureWave(s, paths, records)) return rc;
@@ -1786,7 +1843,7 @@ int x2_adjoint(x2_scene* s, uint32_t first, uint32_t count, const float* d_dloss
     a.lastExtend = s->waveCounters + 1;
     a.shadowQ = s->shadowQ;
     a.shadowCount = s->waveCounters + 2;
-    a.shadowSlots = s->shadowOrder && a.recordsPerPath <= x2::kRecordSegments ? s->waveCounters + 8 : nullptr;
+    a.shadowSlots = s->shadowOrder && !a.vol.head && a.recordsPerPath <= x2::kRecordSegments ? s->waveCounters + 8 : nullptr;
     a.extendSlots = s->extendBins ? s->waveCounters + 8 + x2::kRecordSegments : nullptr;
     a.extendNext = s->waveCounters + 3;
     a.shadowNext = s->waveCounters + 4;
@@ -2155,7 +2212,7 @@ int renderAdaptive(x2_scene* s, uint32_t minSamples, uint32_t maxSamples, float 
     Slot& sl = s->slots[0];
     if (int rc = ensureSlot(sl, ad.tiles)) return rc;
     const uint32_t records = s->config.light_count * s->config.light_samples + 1;
-    uint32_t paths = s->reservePaths ? s->reservePaths : defaultPaths(records);
+    uint32_t paths = s->reservePaths ? s->reservePaths : defaultPaths(records, s->volumeCount ? volumeBytes(s->config, records) : 0.0);
     if (paths > maxItems) paths = uint32_t(maxItems < 1024 ? 1024 : maxItems);
     if (int rc = ensureWave(s, paths, records)) return rc;
     if (int rc = ensureItems(s, maxItems)) return rc;
@@ -2176,7 +2233,8 @@ int renderAdaptive(x2_scene* s, uint32_t minSamples, uint32_t maxSamples, float 
     const WaveGrids grids = waveGrids(paths, records, s->ctx->smCount, s->blocksPerSm);
     const WaveKernels wk = waveKernels(s->traceBlocks, s->shadeBlocks, s->volumeCount != 0, s->triUV != nullptr, s->shortStack != 0,
                                        a.scene.stats != nullptr, s->shadeSplit != 0,
-                                       s->wave.lightJob != nullptr ? s->lightSplit : 0u, s->triOverlap != 0 && s->shortStack != 0 && s->traceBlocks < 9);
+                                       s->wave.lightJob != nullptr ? s->lightSplit : 0u, s->triOverlap != 0 && s->shortStack != 0 && s->traceBlocks < 9,
+                                       a.vol.head != nullptr);
     const uint64_t bound = maxItems * (uint64_t(s->config.max_depth) + 2) / paths + uint64_t(s->config.max_depth) + 64;
     const uint32_t maxIter = uint32_t(std::min<uint64_t>(bound, 0xffffffffu));
 

@@ -140,20 +140,15 @@ __device__ __forceinline__ void cameraPending(const CameraRay& camera, Pending& 
 // through them (pv's T and volume depth change) and, for a camera ray that hits nothing, their opacity as its alpha.
 // kVolumes false compiles the volume code out (the kernels for scenes without volumes: the march's state would
 // otherwise take registers and stack from every surface vertex); a scene with volumes takes the kVolumes form.
-template <bool kVolumes = true>
-__device__ __forceinline__ void afterTrace(const SceneView& s, const Identity& root, Pending& pv, const Hit& hit, V3 cameraPosition,
-                                           V3& radiance, float& alpha) {
+__device__ __forceinline__ void afterHeld(const Pending& pv, const Hit& hit, V3& radiance) {
     if (pv.heldLight != ~0u) {
         const float kept = hit.geom != ~0u && hit.t < pv.heldFar ? 0.0f : 1.0f;
         if (kept > 0.0f) radiance = add(radiance, kept < 1.0f ? mul(pv.held, kept) : pv.held);
     }
-    V3 volumeAlphaT{1, 1, 1};
-    if (kVolumes && s.config.volume_count) {
-        const float tEnd = hit.geom == ~0u ? pv.farT : hit.t;
-        const V3 volumeLight = s.config.volume_estimator == 1 ? volumeRadianceTracked(s, root, pv, pv.origin, pv.dir, pv.nearT, tEnd, volumeAlphaT)
-                                                              : volumeRadiance(s, root, pv, pv.origin, pv.dir, pv.nearT, tEnd, volumeAlphaT);
-        radiance = add(radiance, volumeLight);
-    }
+}
+// What follows the ray's volumes: volumeAlphaT is their transmittance for the alpha.
+__device__ __forceinline__ void afterVolumes(const SceneView& s, const Identity& root, const Pending& pv, const Hit& hit, V3 cameraPosition,
+                                             V3 volumeAlphaT, V3& radiance, float& alpha) {
     // A camera ray that hits nothing: the volumes' opacity (none without volumes: 1 - (1+1+1)/3); a hit adds one (its
     // holdouts' minimum transmittance is zero with no holdouts; shadeVertex).
     if (hit.geom == ~0u && pv.depth == 0) alpha += 1.0f * (1.0f - (volumeAlphaT.x + volumeAlphaT.y + volumeAlphaT.z) / 3.0f);
@@ -162,6 +157,19 @@ __device__ __forceinline__ void afterTrace(const SceneView& s, const Identity& r
         const V3 Lv = mulv(pv.T, visibleLights(s, root, missed ? pv.origin : cameraPosition, pv.dir, missed ? 3.4028234663852886e+38f : hit.t));
         radiance = add(radiance, Lv);
     }
+}
+template <bool kVolumes = true>
+__device__ __forceinline__ void afterTrace(const SceneView& s, const Identity& root, Pending& pv, const Hit& hit, V3 cameraPosition,
+                                           V3& radiance, float& alpha) {
+    afterHeld(pv, hit, radiance);
+    V3 volumeAlphaT{1, 1, 1};
+    if (kVolumes && s.config.volume_count) {
+        const float tEnd = hit.geom == ~0u ? pv.farT : hit.t;
+        const V3 volumeLight = s.config.volume_estimator == 1 ? volumeRadianceTracked(s, root, pv, pv.origin, pv.dir, pv.nearT, tEnd, volumeAlphaT)
+                                                              : volumeRadiance(s, root, pv, pv.origin, pv.dir, pv.nearT, tEnd, volumeAlphaT);
+        radiance = add(radiance, volumeLight);
+    }
+    afterVolumes(s, root, pv, hit, cameraPosition, volumeAlphaT, radiance, alpha);
 }
 
 // A shadow ray and what it carries when nothing occludes [near, far].
@@ -182,10 +190,15 @@ struct LightJob {
     bool hasCull, split, clampHere, rr;
 };
 
+// Volume code in a kernel: none (the scene has no volumes), inline, or in kernels of their own (the wavefront form of a
+// scene with volumes): the sink then gets the stream's branch of a shadow ray's transmittance (volumeBranch) in place
+// of the transmittance, and the ray's own volumes are settled by afterVolumes.
+enum : int { kNoVolumes = 0, kInlineVolumes = 1, kApartVolumes = 2 };
+
 // A vertex's light samples (async_integrator.h:2633-2772): every light of the set that can light the hit, each sample's
 // contribution, MIS-weighted against the lobe, clamped and rouletted, to the sink as a shadow request, in light order.
 // root: the sample's identity (pixel, index, the frame seed, branch 0).
-template <bool kVolumes, int kLobe, class Sink>
+template <int kVolumes, int kLobe, class Sink>
 __device__ __forceinline__ void lightSamples(const SceneView& s, const Identity& root, const LightJob& j, Sink& sink) {
     const x2_config& c = s.config;
     const uint32_t policy = c.sampling;
@@ -249,7 +262,9 @@ __device__ __forceinline__ void lightSamples(const SceneView& s, const Identity&
             q.dir = wi;
             q.near = fmaxf(0.0f, 0.0f);
             q.far = fmaxf((lh.distance - 0.0f) * kHitEpsilonEnd, 2.0f * q.near);
-            if (volumes) {
+            if constexpr (kVolumes == kApartVolumes) {
+                sink.volumeBranch(childBranch(lightAddress, si, 0xfffb), j.depth);
+            } else if (volumes) {
                 // The volumes on the shadow ray's way (transmittance(), async_integrator.h:2722-2731); it matters only
                 // when nothing occludes the ray, and its stream is its own, so it is taken here.
                 Identity tid = lid;
@@ -273,7 +288,7 @@ __device__ __forceinline__ void lightSamples(const SceneView& s, const Identity&
 // kLobe: the lobe kind every vertex of the launch makes (1 Lambert, 2 GGX; 0 any), as the per-lobe shade queues sort
 // them; the kernel then holds one lobe's evaluation and sampling code.
 // kDeferLights: the light samples are not taken here; the sink gets the vertex's LightJob (sink.lights) instead.
-template <bool kVolumes = true, bool kTextures = true, int kLobe = 0, bool kDeferLights = false, class Sink>
+template <int kVolumes = kInlineVolumes, bool kTextures = true, int kLobe = 0, bool kDeferLights = false, class Sink>
 __device__ __forceinline__ bool shadeVertex(const SceneView& s, const Identity& root, uint32_t pixel, uint32_t index, const Pending& pv,
                                             const Hit& hit, V3 va, V3 vb, V3 vc, uint32_t top, V3& radiance, float& alpha, Sink& sink) {
     const x2_config& c = s.config;
@@ -439,7 +454,9 @@ __device__ __forceinline__ bool shadeVertex(const SceneView& s, const Identity& 
                 q.far = shadowFar;
                 q.contribution = direct;
                 q.light = lightIndex;
-                if (volumes) {
+                if constexpr (kVolumes == kApartVolumes) {
+                    sink.volumeBranch(childBranch(sampleBranch, 0xfffb, 0), pv.depth);
+                } else if (volumes) {
                     Identity tid = bid;
                     tid.branch = childBranch(sampleBranch, 0xfffb, 0);
                     Stream vs(tid, pv.depth, 0);

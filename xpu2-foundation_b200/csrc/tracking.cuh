@@ -194,27 +194,17 @@ static __device__ __noinline__ V3 trackedSourceTerm(const SceneView& s, Stream& 
     return vscaled(Li, tr * phaseEval(g, V3{-rayDir.x, -rayDir.y, -rayDir.z}, wi) / pdfL);
 }
 
-// volumeRadiance by tracking: the camera ray's emission, the single scattering of every light (a volume depth on) and
-// the path's throughput through the volumes, as volume.cuh's volumeRadiance returns them. pv's T and volume depth are
-// updated.
-static __device__ __noinline__ V3 volumeRadianceTracked(const SceneView& s, const Identity& root, Pending& pv, V3 org, V3 dir, float tnear, float tfar,
-                                                        V3& alphaTransmittance) {
+// Ratio tracking along a ray: its transmittance w and (a camera ray) the light its volumes emit.
+static __device__ __noinline__ void trackedPass(const SceneView& s, const Identity& root, const Pending& pv, U64 volumeBranch, const Crossing* x,
+                                                uint32_t n, uint32_t regions, float tfar, float& w, V3& emitted) {
     const x2_config& c = s.config;
-    V3 radiance{0, 0, 0};
-    alphaTransmittance = V3{1, 1, 1};
-    Crossing x[kMaxCrossings];
-    uint32_t regions;
-    const uint32_t n = volumeIntervals(s, org, dir, tnear, x, regions);
-    if (n == 0 && regions == 0) return radiance;
-    const U64 volumeBranch = childBranch(pv.branch, 0xfffa, pv.volumeDepth);
+    const V3 org = pv.origin, dir = pv.dir;
     Identity vid = root;
     vid.branch = childBranch(volumeBranch, 0, 0);
     Stream st(vid, pv.depth, 0);
-    const V3 T = pv.T;
-    // Ratio tracking along the ray: its transmittance and (a camera ray) its emission.
     const bool sampleEmission = pv.depth == 0;
-    float w = 1.0f;
-    V3 emitted{0, 0, 0};
+    w = 1.0f;
+    emitted = V3{0, 0, 0};
     auto along = [&](float t, float mu, uint32_t here) {
         V3 e[kMaxVolumes];
         uint32_t chosen = kMaxVolumes;
@@ -232,49 +222,100 @@ static __device__ __noinline__ V3 volumeRadianceTracked(const SceneView& s, cons
         }
         return ratioStep(w, k.sigmaT.x, mu, st);
     };
-    trackIntervals(s, x, n, regions, org, dir, tnear, tfar, st, along);
-    if (sampleEmission) radiance = vplus(radiance, vtimes(T, emitted));
+    trackIntervals(s, x, n, regions, org, dir, pv.nearT, tfar, st, along);
+}
+
+// One scattering sample: delta tracking's collision (none: the ray passed), then every light's source term there, handed
+// to add(light sample, contribution) in their order.
+template <class Add>
+__device__ __forceinline__ void trackedScatter(const SceneView& s, const Identity& root, const Pending& pv, U64 volumeBranch, const Crossing* x,
+                                               uint32_t n, uint32_t regions, float tfar, uint32_t ts, uint32_t samplesPerLight,
+                                               uint32_t scatterCount, float invN, Add& sum) {
+    const x2_config& c = s.config;
+    const V3 org = pv.origin, dir = pv.dir, T = pv.T;
+    Identity did = root;
+    did.branch = childBranch(volumeBranch, 0xfff0, ts);
+    Stream ds(did, pv.depth, 0);
+    float hitT = -1.0f, sigmaT = 0.0f, g = 0.0f;
+    V3 sigmaS{0, 0, 0};
+    auto collide = [&](float t, float mu, uint32_t here) {
+        const VolumeCoefficients k = evalShadersAt(s, here, c.volume_overlap_mode, 0.0f, add(org, mul(dir, t)), kNoGrid, nullptr, nullptr);
+        if (ds.next() * mu < k.sigmaT.x) {
+            hitT = t;
+            sigmaS = k.sigmaS;
+            sigmaT = k.sigmaT.x;
+            g = k.g;
+            return false;
+        }
+        return true;
+    };
+    trackIntervals(s, x, n, regions, org, dir, pv.nearT, tfar, ds, collide);
+    if (hitT < 0.0f || !(sigmaT > 0.0f)) return;
+    const V3 P = add(org, mul(dir, hitT));
+    const V3 albedo = vscaled(sigmaS, 1.0f / sigmaT);
+    for (uint32_t li = 0; li < c.light_count; ++li)
+        for (uint32_t ls = 0; ls < samplesPerLight; ++ls) {
+            Identity sid = root;
+            sid.branch = childBranch(volumeBranch, 1 + li, ls * scatterCount + ts);
+            Stream ss(sid, pv.depth, 0);
+            const float ul[3] = {ss.next(), ss.next(), ss.next()};
+            const V3 Ls = trackedSourceTerm(s, ss, s.lights[li], P, dir, g, ul);
+            sum(li * samplesPerLight + ls, vscaled(vtimes(vtimes(T, albedo), Ls), invN));
+        }
+}
+
+// volumeRadiance by tracking: the camera ray's emission, the single scattering of every light (a volume depth on) and
+// the path's throughput through the volumes, as volume.cuh's volumeRadiance returns them. pv's T and volume depth are
+// updated. (pv holds the ray: org, dir and tnear are its own.)
+static __device__ __noinline__ V3 volumeRadianceTracked(const SceneView& s, const Identity& root, Pending& pv, V3 org, V3 dir, float tnear, float tfar,
+                                                        V3& alphaTransmittance) {
+    const x2_config& c = s.config;
+    V3 radiance{0, 0, 0};
+    alphaTransmittance = V3{1, 1, 1};
+    Crossing x[kMaxCrossings];
+    uint32_t regions;
+    const uint32_t n = volumeIntervals(s, org, dir, tnear, x, regions);
+    if (n == 0 && regions == 0) return radiance;
+    const U64 volumeBranch = childBranch(pv.branch, 0xfffa, pv.volumeDepth);
+    float w;
+    V3 emitted;
+    trackedPass(s, root, pv, volumeBranch, x, n, regions, tfar, w, emitted);
+    if (pv.depth == 0) radiance = vplus(radiance, vtimes(pv.T, emitted));
     alphaTransmittance = V3{w, w, w};
     if (pv.volumeDepth < c.max_volume_depth) {
-        // Single scattering: delta tracking's collision (none: the ray passed), then every light's source term there.
         const bool highQuality = pv.nonMirror == 0;
         const uint32_t samplesPerLight = highQuality ? c.light_samples : 1, scatterCount = highQuality ? c.volume_illumination_samples : 1;
         const float invN = 1.0f / float(samplesPerLight * (scatterCount ? scatterCount : 1));
-        for (uint32_t ts = 0; ts < scatterCount; ++ts) {
-            Identity did = root;
-            did.branch = childBranch(volumeBranch, 0xfff0, ts);
-            Stream ds(did, pv.depth, 0);
-            float hitT = -1.0f, sigmaT = 0.0f, g = 0.0f;
-            V3 sigmaS{0, 0, 0};
-            auto collide = [&](float t, float mu, uint32_t here) {
-                const VolumeCoefficients k = evalShadersAt(s, here, c.volume_overlap_mode, 0.0f, add(org, mul(dir, t)), kNoGrid, nullptr, nullptr);
-                if (ds.next() * mu < k.sigmaT.x) {
-                    hitT = t;
-                    sigmaS = k.sigmaS;
-                    sigmaT = k.sigmaT.x;
-                    g = k.g;
-                    return false;
-                }
-                return true;
-            };
-            trackIntervals(s, x, n, regions, org, dir, tnear, tfar, ds, collide);
-            if (hitT < 0.0f || !(sigmaT > 0.0f)) continue;
-            const V3 P = add(org, mul(dir, hitT));
-            const V3 albedo = vscaled(sigmaS, 1.0f / sigmaT);
-            for (uint32_t li = 0; li < c.light_count; ++li)
-                for (uint32_t ls = 0; ls < samplesPerLight; ++ls) {
-                    Identity sid = root;
-                    sid.branch = childBranch(volumeBranch, 1 + li, ls * scatterCount + ts);
-                    Stream ss(sid, pv.depth, 0);
-                    const float ul[3] = {ss.next(), ss.next(), ss.next()};
-                    const V3 Ls = trackedSourceTerm(s, ss, s.lights[li], P, dir, g, ul);
-                    radiance = vplus(radiance, vscaled(vtimes(vtimes(T, albedo), Ls), invN));
-                }
-        }
+        auto sum = [&](uint32_t, V3 v) { radiance = vplus(radiance, v); };
+        for (uint32_t ts = 0; ts < scatterCount; ++ts)
+            trackedScatter(s, root, pv, volumeBranch, x, n, regions, tfar, ts, samplesPerLight, scatterCount, invN, sum);
         ++pv.volumeDepth;
     }
     pv.T = vscaled(pv.T, w);
     return radiance;
+}
+
+// The parts of it that a wavefront launch makes in kernels of their own (volume.cuh VolumeHead): the walk along the ray,
+// and sample ts of its scattering samples.
+__device__ __forceinline__ void trackedFirstPass(const SceneView& s, const Identity& root, const Pending& pv, float tfar, Crossing* x,
+                                                 VolumeHead& head, V3& vt, V3& radiance) {
+    const x2_config& c = s.config;
+    head = VolumeHead{0, 0, 0, 0, 0.0f, 0.0f, 0.0f, 0};
+    vt = V3{1, 1, 1};
+    radiance = V3{0, 0, 0};
+    uint32_t regions;
+    const uint32_t n = volumeIntervals(s, pv.origin, pv.dir, pv.nearT, x, regions);
+    head.crossings = n;
+    head.regions = regions;
+    if (n == 0 && regions == 0) return;
+    float w;
+    V3 emitted;
+    trackedPass(s, root, pv, childBranch(pv.branch, 0xfffa, pv.volumeDepth), x, n, regions, tfar, w, emitted);
+    if (pv.depth == 0) radiance = vplus(radiance, vtimes(pv.T, emitted));
+    vt = V3{w, w, w};
+    const bool deeper = pv.volumeDepth < c.max_volume_depth;
+    head.flags = kVolumePassed | (deeper ? kVolumeDeeper : 0u) |
+                 (deeper && (pv.nonMirror == 0 ? c.volume_illumination_samples : 1u) > 0 ? kVolumeScatters : 0u);
 }
 
 }  // namespace x2

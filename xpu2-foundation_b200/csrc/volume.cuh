@@ -229,6 +229,82 @@ static __device__ __noinline__ VolumeCoefficients evalShadersAt(const SceneView&
     return c;
 }
 
+// One volume's density lookups along a stretch: what every step reads of its records, in registers. Only for a volume whose
+// maps are axis-aligned (VolumeRec::diagonal, GridRec::diagonal) and a density grid of one channel; the lookups give
+// sampleGrid's values bit for bit.
+struct DensityLookup {
+    V3 scale, offset;  // its world to grid space
+    double m[3], b[3]; // grid space to index
+    const float* values;
+    int lo[3], dims[3];
+    __device__ V3 gridPoint(V3 p) const { return V3{scale.x * p.x + offset.x, scale.y * p.y + offset.y, scale.z * p.z + offset.z}; }
+    __device__ float at(int i, int j, int k) const {
+        const int x = i - lo[0], y = j - lo[1], z = k - lo[2];
+        if (x < 0 || y < 0 || z < 0 || x >= dims[0] || y >= dims[1] || z >= dims[2]) return 0.0f;
+        return __ldg(values + ((size_t(z) * size_t(dims[1]) + size_t(y)) * size_t(dims[0]) + size_t(x)));
+    }
+    __device__ float box(V3 g) const {
+        const double x = double(g.x) * m[0] + b[0], y = double(g.y) * m[1] + b[1], z = double(g.z) * m[2] + b[2];
+        const int i = int(floor(x)), j = int(floor(y)), k = int(floor(z));
+        const double u = x - i, v = y - j, w = z - k;
+        float d[2][2][2];
+        const int xx = i - lo[0], yy = j - lo[1], zz = k - lo[2];
+        if (xx >= 0 && yy >= 0 && zz >= 0 && xx < dims[0] - 1 && yy < dims[1] - 1 && zz < dims[2] - 1) {
+            const size_t sy = size_t(dims[0]), sz = sy * size_t(dims[1]);
+            const float* q = values + sz * size_t(zz) + sy * size_t(yy) + size_t(xx);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) d[c >> 2][(c >> 1) & 1][c & 1] = __ldg(q + (c >> 2) + ((c >> 1) & 1) * sy + (c & 1) * sz);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) d[c >> 2][(c >> 1) & 1][c & 1] = at(i + (c >> 2), j + ((c >> 1) & 1), k + (c & 1));
+        }
+        return boxLerp(boxLerp(boxLerp(d[0][0][0], d[0][0][1], w), boxLerp(d[0][1][0], d[0][1][1], w), v),
+                       boxLerp(boxLerp(d[1][0][0], d[1][0][1], w), boxLerp(d[1][1][0], d[1][1][1], w), v), u);
+    }
+    __device__ float point(V3 g) const {
+        return at(int(round(double(g.x) * m[0] + b[0])), int(round(double(g.y) * m[1] + b[1])), int(round(double(g.z) * m[2] + b[2])));
+    }
+};
+// DensityLookup's nearest voxel with its index made in floats where they decide it: the index's float value is within
+// `guard` of the double that sampleGrid rounds (products and sums of values of at most the stretch's ends' size, each
+// rounded to 2^-24, under 2^-21 of it together), so unless it lies that close to half way between two voxels both round
+// to the same one. Conversions to and from doubles take a quarter of the rate of the rest, six of them a step.
+struct NearestVoxel {
+    const DensityLookup& d;
+    V3 m, b, guard;
+    __device__ NearestVoxel(const DensityLookup& lookup, V3 from, V3 to) : d(lookup) {
+        const V3 g0 = d.gridPoint(from), g1 = d.gridPoint(to);
+        m = V3{float(d.m[0]), float(d.m[1]), float(d.m[2])};
+        b = V3{float(d.b[0]), float(d.b[1]), float(d.b[2])};
+        auto half = [](float g0, float g1, float m, float b) { return 0.5f - 0x1p-20f * (fmaxf(fabsf(g0), fabsf(g1)) * fabsf(m) + fabsf(b) + 1.0f); };
+        guard = V3{half(g0.x, g1.x, m.x, b.x), half(g0.y, g1.y, m.y, b.y), half(g0.z, g1.z, m.z, b.z)};
+    }
+    __device__ float at(V3 p) const {
+        const V3 g = d.gridPoint(p);
+        const float magic = 12582912.0f;  // 1.5 x 2^23: adding it rounds to a whole number in the low mantissa bits
+        const float x = __fmaf_rn(g.x, m.x, b.x), y = __fmaf_rn(g.y, m.y, b.y), z = __fmaf_rn(g.z, m.z, b.z);
+        const float rx = x + magic, ry = y + magic, rz = z + magic;
+        if (fabsf(x - (rx - magic)) < guard.x && fabsf(y - (ry - magic)) < guard.y && fabsf(z - (rz - magic)) < guard.z)
+            return d.at(__float_as_int(rx) - 0x4b400000, __float_as_int(ry) - 0x4b400000, __float_as_int(rz) - 0x4b400000);
+        return d.point(g);
+    }
+};
+__device__ __forceinline__ bool densityLookup(const SceneView& s, const VolumeRec& v, DensityLookup& d) {
+    if (!v.diagonal || v.densityGrid >= s.gridCount) return false;
+    const GridRec& g = s.grids[v.densityGrid];
+    if (!g.diagonal || g.channels != 1) return false;
+    d.scale = V3{v.worldToGrid[0], v.worldToGrid[5], v.worldToGrid[10]};
+    d.offset = V3{v.worldToGrid[3], v.worldToGrid[7], v.worldToGrid[11]};
+    for (int a = 0; a < 3; ++a) {
+        d.m[a] = g.worldToIndex[5 * a];
+        d.b[a] = g.worldToIndex[12 + a];
+        d.lo[a] = g.lo[a];
+        d.dims[a] = g.dims[a];
+    }
+    d.values = g.values;
+    return true;
+}
+
 __device__ __forceinline__ float minFeatureSize(const SceneView& s, uint32_t regions) {
     float m = 3.402823466e+38f;
     for (uint32_t v = 0; v < s.config.volume_count; ++v)
@@ -237,21 +313,44 @@ __device__ __forceinline__ float minFeatureSize(const SceneView& s, uint32_t reg
 }
 
 // ---- crossings (async_cpu.h:1089-1149, with the box meshes' triangles tested one by one) and interiority ----
+// The crossings come one at a time, each the nearest triangle past the last one (lowest index first where two are as near);
+// a triangle's t does not depend on where the search starts, so every triangle is tested once and the search runs over
+// the few that the ray meets (a box: two to four). A ray that meets more than kMet is searched as the backends do,
+// triangle by triangle from each crossing.
 static __device__ __noinline__ uint32_t volumeCrossings(const SceneView& s, V3 o, V3 d, float tnear, Crossing* x) {
     const RayQ r = makeRay(s.bvh, o.x, o.y, o.z, d.x, d.y, d.z);
     const uint32_t tris = 12u * s.config.volume_count;
+    const float inf = __int_as_float(0x7f800000);
+    auto test = [&](uint32_t i, float from, float& th) {
+        const float* v = s.volumeTris + 9 * i;
+        const float4 a = make_float4(v[0], v[1], v[2], 0.0f), b = make_float4(v[3], v[4], v[5], 0.0f), c = make_float4(v[6], v[7], v[8], 0.0f);
+        return triTest(r, a, b, c, from, inf, th);
+    };
+    constexpr uint32_t kMet = 8;
+    float metT[kMet];
+    uint32_t metTri[kMet];
+    uint32_t met = 0;
+    for (uint32_t i = 0; i < tris; ++i) {
+        float th;
+        if (!test(i, tnear, th)) continue;
+#pragma unroll
+        for (uint32_t m = 0; m < kMet; ++m)
+            if (m == met) metT[m] = th, metTri[m] = i;
+        ++met;
+    }
     uint32_t n = 0;
     float t = tnear;
     for (uint32_t k = 0; k < 4 * kMaxCrossings && n < kMaxCrossings; ++k) {
-        float best = __int_as_float(0x7f800000);
+        float best = inf;
         uint32_t hitTri = ~0u;
-        for (uint32_t i = 0; i < tris; ++i) {
-            const float* v = s.volumeTris + 9 * i;
-            const float4 a = make_float4(v[0], v[1], v[2], 0.0f), b = make_float4(v[3], v[4], v[5], 0.0f), c = make_float4(v[6], v[7], v[8], 0.0f);
-            float th;
-            if (triTest(r, a, b, c, t, __int_as_float(0x7f800000), th) && th < best) {
-                best = th;
-                hitTri = i;
+        if (met <= kMet) {
+#pragma unroll
+            for (uint32_t m = 0; m < kMet; ++m)
+                if (m < met && metT[m] >= t && metT[m] < best) best = metT[m], hitTri = metTri[m];
+        } else {
+            for (uint32_t i = 0; i < tris; ++i) {
+                float th;
+                if (test(i, t, th) && th < best) best = th, hitTri = i;
             }
         }
         if (hitTri == ~0u) break;
@@ -338,24 +437,28 @@ struct VolumeStep {  // volume::Step without holdouts
 };
 __device__ __forceinline__ float stepWeight(const VolumeStep& s) { return vlum(vtimes(vscaled(s.sigmaS, s.delta), s.tr)) + 0.0f; }
 
-struct MarchCheckpoint {
-    Stream marching;
+// A place to march again from: 48 bytes, the stream as its next dimension (its words are made again from it).
+struct alignas(16) MarchCheckpoint {
     V3 vt;
     float t, stepStart, stepSize, partial;
-    uint32_t interval, regions, count, visited;
+    uint32_t interval, regions, count, visited, dimension;
 };
+static_assert(sizeof(MarchCheckpoint) == 48, "three 16-byte words");
+// A march's checkpoints, every `stride` steps, the stride doubling once `slots` of them are held.
 struct MarchRecord {
-    static constexpr uint32_t kSlots = 8;
-    MarchCheckpoint at[kSlots];
+    static constexpr uint32_t kSlots = 8;  // of a march inside one thread (in its local memory)
+    MarchCheckpoint* at;
+    uint32_t slots;
     uint32_t used = 0, stride = 8, last = 0;
+    __device__ MarchRecord(MarchCheckpoint* memory, uint32_t n) : at(memory), slots(n) {}
     __device__ bool wants(uint32_t count) const {
         if (count == 0 || count == last || count % stride) return false;
-        return used < kSlots || count % (2 * stride) == 0;
+        return used < slots || count % (2 * stride) == 0;
     }
     __device__ MarchCheckpoint& slot(uint32_t count) {
-        if (used == kSlots) {
-            for (uint32_t i = 0; i < kSlots / 2; ++i) at[i] = at[2 * i + 1];
-            used = kSlots / 2;
+        if (used == slots) {
+            for (uint32_t i = 0; i < slots / 2; ++i) at[i] = at[2 * i + 1];
+            used = slots / 2;
             stride *= 2;
         }
         last = count;
@@ -384,15 +487,45 @@ struct VolumeMarch {
     template <class Emit>
     __device__ void stepping(Emit& emit, Stream& marching, uint32_t regions, float t1, float t, float stepStart, float stepSize, uint32_t interval) {
         const x2_config& c = s.config;
+        // A stretch inside one volume whose lookups DensityLookup makes: evalShadersAt's result for it (sum and max
+        // overlap: that volume's own coefficients), with the volume's records read once a stretch, not once a step.
+        const bool single = __popc(regions) == 1 && c.volume_overlap_mode != kOverlapRnd;
+        const uint32_t only = single ? __ffs(regions) - 1 : 0u;
+        const VolumeRec& vr = s.volumes[only];
+        DensityLookup density;
+        const bool fast = single && vr.interpolation <= kInterpBox && densityLookup(s, vr, density);
+        const V3 gain = vr.gain, albedo = cmax0(vr.colorMult);
+        const float phase = fminf(fmaxf(vr.g, -1.0f), 1.0f);
+        const bool box = vr.interpolation == kInterpBox;
         auto step = [&](float at) {
-            const float rnd = c.volume_overlap_mode == kOverlapRnd ? marching.next() : 0.0f;
             V3 emissions[kDeviceVolumes];
             uint32_t chosen = kMaxVolumes;
-            const VolumeCoefficients k =
-                evalShadersAt(s, regions, c.volume_overlap_mode, rnd, add(org, mul(dir, at)), kNoGrid, sampleEmission ? emissions : nullptr, &chosen);
+            VolumeCoefficients k;
+            const V3 p = add(org, mul(dir, at));
+            if (fast) {
+                const V3 gp = density.gridPoint(p);
+                k.sigmaT = cmax0(vscaled(gain, box ? density.box(gp) : density.point(gp)));
+                k.sigmaS = vtimes(albedo, k.sigmaT);
+                k.g = vlum(vscaled(k.sigmaS, phase));
+                const float normalization = vlum(k.sigmaS);
+                if (normalization > 0.0f) k.g /= normalization;
+            } else {
+                const float rnd = c.volume_overlap_mode == kOverlapRnd ? marching.next() : 0.0f;
+                k = evalShadersAt(s, regions, c.volume_overlap_mode, rnd, p, kNoGrid, sampleEmission ? emissions : nullptr, &chosen);
+            }
             const float delta = at - stepStart;
             if (!emit(VolumeStep{k.sigmaT, k.sigmaS, vt, k.g, stepStart, delta}, count)) stopped = true;
             ++count;
+            if (fast) {
+                if (sampleEmission) {
+                    V3 temperature{0, 0, 0};
+                    if (vr.emissionGrid != kNoGrid && vr.emissionGrid < s.gridCount && s.grids[vr.emissionGrid].channels == 3)
+                        temperature = samplePoint3(s.grids[vr.emissionGrid], density.gridPoint(p));
+                    emitted[only] = vplus(emitted[only], vscaled(vtimes(vt, cmax0(vtimes(temperature, vr.incandescence))), delta));
+                }
+                vt = vtimes(vt, expNeg(k.sigmaT, delta));
+                return;
+            }
             const V3 te = vt;
             if (sampleEmission) {
                 if (c.volume_overlap_mode == kOverlapSum) {
@@ -406,7 +539,7 @@ struct VolumeMarch {
         };
         while (t < t1) {
             if (record && weightsSoFar && record->wants(count))
-                record->slot(count) = MarchCheckpoint{marching, vt, t, stepStart, stepSize, *weightsSoFar, interval, regions, count, visited};
+                record->slot(count) = MarchCheckpoint{vt, t, stepStart, stepSize, *weightsSoFar, interval, regions, count, visited, marching.dimension};
             if (vlum(vt) < c.volume_transmittance_threshold) {
                 reachedThreshold = true;
                 return;
@@ -438,7 +571,11 @@ struct VolumeMarch {
     // The march from its start, or from a checkpoint (the same steps from there, bit for bit).
     template <class Emit>
     __device__ void run(Emit& emit, const MarchCheckpoint* from = nullptr) {
-        Stream marching = from ? from->marching : start;
+        Stream marching = start;
+        if (from) {
+            marching.dimension = from->dimension;
+            marching.group = ~0u;
+        }
         uint32_t regions = from ? from->regions : regionsAtStart;
         if (from) {
             vt = from->vt;
@@ -479,6 +616,18 @@ struct ReplaySteps {
     float total;
     bool weightless;
     const MarchRecord* record;
+    // The last checkpoint before the march's end for which `before` holds (it holds up to some checkpoint and for none
+    // after it: counts, step starts and partial weights only grow), or null.
+    template <class Before>
+    __device__ const MarchCheckpoint* last(const Before& before) const {
+        uint32_t lo = 0, hi = record ? record->used : 0u;
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (record->at[mid].count < count && before(record->at[mid])) lo = mid + 1;
+            else hi = mid;
+        }
+        return lo ? &record->at[lo - 1] : nullptr;
+    }
     __device__ float cdfBefore(const MarchCheckpoint& c) const { return weightless ? float(c.count) / float(count) : c.partial; }
     __device__ float cdf(float& partial, const VolumeStep& s, uint32_t index) const {
         if (index + 1 >= count) return total;
@@ -489,13 +638,7 @@ struct ReplaySteps {
     }
     __device__ __noinline__ VolumeStep pick(float r, float& pdf, float& remapped) const {
         const float rw = r * total;
-        const MarchCheckpoint* from = nullptr;
-        if (record)
-            for (uint32_t j = record->used; j-- > 0;)
-                if (record->at[j].count < count && cdfBefore(record->at[j]) < rw) {
-                    from = &record->at[j];
-                    break;
-                }
+        const MarchCheckpoint* from = last([&](const MarchCheckpoint& c) { return cdfBefore(c) < rw; });
         float partial = from ? from->partial : 0.0f, prev = from ? cdfBefore(*from) : 0.0f, found = total, before = 0.0f;
         VolumeStep chosen{};
         auto emit = [&](const VolumeStep& s, uint32_t i) {
@@ -515,13 +658,7 @@ struct ReplaySteps {
         return chosen;
     }
     __device__ __noinline__ VolumeStep at(float t, float& pdf) const {
-        const MarchCheckpoint* from = nullptr;
-        if (record)
-            for (uint32_t j = record->used; j-- > 0;)
-                if (record->at[j].count < count && record->at[j].stepStart <= t) {
-                    from = &record->at[j];
-                    break;
-                }
+        const MarchCheckpoint* from = last([&](const MarchCheckpoint& c) { return c.stepStart <= t; });
         float partial = from ? from->partial : 0.0f, here = from ? cdfBefore(*from) : 0.0f, kept = 0.0f, keptPrev = 0.0f;
         VolumeStep chosen{};
         auto emit = [&](const VolumeStep& s, uint32_t i) {
@@ -555,11 +692,35 @@ static __device__ __noinline__ V3 volumeTransmittance(const SceneView& s, Stream
         const float stepSize = fs * c.inv_volume_shadow_quality * fmaxf(float(depth - 1), 1.0f);
         float t = t0 + stepSize * u;
         V3 tau{0, 0, 0};
-        while (t < t1) {
-            const float rnd = c.volume_overlap_mode == kOverlapRnd ? st.next() : 0.0f;
-            tau = vplus(tau, evalShadersAt(s, regions, c.volume_overlap_mode, rnd, add(org, mul(dir, t)), kInterpPoint, nullptr, nullptr).sigmaT);
-            if (vlum(vscaled(tau, stepSize * scale)) > tauThreshold) return false;
-            t += stepSize;
+        const VolumeRec& vr = s.volumes[__ffs(regions) - 1];
+        DensityLookup density;
+        if (__popc(regions) == 1 && c.volume_overlap_mode != kOverlapRnd && densityLookup(s, vr, density)) {
+            // One volume, its nearest voxels: four steps' voxels fetched at once, then added and tested in their order.
+            const V3 gain = vr.gain;
+            const NearestVoxel nearest(density, add(org, mul(dir, t0)), add(org, mul(dir, t1)));
+            while (t < t1) {
+                float d[4];
+                bool in[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    in[k] = t < t1;
+                    d[k] = in[k] ? nearest.at(add(org, mul(dir, t))) : 0.0f;
+                    t += stepSize;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (!in[k]) break;
+                    tau = vplus(tau, cmax0(vscaled(gain, d[k])));
+                    if (vlum(vscaled(tau, stepSize * scale)) > tauThreshold) return false;
+                }
+            }
+        } else {
+            while (t < t1) {
+                const float rnd = c.volume_overlap_mode == kOverlapRnd ? st.next() : 0.0f;
+                tau = vplus(tau, evalShadersAt(s, regions, c.volume_overlap_mode, rnd, add(org, mul(dir, t)), kInterpPoint, nullptr, nullptr).sigmaT);
+                if (vlum(vscaled(tau, stepSize * scale)) > tauThreshold) return false;
+                t += stepSize;
+            }
         }
         tr = vtimes(tr, expNeg(tau, stepSize * scale));
         return vlum(tr) > c.volume_transmittance_threshold;
@@ -667,10 +828,67 @@ static __device__ __noinline__ void volumeMultipleScatter(const SceneView& s, co
     }
 }
 
-// What volumeRadiance leaves besides its light: the transmittance the path's throughput takes and the alpha's.
-struct VolumePass {
-    V3 transmittance, alphaTransmittance;
-};
+// One light's scattering sample (integrateVolumeScatteringDirect, async_integrator.h:921-997): its equi-angular part (a
+// bounded light's) and its distance part, each zero where the sample has none.
+static __device__ __noinline__ void scatterSample(const SceneView& s, const Identity& root, U64 volumeBranch, uint32_t pathDepth,
+                                                  const ReplaySteps& lookup, V3 org, V3 dir, V3 T, uint32_t li, uint32_t sample, float firstStart,
+                                                  float rayEnd, float invN, V3& equi, V3& distance) {
+    const x2_light& L = s.lights[li];
+    const bool equiAngular = boundedLight(L);
+    equi = distance = V3{0, 0, 0};
+    Identity sid = root;
+    sid.branch = childBranch(volumeBranch, 1 + li, sample);
+    Stream ss(sid, pathDepth, 0);
+    float D = 0.0f, thetaA = 0.0f, thetaB = 0.0f, offset = 0.0f;
+    float uel[3] = {0.0f, 0.0f, 0.0f};
+    if (equiAngular) {
+        const float ue = ss.next();
+        uel[0] = ss.next();
+        uel[1] = ss.next();
+        uel[2] = ss.next();
+        const V3 pivot = lightPivot(L, uel);
+        offset = dot(add(pivot, mul(org, -1.0f)), dir);
+        const V3 foot = add(org, mul(dir, offset));
+        D = length(add(pivot, mul(foot, -1.0f)));
+        thetaA = mf::atan2(firstStart - offset, D);
+        thetaB = mf::atan2(rayEnd - offset, D);
+        const float te = sampleEquiAngular(ue, D, thetaA, thetaB);
+        const float pdfTe = pdfEquiAngular(te, D, thetaA, thetaB);
+        if (pdfTe != 0.0f && vfinite(pdfTe)) {
+            const float tePrime = te + offset;
+            float pdfK;
+            const VolumeStep vp = lookup.at(tePrime, pdfK);
+            if (!vblack(vp.sigmaS)) {
+                const V3 trScatter = vtimes(vp.tr, expNeg(vp.sigmaT, tePrime - vp.tStart));
+                float mis = 1.0f;
+                const float pdfTd = pdfK * pdfDistanceExponential(tePrime, vlum(vp.sigmaT), vp.tStart, vp.tStart + vp.delta);
+                if (vfinite(pdfTd)) mis = powerHeuristic(pdfTe, pdfTd);
+                const V3 Ls = volumeSourceTerm(s, ss, L, add(org, mul(dir, tePrime)), dir, vp.g, uel, 1.0f);
+                equi = vscaled(vtimes(vtimes(T, vp.sigmaS), vtimes(trScatter, Ls)), invN * mis / pdfTe);
+            }
+        }
+    }
+    const float ud = ss.next();
+    const float udl[3] = {ss.next(), ss.next(), ss.next()};
+    float pdfDensity, udRemapped;
+    const VolumeStep vp = lookup.pick(ud, pdfDensity, udRemapped);
+    if (pdfDensity == 0.0f) return;
+    if (vblack(vp.sigmaS)) return;
+    const float sigmaT = vlum(vp.sigmaT), t0 = vp.tStart, t1 = vp.tStart + vp.delta;
+    const float td = sampleDistanceExponential(udRemapped, sigmaT, t0, t1);
+    const float pdfTd = pdfDensity * pdfDistanceExponential(td, sigmaT, t0, t1);
+    if (pdfTd == 0.0f || !vfinite(pdfTd)) return;
+    const V3 trScatter = vtimes(vp.tr, expNeg(vp.sigmaT, td - t0));
+    float mis = 1.0f;
+    if (equiAngular) {
+        const float pdfTe = pdfEquiAngular(td - offset, D, thetaA, thetaB);
+        if (vfinite(pdfTe)) mis = powerHeuristic(pdfTd, pdfTe);
+    }
+    // (The diagnostic build's shared-pivot switch gives this sample the equi-angular sample's light
+    // point, the pivot its MIS weight was computed with; the reference draws a point of its own.)
+    const V3 Ls = volumeSourceTerm(s, ss, L, add(org, mul(dir, td)), dir, vp.g, equiAngular && mf::sharedPivot() ? uel : udl, 1.0f);
+    distance = vscaled(vtimes(vtimes(T, vp.sigmaS), vtimes(trScatter, Ls)), invN * mis / pdfTd);
+}
 
 // computeRadianceVolume over [tnear, tfar] of a ray (volumeRadiance, async_integrator.h:1152-1291): the camera ray's
 // volume emission, the single scattering of every light at the march's steps (a volume depth on), and the path's
@@ -696,7 +914,8 @@ static __device__ __noinline__ V3 volumeRadiance(const SceneView& s, const Ident
         weights += stepWeight(st);
         return true;
     };
-    MarchRecord record;
+    MarchCheckpoint checkpoints[MarchRecord::kSlots];
+    MarchRecord record(checkpoints, MarchRecord::kSlots);
     march.record = &record;
     march.weightsSoFar = &weights;
     march.run(first);
@@ -723,65 +942,11 @@ static __device__ __noinline__ V3 volumeRadiance(const SceneView& s, const Ident
         if (scatterCount > 0) {
             const float invN = 1.0f / float(samplesPerLight * scatterCount);
             for (uint32_t li = 0; li < c.light_count; ++li) {
-                const x2_light& L = s.lights[li];
-                const bool equiAngular = boundedLight(L);
                 V3 direct{0, 0, 0};
-                for (uint32_t ls = 0; ls < samplesPerLight; ++ls) {
-                    for (uint32_t ts = 0; ts < scatterCount; ++ts) {
-                        Identity sid = root;
-                        sid.branch = childBranch(volumeBranch, 1 + li, ls * scatterCount + ts);
-                        Stream ss(sid, pv.depth, 0);
-                        float D = 0.0f, thetaA = 0.0f, thetaB = 0.0f, offset = 0.0f;
-                        float uel[3] = {0.0f, 0.0f, 0.0f};
-                        if (equiAngular) {
-                            const float ue = ss.next();
-                            uel[0] = ss.next();
-                            uel[1] = ss.next();
-                            uel[2] = ss.next();
-                            const V3 pivot = lightPivot(L, uel);
-                            offset = dot(add(pivot, mul(org, -1.0f)), dir);
-                            const V3 foot = add(org, mul(dir, offset));
-                            D = length(add(pivot, mul(foot, -1.0f)));
-                            thetaA = mf::atan2(firstStart - offset, D);
-                            thetaB = mf::atan2(rayEnd - offset, D);
-                            const float te = sampleEquiAngular(ue, D, thetaA, thetaB);
-                            const float pdfTe = pdfEquiAngular(te, D, thetaA, thetaB);
-                            if (pdfTe != 0.0f && vfinite(pdfTe)) {
-                                const float tePrime = te + offset;
-                                float pdfK;
-                                const VolumeStep vp = lookup.at(tePrime, pdfK);
-                                if (!vblack(vp.sigmaS)) {
-                                    const V3 trScatter = vtimes(vp.tr, expNeg(vp.sigmaT, tePrime - vp.tStart));
-                                    float mis = 1.0f;
-                                    const float pdfTd = pdfK * pdfDistanceExponential(tePrime, vlum(vp.sigmaT), vp.tStart, vp.tStart + vp.delta);
-                                    if (vfinite(pdfTd)) mis = powerHeuristic(pdfTe, pdfTd);
-                                    const V3 Ls = volumeSourceTerm(s, ss, L, add(org, mul(dir, tePrime)), dir, vp.g, uel, 1.0f);
-                                    direct = vplus(direct, vscaled(vtimes(vtimes(T, vp.sigmaS), vtimes(trScatter, Ls)), invN * mis / pdfTe));
-                                }
-                            }
-                        }
-                        const float ud = ss.next();
-                        const float udl[3] = {ss.next(), ss.next(), ss.next()};
-                        float pdfDensity, udRemapped;
-                        const VolumeStep vp = lookup.pick(ud, pdfDensity, udRemapped);
-                        if (pdfDensity == 0.0f) continue;
-                        if (vblack(vp.sigmaS)) continue;
-                        const float sigmaT = vlum(vp.sigmaT), t0 = vp.tStart, t1 = vp.tStart + vp.delta;
-                        const float td = sampleDistanceExponential(udRemapped, sigmaT, t0, t1);
-                        const float pdfTd = pdfDensity * pdfDistanceExponential(td, sigmaT, t0, t1);
-                        if (pdfTd == 0.0f || !vfinite(pdfTd)) continue;
-                        const V3 trScatter = vtimes(vp.tr, expNeg(vp.sigmaT, td - t0));
-                        float mis = 1.0f;
-                        if (equiAngular) {
-                            const float pdfTe = pdfEquiAngular(td - offset, D, thetaA, thetaB);
-                            if (vfinite(pdfTe)) mis = powerHeuristic(pdfTd, pdfTe);
-                        }
-                        // (The diagnostic build's shared-pivot switch gives this sample the equi-angular sample's light
-                        // point, the pivot its MIS weight was computed with; the reference draws a point of its own.)
-                        const V3 Ls = volumeSourceTerm(s, ss, L, add(org, mul(dir, td)), dir, vp.g,
-                                                       equiAngular && mf::sharedPivot() ? uel : udl, 1.0f);
-                        direct = vplus(direct, vscaled(vtimes(vtimes(T, vp.sigmaS), vtimes(trScatter, Ls)), invN * mis / pdfTd));
-                    }
+                for (uint32_t k = 0; k < samplesPerLight * scatterCount; ++k) {
+                    V3 equi, distance;
+                    scatterSample(s, root, volumeBranch, pv.depth, lookup, org, dir, T, li, k, firstStart, rayEnd, invN, equi, distance);
+                    direct = vplus(vplus(direct, equi), distance);
                 }
                 radiance = vplus(radiance, direct);
             }
@@ -791,6 +956,89 @@ static __device__ __noinline__ V3 volumeRadiance(const SceneView& s, const Ident
     }
     pv.T = vtimes(pv.T, vt);
     return radiance;
+}
+
+// ---- the volumes of a wavefront launch in kernels of their own (wavefront.cu): volumeRadiance in three parts ----
+// A ray's volume integral as a launch keeps it a path slot: the first march's result and what its replays need.
+struct VolumeHead {
+    uint32_t crossings, regions, count, flags;  // kVolumePassed, kVolumeScatters
+    float weights, firstStart, lastEnd;
+    uint32_t used;                              // checkpoints held
+};
+enum : uint32_t { kVolumePassed = 1u, kVolumeDeeper = 2u, kVolumeScatters = 4u };
+
+__device__ __forceinline__ VolumeMarch marchOf(const SceneView& s, const Identity& root, const Pending& pv, const Crossing* x, uint32_t n,
+                                               uint32_t regions, float tfar, bool emission) {
+    Identity vid = root;
+    vid.branch = childBranch(childBranch(pv.branch, 0xfffc, pv.volumeDepth), 0, 0);
+    return VolumeMarch{s, x, n, regions, pv.origin, pv.dir, pv.nearT, tfar, pv.depth, emission, Stream(vid, pv.depth, 0), kMarchLimit};
+}
+
+// The first part of volumeRadiance: the crossings, the march, its transmittance (vt) and a camera ray's emission (added to
+// radiance). A march that no scattering sample will replay keeps no weights or checkpoints.
+static __device__ __noinline__ void volumeFirstMarch(const SceneView& s, const Identity& root, const Pending& pv, float tfar, Crossing* x,
+                                                     MarchCheckpoint* checkpoints, uint32_t slots, VolumeHead& head, V3& vt, V3& radiance) {
+    const x2_config& c = s.config;
+    head = VolumeHead{0, 0, 0, 0, 0.0f, 0.0f, 0.0f, 0};
+    vt = V3{1, 1, 1};
+    radiance = V3{0, 0, 0};
+    uint32_t regions;
+    const uint32_t n = volumeIntervals(s, pv.origin, pv.dir, pv.nearT, x, regions);
+    head.crossings = n;
+    head.regions = regions;
+    if (n == 0 && regions == 0) return;
+    const bool sampleEmission = pv.depth == 0, deeper = pv.volumeDepth < c.max_volume_depth;
+    const bool scatters = deeper && (pv.nonMirror == 0 ? c.volume_illumination_samples : 1u) > 0;
+    VolumeMarch march = marchOf(s, root, pv, x, n, regions, tfar, sampleEmission);
+    MarchRecord record(checkpoints, slots);
+    march.record = scatters ? &record : nullptr;
+    float weights = 0.0f, firstStart = 0.0f, lastEnd = 0.0f;
+    march.weightsSoFar = &weights;
+    if (scatters) {
+        auto first = [&](const VolumeStep& st, uint32_t i) {
+            if (i == 0) firstStart = st.tStart;
+            lastEnd = st.tStart + st.delta;
+            weights += stepWeight(st);
+            return true;
+        };
+        march.run(first);
+    } else {
+        auto pass = [](const VolumeStep&, uint32_t) { return true; };
+        march.run(pass);
+    }
+    head.count = march.count;
+    if (march.count == 0) return;
+    vt = march.vt;
+    if (march.reachedThreshold) vt = V3{0, 0, 0};
+    if (sampleEmission)
+        for (uint32_t v = 0; v < c.volume_count; ++v) {
+            if (!(march.visited >> v & 1)) continue;
+            const V3 emission = vtimes(pv.T, march.emitted[v]);
+            if (vblack(emission)) continue;
+            radiance = vplus(radiance, emission);
+        }
+    head.flags = kVolumePassed | (deeper ? kVolumeDeeper : 0u) | (scatters ? kVolumeScatters : 0u);
+    head.weights = weights;
+    head.firstStart = firstStart;
+    head.lastEnd = lastEnd;
+    head.used = record.used;
+}
+
+// The second: sample k of every light's scattering samples (light k / samples, its sample k % samples).
+__device__ __forceinline__ void volumeScatterTask(const SceneView& s, const Identity& root, const Pending& pv, float tfar, const Crossing* x,
+                                                  MarchCheckpoint* checkpoints, uint32_t slots, const VolumeHead& head, uint32_t k, V3& equi,
+                                                  V3& distance) {
+    const x2_config& c = s.config;
+    const bool highQuality = pv.nonMirror == 0;
+    const uint32_t samples = highQuality ? c.light_samples * c.volume_illumination_samples : 1u;
+    VolumeMarch march = marchOf(s, root, pv, x, head.crossings, head.regions, tfar, false);
+    march.record = nullptr;
+    march.weightsSoFar = nullptr;
+    MarchRecord record(checkpoints, slots);
+    record.used = head.used;
+    const ReplaySteps lookup{march, head.count, head.weights != 0.0f ? head.weights : 1.0f, head.weights == 0.0f, &record};
+    scatterSample(s, root, childBranch(pv.branch, 0xfffc, pv.volumeDepth), pv.depth, lookup, pv.origin, pv.dir, pv.T, k / samples, k % samples,
+                  head.firstStart, head.lastEnd, 1.0f / float(samples), equi, distance);
 }
 
 }  // namespace x2

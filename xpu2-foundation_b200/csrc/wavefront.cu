@@ -514,7 +514,8 @@ __device__ __forceinline__ LightJob loadLightJob(const WaveState& w, uint32_t p)
 
 // kDefer: the light samples are deferred to the light kernel (sink.lights stores the vertex's job), and the BSDF
 // sample's shadow record waits in the slot's last record, which the light kernel moves after the light records.
-template <bool kAdjoint = false, bool kDefer = false>
+// kApart: a volume scene's volumes have kernels of their own: each shadow record keeps its transmittance's stream.
+template <bool kAdjoint = false, bool kDefer = false, bool kApart = false>
 struct WaveSink {
     const WaveState& w;
     uint32_t p, n, recordsPerPath;
@@ -532,6 +533,14 @@ struct WaveSink {
     bool ggx, sampled;
 
     bool deferred = false, stashed = false;  // kDefer: a job stored; the BSDF record stashed
+    uint2* branches = nullptr;               // kApart
+    U64 branch = 0;
+    uint32_t branchDepth = 0;
+
+    __device__ void volumeBranch(U64 b, uint32_t d) {
+        branch = b;
+        branchDepth = d;
+    }
 
     __device__ void lights(const LightJob& j) {
         if constexpr (kDefer) {
@@ -549,7 +558,8 @@ struct WaveSink {
         }
         w.sray0[k] = make_float4(q.origin.x, q.origin.y, q.origin.z, q.near);
         w.sray1[k] = make_float4(q.dir.x, q.dir.y, q.dir.z, q.far);
-        w.scontrib[k] = make_float4(q.contribution.x, q.contribution.y, q.contribution.z, 0.0f);
+        w.scontrib[k] = make_float4(q.contribution.x, q.contribution.y, q.contribution.z, kApart ? __uint_as_float(branchDepth) : 0.0f);
+        if (kApart) branches[k] = make_uint2(uint32_t(branch), uint32_t(branch >> 32));
         if (isBsdf) ++nBsdf;
         else ++nNee;
         if (kAdjoint) {
@@ -712,9 +722,144 @@ __device__ __forceinline__ void lightsBody(const WaveArgs& a) {
     warpAddCounters(a.counters, 0, nee, 0, 0, 0, 0);
 }
 
+// The closest hit of slot p's ray as the extend kernel left it, rebuilt as trace() rebuilds it, with its triangle's vertices.
+__device__ __forceinline__ Hit slotHit(const WaveState& w, const SceneView& s, uint32_t p, const Pending& pv, V3& va, V3& vb, V3& vc) {
+    const uint2 hr = w.hit[p];
+    Hit hit;
+    hit.geom = ~0u;
+    hit.prim = 0;
+    hit.t = hit.u = hit.v = 0;
+    hit.normal = hit.origin = hit.below = hit.point = V3{0, 0, 0};
+    va = vb = vc = V3{0, 0, 0};
+    if (hr.x != ~0u) {
+        const float4* tp = reinterpret_cast<const float4*>(s.bvh.tris + hr.x);
+        const float4 A = __ldg(tp), B = __ldg(tp + 1), Cc = __ldg(tp + 2);
+        va = V3{A.x, A.y, A.z};
+        vb = V3{B.x, B.y, B.z};
+        vc = V3{Cc.x, Cc.y, Cc.z};
+        const uint32_t tri = __float_as_uint(A.w);
+        hit.geom = __ldg(s.triMesh + tri);
+        hit.prim = tri - __ldg(s.meshFirst + hit.geom);
+        hit.t = __uint_as_float(hr.y);
+        if (!geometryHit(hit, pv.origin, pv.dir, va, vb, vc)) hit.normal = V3{0, 0, 0};
+    }
+    return hit;
+}
+
+// ---- volumes in kernels of their own (volume.cuh, tracking.cuh) ----
+// Inside shade a warp ran its paths' whole volume integrals side by side, each a march, up to dozens of replays and shadow
+// marches of very different lengths: about 5 lanes of 32 active. Apart, a thread runs one part: a ray's first march
+// (neighbouring slots' rays are alike), one scattering sample (a light's sample k of neighbouring rays in a warp), or
+// one shadow ray's transmittance, and that only where nothing occludes it.
+__device__ __forceinline__ void volumeMarchBody(const WaveArgs& a) {
+    const WaveState& w = a.w;
+    const SceneView& s = a.scene;
+    const uint32_t n = *a.extendCount;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
+        const uint32_t i = base + threadIdx.x;
+        uint32_t p = 0;
+        bool scatters = false;
+        if (i < n) {
+            p = extendAt(a, i);
+            Pending pv;
+            loadPending(w, p, pv);
+            const uint4 m = w.meta[p];
+            const Identity root{m.x, U64(m.y), U64(s.config.seed), 0};
+            V3 va, vb, vc;
+            const Hit hit = slotHit(w, s, p, pv, va, vb, vc);
+            const float tEnd = hit.geom == ~0u ? pv.farT : hit.t;
+            Crossing x[kMaxCrossings];
+            VolumeHead head;
+            V3 vt, light;
+            if (s.config.volume_estimator == 1) trackedFirstPass(s, root, pv, tEnd, x, head, vt, light);
+            else
+                volumeFirstMarch(s, root, pv, tEnd, x, a.vol.checkpoints + size_t(p) * kVolumeCheckpoints, kVolumeCheckpoints, head, vt, light);
+            a.vol.head[p] = head;
+            a.vol.pass[p] = make_float4(vt.x, vt.y, vt.z, 0.0f);
+            a.vol.light[p] = make_float4(light.x, light.y, light.z, tEnd);
+            scatters = (head.flags & kVolumeScatters) != 0;
+            if (scatters)
+                for (uint32_t k = 0; k < head.crossings; ++k) a.vol.crossings[size_t(p) * kMaxCrossings + k] = x[k];
+        }
+        const uint32_t slot = warpReserve(a.vol.count, scatters ? 1u : 0u);
+        if (scatters) a.vol.queue[slot] = p;
+    }
+}
+
+// Sample k of every scattering ray, then sample k + 1: a warp's lanes take the same light's same sample. Tracking: k is the
+// scattering sample, and its thread takes every light at its collision.
+__device__ __forceinline__ void volumeScatterBody(const WaveArgs& a) {
+    const WaveState& w = a.w;
+    const SceneView& s = a.scene;
+    const x2_config& c = s.config;
+    const bool tracked = c.volume_estimator == 1;
+    const uint32_t rays = *a.vol.count;
+    const uint32_t each = tracked ? c.volume_illumination_samples : a.vol.tasks;
+    const uint32_t n = rays * each, stride = gridDim.x * blockDim.x;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const uint32_t k = i / rays, p = a.vol.queue[i - k * rays];
+        Pending pv;
+        loadPending(w, p, pv);
+        const bool highQuality = pv.nonMirror == 0;
+        const uint32_t perLight = highQuality ? c.light_samples : 1u, scatters = highQuality ? c.volume_illumination_samples : 1u;
+        if (k >= (tracked ? scatters : c.light_count * perLight * scatters)) continue;
+        const uint4 m = w.meta[p];
+        const Identity root{m.x, U64(m.y), U64(c.seed), 0};
+        const VolumeHead head = a.vol.head[p];
+        const float tEnd = a.vol.light[p].w;
+        const Crossing* x = a.vol.crossings + size_t(p) * kMaxCrossings;
+        if (tracked) {
+            float4* out = a.vol.parts + 2 * size_t(p) * a.vol.tasks + size_t(k) * c.light_count * perLight;
+            for (uint32_t j = 0; j < c.light_count * perLight; ++j) out[j] = make_float4(0, 0, 0, 0);
+            auto put = [&](uint32_t j, V3 v) { out[j] = make_float4(v.x, v.y, v.z, 0.0f); };
+            trackedScatter(s, root, pv, childBranch(pv.branch, 0xfffa, pv.volumeDepth), x, head.crossings, head.regions, tEnd, k, perLight,
+                           scatters, 1.0f / float(perLight * scatters), put);
+        } else {
+            V3 equi, distance;
+            volumeScatterTask(s, root, pv, tEnd, x, a.vol.checkpoints + size_t(p) * kVolumeCheckpoints, kVolumeCheckpoints, head, k, equi, distance);
+            float4* out = a.vol.parts + 2 * (size_t(p) * a.vol.tasks + k);
+            out[0] = make_float4(equi.x, equi.y, equi.z, 0.0f);
+            out[1] = make_float4(distance.x, distance.y, distance.z, 0.0f);
+        }
+    }
+}
+
+// What the ray's volumes add to its path, summed in volumeRadiance's order; pv's throughput and volume depth as it leaves
+// them, and the transmittance its alpha takes.
+__device__ __forceinline__ V3 volumeSettle(const WaveArgs& a, uint32_t p, Pending& pv, V3& alphaT) {
+    const x2_config& c = a.scene.config;
+    const uint32_t flags = a.vol.head[p].flags;
+    alphaT = V3{1, 1, 1};
+    if (!(flags & kVolumePassed)) return V3{0, 0, 0};
+    const float4 vt = a.vol.pass[p], e = a.vol.light[p];
+    V3 light{e.x, e.y, e.z};
+    if (flags & kVolumeScatters) {
+        const bool highQuality = pv.nonMirror == 0;
+        const uint32_t samples = highQuality ? c.light_samples * c.volume_illumination_samples : 1u;
+        const float4* in = a.vol.parts + 2 * size_t(p) * a.vol.tasks;
+        if (c.volume_estimator == 1) {
+            for (uint32_t k = 0; k < c.light_count * samples; ++k) light = vplus(light, V3{in[k].x, in[k].y, in[k].z});
+        } else {
+            for (uint32_t li = 0; li < c.light_count; ++li) {
+                V3 direct{0, 0, 0};
+                for (uint32_t k = 0; k < samples; ++k) {
+                    const float4 q = in[2 * (li * samples + k)], d = in[2 * (li * samples + k) + 1];
+                    direct = vplus(vplus(direct, V3{q.x, q.y, q.z}), V3{d.x, d.y, d.z});
+                }
+                light = vplus(light, direct);
+            }
+        }
+    }
+    alphaT = V3{vt.x, vt.y, vt.z};
+    pv.T = vtimes(pv.T, alphaT);
+    if (flags & kVolumeDeeper) ++pv.volumeDepth;
+    return light;
+}
+
 // kQueue: -1 every extended path (the per-lobe queues in order when they are on, else the extend queue); 0, 1, 2 one
 // per-lobe queue (GGX, Lambert, the rest), its kernel holding that lobe's code only.
-template <bool kBatch, bool kVolumes, bool kAdjoint = false, bool kTextures = true, int kQueue = -1, bool kDefer = false>
+template <bool kBatch, int kVolumes, bool kAdjoint = false, bool kTextures = true, int kQueue = -1, bool kDefer = false>
 __device__ __forceinline__ void shadeBody(const WaveArgs& a) {
     const WaveState& w = a.w;
     const uint32_t n = kQueue < 0 ? *a.extendCount : a.shadeCount[kQueue];
@@ -737,25 +882,8 @@ __device__ __forceinline__ void shadeBody(const WaveArgs& a) {
             const uint32_t pixel = m.x, index = m.y, request = m.w >> 24;
             const SceneView& s = sceneOf<kBatch>(a, request);
             const Identity root{pixel, U64(index), U64(s.config.seed), 0};
-            const uint2 hr = w.hit[p];
-            Hit hit;
-            hit.geom = ~0u;
-            hit.prim = 0;
-            hit.t = hit.u = hit.v = 0;
-            hit.normal = hit.origin = hit.below = hit.point = V3{0, 0, 0};
-            V3 va{0, 0, 0}, vb{0, 0, 0}, vc{0, 0, 0};
-            if (hr.x != ~0u) {
-                const float4* tp = reinterpret_cast<const float4*>(s.bvh.tris + hr.x);
-                const float4 A = __ldg(tp), B = __ldg(tp + 1), Cc = __ldg(tp + 2);
-                va = V3{A.x, A.y, A.z};
-                vb = V3{B.x, B.y, B.z};
-                vc = V3{Cc.x, Cc.y, Cc.z};
-                const uint32_t tri = __float_as_uint(A.w);
-                hit.geom = __ldg(s.triMesh + tri);
-                hit.prim = tri - __ldg(s.meshFirst + hit.geom);
-                hit.t = __uint_as_float(hr.y);
-                if (!geometryHit(hit, pv.origin, pv.dir, va, vb, vc)) hit.normal = V3{0, 0, 0};
-            }
+            V3 va, vb, vc;
+            const Hit hit = slotHit(w, s, p, pv, va, vb, vc);
             float4 rad4 = w.rad[p];
             V3 radiance{rad4.x, rad4.y, rad4.z};
             float alpha = rad4.w;
@@ -769,7 +897,14 @@ __device__ __forceinline__ void shadeBody(const WaveArgs& a) {
                 if (pv.heldLight != ~0u && !(hit.geom != ~0u && hit.t < pv.heldFar)) creditLightTo(partial, at, s, d, pv.held, pv.heldLight);
             }
             const V3 prior = radiance;
-            afterTrace<kVolumes>(s, root, pv, hit, cameraPosition, radiance, alpha);
+            if constexpr (kVolumes == kApartVolumes) {
+                afterHeld(pv, hit, radiance);
+                V3 alphaT;
+                radiance = add(radiance, volumeSettle(a, p, pv, alphaT));
+                afterVolumes(s, root, pv, hit, cameraPosition, alphaT, radiance, alpha);
+            } else {
+                afterTrace<kVolumes == kInlineVolumes>(s, root, pv, hit, cameraPosition, radiance, alpha);
+            }
             if (kAdjoint && pv.depth == 0 && s.config.visible_lights) {
                 // The light a camera ray sees (afterTrace added it).
                 const bool missed = hit.geom == ~0u;
@@ -778,7 +913,8 @@ __device__ __forceinline__ void shadeBody(const WaveArgs& a) {
             }
             uint32_t next = kDone;
             if (hit.geom != ~0u) {
-                WaveSink<kAdjoint, kDefer> sink{w, p, 0, a.recordsPerPath, false, Pending{}, 0, 0, 0};
+                WaveSink<kAdjoint, kDefer, kVolumes == kApartVolumes> sink{w, p, 0, a.recordsPerPath, false, Pending{}, 0, 0, 0};
+                if (kVolumes == kApartVolumes) sink.branches = a.vol.branch;
                 if (kAdjoint) {
                     sink.adj = &a.adj;
                     sink.s = &s;
@@ -841,16 +977,44 @@ __device__ __forceinline__ void shadowBody(const WaveArgs& a) {
     persistentTrace<true, kStats && !kBatch, kBatch, kShort, kOverlap>(a, n, a.shadowQ, a.shadowNext, shortStacks, seg);
 }
 
+// The unoccluded shadow rays' transmittance through the volumes, into their contributions (a volume scene's shadow queue
+// holds each path's records together).
+__device__ __forceinline__ void volumeShadowBody(const WaveArgs& a) {
+    const WaveState& w = a.w;
+    const SceneView& s = a.scene;
+    const uint32_t n = *a.shadowCount, stride = gridDim.x * blockDim.x;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const uint32_t k = a.shadowQ[i];
+        if (!w.svis[k]) continue;
+        const uint4 m = w.meta[k / a.recordsPerPath];
+        const float4 r0 = w.sray0[k], r1 = w.sray1[k], t = w.scontrib[k];
+        const uint2 b = a.vol.branch[k];
+        const uint32_t depth = __float_as_uint(t.w);
+        const Identity id{m.x, U64(m.y), U64(s.config.seed), (U64(b.y) << 32) | b.x};
+        Stream vs(id, depth, 0);
+        const V3 origin{r0.x, r0.y, r0.z}, dir{r1.x, r1.y, r1.z}, c{t.x, t.y, t.z};
+        const V3 through = s.config.volume_estimator == 1 ? mul(c, trackedTransmittance(s, vs, origin, dir, r0.w, r1.w))
+                                                          : mulv(c, volumeTransmittance(s, vs, origin, dir, r0.w, r1.w, 1.0f, int(depth) + 1));
+        w.scontrib[k] = make_float4(through.x, through.y, through.z, t.w);
+    }
+}
+__global__ void __launch_bounds__(kWaveBlock, 4) wfVolumeMarch(WaveArgs a) { volumeMarchBody(a); }
+__global__ void __launch_bounds__(kWaveBlock, 4) wfVolumeScatter(WaveArgs a) { volumeScatterBody(a); }
+__global__ void __launch_bounds__(kWaveBlock, 4) wfVolumeShadow(WaveArgs a) { volumeShadowBody(a); }
+
 // The kernels, each in a few occupancy variants (blocks of kWaveBlock threads a SM that the register allocation must
 // allow), chosen at launch (x2_wavefront_tune); batches in the compiler's allocation. Shade comes in a form for
 // scenes without volumes (the volume code compiled out) and one for scenes with them.
 __global__ void __launch_bounds__(kWaveBlock) wfExtend(WaveArgs a) { extendBody<false>(a); }
-__global__ void __launch_bounds__(kWaveBlock) wfShade(WaveArgs a) { shadeBody<false, false, false, false>(a); }
+__global__ void __launch_bounds__(kWaveBlock) wfShade(WaveArgs a) { shadeBody<false, kNoVolumes, false, false>(a); }
 // Volume scenes' shade (the march inside it), with the texture lookup compiled in (kTextures) or out.
 template <bool kTextures>
-__global__ void __launch_bounds__(kWaveBlock, 4) wfShadeVolumes(WaveArgs a) { shadeBody<false, true, false, kTextures>(a); }
-__global__ void __launch_bounds__(kWaveBlock, 4) wfShadeBatchVolumes(WaveArgs a) { shadeBody<true, true>(a); }
-__global__ void __launch_bounds__(kWaveBlock, 4) wfShadeAdjoint(WaveArgs a) { shadeBody<false, false, true>(a); }
+__global__ void __launch_bounds__(kWaveBlock, 4) wfShadeVolumes(WaveArgs a) { shadeBody<false, kInlineVolumes, false, kTextures>(a); }
+// The same with the volumes in kernels of their own.
+template <bool kTextures>
+__global__ void __launch_bounds__(kWaveBlock, 4) wfShadeVolumesApart(WaveArgs a) { shadeBody<false, kApartVolumes, false, kTextures>(a); }
+__global__ void __launch_bounds__(kWaveBlock, 4) wfShadeBatchVolumes(WaveArgs a) { shadeBody<true, kInlineVolumes>(a); }
+__global__ void __launch_bounds__(kWaveBlock, 4) wfShadeAdjoint(WaveArgs a) { shadeBody<false, kNoVolumes, true>(a); }
 
 // The adjoint's gradient rows summed in FP64 into grads (one thread a gradient).
 __global__ void wfGradRows(const float* rows, uint32_t rowCount, uint32_t params, double* grads) {
@@ -881,7 +1045,7 @@ __global__ void __launch_bounds__(kWaveBlock, kMinBlocks) wfExtendOcc(WaveArgs a
 }
 template <int kMinBlocks, bool kBatch, bool kTextures = false>
 __global__ void __launch_bounds__(kWaveBlock, kMinBlocks) wfShadeOcc(WaveArgs a) {
-    shadeBody<kBatch, false, false, kTextures>(a);
+    shadeBody<kBatch, kNoVolumes, false, kTextures>(a);
 }
 template <int kMinBlocks>
 __global__ void __launch_bounds__(kWaveBlock, kMinBlocks) wfShadowOcc(WaveArgs a) {
@@ -890,18 +1054,18 @@ __global__ void __launch_bounds__(kWaveBlock, kMinBlocks) wfShadowOcc(WaveArgs a
 // Shade split by lobe (wavefront shape shade_split): one kernel a per-lobe queue, each with one lobe's code.
 template <int kQueue, bool kTextures, int kMinBlocks>
 __global__ void __launch_bounds__(kWaveBlock, kMinBlocks) wfShadeQueue(WaveArgs a) {
-    shadeBody<false, false, false, kTextures, kQueue>(a);
+    shadeBody<false, kNoVolumes, false, kTextures, kQueue>(a);
 }
 // The batch form's shade split by lobe (each path's scene from the request table).
 template <int kQueue, bool kTextures>
 __global__ void __launch_bounds__(kWaveBlock, 4) wfShadeQueueBatch(WaveArgs a) {
-    shadeBody<true, false, false, kTextures, kQueue>(a);
+    shadeBody<true, kNoVolumes, false, kTextures, kQueue>(a);
 }
 // With the light samples split off (light_split): the GGX and Lambert queues' shade without them, and their light
 // kernels.
 template <int kQueue, bool kTextures>
 __global__ void __launch_bounds__(kWaveBlock, 4) wfShadeDefer(WaveArgs a) {
-    shadeBody<false, false, false, kTextures, kQueue, true>(a);
+    shadeBody<false, kNoVolumes, false, kTextures, kQueue, true>(a);
 }
 template <int kQueue, int kMinBlocks>
 __global__ void __launch_bounds__(kWaveBlock, kMinBlocks) wfLightsQueue(WaveArgs a) {
@@ -912,6 +1076,10 @@ __global__ void __launch_bounds__(kWaveBlock, kMinBlocks) wfLightsQueue(WaveArgs
 // nothing but counters. A small queue's kernels are latency, not work (five in a row on a 65,536-sample box pass), and a
 // large queue's fill the tails of one another.
 void launchShade(const WaveKernels& k, const WaveArgs& a, int grid, cudaStream_t st, bool batch, const SideStreams* side) {
+    if (k.volumeMarch) {
+        k.volumeMarch<<<grid, kWaveBlock, 0, st>>>(a);
+        k.volumeScatter<<<grid, kWaveBlock, 0, st>>>(a);
+    }
     if (a.shadeQ) (batch ? wfSortShadeBatch : wfSortShade)<<<grid, kWaveBlock, 0, st>>>(a);
     if (a.shadeQ && k.shadeBy[0]) {
         cudaStream_t on[3] = {st, side ? side->stream[0] : st, side ? side->stream[1] : st};
@@ -937,6 +1105,7 @@ void launchIteration(const WaveKernels& k, const WaveArgs& a, const WaveGrids& g
     k.extend<<<g.work, kWaveBlock, 0, st>>>(a);
     launchShade(k, a, g.work, st, batch, side);
     k.shadow<<<g.shadow, kWaveBlock, 0, st>>>(a);
+    if (k.volumeShadow) k.volumeShadow<<<g.shadow, kWaveBlock, 0, st>>>(a);
 }
 
 WaveGrids waveGrids(uint32_t paths, uint32_t records, int smCount, uint32_t blocksPerSm) {
@@ -950,11 +1119,12 @@ WaveGrids waveGrids(uint32_t paths, uint32_t records, int smCount, uint32_t bloc
 }
 
 WaveKernels waveKernels(uint32_t traceBlocks, uint32_t shadeBlocks, bool volumes, bool textures, bool shortStack, bool counting,
-                        bool shadeSplit, uint32_t lightSplit, bool overlap) {
+                        bool shadeSplit, uint32_t lightSplit, bool overlap, bool volumesApart) {
     const bool lightSplit8 = lightSplit == 2;
     WaveKernels k;
     k.shadeBy[0] = k.shadeBy[1] = k.shadeBy[2] = nullptr;
     k.lightsBy[0] = k.lightsBy[1] = nullptr;
+    k.volumeMarch = k.volumeScatter = k.volumeShadow = nullptr;
     if (shadeSplit && !volumes) {
         // The GGX and Lambert kernels at 4 blocks a SM (128 registers) or, with shade_blocks 5, at 5 (96, more spilled).
         const bool five = shadeBlocks >= 5;
@@ -980,8 +1150,14 @@ WaveKernels waveKernels(uint32_t traceBlocks, uint32_t shadeBlocks, bool volumes
         k.extend = wfExtendCount;
         k.shadow = wfShadowCount;
     }
-    if (volumes) k.shade = textures ? wfShadeVolumes<true> : wfShadeVolumes<false>;
-    else if (textures) k.shade = wfShadeOcc<4, false, true>;
+    if (volumes && volumesApart) {
+        k.shade = textures ? wfShadeVolumesApart<true> : wfShadeVolumesApart<false>;
+        k.volumeMarch = wfVolumeMarch;
+        k.volumeScatter = wfVolumeScatter;
+        k.volumeShadow = wfVolumeShadow;
+    } else if (volumes) {
+        k.shade = textures ? wfShadeVolumes<true> : wfShadeVolumes<false>;
+    } else if (textures) k.shade = wfShadeOcc<4, false, true>;
     else k.shade = shadeBlocks >= 4 ? wfShadeOcc<4, false> : shadeBlocks >= 3 ? wfShadeOcc<3, false> : wfShade;
     return k;
 }
@@ -990,6 +1166,7 @@ WaveKernels waveKernelsBatch(bool volumes, bool textures, bool shadeSplit) {
     WaveKernels k;
     k.shadeBy[0] = k.shadeBy[1] = k.shadeBy[2] = nullptr;
     k.lightsBy[0] = k.lightsBy[1] = nullptr;
+    k.volumeMarch = k.volumeScatter = k.volumeShadow = nullptr;
     if (shadeSplit && !volumes) {
         k.shadeBy[0] = textures ? wfShadeQueueBatch<0, true> : wfShadeQueueBatch<0, false>;
         k.shadeBy[1] = textures ? wfShadeQueueBatch<1, true> : wfShadeQueueBatch<1, false>;
@@ -1014,6 +1191,7 @@ __device__ __forceinline__ void resetQueues(const WaveArgs& a) {
     if (a.extendSlots)
         for (uint32_t o = 0; o < kOctants; ++o) a.extendSlots[o] = 0;
     *a.shadowNext = 0;
+    if (a.vol.count) *a.vol.count = 0;
     if (a.shadeQ) a.shadeCount[0] = a.shadeCount[1] = a.shadeCount[2] = 0;
 }
 __global__ void wfResetQueues(WaveArgs a) {

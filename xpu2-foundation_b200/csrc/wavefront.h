@@ -56,6 +56,21 @@ struct AdjointWave {
     float* texGrad;      // FP32 dL/dtexel, 3 a texel over the scene's textures; null: not wanted
 };
 
+// A volume scene's rays in kernels of their own (march null: the march runs inside shade). Per path slot: the first
+// march's result (VolumeHead), the ray's transmittance and what its volumes emit (and, in light.w, where the ray ends),
+// its crossings and the march's checkpoints, and the parts its scattering samples add (two a sample); per shadow record
+// the branch of its transmittance's stream (its depth waits in scontrib.w); and the slots whose rays scatter.
+constexpr uint32_t kVolumeCheckpoints = 32;
+struct VolumeWave {
+    VolumeHead* head;
+    float4 *pass, *light, *parts;
+    Crossing* crossings;           // kMaxCrossings a slot
+    MarchCheckpoint* checkpoints;  // kVolumeCheckpoints a slot
+    uint2* branch;
+    uint32_t *queue, *count;
+    uint32_t tasks;                // most scattering samples a ray: light_count x light_samples x illumination samples
+};
+
 struct WaveArgs {
     SceneView scene;
     WaveState w;
@@ -85,6 +100,7 @@ struct WaveArgs {
     // warp's lanes run one lobe's code.
     uint32_t* shadeQ;
     uint32_t* shadeCount;
+    VolumeWave vol{};     // volume scenes whose volumes have kernels of their own (head null otherwise)
     AdjointWave adj;      // adjoint launches only (adj.dLdI null otherwise)
     // Adaptive passes (null otherwise): each chunk's 8x8 mask of the pixels it samples (bit y * 8 + x) and each
     // pixel's first sample index of the pass (in place of the chunk's first).
@@ -127,6 +143,11 @@ struct WaveKernels {
     void (*shade)(WaveArgs);
     void (*shadow)(WaveArgs);
     void (*shadeBy[3])(WaveArgs);  // shade split by lobe queue (GGX, Lambert, the rest), or null: shade in one kernel
+    // A volume scene's kernels (null: the march runs inside shade): the rays' first march, their scattering samples, and
+    // the unoccluded shadow rays' transmittance.
+    void (*volumeMarch)(WaveArgs);
+    void (*volumeScatter)(WaveArgs);
+    void (*volumeShadow)(WaveArgs);
     void (*lightsBy[2])(WaveArgs);  // light samples of the GGX and Lambert queues in kernels of their own, or null
 };
 // counting: the traversal kernels that count node visits, triangle tests and lane use (the scene view's stats must
@@ -134,9 +155,11 @@ struct WaveKernels {
 // shadeSplit: shade as one kernel a per-lobe queue (surface scenes); lightSplit (with shadeSplit; 1 or 2, 0 off): the
 // GGX and Lambert queues' light samples in kernels of their own after shade, at 6 (1) or 8 (2) blocks a SM (the wave
 // state's lightJob must be allocated).
+// volumesApart: a volume scene's rays in the volume kernels (WaveArgs::vol set), shade without the march.
 // overlap: the traversal kernels that overlap a lane's node visits and triangle tests (walkStepOverlap; short stack).
 WaveKernels waveKernels(uint32_t traceBlocks, uint32_t shadeBlocks, bool volumes, bool textures, bool shortStack = kDefaultShortStack != 0,
-                        bool counting = false, bool shadeSplit = false, uint32_t lightSplit = 0, bool overlap = false);
+                        bool counting = false, bool shadeSplit = false, uint32_t lightSplit = 0, bool overlap = false,
+                        bool volumesApart = false);
 // Two streams beside a context's own, with the events that fork work onto them and join it again (within one capture or
 // launch sequence).
 struct SideStreams {
