@@ -2669,7 +2669,8 @@ int x2_render_batch(x2_ctx* ctx, const x2_request* req, uint32_t n, x2_completio
         anyVolumes = anyVolumes || v.config.volume_count != 0;
         anyTextures = anyTextures || v.triUV != nullptr;
     }
-    const WaveKernels wk = waveKernelsBatch(anyVolumes, anyTextures, s0->shadeSplit != 0);
+    const WaveKernels wk = waveKernelsBatch(anyVolumes, anyTextures, s0->shadeSplit != 0, s0->lightSplit != 0,
+                                            s0->triOverlap != 0 && s0->shortStack != 0 && s0->traceBlocks < 9);
     std::vector<unsigned long long> items;
     uint32_t iterations = 0;
     if (cudaMalloc(&dViews, sizeof(SceneView) * n) != cudaSuccess || cudaMalloc(&dFilms, sizeof(BatchFilm) * n) != cudaSuccess ||

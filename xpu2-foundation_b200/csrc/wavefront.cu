@@ -682,10 +682,9 @@ __device__ __forceinline__ void reserveShadows(const WaveArgs& a, uint32_t p, ui
 // slot's job through lightSamples — the arithmetic the fused shade runs — its records written from the slot's first,
 // then the BSDF sample's stashed record moved after them, the count and the shadow queue as the fused shade leaves
 // them.
-template <int kQueue>
+template <int kQueue, bool kBatch = false>
 __device__ __forceinline__ void lightsBody(const WaveArgs& a) {
     const WaveState& w = a.w;
-    const SceneView& s = a.scene;
     const uint32_t n = a.shadeCount[kQueue];
     if (blockIdx.x * blockDim.x >= n) return;
     const uint32_t R = a.recordsPerPath;
@@ -699,6 +698,7 @@ __device__ __forceinline__ void lightsBody(const WaveArgs& a) {
             const uint32_t flags = w.lightFlags[p];
             WaveSink<false> sink{w, p, 0, R, false, Pending{}, 0, 0, 0};
             if (flags & 1u) {
+                const SceneView& s = sceneOf<kBatch>(a, kBatch ? requestOf(w, p) : 0u);
                 const LightJob j = loadLightJob(w, p);
                 const Identity root{j.pixel, U64(j.index), U64(s.config.seed), 0};
                 lightSamples<false, kQueue == 0 ? 2 : 1>(s, root, j, sink);
@@ -1039,6 +1039,8 @@ __global__ void __launch_bounds__(kWaveBlock) wfExtendLocal(WaveArgs a) { extend
 __global__ void __launch_bounds__(kWaveBlock) wfShadowLocal(WaveArgs a) { shadowBody<false, 0>(a); }
 __global__ void __launch_bounds__(kWaveBlock) wfExtendBatch(WaveArgs a) { extendBody<true>(a); }
 __global__ void __launch_bounds__(kWaveBlock) wfShadowBatch(WaveArgs a) { shadowBody<true>(a); }
+__global__ void __launch_bounds__(kWaveBlock) wfExtendOverlapBatch(WaveArgs a) { extendBody<true, kShortStack, false, true>(a); }
+__global__ void __launch_bounds__(kWaveBlock) wfShadowOverlapBatch(WaveArgs a) { shadowBody<true, kShortStack, false, true>(a); }
 template <int kMinBlocks>
 __global__ void __launch_bounds__(kWaveBlock, kMinBlocks) wfExtendOcc(WaveArgs a) {
     extendBody<false>(a);
@@ -1070,6 +1072,15 @@ __global__ void __launch_bounds__(kWaveBlock, 4) wfShadeDefer(WaveArgs a) {
 template <int kQueue, int kMinBlocks>
 __global__ void __launch_bounds__(kWaveBlock, kMinBlocks) wfLightsQueue(WaveArgs a) {
     lightsBody<kQueue>(a);
+}
+// The batch form's.
+template <int kQueue, bool kTextures>
+__global__ void __launch_bounds__(kWaveBlock, 4) wfShadeDeferBatch(WaveArgs a) {
+    shadeBody<true, kNoVolumes, false, kTextures, kQueue, true>(a);
+}
+template <int kQueue>
+__global__ void __launch_bounds__(kWaveBlock, 6) wfLightsQueueBatch(WaveArgs a) {
+    lightsBody<kQueue, true>(a);
 }
 
 // With side streams the three queues' kernels (and the two light kernels behind theirs) run side by side: they share
@@ -1162,7 +1173,9 @@ WaveKernels waveKernels(uint32_t traceBlocks, uint32_t shadeBlocks, bool volumes
     return k;
 }
 
-WaveKernels waveKernelsBatch(bool volumes, bool textures, bool shadeSplit) {
+// A batch takes the single launches' forms (its eight uneven requests of 37 M samples: 149 ms with walkStep's traversal and
+// the light samples inside shade).
+WaveKernels waveKernelsBatch(bool volumes, bool textures, bool shadeSplit, bool lightSplit, bool overlap) {
     WaveKernels k;
     k.shadeBy[0] = k.shadeBy[1] = k.shadeBy[2] = nullptr;
     k.lightsBy[0] = k.lightsBy[1] = nullptr;
@@ -1171,10 +1184,16 @@ WaveKernels waveKernelsBatch(bool volumes, bool textures, bool shadeSplit) {
         k.shadeBy[0] = textures ? wfShadeQueueBatch<0, true> : wfShadeQueueBatch<0, false>;
         k.shadeBy[1] = textures ? wfShadeQueueBatch<1, true> : wfShadeQueueBatch<1, false>;
         k.shadeBy[2] = textures ? wfShadeQueueBatch<2, true> : wfShadeQueueBatch<2, false>;
+        if (lightSplit) {
+            k.shadeBy[0] = textures ? wfShadeDeferBatch<0, true> : wfShadeDeferBatch<0, false>;
+            k.shadeBy[1] = textures ? wfShadeDeferBatch<1, true> : wfShadeDeferBatch<1, false>;
+            k.lightsBy[0] = wfLightsQueueBatch<0>;
+            k.lightsBy[1] = wfLightsQueueBatch<1>;
+        }
     }
     k.logic = wfLogicBatch;
-    k.extend = wfExtendBatch;
-    k.shadow = wfShadowBatch;
+    k.extend = overlap ? wfExtendOverlapBatch : wfExtendBatch;
+    k.shadow = overlap ? wfShadowOverlapBatch : wfShadowBatch;
     k.shade = volumes ? wfShadeBatchVolumes : textures ? wfShadeOcc<4, true, true> : wfShadeOcc<4, true>;
     return k;
 }

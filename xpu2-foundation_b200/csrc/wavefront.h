@@ -178,7 +178,7 @@ void launchShade(const WaveKernels& k, const WaveArgs& a, int grid, cudaStream_t
 // An iteration's logic, extend, shade and shadow.
 void launchIteration(const WaveKernels& k, const WaveArgs& a, const WaveGrids& g, cudaStream_t st, bool batch = false,
                      const SideStreams* side = nullptr);
-WaveKernels waveKernelsBatch(bool volumes, bool textures, bool shadeSplit = kDefaultShadeSplit != 0);
+WaveKernels waveKernelsBatch(bool volumes, bool textures, bool shadeSplit, bool lightSplit, bool overlap);
 __global__ void wfSortShade(WaveArgs a);
 __global__ void wfSortShadeBatch(WaveArgs a);
 // The adjoint's logic and shade kernels (dynamic shared memory: the gradient count in floats) and the final sum of the
