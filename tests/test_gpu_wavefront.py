@@ -147,3 +147,23 @@ def test_every_launch_shape_renders_the_same_film(ctx, shape):
     after = scene.counters()
     for k in ("trace", "shadow_nee", "shadow_bsdf", "held", "samples", "errors", "stack_overflows"):
         assert after[k] == base[k], k
+
+
+@pytest.mark.parametrize("cid,n", [(0, 1), (0, 33), (0, 1025), (0, (1 << 22) + 37), (108, 3000), (44, 3000), (33, 700)])
+def test_per_sample_entry_equals_one_thread_a_sample(ctx, cid, n):
+    """integrate() in the wavefront form against integratePairs (a counting run takes it): every sample's radiance and
+    status alike, samples outside the frame refused alike; across a window's end."""
+    s = x2.SyntheticScene(cid)
+    scene = x2.Scene(ctx, s.desc, s.config)
+    rng = np.random.default_rng(n)
+    pixels = rng.integers(0, s.config.width * s.config.height, n, dtype=np.uint32)
+    indices = rng.integers(0, 1 << 20, n, dtype=np.uint32)
+    pixels[n // 2] = s.config.width * s.config.height  # no such pixel
+    rgba, status = scene.integrate(pixels, indices)
+    check = np.unique(np.concatenate([np.arange(min(n, 3000)), np.arange(max(0, n - 300), n), [n // 2]]))
+    scene.count_traversal(True)
+    want, want_status = scene.integrate(pixels[check], indices[check])
+    scene.free()
+    assert np.array_equal(status[check], want_status)
+    assert status[n // 2] == x2.ERROR
+    assert np.array_equal(rgba[check], want)

@@ -8,6 +8,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <string>
 #include <thread>
 #include <vector>
@@ -203,8 +204,12 @@ struct x2_scene {
     x2_chunk* staging = nullptr;  // pinned
     uint32_t stagingCap = 0;
     Counters total{};
-    // the per-sample API's scratch (device pairs/outputs for host callers)
+    // the per-sample API's scratch: its counters, a window's item outputs and its drain's words
     Slot integrateSlot;
+    float4* pairOut = nullptr;
+    uint8_t* pairStatus = nullptr;
+    uint32_t pairCap = 0;
+    uint32_t *pairWords = nullptr, *hostPairWords = nullptr;
     unsigned long long* auditWord = nullptr;
     TraversalStats* stats = nullptr;  // device
     bool counting = false;
@@ -449,10 +454,10 @@ bool volumesApart(x2_scene* s, uint32_t paths, uint32_t records) {
 // path state (slot, light job, queues, `records` shadow records a path, and a volume scene's volume state) would pass
 // kWaveBudgetBytes, as a scene with many lights would.
 constexpr double kWaveBudgetBytes = 12e9;
+static double pathBytes(uint32_t records) { return 128.0 + 16.0 * kLightJobWords + 4.0 * (kOctants + 3 + 1) + 53.0 * records; }
 static uint32_t defaultPaths(uint32_t records, double volumeState = 0.0) {
-    const double perPath = volumeState + 128.0 + 16.0 * kLightJobWords + 4.0 * (kOctants + 3 + 1) + 53.0 * records;
     uint32_t paths = kDefaultPaths;
-    while (paths > (1u << 18) && double(paths) * perPath > kWaveBudgetBytes) paths >>= 1;
+    while (paths > (1u << 18) && double(paths) * (volumeState + pathBytes(records)) > kWaveBudgetBytes) paths >>= 1;
     return paths;
 }
 
@@ -1023,6 +1028,10 @@ int x2_scene_free(x2_scene* s) {
     cudaFree(s->counts);
     for (auto& sl : s->slots) freeSlot(sl);
     freeSlot(s->integrateSlot);
+    cudaFree(s->pairOut);
+    cudaFree(s->pairStatus);
+    cudaFree(s->pairWords);
+    if (s->hostPairWords) cudaFreeHost(s->hostPairWords);
     if (s->staging) cudaFreeHost(s->staging);
     delete s;
     return X2_OK;
@@ -1074,6 +1083,185 @@ int x2_scene_info(x2_scene* s, uint64_t* nodes, uint64_t* bvhBytes, uint64_t* tr
     return X2_OK;
 }
 
+namespace {
+// A single scene's wavefront launch of `count` chunks (sl.chunks) and `items` items over `paths` path slots.
+WaveArgs launchArgs(x2_scene* s, Slot& sl, uint32_t paths, uint32_t records, unsigned long long items, uint32_t count) {
+    WaveArgs a;
+    if (volumesApart(s, paths, records)) {
+        a.vol = s->vol;
+        a.vol.count = s->waveCounters + kWaveCounters - 1;
+    }
+    a.scene = viewOf(s);
+    a.w = s->wave;
+    a.paths = paths;
+    a.recordsPerPath = records;
+    a.chunks = sl.chunks;
+    a.itemCount = items;
+    a.samplesPerChunk = s->samplesPerChunk;
+    a.claimed = s->claimed;
+    a.extendQ = s->extendQ;
+    a.extendCount = s->waveCounters;
+    a.lastExtend = s->waveCounters + 1;
+    a.shadowQ = s->shadowQ;
+    a.shadowCount = s->waveCounters + 2;
+    a.shadowSlots = s->shadowOrder && !a.vol.head && a.recordsPerPath <= x2::kRecordSegments ? s->waveCounters + 8 : nullptr;
+    a.extendSlots = s->extendBins ? s->waveCounters + 8 + x2::kRecordSegments : nullptr;
+    a.extendNext = s->waveCounters + 3;
+    a.shadowNext = s->waveCounters + 4;
+    // Volume scenes are shaded in the extend queue's order: its neighbouring slots hold samples of one pixel, whose
+    // marches are alike; a per-lobe sort (or one by march length) scatters them and the march's lanes diverge more.
+    a.shadeQ = s->lobeQueues && !s->volumeCount ? s->shadeQ : nullptr;
+    a.shadeCount = s->waveCounters + 5;
+    a.adj = AdjointWave{};
+    a.chunkMask = s->launchMask;
+    a.pixelBase = s->launchBase;
+    a.liveChunks = nullptr;
+    a.refill = s->refill;
+    a.triLimit = s->triLimit;
+    a.out = s->out;
+    a.outStatus = s->outStatus;
+    a.counters = sl.counters;
+    a.scenes = nullptr;
+    a.chunkRequest = nullptr;
+    a.chunkItems = nullptr;
+    a.chunkCount = count;
+    return a;
+}
+
+WaveKernels launchKernels(const x2_scene* s, const WaveArgs& a) {
+    return waveKernels(s->traceBlocks, s->shadeBlocks, s->volumeCount != 0, s->triUV != nullptr, s->shortStack != 0, a.scene.stats != nullptr,
+                       s->shadeSplit != 0, s->wave.lightJob != nullptr ? s->lightSplit : 0u,
+                       s->triOverlap != 0 && s->shortStack != 0 && s->traceBlocks < 9, a.vol.head != nullptr);
+}
+
+// A launch as one graph on the context's stream: its iterations in a conditional while node, each iteration's last kernel
+// deciding whether another follows (at most `bound`; past that it raises words[2]), then what tail() enqueues. words: 4
+// device words, cleared here.
+int launchDrain(x2_scene* s, const WaveKernels& wk, const WaveArgs& a, const WaveGrids& grids, uint32_t* words, uint32_t bound, const char* what,
+                const std::function<void()>& tail) {
+    cudaStream_t st = s->ctx->stream;
+    cudaGraph_t graph = nullptr;
+    CUDA_OR(cudaGraphCreate(&graph, 0), X2_ECUDA);
+    cudaError_t err = cudaSuccess;
+    auto check = [&](cudaError_t e) {
+        if (err == cudaSuccess && e != cudaSuccess) err = e;
+        return err == cudaSuccess;
+    };
+    cudaGraphConditionalHandle loop;
+    cudaGraphNode_t node = nullptr;
+    cudaGraphNodeParams cp = {};
+    if (check(cudaGraphConditionalHandleCreate(&loop, graph, 1, cudaGraphCondAssignDefault))) {
+        cp.type = cudaGraphNodeTypeConditional;
+        cp.conditional.handle = loop;
+        cp.conditional.type = cudaGraphCondTypeWhile;
+        cp.conditional.size = 1;
+        check(cudaGraphAddNode(&node, graph, nullptr, 0, &cp));
+    }
+    if (err == cudaSuccess && check(cudaStreamBeginCaptureToGraph(st, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                                                  cudaStreamCaptureModeThreadLocal))) {
+        launchIteration(wk, a, grids, st, false, &s->ctx->side);
+        wfDrainCheck<<<1, 32, 0, st>>>(a, loop, words, bound, words + 2);
+        check(cudaGetLastError());
+        cudaGraph_t body = nullptr;
+        check(cudaStreamEndCapture(st, &body));
+    }
+    if (err == cudaSuccess && check(cudaStreamBeginCaptureToGraph(st, graph, &node, nullptr, 1, cudaStreamCaptureModeThreadLocal))) {
+        tail();
+        check(cudaGetLastError());
+        cudaGraph_t out = nullptr;
+        check(cudaStreamEndCapture(st, &out));
+    }
+    cudaGraphExec_t exec = nullptr;
+    if (err == cudaSuccess) check(cudaGraphInstantiate(&exec, graph, 0));
+    cudaGraphDestroy(graph);
+    if (err != cudaSuccess) {
+        setError("%s: building the launch's graph: %s", what, cudaGetErrorString(err));
+        return X2_ECUDA;
+    }
+    cudaMemsetAsync(words, 0, sizeof(uint32_t) * 4, st);
+    const cudaError_t launched = cudaGraphLaunch(exec, st);
+    cudaGraphExecDestroy(exec);  // released once the launch completes
+    if (launched != cudaSuccess) {
+        setError("%s: graph launch failed: %s", what, cudaGetErrorString(launched));
+        return X2_ECUDA;
+    }
+    return X2_OK;
+}
+
+// What a launch's path slots and queues must start with.
+void clearWave(x2_scene* s, uint32_t paths) {
+    cudaStream_t st = s->ctx->stream;
+    cudaMemsetAsync(s->wave.state, 0, sizeof(uint32_t) * paths, st);
+    cudaMemsetAsync(s->wave.ncount, 0, sizeof(uint32_t) * paths, st);
+    cudaMemsetAsync(s->claimed, 0, sizeof(unsigned long long), st);
+    cudaMemsetAsync(s->waveCounters, 0, sizeof(uint32_t) * kWaveCounters, st);
+}
+
+// The per-sample entry in the wavefront form: the samples of a list, in windows, as a launch's items. One thread a
+// sample, as integratePairs runs them, traces a vertex's up to 18 shadow rays one after another and waits for its warp's
+// longest path (60,000 samples of a field: 3.85 ms); the wavefront traces them side by side and gives each sample the same
+// radiance. integratePairs stays for what this form does not take: several BSDF samples, multiple scattering (whose
+// march would run inside shade), counting runs, the diagnostic build, lists not aligned to pairs, and path state beyond kPairBytes.
+constexpr double kPairBytes = 2e9;
+constexpr uint32_t kPairWindow = 1u << 22;
+uint32_t pairPaths(x2_scene* s, uint64_t n, const uint32_t* pairs) {
+    const x2_config& c = s->config;
+    if (diagnosticKernels() || s->counting || c.bsdf_samples != 1 || (s->volumeCount && c.max_volume_depth > 1) ||
+        reinterpret_cast<uintptr_t>(pairs) % sizeof(uint2))
+        return 0;
+    const uint64_t records = uint64_t(c.light_count) * c.light_samples + 1;
+    const double perPath = pathBytes(uint32_t(records)) + (s->volumeCount ? volumeBytes(c, uint32_t(records)) : 0.0);
+    uint64_t paths = std::min<uint64_t>(std::max<uint64_t>(n, 1024), 1u << 20);
+    while (paths > 1024 && double(paths) * perPath > kPairBytes) paths >>= 1;
+    return double(paths) * perPath > kPairBytes ? 0u : uint32_t(paths);
+}
+int integrateWavefront(x2_scene* s, uint32_t paths, const uint32_t* pairs, uint64_t n, double* rgba, uint32_t* status) {
+    const uint32_t records = s->config.light_count * s->config.light_samples + 1;
+    // The last frame launch's description (x2_wavefront_info) stays its own.
+    const uint32_t framePaths = s->wavePaths;
+    const int rc = ensureWave(s, paths, records);
+    if (framePaths) s->wavePaths = framePaths;
+    if (rc) return rc;
+    const uint32_t window = uint32_t(std::min<uint64_t>(n, kPairWindow));
+    if (window > s->pairCap) {
+        cudaFree(s->pairOut);
+        cudaFree(s->pairStatus);
+        s->pairOut = nullptr;
+        s->pairStatus = nullptr;
+        s->pairCap = 0;
+        if (cudaMalloc(&s->pairOut, sizeof(float4) * window) != cudaSuccess || cudaMalloc(&s->pairStatus, window) != cudaSuccess) {
+            setError("device allocation failed for %u samples' outputs", window);
+            return X2_ENOMEM;
+        }
+        s->pairCap = window;
+    }
+    if (!s->pairWords) CUDA_OR(cudaMalloc(&s->pairWords, sizeof(uint32_t) * 4), X2_ENOMEM);
+    if (!s->hostPairWords) {
+        CUDA_OR(cudaMallocHost(&s->hostPairWords, sizeof(uint32_t) * 4), X2_ENOMEM);
+        std::memset(s->hostPairWords, 0, sizeof(uint32_t) * 4);
+    }
+    cudaStream_t st = s->ctx->stream;
+    const WaveGrids grids = waveGrids(paths, records, s->ctx->smCount, s->blocksPerSm);
+    for (uint64_t first = 0; first < n; first += window) {
+        const uint32_t items = uint32_t(std::min<uint64_t>(window, n - first));
+        clearWave(s, paths);
+        WaveArgs a = launchArgs(s, s->integrateSlot, paths, records, items, 0);
+        a.pairs = pairs + 2 * first;
+        a.out = s->pairOut;
+        a.outStatus = s->pairStatus;
+        const uint64_t bound = uint64_t(items) * (uint64_t(s->config.max_depth) + 2) / paths + uint64_t(s->config.max_depth) + 64;
+        const int done = launchDrain(s, launchKernels(s, a), a, grids, s->pairWords, uint32_t(std::min<uint64_t>(bound, 0xffffffffu)), "x2_integrate", [&] {
+            wfPairsOut<<<(items + 255) / 256, 256, 0, st>>>(s->pairOut, s->pairStatus, items, rgba + 4 * first, status + first);
+        });
+        if (done) return done;
+        // A window that did not drain keeps its word until the caller waits.
+        if (first == 0 || !s->hostPairWords[2])
+            cudaMemcpyAsync(s->hostPairWords, s->pairWords, sizeof(uint32_t) * 4, cudaMemcpyDeviceToHost, st);
+    }
+    return X2_OK;
+}
+}  // namespace
+
 int x2_integrate_device(x2_scene* s, const uint32_t* pairs, uint64_t n, double* rgba, uint32_t* status) {
     if (!s || !s->configured) {
         setError("scene not configured");
@@ -1085,9 +1273,15 @@ int x2_integrate_device(x2_scene* s, const uint32_t* pairs, uint64_t n, double* 
     Slot& sl = s->integrateSlot;
     cudaStream_t st = s->ctx->stream;
     cudaMemsetAsync(sl.counters, 0, sizeof(Counters), st);
-    const int blocks = s->ctx->smCount * s->ctx->renderBlocksPerSm;
-    (s->volumeCount ? integratePairsVolumes : s->triUV ? integratePairsTextured : integratePairs)<<<blocks, kRenderBlock, 0, st>>>(
-        viewOf(s), pairs, n, rgba, status, sl.counters);
+    const uint32_t paths = pairPaths(s, n, pairs);
+    int rc = paths ? integrateWavefront(s, paths, pairs, n, rgba, status) : X2_ENOMEM;
+    if (rc == X2_ENOMEM) {  // not that form's, or no room for its path state (nothing launched)
+        const int blocks = s->ctx->smCount * s->ctx->renderBlocksPerSm;
+        (s->volumeCount ? integratePairsVolumes : s->triUV ? integratePairsTextured : integratePairs)<<<blocks, kRenderBlock, 0, st>>>(
+            viewOf(s), pairs, n, rgba, status, sl.counters);
+        rc = X2_OK;
+    }
+    if (rc) return rc;
     CUDA_OR(cudaGetLastError(), X2_ECUDA);
     cudaMemcpyAsync(sl.hostCounters, sl.counters, sizeof(Counters), cudaMemcpyDeviceToHost, st);
     cudaEventRecord(sl.done, st);
@@ -1125,6 +1319,11 @@ int x2_integrate(x2_scene* s, const uint32_t* pairs, uint64_t n, double* rgba, u
     if (rc == X2_OK && w == X2_OK && s->integrateSlot.busy) {
         accumulate(s->total, *s->integrateSlot.hostCounters);
         s->integrateSlot.busy = false;
+        if (s->hostPairWords && s->hostPairWords[2]) {
+            s->hostPairWords[2] = 0;
+            setError("x2_integrate: the samples did not drain");
+            return X2_EDEVICE;
+        }
     }
     return rc ? rc : w;
 }
@@ -1390,52 +1589,6 @@ int x2_wavefront_tune(x2_scene* s, const x2_wavefront_shape* shape) {
     return X2_OK;
 }
 
-namespace {
-// A single scene's wavefront launch of `count` chunks (sl.chunks) and `items` items over `paths` path slots.
-WaveArgs launchArgs(x2_scene* s, Slot& sl, uint32_t paths, uint32_t records, unsigned long long items, uint32_t count) {
-    WaveArgs a;
-    if (volumesApart(s, paths, records)) {
-        a.vol = s->vol;
-        a.vol.count = s->waveCounters + kWaveCounters - 1;
-    }
-    a.scene = viewOf(s);
-    a.w = s->wave;
-    a.paths = paths;
-    a.recordsPerPath = records;
-    a.chunks = sl.chunks;
-    a.itemCount = items;
-    a.samplesPerChunk = s->samplesPerChunk;
-    a.claimed = s->claimed;
-    a.extendQ = s->extendQ;
-    a.extendCount = s->waveCounters;
-    a.lastExtend = s->waveCounters + 1;
-    a.shadowQ = s->shadowQ;
-    a.shadowCount = s->waveCounters + 2;
-    a.shadowSlots = s->shadowOrder && !a.vol.head && a.recordsPerPath <= x2::kRecordSegments ? s->waveCounters + 8 : nullptr;
-    a.extendSlots = s->extendBins ? s->waveCounters + 8 + x2::kRecordSegments : nullptr;
-    a.extendNext = s->waveCounters + 3;
-    a.shadowNext = s->waveCounters + 4;
-    // Volume scenes are shaded in the extend queue's order: its neighbouring slots hold samples of one pixel, whose
-    // marches are alike; a per-lobe sort (or one by march length) scatters them and the march's lanes diverge more.
-    a.shadeQ = s->lobeQueues && !s->volumeCount ? s->shadeQ : nullptr;
-    a.shadeCount = s->waveCounters + 5;
-    a.adj = AdjointWave{};
-    a.chunkMask = s->launchMask;
-    a.pixelBase = s->launchBase;
-    a.liveChunks = nullptr;
-    a.refill = s->refill;
-    a.triLimit = s->triLimit;
-    a.out = s->out;
-    a.outStatus = s->outStatus;
-    a.counters = sl.counters;
-    a.scenes = nullptr;
-    a.chunkRequest = nullptr;
-    a.chunkItems = nullptr;
-    a.chunkCount = count;
-    return a;
-}
-}  // namespace
-
 int x2_launch_wavefront(x2_scene* s, const x2_chunk* chunks, uint32_t count) {
     if (!s || !s->configured || !s->filmPixels || !s->samplesPerChunk) {
         setError("x2_frame_begin first");
@@ -1471,18 +1624,12 @@ int x2_launch_wavefront(x2_scene* s, const x2_chunk* chunks, uint32_t count) {
     if (int rc = ensureItems(s, items)) return rc;
     cudaStream_t st = s->ctx->stream;
     CUDA_OR(cudaMemcpyAsync(sl.chunks, chunks, sizeof(x2_chunk) * count, cudaMemcpyHostToDevice, st), X2_ECUDA);
-    cudaMemsetAsync(s->wave.state, 0, sizeof(uint32_t) * paths, st);
-    cudaMemsetAsync(s->wave.ncount, 0, sizeof(uint32_t) * paths, st);
-    cudaMemsetAsync(s->claimed, 0, sizeof(unsigned long long), st);
-    cudaMemsetAsync(s->waveCounters, 0, sizeof(uint32_t) * kWaveCounters, st);
+    clearWave(s, paths);
     cudaMemsetAsync(sl.counters, 0, sizeof(Counters), st);
     cudaMemsetAsync(s->outStatus, X2_SKIP, items, st);
     const WaveArgs a = launchArgs(s, sl, paths, records, items, count);
     const WaveGrids grids = waveGrids(paths, records, s->ctx->smCount, s->blocksPerSm);
-    const WaveKernels wk = waveKernels(s->traceBlocks, s->shadeBlocks, s->volumeCount != 0, s->triUV != nullptr, s->shortStack != 0,
-                                       a.scene.stats != nullptr, s->shadeSplit != 0,
-                                       s->wave.lightJob != nullptr ? s->lightSplit : 0u, s->triOverlap != 0 && s->shortStack != 0 && s->traceBlocks < 9,
-                                       a.vol.head != nullptr);
+    const WaveKernels wk = launchKernels(s, a);
     const uint64_t maxIter = items * (uint64_t(s->config.max_depth) + 2) / paths + uint64_t(s->config.max_depth) + 64;
     if (s->waveTiming) {
         // Diagnostic form: no graph; events around every kernel, the iteration's times added once it is done.
@@ -1544,56 +1691,14 @@ int x2_launch_wavefront(x2_scene* s, const x2_chunk* chunks, uint32_t count) {
         s->waveIterations = iterations;
         return X2_OK;
     }
-    // One graph: the launch's iterations in a conditional while node, each iteration's last kernel deciding whether
-    // another follows (at most maxIter; past that it raises the overrun word), then the film reduce. The launch runs
-    // without the host; x2_poll / x2_wait collect it like any launch.
-    cudaGraph_t graph = nullptr;
-    CUDA_OR(cudaGraphCreate(&graph, 0), X2_ECUDA);
-    cudaError_t err = cudaSuccess;
-    auto check = [&](cudaError_t e) {
-        if (err == cudaSuccess && e != cudaSuccess) err = e;
-        return err == cudaSuccess;
-    };
-    cudaGraphConditionalHandle loop;
-    cudaGraphNode_t node = nullptr;
-    cudaGraphNodeParams cp = {};
-    if (check(cudaGraphConditionalHandleCreate(&loop, graph, 1, cudaGraphCondAssignDefault))) {
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = loop;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        check(cudaGraphAddNode(&node, graph, nullptr, 0, &cp));
-    }
+    // One graph: the launch's iterations, then the film reduce. The launch runs without the host; x2_poll / x2_wait
+    // collect it like any launch.
     const uint32_t bound = uint32_t(std::min<uint64_t>(maxIter, 0xffffffffu));
-    if (err == cudaSuccess && check(cudaStreamBeginCaptureToGraph(st, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                                                  cudaStreamCaptureModeThreadLocal))) {
-        launchIteration(wk, a, grids, st, false, &s->ctx->side);
-        wfDrainCheck<<<1, 32, 0, st>>>(a, loop, s->drainWords, bound, s->drainWords + 2);
-        check(cudaGetLastError());
-        cudaGraph_t body = nullptr;
-        check(cudaStreamEndCapture(st, &body));
-    }
-    if (err == cudaSuccess && check(cudaStreamBeginCaptureToGraph(st, graph, &node, nullptr, 1, cudaStreamCaptureModeThreadLocal))) {
-        wfFilmReduce<<<int((64ull * count + 255) / 256), 256, 0, st>>>(a, count, s->sums, s->adaptive ? s->odd : nullptr, s->counts);
-        check(cudaGetLastError());
-        cudaGraph_t out = nullptr;
-        check(cudaStreamEndCapture(st, &out));
-    }
-    cudaGraphExec_t exec = nullptr;
-    if (err == cudaSuccess) check(cudaGraphInstantiate(&exec, graph, 0));
-    cudaGraphDestroy(graph);
-    if (err != cudaSuccess) {
-        setError("x2_launch_wavefront: building the launch's graph: %s", cudaGetErrorString(err));
-        return X2_ECUDA;
-    }
-    cudaMemsetAsync(s->drainWords, 0, sizeof(uint32_t) * 4, st);
     cudaEventRecord(sl.begin, st);
-    const cudaError_t launched = cudaGraphLaunch(exec, st);
-    cudaGraphExecDestroy(exec);  // released once the launch completes
-    if (launched != cudaSuccess) {
-        setError("graph launch failed: %s", cudaGetErrorString(launched));
-        return X2_ECUDA;
-    }
+    if (int rc = launchDrain(s, wk, a, grids, s->drainWords, bound, "x2_launch_wavefront", [&] {
+            wfFilmReduce<<<int((64ull * count + 255) / 256), 256, 0, st>>>(a, count, s->sums, s->adaptive ? s->odd : nullptr, s->counts);
+        }))
+        return rc;
     cudaEventRecord(sl.end, st);
     // The extend kernels counted the traced rays; the launch's counters go to the host as x2_launch's do, with the
     // drain's iteration count and overrun word.
@@ -2231,10 +2336,7 @@ int renderAdaptive(x2_scene* s, uint32_t minSamples, uint32_t maxSamples, float 
     a.pixelBase = ad.base;
     a.liveChunks = ad.words;
     const WaveGrids grids = waveGrids(paths, records, s->ctx->smCount, s->blocksPerSm);
-    const WaveKernels wk = waveKernels(s->traceBlocks, s->shadeBlocks, s->volumeCount != 0, s->triUV != nullptr, s->shortStack != 0,
-                                       a.scene.stats != nullptr, s->shadeSplit != 0,
-                                       s->wave.lightJob != nullptr ? s->lightSplit : 0u, s->triOverlap != 0 && s->shortStack != 0 && s->traceBlocks < 9,
-                                       a.vol.head != nullptr);
+    const WaveKernels wk = launchKernels(s, a);
     const uint64_t bound = maxItems * (uint64_t(s->config.max_depth) + 2) / paths + uint64_t(s->config.max_depth) + 64;
     const uint32_t maxIter = uint32_t(std::min<uint64_t>(bound, 0xffffffffu));
 

@@ -13,6 +13,14 @@
 
 namespace x2 {
 
+bool diagnosticKernels() {
+#ifdef X2_DIAG
+    return true;
+#else
+    return false;
+#endif
+}
+
 cudaError_t uploadSobol(const uint32_t directions[17][32]) {
     return cudaMemcpyToSymbol(c_sobol, directions, sizeof(uint32_t) * 17 * 32);
 }

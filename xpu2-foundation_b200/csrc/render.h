@@ -20,6 +20,9 @@ struct RenderArgs {
     Counters* counters;             // the launch's counters
 };
 
+// Whether render.cu is the diagnostic build (its per-sample kernels then record or round as asked).
+bool diagnosticKernels();
+
 // Fills the Sobol direction table the render kernels read (this device, current context).
 cudaError_t uploadSobol(const uint32_t directions[17][32]);
 

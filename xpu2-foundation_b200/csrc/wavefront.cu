@@ -266,20 +266,31 @@ __device__ __forceinline__ void logicBody(const WaveArgs& a) {
         if (wants) {
             const unsigned long long item = first + __popc(want & ((1u << (threadIdx.x & 31u)) - 1u));
             if (item < itemCount) {
-                unsigned long long chunkFirst;
-                uint32_t perPixel;
-                const uint32_t chunkIndex = chunkOfItem<kBatch>(a, item, chunkFirst, perPixel);
-                const uint32_t offset = uint32_t(item - chunkFirst);
-                const uint32_t position = offset / perPixel, s = offset % perPixel;
-                const x2_chunk chunk = a.chunks[chunkIndex];
-                const uint32_t request = kBatch ? a.chunkRequest[chunkIndex] : 0u;
+                uint32_t pixel, index, request = 0, count = 1;
+                bool sample = true;
+                if (a.pairs) {
+                    const uint2 q = reinterpret_cast<const uint2*>(a.pairs)[item];
+                    pixel = q.x;
+                    index = q.y;
+                } else {
+                    unsigned long long chunkFirst;
+                    uint32_t perPixel;
+                    const uint32_t chunkIndex = chunkOfItem<kBatch>(a, item, chunkFirst, perPixel);
+                    const uint32_t offset = uint32_t(item - chunkFirst);
+                    const uint32_t position = offset / perPixel, s = offset % perPixel;
+                    const x2_chunk chunk = a.chunks[chunkIndex];
+                    request = kBatch ? a.chunkRequest[chunkIndex] : 0u;
+                    const x2_config& config = sceneOf<kBatch>(a, request).config;
+                    const bool masked = a.chunkMask && !((a.chunkMask[chunkIndex] >> position) & 1ull);
+                    pixel = s < chunk.count && !masked ? tilePixelW(chunk.tile, position, config.width, config.height) : ~0u;
+                    sample = pixel != ~0u;
+                    index = sample ? (a.pixelBase ? a.pixelBase[pixel] : chunk.first) + s : 0u;
+                    count = chunk.count;
+                }
                 const SceneView& sv = sceneOf<kBatch>(a, request);
-                const bool masked = a.chunkMask && !((a.chunkMask[chunkIndex] >> position) & 1ull);
-                const uint32_t pixel = s < chunk.count && !masked ? tilePixelW(chunk.tile, position, sv.config.width, sv.config.height) : ~0u;
-                if (pixel == ~0u) {
+                if (!sample) {
                     a.outStatus[item] = uint8_t(X2_SKIP);  // not a sample of this launch
                 } else {
-                    const uint32_t index = (a.pixelBase ? a.pixelBase[pixel] : chunk.first) + s;
                     CameraRay camera;
                     if (!cameraRay(sv, pixel, index, camera)) {
                         a.out[item] = make_float4(0, 0, 0, 0);
@@ -291,7 +302,7 @@ __device__ __forceinline__ void logicBody(const WaveArgs& a) {
                         storePending(w, p, p0, pixel, index, request);
                         w.rad[p] = make_float4(0, 0, 0, 0);
                         if (kAdjoint) {
-                            const float inv = 1.0f / float(chunk.count);
+                            const float inv = 1.0f / float(count);
                             a.adj.delta[p] = make_float4(a.adj.dLdI[3ull * pixel] * inv, a.adj.dLdI[3ull * pixel + 1] * inv,
                                                          a.adj.dLdI[3ull * pixel + 2] * inv, 0.0f);
                             a.adj.vcount[p] = 0;
@@ -1307,6 +1318,19 @@ __global__ void wfFilmReduceBatch(WaveArgs a, const BatchFilm* __restrict__ film
         for (int k = 0; k < 4; ++k)
             if (o[k] != 0.0) atomicAdd(f.odd + 4ull * pixel + k, o[k]);
     atomicAdd(f.counts + pixel, n);
+}
+
+__global__ void wfPairsOut(const float4* __restrict__ out, const uint8_t* __restrict__ outStatus, uint32_t n, double* __restrict__ rgba,
+                           uint32_t* __restrict__ status) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float4 v = out[i];
+    const size_t q = 4 * size_t(i);
+    rgba[q] = double(v.x);
+    rgba[q + 1] = double(v.y);
+    rgba[q + 2] = double(v.z);
+    rgba[q + 3] = double(v.w);
+    status[i] = outStatus[i];
 }
 
 }  // namespace x2

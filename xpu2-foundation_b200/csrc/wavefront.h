@@ -111,6 +111,8 @@ struct WaveArgs {
     const uint32_t* liveChunks;
     uint32_t refill;       // a warp fetches new rays once this many of its lanes are idle (1..32)
     uint32_t triLimit;     // triangle tests a lane makes a traversal step
+    // The per-sample entry (null: items are chunks' samples): item i is sample (pairs[2 i], pairs[2 i + 1]) as (pixel, index).
+    const uint32_t* pairs = nullptr;
     float4* out;          // per item: rgb, alpha
     uint8_t* outStatus;   // per item: SampleStatus (Skip for items that are not samples)
     Counters* counters;
@@ -194,5 +196,7 @@ __global__ void wfDrainCheck(WaveArgs a, cudaGraphConditionalHandle loop, uint32
                              uint32_t* overrun);
 __global__ void wfFilmReduce(WaveArgs a, uint32_t chunkCount, double* sums, double* odd, uint32_t* counts);
 __global__ void wfFilmReduceBatch(WaveArgs a, const BatchFilm* films);
+// The per-sample entry's outputs from a launch's items: rgb and alpha as doubles, the status as a word.
+__global__ void wfPairsOut(const float4* out, const uint8_t* outStatus, uint32_t n, double* rgba, uint32_t* status);
 
 }  // namespace x2
