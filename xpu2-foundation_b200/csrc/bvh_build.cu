@@ -309,8 +309,70 @@ __global__ void restructure(uint32_t n, uint32_t* left, uint32_t* right, uint32_
     }
 }
 
+// The wide nodes' cuts by least surface-area cost (Ylitie, Karras and Laine 2017, section 4): for every binary node and i =
+// 1..7, the least cost c[7 node + i - 1] of giving its subtree at most i of a wide node's slots, bottom up as refit. One
+// slot is a leaf (a subtree of at most three triangles, kWideTri an area and triangle) or a wide node of its own (kWideNode
+// an area, over the best split of eight slots between the two children); more are the best split of them, or fewer.
+// choice: bits 3 (j - 2) the left child's share of the best split of j = 2..8 slots, bits 21 + (i - 2) whether i = 2..7
+// slots are split (else i - 1 serve as well). Opening the largest subtree first instead left wide nodes of 7.1 triangles
+// on the 12.3M-triangle field (small subtrees got nodes of their own); a ray's triangle tests ride along with its node
+// visits (walkStepOverlap: 7 of 32 lanes test in nearly every step), so a test is cheap beside a visit.
+constexpr float kWideNode = 1.0f, kWideTri = 0.6f;
+__global__ void wideCosts(uint32_t n, const uint32_t* __restrict__ left, const uint32_t* __restrict__ right, const uint32_t* __restrict__ parent,
+                          const Aabb* __restrict__ box, const uint32_t* __restrict__ count, float* c, uint32_t* choice, unsigned* flags) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n || n == 1) return;
+    uint32_t node = parent[n - 1 + k];
+    for (;;) {
+        if (atomicAdd(&flags[node], 1u) == 0u) return;  // the first arrival leaves the node to the second
+        __threadfence();
+        float l[7], r[7];
+        auto load = [&](uint32_t child, float* v) {
+            const float leaf = kWideTri * area(box[child]);
+            for (int i = 0; i < 7; ++i) v[i] = isLeafNode(child, n) ? leaf : __ldcg(c + 7 * size_t(child) + i);
+        };
+        load(left[node], l);
+        load(right[node], r);
+        uint32_t bits = 0;
+        float split[9];
+#pragma unroll
+        for (int j = 2; j <= 8; ++j) {
+            float best = FLT_MAX;
+            uint32_t share = 1;
+#pragma unroll
+            for (int i = 1; i < j; ++i) {
+                if (i > 7 || j - i > 7) continue;
+                const float cost = l[i - 1] + r[j - i - 1];
+                if (cost < best) {
+                    best = cost;
+                    share = uint32_t(i);
+                }
+            }
+            split[j] = best;
+            bits |= share << (3 * (j - 2));
+        }
+        const float a = area(box[node]);
+        const uint32_t triangles = count[node];
+        float least = triangles <= 3 ? kWideTri * a * float(triangles) : kWideNode * a + split[8];
+        c[7 * size_t(node)] = least;
+#pragma unroll
+        for (int i = 2; i <= 7; ++i) {
+            if (split[i] < least) {
+                least = split[i];
+                bits |= 1u << (21 + i - 2);
+            }
+            c[7 * size_t(node) + i - 1] = least;
+        }
+        choice[node] = bits;
+        __threadfence();
+        if (node == 0) return;
+        node = parent[node];
+    }
+}
+
 struct CollapseArgs {
     uint32_t n;
+    const uint32_t* choice;     // each binary node's cuts (wideCosts)
     const uint32_t* left;
     const uint32_t* right;
     const Aabb* box;
@@ -330,8 +392,6 @@ struct CollapseArgs {
 };
 
 
-// One wide node from binary node `b`: open the largest-area internal node until eight children; binary subtrees of
-// at most three triangles become leaves; order the slots by direction octant; quantise the child boxes.
 // The leaf-order triangles with each vertex's coordinates rotated: (y, z, x) for rays whose dominant axis is x, and
 // (z, x, y) for y (traverse.cuh triTestRotated); the scene index stays in v0.w.
 __global__ void rotateTriangles(const TriRec* __restrict__ tris, uint32_t n, TriRec* __restrict__ yzx, TriRec* __restrict__ zxy) {
@@ -360,6 +420,8 @@ __global__ void checkLeafTriangles(const unsigned* __restrict__ seen, uint32_t n
     if (i < n && seen[i] != 1u) atomicAdd(bad, 1u);
 }
 
+// One wide node from a binary node: its children as wideCosts chose them; binary subtrees of at most three triangles become
+// leaves; the slots ordered by direction octant; the child boxes quantised.
 __global__ void collapse(CollapseArgs a) {
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= a.queueInCount) return;
@@ -370,29 +432,26 @@ __global__ void collapse(CollapseArgs a) {
     if (isLeafNode(item.x, n)) {
         c[nc++] = item.x;
     } else {
-        c[nc++] = a.left[item.x];
-        c[nc++] = a.right[item.x];
-    }
-    while (nc < 8) {
-        // Subtrees of more than three triangles first (each would otherwise become a node of its own); then the small
-        // ones, whose triangles stay in this node either way but get tighter boxes.
-        int best = -1;
-        float bestArea = -1.0f;
-        bool bestBig = false;
-        for (int i = 0; i < nc; ++i) {
-            if (isLeafNode(c[i], n)) continue;
-            const bool big = a.count[c[i]] > 3;
-            const float s = area(a.box[c[i]]);
-            if ((big && !bestBig) || (big == bestBig && s > bestArea)) {
-                bestArea = s;
-                best = i;
-                bestBig = big;
+        // The node's eight slots shared out down the binary tree as wideCosts chose.
+        uint2 open[8];  // (binary node, slots)
+        int top = 0;
+        const uint32_t share = (a.choice[item.x] >> (3 * (8 - 2))) & 7u;
+        open[top++] = make_uint2(a.right[item.x], 8u - share);
+        open[top++] = make_uint2(a.left[item.x], share);
+        while (top) {
+            const uint2 e = open[--top];
+            uint32_t slots = e.y;
+            if (isLeafNode(e.x, n)) slots = 1;
+            const uint32_t bits = slots > 1 ? a.choice[e.x] : 0u;
+            while (slots > 1 && !((bits >> (21 + slots - 2)) & 1u)) --slots;
+            if (slots == 1) {
+                c[nc++] = e.x;
+            } else {
+                const uint32_t part = (bits >> (3 * (slots - 2))) & 7u;
+                open[top++] = make_uint2(a.right[e.x], slots - part);
+                open[top++] = make_uint2(a.left[e.x], part);
             }
         }
-        if (best < 0) break;
-        const uint32_t b = c[best];
-        c[best] = a.left[b];
-        c[nc++] = a.right[b];
     }
     // Node bounds and the octant ordering of the slots.
     Aabb nb;
@@ -552,7 +611,8 @@ int buildBvh(const float* dVertices, const uint32_t* dTriangles, uint32_t n, cud
     Aabb *triBox = nullptr, *box = nullptr;
     uint64_t *keys = nullptr, *keysSorted = nullptr;
     uint32_t *values = nullptr, *order = nullptr, *left = nullptr, *right = nullptr, *parent = nullptr, *count = nullptr;
-    float* cost = nullptr;
+    float *cost = nullptr, *wide = nullptr;
+    uint32_t* choice = nullptr;
     unsigned *flags = nullptr, *sceneBox = nullptr, *counters = nullptr;
     uint2 *qa = nullptr, *qb = nullptr;
     void* temp = nullptr;
@@ -601,6 +661,11 @@ int buildBvh(const float* dVertices, const uint32_t* dTriangles, uint32_t n, cud
         restructure<<<grid, kBlock, 0, stream>>>(n, left, right, parent, box, count, cost, flags);
         CK(cudaGetLastError());
     }
+    CK(cudaMallocAsync(&wide, sizeof(float) * 7 * size_t(n), stream));
+    CK(cudaMallocAsync(&choice, sizeof(uint32_t) * n, stream));
+    CK(cudaMemsetAsync(flags, 0, sizeof(unsigned) * n, stream));
+    wideCosts<<<grid, kBlock, 0, stream>>>(n, left, right, parent, box, count, wide, choice, flags);
+    CK(cudaGetLastError());
     // Wide node 0 is the root; counters: [0] wide nodes, [1] triangles placed, [2] next queue size, [3] overflow.
     host[0] = 1;
     CK(cudaMemcpyAsync(counters, host, sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
@@ -608,6 +673,7 @@ int buildBvh(const float* dVertices, const uint32_t* dTriangles, uint32_t n, cud
     while (queueCount) {
         CollapseArgs a;
         a.n = n;
+        a.choice = choice;
         a.left = left;
         a.right = right;
         a.box = box;
@@ -676,6 +742,8 @@ fail:
     cudaFreeAsync(parent, stream);
     cudaFreeAsync(count, stream);
     cudaFreeAsync(cost, stream);
+    cudaFreeAsync(wide, stream);
+    cudaFreeAsync(choice, stream);
     cudaFreeAsync(flags, stream);
     cudaFreeAsync(sceneBox, stream);
     cudaFreeAsync(counters, stream);
