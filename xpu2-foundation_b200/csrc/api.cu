@@ -210,6 +210,8 @@ struct x2_scene {
     uint8_t* pairStatus = nullptr;
     uint32_t pairCap = 0;
     uint32_t *pairWords = nullptr, *hostPairWords = nullptr;
+    float4* stepLists = nullptr;  // the plain megakernel's lists
+    size_t stepThreads = 0;
     unsigned long long* auditWord = nullptr;
     TraversalStats* stats = nullptr;  // device
     bool counting = false;
@@ -1028,6 +1030,7 @@ int x2_scene_free(x2_scene* s) {
     cudaFree(s->counts);
     for (auto& sl : s->slots) freeSlot(sl);
     freeSlot(s->integrateSlot);
+    cudaFree(s->stepLists);
     cudaFree(s->pairOut);
     cudaFree(s->pairStatus);
     cudaFree(s->pairWords);
@@ -1415,6 +1418,24 @@ int x2_frame_begin_adaptive(x2_scene* s, uint32_t samplesPerChunk) {
     return X2_OK;
 }
 
+namespace {
+// renderSteps's lists for `threads` threads, kept with the scene (launches run one after another on the context's
+// stream), or null when the device has no room for them.
+float4* stepLists(x2_scene* s, size_t threads) {
+    if (threads <= s->stepThreads) return s->stepLists;
+    cudaFree(s->stepLists);
+    s->stepLists = nullptr;
+    s->stepThreads = 0;
+    if (cudaMalloc(&s->stepLists, sizeof(float4) * kStepListWords * threads) != cudaSuccess) {
+        cudaGetLastError();
+        s->stepLists = nullptr;
+        return nullptr;
+    }
+    s->stepThreads = threads;
+    return s->stepLists;
+}
+}  // namespace
+
 int x2_launch(x2_scene* s, const x2_chunk* chunks, uint32_t count) {
     if (!s || !s->configured || !s->filmPixels || !s->samplesPerChunk) {
         setError("x2_frame_begin first");
@@ -1460,12 +1481,19 @@ int x2_launch(x2_scene* s, const x2_chunk* chunks, uint32_t count) {
     // The bounce-at-a-time form for surface scenes (renderSteps); renderChunks for volumes, counting launches and
     // vertices with more shadow rays than its list holds.
     void (*kernel)(RenderArgs) = s->volumeCount ? renderChunksVolumes : s->triUV ? renderChunksTextured : renderChunks;
-    if (!s->volumeCount && !a.scene.stats &&
-        uint64_t(s->config.light_count) * s->config.light_samples + s->config.bsdf_samples <= kStepRecords)
-        kernel = s->triUV ? renderStepsTextured<4> : renderSteps<4>;
     int perSm = 0;
+    a.lists = nullptr;
+    if (!s->volumeCount && !a.scene.stats &&
+        uint64_t(s->config.light_count) * s->config.light_samples + s->config.bsdf_samples <= kStepRecords) {
+        auto* steps = s->triUV ? renderStepsTextured<4> : renderSteps<4>;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, steps, kRenderBlock, 0);
+        a.lists = stepLists(s, size_t(s->ctx->smCount) * std::max(perSm, 1) * kRenderBlock);
+        if (a.lists) kernel = steps;  // else no room for its lists: the kernel that needs none
+    }
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, kRenderBlock, 0);
-    const int blocks = s->ctx->smCount * std::max(perSm, 1);
+    // No more blocks than the items fill (a small launch's idle blocks would each claim and find nothing).
+    const int blocks = int(std::min<unsigned long long>((unsigned long long)s->ctx->smCount * std::max(perSm, 1),
+                                                        (a.itemCount + kRenderBlock - 1) / kRenderBlock));
     cudaEventRecord(sl->begin, st);
     kernel<<<blocks, kRenderBlock, 0, st>>>(a);
     CUDA_OR(cudaGetLastError(), X2_ECUDA);

@@ -5,8 +5,8 @@
 // pixel (warp-aggregated atomics) instead of one a sample. The film is the reference's: FP64 sums (rgb + alpha), FP64
 // odd-index sums (adaptive frames), U32 counts (async_gpu.cu:320-364).
 //
-// renderSteps (surface scenes): a bounce at a time, a lane taking the next item as soon as its sample is done, rays
-// walked a node a step across the warp (below). renderChunks (volumes, counting launches): persistent warps claim 32
+// renderSteps (surface scenes): a bounce at a time, a lane taking the next item as soon as its sample is done, the
+// warp's rays walked a node a step by whichever lanes are free (below). renderChunks (volumes, counting launches): persistent warps claim 32
 // items at a time (one atomic a warp) and each lane runs its sample's whole path (integrate).
 #include "integrator.cuh"
 #include "render.h"
@@ -167,15 +167,24 @@ __global__ void __launch_bounds__(kRenderBlock) renderChunksVolumes(RenderArgs a
 
 // renderSteps: the plain megakernel for surface scenes, a bounce at a time. A lane holds one sample's path (its pending
 // rays on a local stack, its radiance) and takes the launch's next item as soon as the sample is done, so a warp never
-// waits for its longest path (path regeneration). A warp step is one vertex of every live lane's path: the closest hit
-// of its next pending ray, walked a node a step together with the warp's other rays (walkStep); the vertex shaded
-// (afterTrace, shadeVertex) with its shadow rays written to a list of the lane's own; then the lists walked together,
-// a lane whose ray is done starting its next one at once; then the unoccluded rays' contributions added in the list's
-// order. That is the order in which integrate (one thread a sample, shadow rays traced as they come) adds them, and
-// the steps visit the nodes and test the triangles traceClosest / traceAny do, so a sample's radiance is the same bit
-// for bit. Scenes with volumes, vertices with more than kStepRecords shadow rays and counting launches use renderChunks.
+// waits for its longest path (path regeneration). A warp step is one vertex of every live lane's path: the shadow rays
+// its lanes' last vertices made and the closest hits of their next pending rays, walked a node a step by whichever
+// lanes are free; then the unoccluded rays' contributions added in their list's order and the next vertices shaded
+// (afterTrace, shadeVertex), their shadow rays written to the lanes' lists. That is the order in which integrate (one
+// thread a sample, shadow rays traced as they come) adds them, and the steps visit the nodes and test the triangles
+// traceClosest / traceAny do, so a sample's radiance is the same bit for bit. Scenes with volumes, vertices with more
+// than kStepRecords shadow rays and counting launches use renderChunks.
+//
+// The walk's rays are the warp's, not their lane's: a vertex makes anything from no shadow ray to one a light, and with
+// each lane walking its own list a warp waited for its longest (9.5 of 32 lanes active). So the lists lie in global
+// memory (RenderArgs::lists, a warp's own few kilobytes of it, in L1 and L2), the warp's rays are numbered through a
+// shared table, closest hits first (their walks are the longest), and a lane whose ray is done takes the next number once
+// kStepRefill lanes are free; a ray's outcome goes back to its owner through shared memory.
+constexpr uint32_t kStepRefill = 4;
+constexpr uint32_t kStepClosest = 31;  // in a ray's number: the owner's pending ray, not a list entry
+
 struct StepSink {
-    ShadowReq* reqs;
+    float4* list;
     uint32_t& n;
     Pending* stack;
     uint32_t& size;
@@ -184,8 +193,14 @@ struct StepSink {
     __device__ void shadow(const ShadowReq& q, bool fromBsdf) {
         if (fromBsdf) ++bsdf;
         else ++nee;
-        if (n < kStepRecords) reqs[n++] = q;
-        else full = true;
+        if (n < kStepRecords) {
+            float4* e = list + 3 * n++;
+            e[0] = make_float4(q.origin.x, q.origin.y, q.origin.z, q.near);
+            e[1] = make_float4(q.dir.x, q.dir.y, q.dir.z, q.far);
+            e[2] = make_float4(q.contribution.x, q.contribution.y, q.contribution.z, 0.0f);
+        } else {
+            full = true;
+        }
     }
     __device__ void held() { ++heldRays; }
     __device__ void vertex(uint32_t, const Bsdf&, V3, const TexHit*) {}
@@ -193,11 +208,16 @@ struct StepSink {
     __device__ void push(const Pending& p) { stack[size++] = p; }
 };
 
+static_assert(kStepRecords < kStepClosest, "a ray's number has five bits for the list entry");
 template <bool kTextures>
 __device__ __forceinline__ void renderStepsBody(const RenderArgs& a) {
+    constexpr uint32_t kWarps = kRenderBlock / 32, kRays = 32 * (kStepRecords + 1);
     __shared__ uint2 shortStacks[kShortStack * kRenderBlock];
+    __shared__ uint16_t numbers[kWarps][kRays];   // the warp's rays: owner lane | list entry << 5
+    __shared__ uint32_t unoccluded[kWarps][32];   // by owner: its list's unoccluded entries
+    __shared__ uint32_t closest[kWarps][32][3];   // by owner: its pending ray's hit (triangle, leaf order, t bits)
     const unsigned full = 0xffffffffu;
-    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const SceneView& s = a.scene;
     const Bvh8 bvh = s.bvh;
     uint32_t* overflow = s.overflow;
@@ -206,13 +226,11 @@ __device__ __forceinline__ void renderStepsBody(const RenderArgs& a) {
     walk.shortStack = shortStacks + threadIdx.x;
     walk.nodes = walk.tris = 0;
     Pending stack[kMaxPending];
-    ShadowReq reqs[kStepRecords];
+    float4* const lists = a.lists + (size_t(blockIdx.x) * kRenderBlock + 32 * warp) * kStepListWords;  // the warp's
+    float4* const list = lists + lane * kStepListWords;
     uint32_t size = 0, n = 0, pixel = 0, index = 0;
-    uint32_t hitTri = ~0u, hitLeaf = 0;  // the closest hit of the pending stack's top ray, once walked
-    float hitT = 0.0f;
     V3 cameraPosition{0, 0, 0}, radiance{0, 0, 0};
     float alpha = 0.0f;
-    RayQ r;
     unsigned long long trace = 0, nee = 0, bsdf = 0, held = 0, samples = 0, errors = 0;
     bool live = false, drained = false;
     for (;;) {
@@ -249,49 +267,70 @@ __device__ __forceinline__ void renderStepsBody(const RenderArgs& a) {
             if (drained) break;
             continue;
         }
-        // Each live lane's rays, walked a step at a time with the warp's others: the last vertex's shadow rays in
-        // order, then the closest hit of the next pending ray; a lane whose ray is done starts its next at once.
-        uint32_t j = 0, vis = 0;
-        bool tracing = live && (n > 0 || size > 0), any = n > 0;
-        if (tracing) {
-            const V3 o = any ? reqs[0].origin : stack[size - 1].origin, d = any ? reqs[0].dir : stack[size - 1].dir;
-            r = makeRay(bvh, o.x, o.y, o.z, d.x, d.y, d.z);
-            if (any) walkStart<true, kShortStack>(walk, r, reqs[0].near, reqs[0].far);
-            else walkStart<false, kShortStack>(walk, r, stack[size - 1].nearT, stack[size - 1].farT);
+        // The warp's rays, numbered: the pending rays, then the lists' entries.
+        const bool pending = live && size > 0;
+        const uint32_t pendings = __ballot_sync(full, pending);
+        if (pending) {
+            const Pending& next = stack[size - 1];
+            list[3 * kStepRecords] = make_float4(next.origin.x, next.origin.y, next.origin.z, next.nearT);
+            list[3 * kStepRecords + 1] = make_float4(next.dir.x, next.dir.y, next.dir.z, next.farT);
+            numbers[warp][__popc(pendings & ((1u << lane) - 1u))] = uint16_t(lane | (kStepClosest << 5));
         }
+        const uint32_t entries = live ? n : 0u;
+        uint32_t last = entries;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t v = __shfl_up_sync(full, last, off);
+            if (lane >= uint32_t(off)) last += v;
+        }
+        const uint32_t rays = __popc(pendings) + __shfl_sync(full, last, 31), firstEntry = __popc(pendings) + last - entries;
+        for (uint32_t k = 0; k < entries; ++k) numbers[warp][firstEntry + k] = uint16_t(lane | (k << 5));
+        unoccluded[warp][lane] = 0;
+        __syncwarp();
+        uint32_t next = 0, number = 0;
+        bool walking = false, any = false;
+        RayQ r;
         for (;;) {
-            const uint32_t lanes = __ballot_sync(full, tracing);
+            uint32_t lanes = __ballot_sync(full, walking);
+            if (next < rays && 32 - __popc(lanes) >= int(kStepRefill)) {
+                const uint32_t mine = next + __popc(~lanes & ((1u << lane) - 1u));
+                if (!walking && mine < rays) {
+                    number = numbers[warp][mine];
+                    any = (number >> 5) != kStepClosest;
+                    const float4* e = lists + (number & 31u) * kStepListWords + 3 * (any ? number >> 5 : kStepRecords);
+                    const float4 r0 = e[0], r1 = e[1];
+                    r = makeRay(bvh, r0.x, r0.y, r0.z, r1.x, r1.y, r1.z);
+                    if (any) walkStart<true, kShortStack>(walk, r, r0.w, r1.w);
+                    else walkStart<false, kShortStack>(walk, r, r0.w, r1.w);
+                    walking = true;
+                }
+                next += 32 - __popc(lanes);
+                lanes = __ballot_sync(full, walking);
+            }
             if (!lanes) break;
-            if (tracing && walkStepOverlapKind<kShortStack>(bvh, r, walk, deep, overflow, lanes, any)) {
-                if (any) {
-                    if (!walk.best) vis |= 1u << j;
-                    ++j;
-                } else {
-                    hitTri = walk.best;
-                    hitLeaf = walk.bestLeaf;
-                    hitT = walk.tmax;
+            if (walking && walkStepOverlapKind<kShortStack>(bvh, r, walk, deep, overflow, lanes, any)) {
+                const uint32_t owner = number & 31u;
+                if (!any) {
+                    closest[warp][owner][0] = walk.best;
+                    closest[warp][owner][1] = walk.bestLeaf;
+                    closest[warp][owner][2] = __float_as_uint(walk.tmax);
+                } else if (!walk.best) {
+                    atomicOr(&unoccluded[warp][owner], 1u << (number >> 5));
                 }
-                tracing = false;
-                if (any && j < n) {
-                    const ShadowReq& q = reqs[j];
-                    r = makeRay(bvh, q.origin.x, q.origin.y, q.origin.z, q.dir.x, q.dir.y, q.dir.z);
-                    walkStart<true, kShortStack>(walk, r, q.near, q.far);
-                    tracing = true;
-                } else if (any && size > 0) {
-                    const Pending& next = stack[size - 1];
-                    r = makeRay(bvh, next.origin.x, next.origin.y, next.origin.z, next.dir.x, next.dir.y, next.dir.z);
-                    walkStart<false, kShortStack>(walk, r, next.nearT, next.farT);
-                    any = false;
-                    tracing = true;
-                }
+                walking = false;
             }
         }
+        __syncwarp();
         // The shadow rays' contributions in the list's order, then the next vertex: the hit rebuilt as trace() does,
         // afterTrace and shadeVertex, its shadow rays to the list.
-        for (uint32_t k = 0; k < n; ++k)
-            if ((vis >> k) & 1u) radiance = add(radiance, reqs[k].contribution);
+        for (uint32_t vis = entries ? unoccluded[warp][lane] : 0u; vis; vis &= vis - 1) {
+            const float4 c = list[3 * (__ffs(vis) - 1) + 2];
+            radiance = add(radiance, V3{c.x, c.y, c.z});
+        }
         n = 0;
-        if (live && size > 0) {
+        if (pending) {
+            const uint32_t hitTri = closest[warp][lane][0], hitLeaf = closest[warp][lane][1];
+            const float hitT = __uint_as_float(closest[warp][lane][2]);
             Pending pv = stack[--size];
             const uint32_t top = size;
             ++trace;
@@ -315,7 +354,7 @@ __device__ __forceinline__ void renderStepsBody(const RenderArgs& a) {
             const Identity root{pixel, U64(index), U64(s.config.seed), 0};
             afterTrace<false>(s, root, pv, hit, cameraPosition, radiance, alpha);
             if (hit.geom != ~0u) {
-                StepSink sink{reqs, n, stack, size, nee, bsdf, held, false};
+                StepSink sink{list, n, stack, size, nee, bsdf, held, false};
                 if (!shadeVertex<false, kTextures>(s, root, pixel, index, pv, hit, va, vb, vc, top, radiance, alpha, sink) || sink.full) {
                     ++errors;
                     live = false;

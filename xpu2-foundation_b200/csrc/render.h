@@ -18,7 +18,11 @@ struct RenderArgs {
     double* odd;                    // null unless the frame is adaptive
     uint32_t* counts;
     Counters* counters;             // the launch's counters
+    float4* lists;                  // renderSteps: kStepListWords a thread of the grid
 };
+// A renderSteps thread's rays in memory the warp's other lanes can walk them from: a vertex's shadow rays (origin and near,
+// direction and far, contribution) and the next pending ray (origin and near, direction and far).
+constexpr size_t kStepListWords = 3 * size_t(kStepRecords) + 2;
 
 // Whether render.cu is the diagnostic build (its per-sample kernels then record or round as asked).
 bool diagnosticKernels();
