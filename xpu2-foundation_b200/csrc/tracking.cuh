@@ -110,21 +110,31 @@ __device__ __forceinline__ bool trackStretch(const SceneView& s, uint32_t region
         }
     if (!count) return true;
     if (count == 1) {
+        // One loop, a draw or a cell a pass, left by its condition alone (no return inside it): a warp's lanes meet again at
+        // every pass, wherever in the grid each of them is. As a loop over cells with one over collisions inside and
+        // returns out of both, the walks ran at 2.8 lanes of 32.
         MajorantWalk w;
-        if (!majorantStart(s.volumes[only], org, dir, t0, t1, w)) return true;
-        for (int cells = 0; cells < 4 * kMajorantCells; ++cells) {
-            float exitT;
-            const float mu = majorantHere(w, exitT);
-            if (mu > 0.0f) {
-                for (float t = w.t;;) {
-                    t -= mf::log(1.0f - st.next()) / mu;
-                    if (!(t < exitT)) break;
-                    if (!visit(t, mu, regions)) return false;
-                }
+        bool going = majorantStart(s.volumes[only], org, dir, t0, t1, w), through = true, inside = false;
+        float exitT = 0.0f, t = 0.0f, mu = 0.0f;
+        int cells = 0;
+        while (going) {
+            if (!inside) {
+                mu = majorantHere(w, exitT);
+                t = w.t;
+                inside = mu > 0.0f;
             }
-            if (exitT >= w.tEnd || !majorantNext(w)) return true;
+            bool leaves = !inside;  // the cell
+            if (inside) {
+                t -= mf::log(1.0f - st.next()) / mu;
+                leaves = !(t < exitT);
+                if (!leaves) through = going = visit(t, mu, regions);
+            }
+            if (leaves) {
+                inside = false;
+                going = !(exitT >= w.tEnd) && majorantNext(w) && ++cells < 4 * kMajorantCells;
+            }
         }
-        return true;
+        return through;
     }
     if (!(bound > 0.0f)) return true;
     for (float t = t0;;) {
@@ -139,29 +149,71 @@ template <class Visit>
 __device__ __forceinline__ void trackIntervals(const SceneView& s, const Crossing* x, uint32_t n, uint32_t regions, V3 org, V3 dir, float tnear,
                                                float tfar, Stream& st, Visit& visit) {
     float tStart = tnear;
-    for (uint32_t i = 0; i < n; ++i) {
-        if (x[i].t > tfar) break;
-        if (x[i].t - tStart > kVolumeEpsilon) {
-            if (regions && !trackStretch(s, regions, org, dir, tStart, x[i].t, st, visit)) return;
-            tStart = x[i].t;
+    bool more = true, through = true;
+    for (uint32_t i = 0; more && through; ++i) {
+        more = i < n && x[i].t <= tfar;  // the stretch to crossing i; the last ends at tfar
+        const float t0 = tStart, t1 = more ? x[i].t : tfar;
+        if (t1 - tStart > kVolumeEpsilon) {
+            tStart = t1;
+            if (regions && (more || tfar < kFarLimit)) through = trackStretch(s, regions, org, dir, t0, t1, st, visit);
         }
-        applyCrossing(regions, x[i]);
+        if (more) applyCrossing(regions, x[i]);
     }
-    if (tfar - tStart > kVolumeEpsilon && regions && tfar < kFarLimit) trackStretch(s, regions, org, dir, tStart, tfar, st, visit);
 }
 
 // The ratio-tracking weight's step at a tentative collision, with Russian roulette below 0.1; false once it is zero.
 __device__ __forceinline__ bool ratioStep(float& w, float sigmaT, float mu, Stream& st) {
     w *= 1.0f - fminf(sigmaT / mu, 1.0f);
-    if (w < 0.1f) {
-        if (st.next() >= w) {
-            w = 0.0f;
-            return false;
-        }
-        w = 1.0f;
-    }
-    return true;
+    if (w < 0.1f) w = st.next() >= w ? 0.0f : 1.0f;
+    return w > 0.0f;
 }
+
+// The coefficients at a collision: evalShadersAt's, by DensityLookup in a scene of one volume whose maps it takes (sum and
+// max overlap: that volume's own).
+struct TrackedLookup {
+    const SceneView& s;
+    const VolumeRec* one;
+    DensityLookup density;
+    __device__ explicit TrackedLookup(const SceneView& scene) : s(scene), one(nullptr) {
+        if (s.config.volume_count == 1 && s.volumes[0].interpolation <= kInterpBox && densityLookup(s, s.volumes[0], density)) one = s.volumes;
+    }
+    __device__ __forceinline__ V3 extinction(V3 gp, bool box) const { return cmax0(vscaled(one->gain, box ? density.box(gp) : density.point(gp))); }
+    // sigma_t at the nearest voxel.
+    __device__ __forceinline__ float nearest(uint32_t here, V3 p) const {
+        if (one) return extinction(density.gridPoint(p), false).x;
+        return evalShadersAt(s, here, s.config.volume_overlap_mode, 0.0f, p, kInterpPoint, nullptr, nullptr).sigmaT.x;
+    }
+    __device__ __forceinline__ VolumeCoefficients at(uint32_t here, V3 p) const {
+        if (!one) return evalShadersAt(s, here, s.config.volume_overlap_mode, 0.0f, p, kNoGrid, nullptr, nullptr);
+        VolumeCoefficients k;
+        k.sigmaT = extinction(density.gridPoint(p), one->interpolation == kInterpBox);
+        k.sigmaS = vtimes(cmax0(one->colorMult), k.sigmaT);
+        k.g = vlum(vscaled(k.sigmaS, fminf(fmaxf(one->g, -1.0f), 1.0f)));
+        const float normalization = vlum(k.sigmaS);
+        if (normalization > 0.0f) k.g /= normalization;
+        return k;
+    }
+    // sigma_t and the light the volumes emit there.
+    __device__ __forceinline__ float withEmission(uint32_t here, V3 p, V3& sum) const {
+        sum = V3{0, 0, 0};
+        if (one) {
+            const V3 gp = density.gridPoint(p);
+            if (one->emissionGrid != kNoGrid && one->emissionGrid < s.gridCount && s.grids[one->emissionGrid].channels == 3)
+                sum = vplus(sum, cmax0(vtimes(samplePoint3(s.grids[one->emissionGrid], gp), one->incandescence)));
+            return extinction(gp, one->interpolation == kInterpBox).x;
+        }
+        V3 e[kDeviceVolumes];
+        uint32_t chosen = kMaxVolumes;
+        const VolumeCoefficients k = evalShadersAt(s, here, s.config.volume_overlap_mode, 0.0f, p, kNoGrid, e, &chosen);
+        if (s.config.volume_overlap_mode == kOverlapSum) {
+            for (uint32_t v = 0; v < s.config.volume_count; ++v)
+                if (here >> v & 1) sum = vplus(sum, e[v]);
+        } else if (chosen < kMaxVolumes) {
+            sum = e[0];
+        }
+        return k.sigmaT.x;
+    }
+};
 
 // Ratio tracking: an unbiased estimate of the (grey) transmittance of [tnear, tfar] at the nearest voxel.
 static __device__ __noinline__ float trackedTransmittance(const SceneView& s, Stream& st, V3 org, V3 dir, float tnear, float tfar) {
@@ -170,10 +222,8 @@ static __device__ __noinline__ float trackedTransmittance(const SceneView& s, St
     const uint32_t n = volumeIntervals(s, org, dir, tnear, x, regions);
     if (n == 0 && regions == 0) return 1.0f;
     float w = 1.0f;
-    auto visit = [&](float t, float mu, uint32_t here) {
-        const V3 p = add(org, mul(dir, t));
-        return ratioStep(w, evalShadersAt(s, here, s.config.volume_overlap_mode, 0.0f, p, kInterpPoint, nullptr, nullptr).sigmaT.x, mu, st);
-    };
+    const TrackedLookup lookup(s);
+    auto visit = [&](float t, float mu, uint32_t here) { return ratioStep(w, lookup.nearest(here, add(org, mul(dir, t))), mu, st); };
     trackIntervals(s, x, n, regions, org, dir, tnear, tfar, st, visit);
     return w;
 }
@@ -197,7 +247,6 @@ static __device__ __noinline__ V3 trackedSourceTerm(const SceneView& s, Stream& 
 // Ratio tracking along a ray: its transmittance w and (a camera ray) the light its volumes emit.
 static __device__ __noinline__ void trackedPass(const SceneView& s, const Identity& root, const Pending& pv, U64 volumeBranch, const Crossing* x,
                                                 uint32_t n, uint32_t regions, float tfar, float& w, V3& emitted) {
-    const x2_config& c = s.config;
     const V3 org = pv.origin, dir = pv.dir;
     Identity vid = root;
     vid.branch = childBranch(volumeBranch, 0, 0);
@@ -205,22 +254,14 @@ static __device__ __noinline__ void trackedPass(const SceneView& s, const Identi
     const bool sampleEmission = pv.depth == 0;
     w = 1.0f;
     emitted = V3{0, 0, 0};
+    const TrackedLookup lookup(s);
     auto along = [&](float t, float mu, uint32_t here) {
-        V3 e[kMaxVolumes];
-        uint32_t chosen = kMaxVolumes;
         const V3 p = add(org, mul(dir, t));
-        const VolumeCoefficients k = evalShadersAt(s, here, c.volume_overlap_mode, 0.0f, p, kNoGrid, sampleEmission ? e : nullptr, &chosen);
-        if (sampleEmission) {
-            V3 sum{0, 0, 0};
-            if (c.volume_overlap_mode == kOverlapSum) {
-                for (uint32_t v = 0; v < c.volume_count; ++v)
-                    if (here >> v & 1) sum = vplus(sum, e[v]);
-            } else if (chosen < kMaxVolumes) {
-                sum = e[0];
-            }
-            emitted = vplus(emitted, vscaled(sum, w / mu));
-        }
-        return ratioStep(w, k.sigmaT.x, mu, st);
+        if (!sampleEmission) return ratioStep(w, lookup.at(here, p).sigmaT.x, mu, st);
+        V3 sum;
+        const float sigmaT = lookup.withEmission(here, p, sum);
+        emitted = vplus(emitted, vscaled(sum, w / mu));
+        return ratioStep(w, sigmaT, mu, st);
     };
     trackIntervals(s, x, n, regions, org, dir, pv.nearT, tfar, st, along);
 }
@@ -238,8 +279,9 @@ __device__ __forceinline__ void trackedScatter(const SceneView& s, const Identit
     Stream ds(did, pv.depth, 0);
     float hitT = -1.0f, sigmaT = 0.0f, g = 0.0f;
     V3 sigmaS{0, 0, 0};
+    const TrackedLookup lookup(s);
     auto collide = [&](float t, float mu, uint32_t here) {
-        const VolumeCoefficients k = evalShadersAt(s, here, c.volume_overlap_mode, 0.0f, add(org, mul(dir, t)), kNoGrid, nullptr, nullptr);
+        const VolumeCoefficients k = lookup.at(here, add(org, mul(dir, t)));
         if (ds.next() * mu < k.sigmaT.x) {
             hitT = t;
             sigmaS = k.sigmaS;

@@ -279,14 +279,15 @@ struct NearestVoxel {
         auto half = [](float g0, float g1, float m, float b) { return 0.5f - 0x1p-20f * (fmaxf(fabsf(g0), fabsf(g1)) * fabsf(m) + fabsf(b) + 1.0f); };
         guard = V3{half(g0.x, g1.x, m.x, b.x), half(g0.y, g1.y, m.y, b.y), half(g0.z, g1.z, m.z, b.z)};
     }
-    __device__ float at(V3 p) const {
+    // The voxel's value; false where the floats do not decide its index.
+    __device__ bool at(V3 p, float& value) const {
         const V3 g = d.gridPoint(p);
         const float magic = 12582912.0f;  // 1.5 x 2^23: adding it rounds to a whole number in the low mantissa bits
         const float x = __fmaf_rn(g.x, m.x, b.x), y = __fmaf_rn(g.y, m.y, b.y), z = __fmaf_rn(g.z, m.z, b.z);
         const float rx = x + magic, ry = y + magic, rz = z + magic;
-        if (fabsf(x - (rx - magic)) < guard.x && fabsf(y - (ry - magic)) < guard.y && fabsf(z - (rz - magic)) < guard.z)
-            return d.at(__float_as_int(rx) - 0x4b400000, __float_as_int(ry) - 0x4b400000, __float_as_int(rz) - 0x4b400000);
-        return d.point(g);
+        const bool sure = fabsf(x - (rx - magic)) < guard.x && fabsf(y - (ry - magic)) < guard.y && fabsf(z - (rz - magic)) < guard.z;
+        if (sure) value = d.at(__float_as_int(rx) - 0x4b400000, __float_as_int(ry) - 0x4b400000, __float_as_int(rz) - 0x4b400000);
+        return sure;
     }
 };
 __device__ __forceinline__ bool densityLookup(const SceneView& s, const VolumeRec& v, DensityLookup& d) {
@@ -448,6 +449,7 @@ static_assert(sizeof(MarchCheckpoint) == 48, "three 16-byte words");
 struct MarchRecord {
     static constexpr uint32_t kSlots = 8;  // of a march inside one thread (in its local memory)
     MarchCheckpoint* at;
+    MarchCheckpoint* first = nullptr;  // where the first step is kept (its stepSize 0: not kept), or null
     uint32_t slots;
     uint32_t used = 0, stride = 8, last = 0;
     __device__ MarchRecord(MarchCheckpoint* memory, uint32_t n) : at(memory), slots(n) {}
@@ -538,6 +540,8 @@ struct VolumeMarch {
             vt = vtimes(vt, expNeg(k.sigmaT, delta));
         };
         while (t < t1) {
+            if (record && count == 0 && record->first)
+                *record->first = MarchCheckpoint{vt, t, stepStart, stepSize, 0.0f, interval, regions, 0u, visited, marching.dimension};
             if (record && weightsSoFar && record->wants(count))
                 record->slot(count) = MarchCheckpoint{vt, t, stepStart, stepSize, *weightsSoFar, interval, regions, count, visited, marching.dimension};
             if (vlum(vt) < c.volume_transmittance_threshold) {
@@ -636,11 +640,57 @@ struct ReplaySteps {
         if (partial > total) partial = total;
         return partial;
     }
+    // The steps from a checkpoint in registers, while they lie in its stretch and the stretch is in one volume whose lookups
+    // DensityLookup makes: VolumeMarch::run keeps the march's state in memory (the replays' callers hold it), a dozen
+    // loads and stores a step. False where the stretch ends before emit does (emit's state is then the caller's to
+    // reset); a step's g is left to the caller (phaseOf).
+    template <class Emit>
+    __device__ __forceinline__ bool replay(const MarchCheckpoint* from, Emit& emit) const {
+        const SceneView& s = m.s;
+        const uint32_t regions = from->regions;
+        if (__popc(regions) != 1 || s.config.volume_overlap_mode == kOverlapRnd) return false;
+        const VolumeRec& vr = s.volumes[__ffs(regions) - 1];
+        DensityLookup density;
+        if (vr.interpolation > kInterpBox || !densityLookup(s, vr, density)) return false;
+        const V3 gain = vr.gain, albedo = cmax0(vr.colorMult), org = m.org, dir = m.dir;
+        const bool box = vr.interpolation == kInterpBox;
+        V3 vt = from->vt;
+        float t = from->t, stepStart = from->stepStart;
+        const float stepSize = from->stepSize, t1 = from->interval < m.n ? m.x[from->interval].t : m.tfar;
+        bool inside = true, found = false;
+        for (uint32_t i = from->count; inside; ++i) {
+            const bool rest = !(t < t1);  // the stretch's last, shorter step
+            inside = !rest || t - t1 > kVolumeEpsilon;
+            if (inside) {
+                const float at = rest ? t1 : t;
+                const V3 gp = density.gridPoint(add(org, mul(dir, at)));
+                const V3 sigmaT = cmax0(vscaled(gain, box ? density.box(gp) : density.point(gp)));
+                const float delta = at - stepStart;
+                found = !emit(VolumeStep{sigmaT, vtimes(albedo, sigmaT), vt, 0.0f, stepStart, delta}, i);
+                inside = !found && !rest;
+                vt = vtimes(vt, expNeg(sigmaT, delta));
+                stepStart = t;
+                t += stepSize;
+            }
+        }
+        return found;
+    }
+    __device__ __forceinline__ float phaseOf(const MarchCheckpoint* from, V3 sigmaS) const {
+        float g = vlum(vscaled(sigmaS, fminf(fmaxf(m.s.volumes[__ffs(from->regions) - 1].g, -1.0f), 1.0f)));
+        const float normalization = vlum(sigmaS);
+        if (normalization > 0.0f) g /= normalization;
+        return g;
+    }
+    // Where a replay starts that no checkpoint shortens.
+    __device__ __forceinline__ const MarchCheckpoint* start() const {
+        return record && record->first && record->first->stepSize > 0.0f ? record->first : nullptr;
+    }
     __device__ __noinline__ VolumeStep pick(float r, float& pdf, float& remapped) const {
         const float rw = r * total;
         const MarchCheckpoint* from = last([&](const MarchCheckpoint& c) { return cdfBefore(c) < rw; });
-        float partial = from ? from->partial : 0.0f, prev = from ? cdfBefore(*from) : 0.0f, found = total, before = 0.0f;
+        float partial, prev, found, before;
         VolumeStep chosen{};
+        auto reset = [&] { partial = from ? from->partial : 0.0f, prev = from ? cdfBefore(*from) : 0.0f, found = total, before = 0.0f; };
         auto emit = [&](const VolumeStep& s, uint32_t i) {
             const float here = cdf(partial, s, i);
             chosen = s;
@@ -651,7 +701,14 @@ struct ReplaySteps {
             prev = here;
             return true;
         };
-        m.run(emit, from);
+        reset();
+        const MarchCheckpoint* begin = from ? from : start();
+        if (begin && replay(begin, emit)) {
+            chosen.g = phaseOf(begin, chosen.sigmaS);
+        } else {
+            reset();
+            m.run(emit, from);
+        }
         const float value = found - before;
         pdf = value / total;
         remapped = (rw - before) / value;
@@ -659,8 +716,9 @@ struct ReplaySteps {
     }
     __device__ __noinline__ VolumeStep at(float t, float& pdf) const {
         const MarchCheckpoint* from = last([&](const MarchCheckpoint& c) { return c.stepStart <= t; });
-        float partial = from ? from->partial : 0.0f, here = from ? cdfBefore(*from) : 0.0f, kept = 0.0f, keptPrev = 0.0f;
+        float partial, here, kept, keptPrev;
         VolumeStep chosen{};
+        auto reset = [&] { partial = from ? from->partial : 0.0f, here = from ? cdfBefore(*from) : 0.0f, kept = 0.0f, keptPrev = 0.0f; };
         auto emit = [&](const VolumeStep& s, uint32_t i) {
             if (i > 0 && s.tStart > t) return false;
             const float before = here;
@@ -668,7 +726,14 @@ struct ReplaySteps {
             chosen = s, kept = here, keptPrev = i > 0 ? before : 0.0f;
             return i + 1 < count;
         };
-        m.run(emit, from);
+        reset();
+        const MarchCheckpoint* begin = from ? from : start();
+        if (begin && replay(begin, emit)) {
+            chosen.g = phaseOf(begin, chosen.sigmaS);
+        } else {
+            reset();
+            m.run(emit, from);
+        }
         pdf = (kept - keptPrev) / total;
         return chosen;
     }
@@ -682,59 +747,73 @@ static __device__ __noinline__ V3 volumeTransmittance(const SceneView& s, Stream
     const uint32_t n = volumeIntervals(s, org, dir, tnear, x, regions);
     V3 tr{1, 1, 1};
     if (n == 0 && regions == 0) return tr;
+    // Loops that leave by their conditions alone (no return or break inside them), so that a warp's lanes meet again at
+    // every step whatever each of them found there.
     float tStart = tnear;
-    auto segment = [&](float t0, float t1) -> bool {
-        if (!regions) return true;
-        if (t1 >= kFarLimit) return false;
-        const float fs = minFeatureSize(s, regions);
-        const float tauThreshold = c.volume_transmittance_threshold == 0.0f ? 3.402823466e+38f : -mf::log(c.volume_transmittance_threshold / vlum(tr));
-        const float u = st.next();
-        const float stepSize = fs * c.inv_volume_shadow_quality * fmaxf(float(depth - 1), 1.0f);
-        float t = t0 + stepSize * u;
-        V3 tau{0, 0, 0};
-        const VolumeRec& vr = s.volumes[__ffs(regions) - 1];
-        DensityLookup density;
-        if (__popc(regions) == 1 && c.volume_overlap_mode != kOverlapRnd && densityLookup(s, vr, density)) {
-            // One volume, its nearest voxels: four steps' voxels fetched at once, then added and tested in their order.
-            const V3 gain = vr.gain;
-            const NearestVoxel nearest(density, add(org, mul(dir, t0)), add(org, mul(dir, t1)));
-            while (t < t1) {
-                float d[4];
-                bool in[4];
+    bool through = true, more = true;
+    for (uint32_t i = 0; more && through; ++i) {
+        more = i < n && x[i].t <= tfar;  // the stretch to crossing i; the last ends at tfar
+        const float t0 = tStart, t1 = more ? x[i].t : tfar;
+        if (t1 - tStart > kVolumeEpsilon) {
+            tStart = t1;
+            if (regions && t1 >= kFarLimit) {
+                through = false;
+            } else if (regions) {
+                const float fs = minFeatureSize(s, regions);
+                const float tauThreshold = c.volume_transmittance_threshold == 0.0f ? 3.402823466e+38f : -mf::log(c.volume_transmittance_threshold / vlum(tr));
+                const float u = st.next();
+                const float stepSize = fs * c.inv_volume_shadow_quality * fmaxf(float(depth - 1), 1.0f);
+                float t = t0 + stepSize * u;
+                V3 tau{0, 0, 0};
+                const VolumeRec& vr = s.volumes[__ffs(regions) - 1];
+                DensityLookup density;
+                if (__popc(regions) == 1 && c.volume_overlap_mode != kOverlapRnd && densityLookup(s, vr, density)) {
+                    // One volume, its nearest voxels: four steps' voxels fetched at once, then added and tested in their
+                    // order. An index its float does not decide (under one in a hundred) is made in doubles afterwards.
+                    const V3 gain = vr.gain;
+                    const NearestVoxel nearest(density, add(org, mul(dir, t0)), add(org, mul(dir, t1)));
+                    while (t < t1 && through) {
+                        float at[4], d[4];
+                        uint32_t unsure = 0;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    in[k] = t < t1;
-                    d[k] = in[k] ? nearest.at(add(org, mul(dir, t))) : 0.0f;
-                    t += stepSize;
+                        for (int k = 0; k < 4; ++k) {
+                            at[k] = t;
+                            d[k] = 0.0f;
+                            if (t < t1 && !nearest.at(add(org, mul(dir, t)), d[k])) unsure |= 1u << k;
+                            t += stepSize;
+                        }
+#pragma unroll 1
+                        for (; unsure; unsure &= unsure - 1) {
+                            const int k = __ffs(unsure) - 1;
+                            const float v = density.point(density.gridPoint(add(org, mul(dir, k == 0 ? at[0] : k == 1 ? at[1] : k == 2 ? at[2] : at[3]))));
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                if (j == k) d[j] = v;
+                        }
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            if (at[k] < t1 && through) {
+                                tau = vplus(tau, cmax0(vscaled(gain, d[k])));
+                                through = !(vlum(vscaled(tau, stepSize * scale)) > tauThreshold);
+                            }
+                    }
+                } else {
+                    while (t < t1 && through) {
+                        const float rnd = c.volume_overlap_mode == kOverlapRnd ? st.next() : 0.0f;
+                        tau = vplus(tau, evalShadersAt(s, regions, c.volume_overlap_mode, rnd, add(org, mul(dir, t)), kInterpPoint, nullptr, nullptr).sigmaT);
+                        through = !(vlum(vscaled(tau, stepSize * scale)) > tauThreshold);
+                        t += stepSize;
+                    }
                 }
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    if (!in[k]) break;
-                    tau = vplus(tau, cmax0(vscaled(gain, d[k])));
-                    if (vlum(vscaled(tau, stepSize * scale)) > tauThreshold) return false;
+                if (through) {
+                    tr = vtimes(tr, expNeg(tau, stepSize * scale));
+                    through = vlum(tr) > c.volume_transmittance_threshold;
                 }
             }
-        } else {
-            while (t < t1) {
-                const float rnd = c.volume_overlap_mode == kOverlapRnd ? st.next() : 0.0f;
-                tau = vplus(tau, evalShadersAt(s, regions, c.volume_overlap_mode, rnd, add(org, mul(dir, t)), kInterpPoint, nullptr, nullptr).sigmaT);
-                if (vlum(vscaled(tau, stepSize * scale)) > tauThreshold) return false;
-                t += stepSize;
-            }
         }
-        tr = vtimes(tr, expNeg(tau, stepSize * scale));
-        return vlum(tr) > c.volume_transmittance_threshold;
-    };
-    for (uint32_t i = 0; i < n; ++i) {
-        if (x[i].t > tfar) break;
-        if (x[i].t - tStart > kVolumeEpsilon) {
-            if (!segment(tStart, x[i].t)) return V3{0, 0, 0};
-            tStart = x[i].t;
-        }
-        applyCrossing(regions, x[i]);
+        if (more) applyCrossing(regions, x[i]);
     }
-    if (tfar - tStart > kVolumeEpsilon && !segment(tStart, tfar)) return V3{0, 0, 0};
-    return tr;
+    return through ? tr : V3{0, 0, 0};
 }
 
 // estimateInScatteringSourceTermDirect (async_integrator.h:573-591): a light sample from a point in a volume, its
@@ -990,7 +1069,9 @@ static __device__ __noinline__ void volumeFirstMarch(const SceneView& s, const I
     const bool sampleEmission = pv.depth == 0, deeper = pv.volumeDepth < c.max_volume_depth;
     const bool scatters = deeper && (pv.nonMirror == 0 ? c.volume_illumination_samples : 1u) > 0;
     VolumeMarch march = marchOf(s, root, pv, x, n, regions, tfar, sampleEmission);
-    MarchRecord record(checkpoints, slots);
+    MarchRecord record(checkpoints, slots - 1);
+    record.first = checkpoints + slots - 1;
+    if (scatters) record.first->stepSize = 0.0f;
     march.record = scatters ? &record : nullptr;
     float weights = 0.0f, firstStart = 0.0f, lastEnd = 0.0f;
     march.weightsSoFar = &weights;
@@ -1034,7 +1115,8 @@ __device__ __forceinline__ void volumeScatterTask(const SceneView& s, const Iden
     VolumeMarch march = marchOf(s, root, pv, x, head.crossings, head.regions, tfar, false);
     march.record = nullptr;
     march.weightsSoFar = nullptr;
-    MarchRecord record(checkpoints, slots);
+    MarchRecord record(checkpoints, slots - 1);
+    record.first = checkpoints + slots - 1;
     record.used = head.used;
     const ReplaySteps lookup{march, head.count, head.weights != 0.0f ? head.weights : 1.0f, head.weights == 0.0f, &record};
     scatterSample(s, root, childBranch(pv.branch, 0xfffc, pv.volumeDepth), pv.depth, lookup, pv.origin, pv.dir, pv.T, k / samples, k % samples,
