@@ -265,6 +265,10 @@ struct x2_scene {
     float4* adelta = nullptr;
     uint2* aaux = nullptr;
     float4* atex = nullptr;
+    float *adjGradRows = nullptr, *adjTexGrad = nullptr;  // the gradients' rows, the texels', the FP64 sums
+    double* adjGrads = nullptr;
+    uint32_t adjParams = 0;
+    uint64_t adjTexels = 0;
     uint32_t adjPaths = 0, adjVerts = 0, adjRecords = 0;  // paths the adjoint's buffers hold; their vertices, records
 };
 
@@ -992,6 +996,9 @@ int x2_scene_free(x2_scene* s) {
     if (s->ctx) cudaSetDevice(s->ctx->device);
     if (s->ctx) cudaStreamSynchronize(s->ctx->stream);
     freeAdjointWave(s);
+    cudaFree(s->adjGradRows);
+    cudaFree(s->adjGrads);
+    cudaFree(s->adjTexGrad);
     delete s->adaptiveState;
     s->adaptiveState = nullptr;
     cudaFree(s->bvh.nodes);
@@ -1137,12 +1144,12 @@ WaveKernels launchKernels(const x2_scene* s, const WaveArgs& a) {
                        s->triOverlap != 0 && s->shortStack != 0 && s->traceBlocks < 9, a.vol.head != nullptr);
 }
 
-// A launch as one graph on the context's stream: its iterations in a conditional while node, each iteration's last kernel
-// deciding whether another follows (at most `bound`; past that it raises words[2]), then what tail() enqueues. words: 4
-// device words, cleared here.
-int launchDrain(x2_scene* s, const WaveKernels& wk, const WaveArgs& a, const WaveGrids& grids, uint32_t* words, uint32_t bound, const char* what,
+// A launch as one graph on the context's stream: its iterations (what iteration() enqueues) in a conditional while node,
+// each iteration's last kernel deciding whether another follows (at most `bound`; past that it raises words[2]), then what
+// tail() enqueues. words: 4 device words, cleared here.
+int launchDrain(x2_ctx* ctx, const WaveArgs& a, uint32_t* words, uint32_t bound, const char* what, const std::function<void()>& iteration,
                 const std::function<void()>& tail) {
-    cudaStream_t st = s->ctx->stream;
+    cudaStream_t st = ctx->stream;
     cudaGraph_t graph = nullptr;
     CUDA_OR(cudaGraphCreate(&graph, 0), X2_ECUDA);
     cudaError_t err = cudaSuccess;
@@ -1162,7 +1169,7 @@ int launchDrain(x2_scene* s, const WaveKernels& wk, const WaveArgs& a, const Wav
     }
     if (err == cudaSuccess && check(cudaStreamBeginCaptureToGraph(st, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
                                                                   cudaStreamCaptureModeThreadLocal))) {
-        launchIteration(wk, a, grids, st, false, &s->ctx->side);
+        iteration();
         wfDrainCheck<<<1, 32, 0, st>>>(a, loop, words, bound, words + 2);
         check(cudaGetLastError());
         cudaGraph_t body = nullptr;
@@ -1253,7 +1260,9 @@ int integrateWavefront(x2_scene* s, uint32_t paths, const uint32_t* pairs, uint6
         a.out = s->pairOut;
         a.outStatus = s->pairStatus;
         const uint64_t bound = uint64_t(items) * (uint64_t(s->config.max_depth) + 2) / paths + uint64_t(s->config.max_depth) + 64;
-        const int done = launchDrain(s, launchKernels(s, a), a, grids, s->pairWords, uint32_t(std::min<uint64_t>(bound, 0xffffffffu)), "x2_integrate", [&] {
+        const WaveKernels wk = launchKernels(s, a);
+        const int done = launchDrain(s->ctx, a, s->pairWords, uint32_t(std::min<uint64_t>(bound, 0xffffffffu)), "x2_integrate",
+                                     [&] { launchIteration(wk, a, grids, st, false, &s->ctx->side); }, [&] {
             wfPairsOut<<<(items + 255) / 256, 256, 0, st>>>(s->pairOut, s->pairStatus, items, rgba + 4 * first, status + first);
         });
         if (done) return done;
@@ -1723,9 +1732,11 @@ int x2_launch_wavefront(x2_scene* s, const x2_chunk* chunks, uint32_t count) {
     // collect it like any launch.
     const uint32_t bound = uint32_t(std::min<uint64_t>(maxIter, 0xffffffffu));
     cudaEventRecord(sl.begin, st);
-    if (int rc = launchDrain(s, wk, a, grids, s->drainWords, bound, "x2_launch_wavefront", [&] {
-            wfFilmReduce<<<int((64ull * count + 255) / 256), 256, 0, st>>>(a, count, s->sums, s->adaptive ? s->odd : nullptr, s->counts);
-        }))
+    if (int rc = launchDrain(s->ctx, a, s->drainWords, bound, "x2_launch_wavefront", [&] { launchIteration(wk, a, grids, st, false, &s->ctx->side); },
+                             [&] {
+                                 wfFilmReduce<<<int((64ull * count + 255) / 256), 256, 0, st>>>(
+                                     a, count, s->sums, s->adaptive ? s->odd : nullptr, s->counts);
+                             }))
         return rc;
     cudaEventRecord(sl.end, st);
     // The extend kernels counted the traced rays; the launch's counters go to the host as x2_launch's do, with the
@@ -1937,18 +1948,29 @@ int x2_adjoint(x2_scene* s, uint32_t first, uint32_t count, const float* d_dloss
     }
     Slot& sl = s->slots[0];
     if (int rc = ensureSlot(sl, tiles)) return rc;
+    // The gradient rows, the FP64 gradients and the texels' (kept with the scene).
     constexpr uint32_t kRows = 1024;
-    float* rows = nullptr;
-    double* grads = nullptr;
-    float* texGrad = nullptr;
     const uint64_t texGrads = d_texture_grad ? 3 * texelCount(s) : 0;
-    if (cudaMalloc(&rows, sizeof(float) * size_t(kRows) * params) != cudaSuccess || cudaMalloc(&grads, sizeof(double) * params) != cudaSuccess ||
-        (texGrads && cudaMalloc(&texGrad, sizeof(float) * texGrads) != cudaSuccess)) {
-        cudaFree(rows);
-        cudaFree(grads);
-        setError("x2_adjoint: allocation failed");
-        return X2_ENOMEM;
+    if (params > s->adjParams || texGrads > s->adjTexels) {
+        cudaFree(s->adjGradRows);
+        cudaFree(s->adjGrads);
+        cudaFree(s->adjTexGrad);
+        s->adjGradRows = s->adjTexGrad = nullptr;
+        s->adjGrads = nullptr;
+        s->adjParams = 0;
+        s->adjTexels = 0;
+        if (cudaMalloc(&s->adjGradRows, sizeof(float) * size_t(kRows) * params) != cudaSuccess ||
+            cudaMalloc(&s->adjGrads, sizeof(double) * params) != cudaSuccess ||
+            (texGrads && cudaMalloc(&s->adjTexGrad, sizeof(float) * texGrads) != cudaSuccess)) {
+            setError("x2_adjoint: allocation failed");
+            return X2_ENOMEM;
+        }
+        s->adjParams = params;
+        s->adjTexels = texGrads;
     }
+    float* const rows = s->adjGradRows;
+    double* const grads = s->adjGrads;
+    float* const texGrad = texGrads ? s->adjTexGrad : nullptr;
     cudaStream_t st = s->ctx->stream;
     std::vector<x2_chunk> chunks(tiles);
     for (uint32_t t = 0; t < tiles; ++t) chunks[t] = x2_chunk{t, first, count, 0};
@@ -1997,67 +2019,32 @@ int x2_adjoint(x2_scene* s, uint32_t first, uint32_t count, const float* d_dloss
     a.pixelBase = nullptr;
     a.liveChunks = nullptr;
     const size_t shared = sizeof(float) * params;
-    if (shared > 48 * 1024) {
-        cudaFuncSetAttribute(wfLogicAdjoint, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shared));
-        cudaFuncSetAttribute(wfShadeAdjoint, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shared));
-    }
-    // Logic in a grid of a few blocks a SM (each block's partials go to a gradient row once a launch).
-    const int gridLogic = std::min(int((paths + kWaveBlock - 1) / kWaveBlock), s->ctx->smCount * 8);
+    const AdjointKernels adj = adjointKernels(s->triUV != nullptr);
+    if (shared > 48 * 1024)
+        for (auto* k : {adj.logic, adj.shade, adj.shadeBy[0], adj.shadeBy[1], adj.shadeBy[2]})
+            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(shared));
     const WaveGrids grids = waveGrids(paths, records, s->ctx->smCount, s->blocksPerSm);
-    const WaveKernels wk = waveKernels(s->traceBlocks, s->shadeBlocks, false, s->triUV != nullptr);
+    const WaveKernels wk = waveKernels(s->traceBlocks, s->shadeBlocks, false, s->triUV != nullptr, s->shortStack != 0, false, false, 0,
+                                       s->triOverlap != 0 && s->shortStack != 0 && s->traceBlocks < 9);
     const uint64_t maxIter = items * (uint64_t(s->config.max_depth) + 2) / paths + uint64_t(s->config.max_depth) + 64;
-    constexpr int kIter = 8;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    int rc = X2_OK;
-    if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-        setError("x2_adjoint: stream capture failed");
-        rc = X2_ECUDA;
-    } else {
-        for (int it = 0; it < kIter; ++it) {
-            wfResetQueues<<<1, 32, 0, st>>>(a);
-            wfLogicAdjoint<<<gridLogic, kWaveBlock, shared, st>>>(a);
-            wk.extend<<<grids.work, kWaveBlock, 0, st>>>(a);
-            if (a.shadeQ) wfSortShade<<<grids.work, kWaveBlock, 0, st>>>(a);
-            wfShadeAdjoint<<<grids.work, kWaveBlock, shared, st>>>(a);
-            wk.shadow<<<grids.shadow, kWaveBlock, 0, st>>>(a);
-        }
-        wfResetQueues<<<1, 32, 0, st>>>(a);
-        if (cudaStreamEndCapture(st, &graph) != cudaSuccess || cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) {
-            setError("x2_adjoint: graph capture failed");
-            rc = X2_ECUDA;
-        }
+    int rc = launchDrain(
+        s->ctx, a, s->drainWords, uint32_t(std::min<uint64_t>(maxIter, 0xffffffffu)), "x2_adjoint",
+        [&] { launchAdjointIteration(wk, adj, a, grids, s->ctx->smCount * 8, shared, st, &s->ctx->side); },
+        [&] {
+            wfGradRows<<<(params + 31) / 32, dim3(32, 32), 0, st>>>(rows, kRows, params, grads);
+            addInto<<<(params + 255) / 256, 256, 0, st>>>(d_albedo_grad, grads, 3 * s->materialCount);
+            if (d_roughness_grad) addInto<<<(params + 255) / 256, 256, 0, st>>>(d_roughness_grad, grads + 3 * s->materialCount, s->materialCount);
+            addInto<<<(params + 255) / 256, 256, 0, st>>>(d_radiance_grad, grads + 4 * s->materialCount, 3 * s->lightCount);
+            if (texGrads) addFloatInto<<<unsigned((texGrads + 255) / 256), 256, 0, st>>>(d_texture_grad, texGrad, texGrads);
+        });
+    if (rc) return rc;
+    cudaMemcpyAsync(s->hostDrain, s->drainWords, sizeof(uint32_t) * 4, cudaMemcpyDeviceToHost, st);
+    if ((rc = x2_synchronize(s->ctx, 600000)) != X2_OK) return rc;
+    if (s->hostDrain[2]) {
+        setError("x2_adjoint: the wavefront did not drain after %u iterations", s->hostDrain[0]);
+        return X2_EDEVICE;
     }
-    uint32_t iterations = 0;
-    while (rc == X2_OK) {
-        if (cudaGraphLaunch(exec, st) != cudaSuccess) {
-            setError("x2_adjoint: graph launch failed");
-            rc = X2_ECUDA;
-            break;
-        }
-        iterations += kIter;
-        cudaMemcpyAsync(s->hostLast, s->waveCounters + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-        if ((rc = x2_synchronize(s->ctx, 600000)) != X2_OK) break;
-        if (s->hostLast[0] == 0) break;
-        if (iterations > maxIter) {
-            setError("x2_adjoint: the wavefront did not drain after %u iterations", iterations);
-            rc = X2_EDEVICE;
-        }
-    }
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-    if (rc == X2_OK) {
-        wfGradRows<<<(params + 255) / 256, 256, 0, st>>>(rows, kRows, params, grads);
-        addInto<<<(params + 255) / 256, 256, 0, st>>>(d_albedo_grad, grads, 3 * s->materialCount);
-        if (d_roughness_grad) addInto<<<(params + 255) / 256, 256, 0, st>>>(d_roughness_grad, grads + 3 * s->materialCount, s->materialCount);
-        addInto<<<(params + 255) / 256, 256, 0, st>>>(d_radiance_grad, grads + 4 * s->materialCount, 3 * s->lightCount);
-        if (texGrads) addFloatInto<<<unsigned((texGrads + 255) / 256), 256, 0, st>>>(d_texture_grad, texGrad, texGrads);
-        rc = cudaGetLastError() == cudaSuccess ? x2_synchronize(s->ctx, 600000) : X2_ECUDA;
-    }
-    cudaFree(rows);
-    cudaFree(grads);
-    cudaFree(texGrad);
-    return rc;
+    return X2_OK;
 }
 
 // ---- adaptive sampling (row f2): the reference's adaptive frame (async_render.h, async_adaptive.h) on the device ----
@@ -2864,49 +2851,18 @@ int x2_render_batch(x2_ctx* ctx, const x2_request* req, uint32_t n, x2_completio
         a.chunkItems = dChunkItems;
         a.chunkCount = c1 - c0;
         const uint64_t maxIter = windowItems * (uint64_t(maxDepth) + 2) / paths + uint64_t(maxDepth) + 64;
-        constexpr int kIter = 8;
-        cudaGraph_t graph = nullptr;
-        cudaGraphExec_t exec = nullptr;
-        if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-            setError("stream capture failed");
-            rc = X2_ECUDA;
-            break;
-        }
-        for (int it = 0; it < kIter; ++it) {
-            wfResetQueues<<<1, 32, 0, st>>>(a);
-            launchIteration(wk, a, grids, st, true, &ctx->side);
-        }
-        wfResetQueues<<<1, 32, 0, st>>>(a);
-        if (cudaStreamEndCapture(st, &graph) != cudaSuccess || cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) {
-            if (graph) cudaGraphDestroy(graph);
-            setError("batch graph capture failed");
-            rc = X2_ECUDA;
-            break;
-        }
-        for (uint64_t it = 0;;) {
-            if (cudaGraphLaunch(exec, st) != cudaSuccess) {
-                setError("graph launch failed");
-                rc = X2_ECUDA;
-                break;
-            }
-            it += kIter;
-            iterations += kIter;
-            cudaMemcpyAsync(s0->hostLast, s0->waveCounters + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-            if ((rc = x2_synchronize(ctx, 600000)) != X2_OK) break;
-            if (s0->hostLast[0] == 0) break;
-            if (it > maxIter) {
-                setError("batch window did not drain after %llu iterations", (unsigned long long)it);
-                rc = X2_EDEVICE;
-                break;
-            }
-        }
-        cudaGraphExecDestroy(exec);
-        cudaGraphDestroy(graph);
+        rc = launchDrain(
+            ctx, a, s0->drainWords, uint32_t(std::min<uint64_t>(maxIter, 0xffffffffu)), "x2_render_batch",
+            [&] { launchIteration(wk, a, grids, st, true, &ctx->side); },
+            [&] { wfFilmReduceBatch<<<int((64ull * (c1 - c0) + 255) / 256), 256, 0, st>>>(a, dFilms); });
         if (rc) break;
-        wfFilmReduceBatch<<<int((64ull * (c1 - c0) + 255) / 256), 256, 0, st>>>(a, dFilms);
-        if (cudaGetLastError() != cudaSuccess) {
-            setError("batch film reduction failed to launch");
-            rc = X2_ECUDA;
+        // The next window rewrites the host's tables: this one is waited for.
+        cudaMemcpyAsync(s0->hostDrain, s0->drainWords, sizeof(uint32_t) * 4, cudaMemcpyDeviceToHost, st);
+        if ((rc = x2_synchronize(ctx, 600000)) != X2_OK) break;
+        iterations += s0->hostDrain[0];
+        if (s0->hostDrain[2]) {
+            setError("batch window did not drain after %u iterations", s0->hostDrain[0]);
+            rc = X2_EDEVICE;
         }
     }
     if (!rc) {

@@ -1026,13 +1026,24 @@ template <bool kTextures>
 __global__ void __launch_bounds__(kWaveBlock, 4) wfShadeVolumesApart(WaveArgs a) { shadeBody<false, kApartVolumes, false, kTextures>(a); }
 __global__ void __launch_bounds__(kWaveBlock, 4) wfShadeBatchVolumes(WaveArgs a) { shadeBody<true, kInlineVolumes>(a); }
 __global__ void __launch_bounds__(kWaveBlock, 4) wfShadeAdjoint(WaveArgs a) { shadeBody<false, kNoVolumes, true>(a); }
+// Split by lobe, as the primal's.
+template <int kQueue, bool kTextures>
+__global__ void __launch_bounds__(kWaveBlock, 4) wfShadeAdjointQueue(WaveArgs a) {
+    shadeBody<false, kNoVolumes, true, kTextures, kQueue>(a);
+}
 
-// The adjoint's gradient rows summed in FP64 into grads (one thread a gradient).
+// The adjoint's gradient rows summed in FP64 into grads: a block 32 neighbouring gradients, 32 threads each a share of the
+// rows (one thread a gradient ran its 1024 rows' additions one after another).
 __global__ void wfGradRows(const float* rows, uint32_t rowCount, uint32_t params, double* grads) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= params) return;
+    __shared__ double part[32][33];
+    const uint32_t i = blockIdx.x * 32 + threadIdx.x;
     double sum = 0.0;
-    for (uint32_t r = 0; r < rowCount; ++r) sum += double(rows[size_t(r) * params + i]);
+    if (i < params)
+        for (uint32_t r = threadIdx.y; r < rowCount; r += 32) sum += double(rows[size_t(r) * params + i]);
+    part[threadIdx.y][threadIdx.x] = sum;
+    __syncthreads();
+    if (threadIdx.y || i >= params) return;
+    for (uint32_t k = 1; k < 32; ++k) sum += part[k][threadIdx.x];
     grads[i] += sum;
 }
 __global__ void __launch_bounds__(kWaveBlock) wfShadow(WaveArgs a) { shadowBody<false>(a); }
@@ -1207,6 +1218,36 @@ WaveKernels waveKernelsBatch(bool volumes, bool textures, bool shadeSplit, bool 
     k.shadow = overlap ? wfShadowOverlapBatch : wfShadowBatch;
     k.shade = volumes ? wfShadeBatchVolumes : textures ? wfShadeOcc<4, true, true> : wfShadeOcc<4, true>;
     return k;
+}
+
+AdjointKernels adjointKernels(bool textures) {
+    AdjointKernels k;
+    k.logic = wfLogicAdjoint;
+    k.shade = wfShadeAdjoint;
+    k.shadeBy[0] = textures ? wfShadeAdjointQueue<0, true> : wfShadeAdjointQueue<0, false>;
+    k.shadeBy[1] = textures ? wfShadeAdjointQueue<1, true> : wfShadeAdjointQueue<1, false>;
+    k.shadeBy[2] = textures ? wfShadeAdjointQueue<2, true> : wfShadeAdjointQueue<2, false>;
+    return k;
+}
+
+void launchAdjointIteration(const WaveKernels& k, const AdjointKernels& adj, const WaveArgs& a, const WaveGrids& g, int creditBlocks,
+                            size_t shared, cudaStream_t st, const SideStreams* side) {
+    adj.logic<<<std::min(g.logic, creditBlocks), kWaveBlock, shared, st>>>(a);
+    k.extend<<<g.work, kWaveBlock, 0, st>>>(a);
+    if (a.shadeQ) {
+        wfSortShade<<<g.work, kWaveBlock, 0, st>>>(a);
+        cudaStream_t on[3] = {st, side->stream[0], side->stream[1]};
+        cudaEventRecord(side->fork, st);
+        for (int j = 0; j < 2; ++j) cudaStreamWaitEvent(side->stream[j], side->fork, 0);
+        for (int q = 0; q < 3; ++q) adj.shadeBy[q]<<<std::min(g.work, creditBlocks), kWaveBlock, shared, on[q]>>>(a);
+        for (int j = 0; j < 2; ++j) {
+            cudaEventRecord(side->join[j], side->stream[j]);
+            cudaStreamWaitEvent(st, side->join[j], 0);
+        }
+    } else {
+        adj.shade<<<std::min(g.work, creditBlocks), kWaveBlock, shared, st>>>(a);
+    }
+    k.shadow<<<g.shadow, kWaveBlock, 0, st>>>(a);
 }
 
 // Queue counters for the next iteration: the extend and shadow counts start at zero; the previous extend count is kept

@@ -185,8 +185,17 @@ __global__ void wfSortShade(WaveArgs a);
 __global__ void wfSortShadeBatch(WaveArgs a);
 // The adjoint's logic and shade kernels (dynamic shared memory: the gradient count in floats) and the final sum of the
 // gradient rows into FP64 (added to grads).
-__global__ void wfLogicAdjoint(WaveArgs a);
-__global__ void wfShadeAdjoint(WaveArgs a);
+struct AdjointKernels {
+    void (*logic)(WaveArgs);
+    void (*shade)(WaveArgs);       // every extended path
+    void (*shadeBy[3])(WaveArgs);  // one per-lobe queue each
+};
+AdjointKernels adjointKernels(bool textures);
+// An iteration of the adjoint: its logic, extend (k's), the sort and the per-lobe shade kernels side by side (or one shade
+// kernel without the queues), shadow (k's). The crediting kernels run in at most creditBlocks blocks, each of which zeroes
+// its partials and adds them to a gradient row once.
+void launchAdjointIteration(const WaveKernels& k, const AdjointKernels& adj, const WaveArgs& a, const WaveGrids& g, int creditBlocks,
+                            size_t shared, cudaStream_t st, const SideStreams* side);
 __global__ void wfGradRows(const float* rows, uint32_t rowCount, uint32_t params, double* grads);
 __global__ void wfResetQueues(WaveArgs a);
 // The drain loop's test, last in the body of a conditional while node: go on while the iteration extended a ray, at
