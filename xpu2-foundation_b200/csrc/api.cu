@@ -1348,7 +1348,12 @@ int x2_trace_rays_device(x2_scene* s, const float* rays, uint64_t n, uint32_t* t
         setError("null rays");
         return X2_EINVAL;
     }
-    traceRays<<<s->ctx->smCount * 8, 128, 0, s->ctx->stream>>>(viewOf(s), rays, n, tri, t, occluded);
+    if (int rc = ensureSlot(s->integrateSlot, 1)) return rc;
+    int perSm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, traceRays, kRenderBlock, 0);
+    const int blocks = int(std::min<uint64_t>(uint64_t(s->ctx->smCount) * std::max(perSm, 1), (2 * n + kRenderBlock - 1) / kRenderBlock));
+    cudaMemsetAsync(s->integrateSlot.claimed, 0, sizeof(unsigned long long), s->ctx->stream);
+    traceRays<<<blocks, kRenderBlock, 0, s->ctx->stream>>>(viewOf(s), rays, n, tri, t, occluded, s->integrateSlot.claimed);
     CUDA_OR(cudaGetLastError(), X2_ECUDA);
     return X2_OK;
 }

@@ -422,18 +422,54 @@ __global__ void __launch_bounds__(kRenderBlock) integratePairsVolumes(SceneView 
 }
 
 // Closest hit and occlusion for n rays (8 floats each: origin, direction, near, far).
-__global__ void traceRays(SceneView s, const float* __restrict__ rays, unsigned long long n, uint32_t* __restrict__ tri, float* __restrict__ t,
-                          uint32_t* __restrict__ occluded) {
-    const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const float* r = rays + 8 * i;
-        const RayQ q = makeRay(s.bvh, r[0], r[1], r[2], r[3], r[4], r[5]);
-        float th;
-        uint32_t leaf;
-        const uint32_t id = traceClosest<false>(s.bvh, q, r[6], r[7], th, &leaf, s.overflow, nullptr);
-        if (tri) tri[i] = id;
-        if (t) t[i] = id == ~0u ? 0.0f : th;
-        if (occluded) occluded[i] = traceAny<false>(s.bvh, q, r[6], r[7], s.overflow, nullptr) ? 1u : 0u;
+// The ray entry: query 2 i is ray i's closest hit (when a caller wants it), 2 i + 1 its occlusion, walked a node a step by
+// persistent warps whose idle lanes take the next queries (as the wavefront's traversal kernels). One thread a ray, both
+// walks one after the other, took 0.225 ms for 262,139 scattered rays: a warp waited for its longest walk twice.
+__global__ void __launch_bounds__(kRenderBlock) traceRays(SceneView s, const float* __restrict__ rays, unsigned long long n,
+                                                          uint32_t* __restrict__ tri, float* __restrict__ t, uint32_t* __restrict__ occluded,
+                                                          unsigned long long* next) {
+    __shared__ uint2 shortStacks[kShortStack * kRenderBlock];
+    const unsigned full = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31u;
+    Walk<kShortStack> walk;
+    uint2 deep[kStack - kShortStack];
+    walk.shortStack = shortStacks + threadIdx.x;
+    walk.nodes = walk.tris = 0;
+    const bool wantHit = tri || t, wantOccluded = occluded != nullptr;
+    const unsigned long long kinds = (wantHit ? 1u : 0u) + (wantOccluded ? 1u : 0u), queries = n * kinds;
+    unsigned long long ray = 0;
+    bool walking = false, any = false, drained = queries == 0;
+    RayQ r;
+    for (;;) {
+        uint32_t lanes = __ballot_sync(full, walking);
+        if (!drained && 32 - __popc(lanes) >= 8) {
+            const uint32_t want = 32 - __popc(lanes);
+            unsigned long long base = 0;
+            if (lane == 0) base = atomicAdd(next, (unsigned long long)want);
+            base = __shfl_sync(full, base, 0);
+            drained = base + want >= queries;
+            const unsigned long long q = base + __popc(~lanes & ((1u << lane) - 1u));
+            if (!walking && q < queries) {
+                ray = kinds == 2 ? q >> 1 : q;
+                any = kinds == 2 ? (q & 1u) != 0 : wantOccluded;
+                const float* v = rays + 8 * ray;
+                r = makeRay(s.bvh, v[0], v[1], v[2], v[3], v[4], v[5]);
+                if (any) walkStart<true, kShortStack>(walk, r, v[6], v[7]);
+                else walkStart<false, kShortStack>(walk, r, v[6], v[7]);
+                walking = true;
+            }
+            lanes = __ballot_sync(full, walking);
+        }
+        if (!lanes) break;
+        if (walking && walkStepOverlapKind<kShortStack>(s.bvh, r, walk, deep, s.overflow, lanes, any)) {
+            if (any) {
+                occluded[ray] = walk.best;
+            } else {
+                if (tri) tri[ray] = walk.best;
+                if (t) t[ray] = walk.best == ~0u ? 0.0f : walk.tmax;
+            }
+            walking = false;
+        }
     }
 }
 

@@ -46,7 +46,8 @@ __global__ void integratePairsTextured(SceneView s, const uint32_t* pairs, unsig
                                        Counters* counters);
 __global__ void integratePairsVolumes(SceneView s, const uint32_t* pairs, unsigned long long n, double* rgba, uint32_t* status,
                                       Counters* counters);
-__global__ void traceRays(SceneView s, const float* rays, unsigned long long n, uint32_t* tri, float* t, uint32_t* occluded);
+__global__ void traceRays(SceneView s, const float* rays, unsigned long long n, uint32_t* tri, float* t, uint32_t* occluded,
+                          unsigned long long* next);
 __global__ void sampleWords(const x2_identity* ids, const uint32_t* dims, unsigned long long n, uint32_t policy, uint32_t* out);
 __global__ void auditCounts(const uint32_t* counts, const uint32_t* expected, uint32_t spp, uint32_t pixels, unsigned long long* firstBad);
 
