@@ -405,7 +405,7 @@ int x2_render_workgrid(x2_scene* scene, x2_workgrid* grid, uint32_t chunks_per_l
  * material), each material's roughness (a GGX lobe's; 1 float a material) and each light's radiance (3 floats a
  * light); host arrays, null leaves a set as it is. Waits. */
 int x2_scene_set_params(x2_scene* scene, const float* albedo, const float* roughness, const float* radiance);
-/* A texture's texels set in place (host array, the texture's width x height x 3 floats). Waits. */
+/* A texture's texels set in place (host or device array, the texture's width x height x 3 floats). Waits. */
 int x2_scene_set_texture(x2_scene* scene, uint32_t texture, const float* rgb);
 /* The adjoint of samples [first, first + count) of every pixel (the film's mean image): given dL/dimage (device, 3
  * floats a pixel), adds dL/dalbedo (device, 3 doubles a material: for a textured material its diffuse multiplier),

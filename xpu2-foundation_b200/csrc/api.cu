@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstring>
 #include <functional>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -69,9 +70,13 @@ void sobolDirections(uint32_t out[17][32]) {
         }                                                                                           \
     } while (0)
 
-// Waits for an event with a deadline (no unbounded cudaEventSynchronize).
+// Waits for an event with a deadline (no unbounded cudaEventSynchronize). The first kSpinMs polls without sleeping: a
+// sleep of 50 us lasts over 100, and a small frame's calls wait three or four times (the 256x256 box pass at one sample:
+// 0.3 of its 1.2 ms).
+constexpr int kSpinMs = 2;
 int waitEvent(cudaEvent_t e, int timeoutMs) {
-    const auto until = std::chrono::steady_clock::now() + std::chrono::milliseconds(timeoutMs < 0 ? 0 : timeoutMs);
+    const auto begin = std::chrono::steady_clock::now();
+    const auto until = begin + std::chrono::milliseconds(timeoutMs < 0 ? 0 : timeoutMs), spin = begin + std::chrono::milliseconds(kSpinMs);
     for (;;) {
         const cudaError_t q = cudaEventQuery(e);
         if (q == cudaSuccess) return X2_OK;
@@ -79,11 +84,13 @@ int waitEvent(cudaEvent_t e, int timeoutMs) {
             setError("device error while waiting: %s", cudaGetErrorString(q));
             return X2_ECUDA;
         }
-        if (std::chrono::steady_clock::now() >= until) {
+        const auto now = std::chrono::steady_clock::now();
+        if (now >= until) {
             setError("wait timed out after %d ms", timeoutMs);
             return X2_ETIMEOUT;
         }
-        std::this_thread::sleep_for(std::chrono::microseconds(50));
+        if (now < spin) std::this_thread::yield();
+        else std::this_thread::sleep_for(std::chrono::microseconds(50));
     }
 }
 
@@ -110,12 +117,27 @@ struct Slot {
 
 using namespace x2;
 
+// A launch's instantiated graph and the bytes of what it was made with.
+struct KeptGraph {
+    cudaGraphExec_t exec = nullptr;
+    std::vector<unsigned char> key;
+    void drop() {
+        if (exec) cudaGraphExecDestroy(exec);
+        exec = nullptr;
+        key.clear();
+    }
+};
+
 struct x2_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     int smCount = 0;
     int renderBlocksPerSm = 0;
     x2::SideStreams side;  // for kernels of one iteration that run side by side
+    std::mutex scratchMutex;
+    unsigned char* scratch = nullptr;  // a host caller's arrays during x2_integrate or x2_trace_rays
+    size_t scratchBytes = 0;
+    bool scratchLent = false;
 };
 
 // An adaptive frame's device state (adaptive.h AdaptiveArgs) and its host-side layout.
@@ -216,8 +238,10 @@ struct x2_scene {
     TraversalStats* stats = nullptr;  // device
     bool counting = false;
     float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};  // the vertices' bounds
-    // wavefront
+    // wavefront (its arrays in one allocation, its device and pinned words in one each)
     WaveState wave{};
+    unsigned char *waveMemory = nullptr, *deviceWords = nullptr;
+    uint32_t* hostWords = nullptr;
     uint32_t wavePaths = 0, waveRecords = 0, reservePaths = 0;  // the last launch's paths; records a path
     uint32_t waveCap = 0;                                          // paths the wave's buffers hold
     uint32_t* extendQ = nullptr;
@@ -244,6 +268,7 @@ struct x2_scene {
     uint32_t waveIterations = 0;       // of the last wavefront launch
     // The asynchronous wavefront launch's drain: [0] its iterations, [1] a running total, [2] its overrun word
     // (device; 4 words), their host copy (pinned), the launch they belong to (0: none pending) and its bound.
+    KeptGraph frameGraph, pairGraph, adaptiveGraph;  // the last frame launch's, per-sample launch's and adaptive frame's graph
     uint32_t* drainWords = nullptr;
     uint32_t* hostDrain = nullptr;
     uint64_t drainSeq = 0;
@@ -258,6 +283,7 @@ struct x2_scene {
     AdaptiveState* adaptiveState = nullptr;
     // the adjoint's wavefront state (x2_adjoint): vertex records, scales, counts, dL/dI shares, record auxiliaries
     x2::VolumeWave vol{};                 // a volume scene's wavefront state (its volumes in kernels of their own)
+    unsigned char* volMemory = nullptr;
     uint32_t volPaths = 0, volRecords = 0, volTasks = 0;  // the paths, records and samples its buffers hold
     uint4* avert = nullptr;
     float4* ascale = nullptr;
@@ -276,6 +302,7 @@ namespace {
 
 SceneView viewOf(const x2_scene* s) {
     SceneView v;
+    std::memset(&v, 0, sizeof(v));
     v.bvh = Bvh8{s->bvh.nodes, s->bvh.tris, s->bvh.nodeCount, s->bvh.triCount, {s->lo[0], s->lo[1], s->lo[2]}, {s->hi[0], s->hi[1], s->hi[2]},
                  {s->bvh.rot[0], s->bvh.rot[1], s->bvh.tris}};
     v.triMesh = s->triMesh;
@@ -359,15 +386,35 @@ void retire(x2_scene* s, Slot& sl, x2_completion* out) {
     sl.busy = false;
 }
 
+// Several arrays in one allocation: a first pass over the takes sizes it (base null), a second places them, 256 bytes
+// aligned. (A new scene's first launch made some thirty allocations, a good part of its time.)
+struct Carve {
+    unsigned char* base = nullptr;
+    size_t size = 0;
+    template <class T>
+    void take(T*& p, size_t n) {
+        size = (size + 255) & ~size_t(255);
+        if (base) p = reinterpret_cast<T*>(base + size);
+        size += sizeof(T) * n;
+    }
+};
+template <class Place>
+bool carve(unsigned char** memory, const Place& place) {
+    Carve m;
+    place(m);
+    if (cudaMalloc(memory, m.size) != cudaSuccess) {
+        *memory = nullptr;
+        return false;
+    }
+    m = Carve{*memory, 0};
+    place(m);
+    return true;
+}
+
 void freeWave(x2_scene* s) {
-    WaveState& w = s->wave;
-    void* ptrs[] = {w.ray0, w.ray1, w.T, w.held, w.meta, w.branch, w.rad, w.hit, w.state, w.item, w.ncount, w.sray0, w.sray1, w.scontrib, w.svis,
-                    w.lightJob, w.lightFlags};
-    for (void* p : ptrs) cudaFree(p);
-    w = WaveState{};
-    cudaFree(s->extendQ);
-    cudaFree(s->shadowQ);
-    cudaFree(s->shadeQ);
+    cudaFree(s->waveMemory);
+    s->waveMemory = nullptr;
+    s->wave = WaveState{};
     s->extendQ = s->shadowQ = s->shadeQ = nullptr;
     s->wavePaths = s->waveRecords = s->waveCap = 0;
 }
@@ -383,23 +430,27 @@ int ensureWave(x2_scene* s, uint32_t paths, uint32_t records) {
     freeWave(s);
     WaveState& w = s->wave;
     const size_t P = paths, R = size_t(paths) * records;
-    bool ok = cudaMalloc(&w.ray0, sizeof(float4) * P) == cudaSuccess && cudaMalloc(&w.ray1, sizeof(float4) * P) == cudaSuccess &&
-              cudaMalloc(&w.T, sizeof(float4) * P) == cudaSuccess && cudaMalloc(&w.held, sizeof(float4) * P) == cudaSuccess &&
-              cudaMalloc(&w.meta, sizeof(uint4) * P) == cudaSuccess && cudaMalloc(&w.branch, sizeof(uint2) * P) == cudaSuccess &&
-              cudaMalloc(&w.rad, sizeof(float4) * P) == cudaSuccess && cudaMalloc(&w.hit, sizeof(uint2) * P) == cudaSuccess &&
-              cudaMalloc(&w.state, sizeof(uint32_t) * P) == cudaSuccess && cudaMalloc(&w.item, sizeof(uint32_t) * P) == cudaSuccess &&
-              cudaMalloc(&w.ncount, sizeof(uint32_t) * P) == cudaSuccess && cudaMalloc(&w.sray0, sizeof(float4) * R) == cudaSuccess &&
-              cudaMalloc(&w.sray1, sizeof(float4) * R) == cudaSuccess && cudaMalloc(&w.scontrib, sizeof(float4) * R) == cudaSuccess &&
-              cudaMalloc(&w.svis, R) == cudaSuccess && cudaMalloc(&s->extendQ, sizeof(uint32_t) * kOctants * P) == cudaSuccess &&
-              cudaMalloc(&s->shadowQ, sizeof(uint32_t) * R) == cudaSuccess && cudaMalloc(&s->shadeQ, sizeof(uint32_t) * 3 * P) == cudaSuccess &&
-              cudaMalloc(&w.lightJob, sizeof(uint4) * kLightJobWords * P) == cudaSuccess &&
-              cudaMalloc(&w.lightFlags, sizeof(uint32_t) * P) == cudaSuccess;
-    if (ok && !s->waveCounters) ok = cudaMalloc(&s->waveCounters, sizeof(uint32_t) * kWaveCounters) == cudaSuccess;
-    if (ok && !s->claimed) ok = cudaMalloc(&s->claimed, sizeof(unsigned long long)) == cudaSuccess;
-    if (ok && !s->hostLast) ok = cudaMallocHost(&s->hostLast, sizeof(uint32_t) * 4) == cudaSuccess;
-    if (ok && !s->drainWords) ok = cudaMalloc(&s->drainWords, sizeof(uint32_t) * 4) == cudaSuccess;
-    if (ok && !s->hostDrain) ok = cudaMallocHost(&s->hostDrain, sizeof(uint32_t) * 4) == cudaSuccess;
+    auto place = [&](Carve& m) {
+        m.take(w.ray0, P), m.take(w.ray1, P), m.take(w.T, P), m.take(w.held, P), m.take(w.meta, P), m.take(w.branch, P), m.take(w.rad, P);
+        m.take(w.hit, P), m.take(w.state, P), m.take(w.item, P), m.take(w.ncount, P), m.take(w.sray0, R), m.take(w.sray1, R);
+        m.take(w.scontrib, R), m.take(w.svis, R), m.take(s->extendQ, kOctants * P), m.take(s->shadowQ, R), m.take(s->shadeQ, 3 * P);
+        m.take(w.lightJob, kLightJobWords * P), m.take(w.lightFlags, P);
+    };
+    bool ok = carve(&s->waveMemory, place);
+    if (ok && !s->deviceWords) ok = carve(&s->deviceWords, [&](Carve& m) {
+        m.take(s->waveCounters, kWaveCounters), m.take(s->claimed, 1), m.take(s->drainWords, 4), m.take(s->pairWords, 4);
+    });
+    if (ok && !s->hostWords) {
+        ok = cudaMallocHost(&s->hostWords, sizeof(uint32_t) * 12) == cudaSuccess;
+        if (ok) {
+            std::memset(s->hostWords, 0, sizeof(uint32_t) * 12);
+            s->hostLast = s->hostWords;
+            s->hostDrain = s->hostWords + 4;
+            s->hostPairWords = s->hostWords + 8;
+        }
+    }
     if (!ok) {
+        cudaGetLastError();
         freeWave(s);
         setError("device allocation failed for %u wavefront paths", paths);
         return X2_ENOMEM;
@@ -411,8 +462,8 @@ int ensureWave(x2_scene* s, uint32_t paths, uint32_t records) {
 
 void freeVolumeWave(x2_scene* s) {
     x2::VolumeWave& v = s->vol;
-    void* ptrs[] = {v.head, v.pass, v.light, v.parts, v.crossings, v.checkpoints, v.branch, v.queue};
-    for (void* p : ptrs) cudaFree(p);
+    cudaFree(s->volMemory);
+    s->volMemory = nullptr;
     v = x2::VolumeWave{};
     s->volPaths = s->volRecords = s->volTasks = 0;
 }
@@ -439,12 +490,11 @@ bool volumesApart(x2_scene* s, uint32_t paths, uint32_t records) {
     freeVolumeWave(s);
     x2::VolumeWave& v = s->vol;
     const size_t P = paths;
-    if (cudaMalloc(&v.head, sizeof(x2::VolumeHead) * P) != cudaSuccess || cudaMalloc(&v.pass, sizeof(float4) * P) != cudaSuccess ||
-        cudaMalloc(&v.light, sizeof(float4) * P) != cudaSuccess ||
-        cudaMalloc(&v.parts, sizeof(float4) * 2 * P * std::max<uint64_t>(tasks, 1)) != cudaSuccess ||
-        cudaMalloc(&v.crossings, sizeof(x2::Crossing) * x2::kMaxCrossings * P) != cudaSuccess ||
-        cudaMalloc(&v.checkpoints, sizeof(x2::MarchCheckpoint) * x2::kVolumeCheckpoints * P) != cudaSuccess ||
-        cudaMalloc(&v.branch, sizeof(uint2) * records * P) != cudaSuccess || cudaMalloc(&v.queue, sizeof(uint32_t) * P) != cudaSuccess) {
+    if (!carve(&s->volMemory, [&](Carve& m) {
+            m.take(v.head, P), m.take(v.pass, P), m.take(v.light, P), m.take(v.parts, 2 * P * std::max<uint64_t>(tasks, 1));
+            m.take(v.crossings, x2::kMaxCrossings * P), m.take(v.checkpoints, x2::kVolumeCheckpoints * P), m.take(v.branch, records * P);
+            m.take(v.queue, P);
+        })) {
         cudaGetLastError();  // not enough memory: the form that needs none
         freeVolumeWave(s);
         return false;
@@ -635,6 +685,7 @@ int x2_close(x2_ctx* ctx) {
         cudaEventDestroy(ctx->side.join[j]);
     }
     cudaEventDestroy(ctx->side.fork);
+    cudaFree(ctx->scratch);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
     return X2_OK;
@@ -1021,17 +1072,15 @@ int x2_scene_free(x2_scene* s) {
     cudaFree(s->grids);
     for (float* g : s->gridValues) cudaFree(g);
     for (float* m : s->majorants) cudaFree(m);
+    s->frameGraph.drop();
+    s->pairGraph.drop();
+    s->adaptiveGraph.drop();
     freeWave(s);
     freeVolumeWave(s);
     cudaFree(s->out);
     cudaFree(s->outStatus);
-    cudaFree(s->extendQ);
-    cudaFree(s->shadowQ);
-    cudaFree(s->waveCounters);
-    cudaFree(s->claimed);
-    if (s->hostLast) cudaFreeHost(s->hostLast);
-    cudaFree(s->drainWords);
-    if (s->hostDrain) cudaFreeHost(s->hostDrain);
+    cudaFree(s->deviceWords);
+    if (s->hostWords) cudaFreeHost(s->hostWords);
     cudaFree(s->sums);
     cudaFree(s->odd);
     cudaFree(s->counts);
@@ -1040,8 +1089,6 @@ int x2_scene_free(x2_scene* s) {
     cudaFree(s->stepLists);
     cudaFree(s->pairOut);
     cudaFree(s->pairStatus);
-    cudaFree(s->pairWords);
-    if (s->hostPairWords) cudaFreeHost(s->hostPairWords);
     if (s->staging) cudaFreeHost(s->staging);
     delete s;
     return X2_OK;
@@ -1097,6 +1144,7 @@ namespace {
 // A single scene's wavefront launch of `count` chunks (sl.chunks) and `items` items over `paths` path slots.
 WaveArgs launchArgs(x2_scene* s, Slot& sl, uint32_t paths, uint32_t records, unsigned long long items, uint32_t count) {
     WaveArgs a;
+    std::memset(static_cast<void*>(&a), 0, sizeof(a));  // its padding too: launches are compared by their bytes
     if (volumesApart(s, paths, records)) {
         a.vol = s->vol;
         a.vol.count = s->waveCounters + kWaveCounters - 1;
@@ -1147,9 +1195,27 @@ WaveKernels launchKernels(const x2_scene* s, const WaveArgs& a) {
 // A launch as one graph on the context's stream: its iterations (what iteration() enqueues) in a conditional while node,
 // each iteration's last kernel deciding whether another follows (at most `bound`; past that it raises words[2]), then what
 // tail() enqueues. words: 4 device words, cleared here.
+// A launch whose key (everything its kernels are launched with) is the last one's launches that one's graph again: building
+// and instantiating one takes the host about 0.2 ms.
+struct DrainKey {
+    WaveKernels kernels;
+    WaveArgs args;
+    WaveGrids grids;
+    uint32_t bound, tail;
+    const void* out[3];
+};
 int launchDrain(x2_ctx* ctx, const WaveArgs& a, uint32_t* words, uint32_t bound, const char* what, const std::function<void()>& iteration,
-                const std::function<void()>& tail) {
+                const std::function<void()>& tail, KeptGraph* kept = nullptr, const DrainKey* key = nullptr) {
     cudaStream_t st = ctx->stream;
+    if (kept && kept->exec && kept->key.size() == sizeof(*key) && !std::memcmp(kept->key.data(), key, sizeof(*key))) {
+        cudaMemsetAsync(words, 0, sizeof(uint32_t) * 4, st);
+        const cudaError_t again = cudaGraphLaunch(kept->exec, st);
+        if (again != cudaSuccess) {
+            setError("%s: graph launch failed: %s", what, cudaGetErrorString(again));
+            return X2_ECUDA;
+        }
+        return X2_OK;
+    }
     cudaGraph_t graph = nullptr;
     CUDA_OR(cudaGraphCreate(&graph, 0), X2_ECUDA);
     cudaError_t err = cudaSuccess;
@@ -1190,12 +1256,66 @@ int launchDrain(x2_ctx* ctx, const WaveArgs& a, uint32_t* words, uint32_t bound,
     }
     cudaMemsetAsync(words, 0, sizeof(uint32_t) * 4, st);
     const cudaError_t launched = cudaGraphLaunch(exec, st);
-    cudaGraphExecDestroy(exec);  // released once the launch completes
+    if (kept && launched == cudaSuccess) {
+        if (kept->exec) cudaGraphExecDestroy(kept->exec);  // released once its last launch completes
+        kept->exec = exec;
+        kept->key.assign(reinterpret_cast<const unsigned char*>(key), reinterpret_cast<const unsigned char*>(key) + sizeof(*key));
+    } else {
+        cudaGraphExecDestroy(exec);
+    }
     if (launched != cudaSuccess) {
         setError("%s: graph launch failed: %s", what, cudaGetErrorString(launched));
         return X2_ECUDA;
     }
     return X2_OK;
+}
+// The key of a launch, its padding zero.
+DrainKey drainKey(const WaveKernels& k, const WaveArgs& a, const WaveGrids& g, uint32_t bound, uint32_t tail, const void* o0, const void* o1,
+                  const void* o2) {
+    DrainKey key;
+    std::memset(static_cast<void*>(&key), 0, sizeof(key));
+    key.kernels = k;
+    key.args = a;
+    key.grids = g;
+    key.bound = bound;
+    key.tail = tail;
+    key.out[0] = o0;
+    key.out[1] = o1;
+    key.out[2] = o2;
+    return key;
+}
+
+// Device memory for a host caller's arrays during one call: the context keeps one piece of at most kCallScratch bytes (a
+// scene's first call then allocates nothing), lent to one call at a time; a call that finds it lent or too small
+// allocates its own, and leaves it in place of a smaller one (dropScratch, once the call has waited).
+constexpr size_t kCallScratch = 64u << 20;
+unsigned char* callScratch(x2_ctx* ctx, size_t bytes) {
+    {
+        std::lock_guard<std::mutex> lock(ctx->scratchMutex);
+        if (!ctx->scratchLent && bytes <= ctx->scratchBytes) {
+            ctx->scratchLent = true;
+            return ctx->scratch;
+        }
+    }
+    unsigned char* p = nullptr;
+    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        setError("device allocation failed for a call's %zu bytes", bytes);
+        return nullptr;
+    }
+    return p;
+}
+void dropScratch(x2_ctx* ctx, unsigned char* p, size_t bytes) {
+    std::lock_guard<std::mutex> lock(ctx->scratchMutex);
+    if (p == ctx->scratch) {
+        ctx->scratchLent = false;
+    } else if (!ctx->scratchLent && bytes <= kCallScratch && bytes > ctx->scratchBytes) {
+        cudaFree(ctx->scratch);
+        ctx->scratch = p;
+        ctx->scratchBytes = bytes;
+    } else {
+        cudaFree(p);
+    }
 }
 
 // What a launch's path slots and queues must start with.
@@ -1245,11 +1365,6 @@ int integrateWavefront(x2_scene* s, uint32_t paths, const uint32_t* pairs, uint6
         }
         s->pairCap = window;
     }
-    if (!s->pairWords) CUDA_OR(cudaMalloc(&s->pairWords, sizeof(uint32_t) * 4), X2_ENOMEM);
-    if (!s->hostPairWords) {
-        CUDA_OR(cudaMallocHost(&s->hostPairWords, sizeof(uint32_t) * 4), X2_ENOMEM);
-        std::memset(s->hostPairWords, 0, sizeof(uint32_t) * 4);
-    }
     cudaStream_t st = s->ctx->stream;
     const WaveGrids grids = waveGrids(paths, records, s->ctx->smCount, s->blocksPerSm);
     for (uint64_t first = 0; first < n; first += window) {
@@ -1261,10 +1376,12 @@ int integrateWavefront(x2_scene* s, uint32_t paths, const uint32_t* pairs, uint6
         a.outStatus = s->pairStatus;
         const uint64_t bound = uint64_t(items) * (uint64_t(s->config.max_depth) + 2) / paths + uint64_t(s->config.max_depth) + 64;
         const WaveKernels wk = launchKernels(s, a);
-        const int done = launchDrain(s->ctx, a, s->pairWords, uint32_t(std::min<uint64_t>(bound, 0xffffffffu)), "x2_integrate",
+        const uint32_t most = uint32_t(std::min<uint64_t>(bound, 0xffffffffu));
+        const DrainKey key = drainKey(wk, a, grids, most, items, rgba + 4 * first, status + first, nullptr);
+        const int done = launchDrain(s->ctx, a, s->pairWords, most, "x2_integrate",
                                      [&] { launchIteration(wk, a, grids, st, false, &s->ctx->side); }, [&] {
             wfPairsOut<<<(items + 255) / 256, 256, 0, st>>>(s->pairOut, s->pairStatus, items, rgba + 4 * first, status + first);
-        });
+        }, &s->pairGraph, &key);
         if (done) return done;
         // A window that did not drain keeps its word until the caller waits.
         if (first == 0 || !s->hostPairWords[2])
@@ -1313,21 +1430,18 @@ int x2_integrate(x2_scene* s, const uint32_t* pairs, uint64_t n, double* rgba, u
         return X2_EINVAL;
     }
     cudaStream_t st = s->ctx->stream;
-    uint32_t *dPairs = nullptr, *dStatus = nullptr;
-    double* dRgba = nullptr;
-    CUDA_OR(cudaMallocAsync(&dPairs, sizeof(uint32_t) * 2 * n, st), X2_ENOMEM);
-    CUDA_OR(cudaMallocAsync(&dRgba, sizeof(double) * 4 * n, st), X2_ENOMEM);
-    CUDA_OR(cudaMallocAsync(&dStatus, sizeof(uint32_t) * n, st), X2_ENOMEM);
+    unsigned char* scratch = callScratch(s->ctx, 44 * n);
+    if (!scratch) return X2_ENOMEM;
+    double* dRgba = reinterpret_cast<double*>(scratch);
+    uint32_t *dPairs = reinterpret_cast<uint32_t*>(dRgba + 4 * n), *dStatus = dPairs + 2 * n;
     cudaMemcpyAsync(dPairs, pairs, sizeof(uint32_t) * 2 * n, cudaMemcpyHostToDevice, st);
     int rc = x2_integrate_device(s, dPairs, n, dRgba, dStatus);
     if (rc == X2_OK) {
         cudaMemcpyAsync(rgba, dRgba, sizeof(double) * 4 * n, cudaMemcpyDeviceToHost, st);
         cudaMemcpyAsync(status, dStatus, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, st);
     }
-    cudaFreeAsync(dPairs, st);
-    cudaFreeAsync(dRgba, st);
-    cudaFreeAsync(dStatus, st);
     const int w = x2_synchronize(s->ctx, 600000);
+    dropScratch(s->ctx, scratch, 44 * n);
     if (rc == X2_OK && w == X2_OK && s->integrateSlot.busy) {
         accumulate(s->total, *s->integrateSlot.hostCounters);
         s->integrateSlot.busy = false;
@@ -1367,12 +1481,10 @@ int x2_trace_rays(x2_scene* s, const float* rays, uint64_t n, uint32_t* tri, flo
         return X2_EINVAL;
     }
     cudaStream_t st = s->ctx->stream;
-    float *dRays = nullptr, *dT = nullptr;
-    uint32_t *dTri = nullptr, *dOcc = nullptr;
-    CUDA_OR(cudaMallocAsync(&dRays, sizeof(float) * 8 * n, st), X2_ENOMEM);
-    CUDA_OR(cudaMallocAsync(&dT, sizeof(float) * n, st), X2_ENOMEM);
-    CUDA_OR(cudaMallocAsync(&dTri, sizeof(uint32_t) * n, st), X2_ENOMEM);
-    CUDA_OR(cudaMallocAsync(&dOcc, sizeof(uint32_t) * n, st), X2_ENOMEM);
+    unsigned char* scratch = callScratch(s->ctx, 44 * n);
+    if (!scratch) return X2_ENOMEM;
+    float *dRays = reinterpret_cast<float*>(scratch), *dT = dRays + 8 * n;
+    uint32_t *dTri = reinterpret_cast<uint32_t*>(dT + n), *dOcc = dTri + n;
     cudaMemcpyAsync(dRays, rays, sizeof(float) * 8 * n, cudaMemcpyHostToDevice, st);
     const int rc = x2_trace_rays_device(s, dRays, n, dTri, dT, dOcc);
     if (rc == X2_OK) {
@@ -1380,11 +1492,8 @@ int x2_trace_rays(x2_scene* s, const float* rays, uint64_t n, uint32_t* tri, flo
         cudaMemcpyAsync(t, dT, sizeof(float) * n, cudaMemcpyDeviceToHost, st);
         cudaMemcpyAsync(occluded, dOcc, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, st);
     }
-    cudaFreeAsync(dRays, st);
-    cudaFreeAsync(dT, st);
-    cudaFreeAsync(dTri, st);
-    cudaFreeAsync(dOcc, st);
     const int w = x2_synchronize(s->ctx, 600000);
+    dropScratch(s->ctx, scratch, 44 * n);
     return rc ? rc : w;
 }
 
@@ -1733,15 +1842,17 @@ int x2_launch_wavefront(x2_scene* s, const x2_chunk* chunks, uint32_t count) {
         s->waveIterations = iterations;
         return X2_OK;
     }
-    // One graph: the launch's iterations, then the film reduce. The launch runs without the host; x2_poll / x2_wait
+    // One graph, kept for the next launch like it: the launch's iterations, then the film reduce. The launch runs without the host; x2_poll / x2_wait
     // collect it like any launch.
     const uint32_t bound = uint32_t(std::min<uint64_t>(maxIter, 0xffffffffu));
     cudaEventRecord(sl.begin, st);
+    const DrainKey key = drainKey(wk, a, grids, bound, count, s->sums, s->adaptive ? s->odd : nullptr, s->counts);
     if (int rc = launchDrain(s->ctx, a, s->drainWords, bound, "x2_launch_wavefront", [&] { launchIteration(wk, a, grids, st, false, &s->ctx->side); },
                              [&] {
                                  wfFilmReduce<<<int((64ull * count + 255) / 256), 256, 0, st>>>(
                                      a, count, s->sums, s->adaptive ? s->odd : nullptr, s->counts);
-                             }))
+                             },
+                             &s->frameGraph, &key))
         return rc;
     cudaEventRecord(sl.end, st);
     // The extend kernels counted the traced rays; the launch's counters go to the host as x2_launch's do, with the
@@ -1828,7 +1939,7 @@ int x2_scene_set_texture(x2_scene* s, uint32_t texture, const float* rgb) {
     if (int rc = x2_wait(s, 600000, nullptr)) return rc;
     const TexRec& t = s->hostTextures[texture];
     cudaStream_t st = s->ctx->stream;
-    CUDA_OR(cudaMemcpyAsync(s->texels + 3 * t.first, rgb, sizeof(float) * 3 * size_t(t.width) * t.height, cudaMemcpyHostToDevice, st), X2_ECUDA);
+    CUDA_OR(cudaMemcpyAsync(s->texels + 3 * t.first, rgb, sizeof(float) * 3 * size_t(t.width) * t.height, cudaMemcpyDefault, st), X2_ECUDA);
     CUDA_OR(cudaStreamSynchronize(st), X2_ECUDA);
     return X2_OK;
 }
@@ -2360,75 +2471,97 @@ int renderAdaptive(x2_scene* s, uint32_t minSamples, uint32_t maxSamples, float 
     const uint64_t bound = maxItems * (uint64_t(s->config.max_depth) + 2) / paths + uint64_t(s->config.max_depth) + 64;
     const uint32_t maxIter = uint32_t(std::min<uint64_t>(bound, 0xffffffffu));
 
-    // The graph, built in segments: each captured onto the graph after the last segment's end nodes.
-    GraphSegments g;
-    g.st = st;
-    CUDA_OR(cudaGraphCreate(&g.graph, 0), X2_ECUDA);
-    const uint32_t pixels = ad.width * ad.height;
-    const int compactBlocks = int((ad.tiles + x2::kCompactBlock - 1) / x2::kCompactBlock);
-    for (size_t k = 0; k < passes.size() && g.err == cudaSuccess; ++k) {
-        const uint32_t size = passes[k].second - passes[k].first;
-        const uint32_t uniform = passes[k].first < minSamples ? 1u : 0u;
-        a.samplesPerChunk = size;
-        a.itemCount = (unsigned long long)ad.tiles * 64ull * size;
-        x2::AdaptiveArgs pass = chain;
-        if (!uniform) {
-            if (!g.begin(g.graph, true)) break;
-            x2::chainPixelErrors<<<(pixels + 255) / 256, 256, 0, st>>>(chain, s->sums, s->odd, s->counts);
-            if (cellular) {
-                // The next generation from the film so far; the pass's masks come from it.
-                const uint8_t* aliveIn = ad.alive + size_t(generation % 2) * ad.tiles;
-                uint8_t* aliveOut = ad.alive + size_t((generation + 1) % 2) * ad.tiles;
-                ++generation;
-                cudaMemsetAsync(chain.liveTiles, 0, sizeof(uint32_t), st);
-                x2::tileRatios<<<(ad.tiles + 255) / 256, 256, 0, st>>>(chain);
-                x2::nextGeneration<<<(ad.tiles + 255) / 256, 256, 0, st>>>(chain, aliveIn, aliveOut);
-                pass.alive = aliveOut;
-            }
-            g.check(cudaGetLastError());
-            if (!g.end(true)) break;
-            if (!cellular && !appendTrees(g, chain, ad, s->ctx->smCount)) break;
-        }
-        if (!g.begin(g.graph, true)) break;
-        x2::tileMasks<<<(ad.tiles + 255) / 256, 256, 0, st>>>(pass, uniform, size);
-        x2::compactCount<<<compactBlocks, x2::kCompactBlock, 0, st>>>(chain);
-        x2::compactWrite<<<compactBlocks, x2::kCompactBlock, 0, st>>>(chain, size);
-        cudaMemsetAsync(s->wave.state, 0, sizeof(uint32_t) * paths, st);
-        cudaMemsetAsync(s->wave.ncount, 0, sizeof(uint32_t) * paths, st);
-        cudaMemsetAsync(s->claimed, 0, sizeof(unsigned long long), st);
-        cudaMemsetAsync(s->waveCounters, 0, sizeof(uint32_t) * kWaveCounters, st);
-        cudaMemsetAsync(s->outStatus, X2_SKIP, a.itemCount, st);
-        cudaMemsetAsync(ad.words + 2, 0, sizeof(uint32_t), st);
-        g.check(cudaGetLastError());
-        if (!g.end(true)) break;
-        // The pass's drain: a while node whose body is one iteration and the test that decides the next.
-        cudaGraphConditionalHandle loop;
-        cudaGraph_t body = g.whileNode(&loop);
-        if (!body || !g.begin(body, false)) break;
-        launchIteration(wk, a, grids, st, false, &s->ctx->side);
-        wfDrainCheck<<<1, 32, 0, st>>>(a, loop, ad.words + 2, maxIter, ad.words + 4);
-        g.check(cudaGetLastError());
-        if (!g.end(false)) break;
-        if (!g.begin(g.graph, true)) break;
-        wfFilmReduce<<<int((64ull * ad.tiles + 255) / 256), 256, 0, st>>>(a, ad.tiles, s->sums, s->odd, s->counts);
-        g.check(cudaGetLastError());
-        g.end(true);
-    }
-    cudaError_t err = g.err;
+    // The frame's graph, kept for the next frame like it (a frame's worth of passes is some hundred nodes to build and
+    // instantiate).
+    struct AdaptiveKey {
+        DrainKey drain;
+        x2::AdaptiveArgs chain;
+        uint32_t minSamples, maxSamples, cellular;
+    };
+    AdaptiveKey key;
+    std::memset(static_cast<void*>(&key), 0, sizeof(key));
+    key.drain = drainKey(wk, a, grids, maxIter, most, s->sums, s->odd, s->counts);
+    key.chain = chain;
+    key.minSamples = minSamples;
+    key.maxSamples = maxSamples;
+    key.cellular = cellular ? 1 : 0;
+    KeptGraph& kept = s->adaptiveGraph;
+    cudaError_t err = cudaSuccess;
     auto check = [&](cudaError_t e) {
         if (err == cudaSuccess && e != cudaSuccess) err = e;
         return err == cudaSuccess;
     };
-    cudaGraph_t graph = g.graph;
-    cudaGraphExec_t exec = nullptr;
-    if (err == cudaSuccess) check(cudaGraphInstantiate(&exec, graph, 0));
-    cudaGraphDestroy(graph);
-    if (err != cudaSuccess) {
-        setError("x2_render_adaptive: building the frame's graph: %s", cudaGetErrorString(err));
-        return X2_ECUDA;
+    const bool again = kept.exec && kept.key.size() == sizeof(key) && !std::memcmp(kept.key.data(), &key, sizeof(key));
+    if (!again) {
+        kept.drop();
+        // Built in segments: each captured onto the graph after the last segment's end nodes.
+        GraphSegments g;
+        g.st = st;
+        CUDA_OR(cudaGraphCreate(&g.graph, 0), X2_ECUDA);
+        const uint32_t pixels = ad.width * ad.height;
+        const int compactBlocks = int((ad.tiles + x2::kCompactBlock - 1) / x2::kCompactBlock);
+        for (size_t k = 0; k < passes.size() && g.err == cudaSuccess; ++k) {
+            const uint32_t size = passes[k].second - passes[k].first;
+            const uint32_t uniform = passes[k].first < minSamples ? 1u : 0u;
+            a.samplesPerChunk = size;
+            a.itemCount = (unsigned long long)ad.tiles * 64ull * size;
+            x2::AdaptiveArgs pass = chain;
+            if (!uniform) {
+                if (!g.begin(g.graph, true)) break;
+                x2::chainPixelErrors<<<(pixels + 255) / 256, 256, 0, st>>>(chain, s->sums, s->odd, s->counts);
+                if (cellular) {
+                    // The next generation from the film so far; the pass's masks come from it.
+                    const uint8_t* aliveIn = ad.alive + size_t(generation % 2) * ad.tiles;
+                    uint8_t* aliveOut = ad.alive + size_t((generation + 1) % 2) * ad.tiles;
+                    ++generation;
+                    cudaMemsetAsync(chain.liveTiles, 0, sizeof(uint32_t), st);
+                    x2::tileRatios<<<(ad.tiles + 255) / 256, 256, 0, st>>>(chain);
+                    x2::nextGeneration<<<(ad.tiles + 255) / 256, 256, 0, st>>>(chain, aliveIn, aliveOut);
+                    pass.alive = aliveOut;
+                }
+                g.check(cudaGetLastError());
+                if (!g.end(true)) break;
+                if (!cellular && !appendTrees(g, chain, ad, s->ctx->smCount)) break;
+            }
+            if (!g.begin(g.graph, true)) break;
+            x2::tileMasks<<<(ad.tiles + 255) / 256, 256, 0, st>>>(pass, uniform, size);
+            x2::compactCount<<<compactBlocks, x2::kCompactBlock, 0, st>>>(chain);
+            x2::compactWrite<<<compactBlocks, x2::kCompactBlock, 0, st>>>(chain, size);
+            cudaMemsetAsync(s->wave.state, 0, sizeof(uint32_t) * paths, st);
+            cudaMemsetAsync(s->wave.ncount, 0, sizeof(uint32_t) * paths, st);
+            cudaMemsetAsync(s->claimed, 0, sizeof(unsigned long long), st);
+            cudaMemsetAsync(s->waveCounters, 0, sizeof(uint32_t) * kWaveCounters, st);
+            cudaMemsetAsync(s->outStatus, X2_SKIP, a.itemCount, st);
+            cudaMemsetAsync(ad.words + 2, 0, sizeof(uint32_t), st);
+            g.check(cudaGetLastError());
+            if (!g.end(true)) break;
+            // The pass's drain: a while node whose body is one iteration and the test that decides the next.
+            cudaGraphConditionalHandle loop;
+            cudaGraph_t body = g.whileNode(&loop);
+            if (!body || !g.begin(body, false)) break;
+            launchIteration(wk, a, grids, st, false, &s->ctx->side);
+            wfDrainCheck<<<1, 32, 0, st>>>(a, loop, ad.words + 2, maxIter, ad.words + 4);
+            g.check(cudaGetLastError());
+            if (!g.end(false)) break;
+            if (!g.begin(g.graph, true)) break;
+            wfFilmReduce<<<int((64ull * ad.tiles + 255) / 256), 256, 0, st>>>(a, ad.tiles, s->sums, s->odd, s->counts);
+            g.check(cudaGetLastError());
+            g.end(true);
+        }
+        err = g.err;
+        cudaGraph_t graph = g.graph;
+        if (err == cudaSuccess) check(cudaGraphInstantiate(&kept.exec, graph, 0));
+        cudaGraphDestroy(graph);
+        if (err != cudaSuccess) {
+            kept.exec = nullptr;
+            setError("x2_render_adaptive: building the frame's graph: %s", cudaGetErrorString(err));
+            return X2_ECUDA;
+        }
+        const unsigned char* bytes = reinterpret_cast<const unsigned char*>(&key);
+        kept.key.assign(bytes, bytes + sizeof(key));
     }
     cudaEventRecord(sl.begin, st);
-    check(cudaGraphLaunch(exec, st));
+    check(cudaGraphLaunch(kept.exec, st));
     cudaEventRecord(sl.end, st);
     cudaMemcpyAsync(sl.hostCounters, sl.counters, sizeof(Counters), cudaMemcpyDeviceToHost, st);
     cudaMemcpyAsync(ad.hostWords, ad.words, sizeof(uint32_t) * 8, cudaMemcpyDeviceToHost, st);
@@ -2439,7 +2572,6 @@ int renderAdaptive(x2_scene* s, uint32_t minSamples, uint32_t maxSamples, float 
     sl.seq = s->nextSeq++;
     s->lastItems = 0;  // the passes' per-item outputs are not kept
     int rc = x2_synchronize(s->ctx, 600000);
-    cudaGraphExecDestroy(exec);
     if (err != cudaSuccess) {
         setError("x2_render_adaptive: graph launch failed: %s", cudaGetErrorString(err));
         return X2_ECUDA;

@@ -510,7 +510,11 @@ class Scene:
         _check(library().x2_scene_set_params(self._h, _ptr(a), _ptr(g), _ptr(r)))
 
     def set_texture(self, texture, rgb):
-        """x2_scene_set_texture: texture `texture`'s texels (height x width x 3 floats) set in place."""
+        """x2_scene_set_texture: texture `texture`'s texels (height x width x 3 floats) set in place; a contiguous float32
+        CUDA tensor on the context's device is copied there, without a way through the host (its stream must be idle)."""
+        if getattr(rgb, "is_cuda", False):
+            _check(library().x2_scene_set_texture(self._h, texture, C.c_void_p(rgb.data_ptr())))
+            return
         a = np.ascontiguousarray(rgb, np.float32)
         _check(library().x2_scene_set_texture(self._h, texture, _ptr(a)))
 

@@ -7,7 +7,6 @@ identity and credits each contribution to the light it reached, the Lambert vert
 read) and the GGX vertices it passed. The adjoint takes its own samples (`adjoint_first`, `adjoint_count`),
 decorrelated from the primal's unless the caller picks the same ones.
 """
-import numpy as np
 import torch
 
 
@@ -20,17 +19,24 @@ class Render(torch.autograd.Function):
     def forward(ctx, albedo, radiance, roughness, texture, scene, first, count, adjoint_first, adjoint_count):
         scene.set_params(_host(albedo), _host(radiance), _host(roughness))
         if texture is not None:
-            scene.set_texture(0, _host(texture))
+            # Texels that already lie on the scene's device as the library keeps them go there directly.
+            here = texture.is_cuda and texture.device.index == scene.ctx.device and texture.dtype == torch.float32
+            if here:
+                texels = texture.detach().contiguous()
+                torch.cuda.current_stream(texels.device).synchronize()
+            scene.set_texture(0, texels if here else _host(texture))
         scene.frame_begin(count)
         scene.render_frame_wavefront(first, count)
         scene.wait()
-        sums, counts = scene.film()
         cfg = scene.config
-        image = (sums[:, :3] / np.maximum(counts, 1)[:, None]).reshape(cfg.height, cfg.width, 3)
+        # The film's mean where the film lies: its FP64 sums over its counts, rounded to float as on the host.
+        sums, _, counts = scene.film_tensors()
+        image = (sums[:, :3] / counts.clamp(min=1)[:, None]).to(torch.float32).reshape(cfg.height, cfg.width, 3)
+        torch.cuda.current_stream(image.device).synchronize()  # before the library's stream may write the film again
         ctx.scene = scene
         ctx.adjoint = (adjoint_first, adjoint_count)
         ctx.params = [(p.shape, p.dtype, p.device) if p is not None else None for p in (albedo, radiance, roughness, texture)]
-        return torch.from_numpy(image.astype(np.float32)).to(albedo.device)
+        return image.to(albedo.device)
 
     @staticmethod
     def backward(ctx, grad_image):
