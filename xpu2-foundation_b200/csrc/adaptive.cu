@@ -60,6 +60,8 @@ __global__ void treeRoots(AdaptiveArgs a) {
     }
 }
 
+constexpr int kTableAhead = 8;
+
 // Row y of region r: its running error sums left to right (in double, as the table keeps them) into table row y + 1;
 // the thread of row 0 also clears table row 0. A pixel without both halves marks its region not ready.
 __global__ void tableRows(AdaptiveArgs a) {
@@ -77,10 +79,18 @@ __global__ void tableRows(AdaptiveArgs a) {
     bool missing = false;
     double run = 0.0;
     out[0] = 0.0;
-    for (int x = 0; x < w; ++x) {
-        missing |= e[x] < 0.0f;
-        run += double(e[x]);
-        out[x + 1] = run;
+    // Eight errors fetched at once, added in their order: one at a time each waited for its own load behind the store.
+    for (int x = 0; x < w; x += kTableAhead) {
+        float v[kTableAhead];
+#pragma unroll
+        for (int k = 0; k < kTableAhead; ++k) v[k] = x + k < w ? e[x + k] : 0.0f;
+#pragma unroll
+        for (int k = 0; k < kTableAhead; ++k)
+            if (x + k < w) {
+                missing |= v[k] < 0.0f;
+                run += double(v[k]);
+                out[x + k + 1] = run;
+            }
     }
     if (missing) a.regions.ready[r] = 0;
 }
@@ -95,9 +105,16 @@ __global__ void tableColumns(AdaptiveArgs a) {
     const int x = int(i - a.regions.colStart[r]) + 1, w1 = b[2] - b[0] + 1, h = b[3] - b[1];
     double* col = a.sat + a.regions.satOffset[r] + x;
     double run = col[w1];
-    for (int y = 2; y <= h; ++y) {
-        run += col[size_t(y) * size_t(w1)];
-        col[size_t(y) * size_t(w1)] = run;
+    for (int y = 2; y <= h; y += kTableAhead) {
+        double v[kTableAhead];
+#pragma unroll
+        for (int k = 0; k < kTableAhead; ++k) v[k] = y + k <= h ? col[size_t(y + k) * size_t(w1)] : 0.0;
+#pragma unroll
+        for (int k = 0; k < kTableAhead; ++k)
+            if (y + k <= h) {
+                run += v[k];
+                col[size_t(y + k) * size_t(w1)] = run;
+            }
     }
 }
 

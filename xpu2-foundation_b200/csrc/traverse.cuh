@@ -2,9 +2,9 @@
 //
 // A node is five 16-byte read-only loads. Its eight children are tested with one FMA a slab (Ylitie et al. 2017:
 // the ray is expressed in the node's quantised frame once, t = q * (2^e / d) + (p - o) / d, two slabs an instruction),
-// widened by a bound on the roundings so the quantised boxes stay conservative (visitNode). Hit children enter a 32-bit mask: internal
-// children on bits 24..31 in near-to-far order for the ray's octant (the build places each child in the slot of
-// the octant it lies toward), leaf triangles on bits 0..23. The stack holds (child base, mask | imask) pairs and
+// widened by a bound on the roundings so the quantised boxes stay conservative (visitNode). Hit children enter a 32-bit
+// mask: internal children on bits 24..31 in near-to-far order for the ray's octant (the build places each child in the
+// slot of the octant it lies toward), leaf triangles on bits 0..23. The stack holds (child base, mask | imask) pairs and
 // lives in registers/local memory; an overflow is counted, never silent.
 //
 // The triangle test is Woop, Benthin and Wald's watertight test in fp32 without contraction (the library is built
@@ -138,9 +138,11 @@ __device__ __forceinline__ void fma2(unsigned long long a, unsigned long long b,
 // One node: the hit mask (bits 24..31 internal children in traversal order, 0..23 leaf triangles), its child and
 // triangle bases and its internal-child mask.
 //
-// The traversals are bound by instruction issue (with the ALU pipe behind it), so the test is written for few
-// instructions: a child's near and far slab distances of an axis are one packed FMA, (2^15 + q) s + c with
-// s = 2^e * (1/d), a = (p - o) * (1/d) and c = a - 2^15 s -+ w, the byte placed in the float's mantissa by one permute.
+// The walks wait for their nodes at seven or eight warps a scheduler (shadow rays of the 12.3M-triangle field: issue slots
+// 70 % busy, the ALU pipe 59 %, L1's data path 46 %), with the test's instructions close behind, so it is written for
+// few of them (prefetching the next node into L1 cost 2 % of the shadow rays' time): a child's near and far slab
+// distances of an axis are one packed FMA, (2^15 + q) s + c with s = 2^e * (1/d), a = (p - o) * (1/d) and
+// c = a - 2^15 s -+ w, the byte placed in the float's mantissa by one permute.
 //
 // Conservative by construction: the quantised child boxes contain the exact ones (the build rounds outward), and every
 // slab is widened by w = 2^-20 L |1/d| + 2^-7 |s| each way, L the L1 distance from the ray's origin to the scene's
