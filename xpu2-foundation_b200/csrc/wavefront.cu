@@ -7,13 +7,16 @@
 //           claim a new sample for an empty slot (regeneration: a camera ray), and append every slot with a ray to
 //           trace to the extend queue (warp-aggregated atomics);
 //   extend  closest hit of every queued ray (traverse.cuh);
+//   (a scene with volumes: the rays' marches or walks and their scattering samples, kernels of their own);
 //   sort    the extended paths into per-lobe queues by their hit's material (GGX, Lambert, none or missed);
-//   shade   each queued path's vertex, the queues in that order (integrator.cuh shadeVertex): its shadow rays go to fixed per-path record slots
-//           and, by one warp-aggregated reservation a warp, to the shadow queue; its child becomes the slot's ray;
-//   shadow  any hit of every queued shadow ray, a visibility flag each.
-// Iterations are captured once as a CUDA graph and replayed until every item is done. The per-item output (rgb,
-// alpha, status) is then summed into the film in sample order by filmReduce, so the film does not depend on the
-// order paths finish in.
+//   shade   each queued path's vertex (integrator.cuh shadeVertex), a kernel a queue, its light samples in a kernel behind
+//           it: its shadow rays go to fixed per-path record slots and, by one warp-aggregated reservation a warp, to the
+//           shadow queue; its child becomes the slot's ray;
+//   shadow  any hit of every queued shadow ray, a visibility flag each (then, with volumes, the unoccluded rays'
+//           transmittance).
+// A launch is one CUDA graph whose iterations run in a conditional while node until every item is done (wfDrainCheck). The
+// per-item output (rgb, alpha, status) is then summed into the film in sample order by filmReduce, so the film does not
+// depend on the order paths finish in, or, for the per-sample entry's list of samples, handed out as it is (wfPairsOut).
 #include "credits.cuh"
 #include "wavefront.h"
 

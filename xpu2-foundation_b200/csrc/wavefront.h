@@ -6,9 +6,8 @@ namespace x2 {
 
 constexpr int kWaveBlock = 128;
 constexpr uint32_t kRecordSegments = 64;
-// Launch-shape defaults (x2_wavefront_tune changes them a scene). Paths in flight: 2^22 (each launch of the traversal
-// kernels then has four times the rays of 2^20 for the same ramp-down at its end: 145.3 -> 143.0 -> 155.4 ms for
-// 2^21, 2^22, 2^20 on config 1's 4096 tiles).
+// Launch-shape defaults (x2_wavefront_tune changes them a scene), the 12.3M-triangle frame's best: 2^23 paths in flight
+// 822.5 ms, 2^22 827.4; refill at 4 idle lanes 840.5, 6 824.4, 8 822.5, 12 835.7, 16 871.4; 32 blocks a SM 822.5, 16 828.3.
 constexpr uint32_t kDefaultPaths = 1u << 23;
 constexpr uint32_t kDefaultRefill = 8, kDefaultBlocksPerSm = 32, kDefaultTraceBlocks = 0, kDefaultShadeBlocks = 4,
                    kDefaultTriLimit = 1, kDefaultShadowOrder = 0, kDefaultExtendBins = 0, kDefaultShortStack = 1,
