@@ -1,6 +1,6 @@
 """The ray entry (x2_trace_rays: closest hit and occlusion, each ray's two queries walked apart) and the BVH build's cuts of
 the wide nodes, against every triangle tested in double precision: triangle counts about the sizes of a leaf and of a
-wide node, ray counts about a warp's."""
+wide node, ray counts about a warp's, and one beyond a lane for every query."""
 import ctypes as C
 
 import numpy as np
@@ -48,7 +48,7 @@ def every_triangle(v, o, d, far):
     return hit.min(1), hit.argmin(1), unclear
 
 
-@pytest.mark.parametrize("triangles,rays", [(1, 1), (2, 31), (3, 33), (4, 500), (5, 500), (8, 129), (9, 500), (24, 500), (25, 500), (300, 4097)])
+@pytest.mark.parametrize("triangles,rays", [(1, 1), (2, 31), (3, 33), (4, 500), (5, 500), (8, 129), (9, 500), (24, 500), (25, 500), (300, 4097), (5, 90001)])
 def test_rays_against_every_triangle(ctx, triangles, rays):
     scene, v = soup(ctx, triangles, 100 + triangles)
     rng = np.random.default_rng(triangles)

@@ -132,7 +132,7 @@ struct x2_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     int smCount = 0;
-    int renderBlocksPerSm = 0;
+    int renderBlocksPerSm = 0, rayBlocksPerSm = 0;
     x2::SideStreams side;  // for kernels of one iteration that run side by side
     std::mutex scratchMutex;
     unsigned char* scratch = nullptr;  // a host caller's arrays during x2_integrate or x2_trace_rays
@@ -672,6 +672,8 @@ int x2_open(int device, x2_ctx** out) {
     cudaDeviceGetAttribute(&ctx->smCount, cudaDevAttrMultiProcessorCount, device);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->renderBlocksPerSm, renderChunks, kRenderBlock, 0);
     if (ctx->renderBlocksPerSm < 1) ctx->renderBlocksPerSm = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->rayBlocksPerSm, traceRays, kRenderBlock, 0);
+    if (ctx->rayBlocksPerSm < 1) ctx->rayBlocksPerSm = 1;
     *out = ctx;
     return X2_OK;
 }
@@ -1462,12 +1464,21 @@ int x2_trace_rays_device(x2_scene* s, const float* rays, uint64_t n, uint32_t* t
         setError("null rays");
         return X2_EINVAL;
     }
-    if (int rc = ensureSlot(s->integrateSlot, 1)) return rc;
-    int perSm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, traceRays, kRenderBlock, 0);
-    const int blocks = int(std::min<uint64_t>(uint64_t(s->ctx->smCount) * std::max(perSm, 1), (2 * n + kRenderBlock - 1) / kRenderBlock));
-    cudaMemsetAsync(s->integrateSlot.claimed, 0, sizeof(unsigned long long), s->ctx->stream);
-    traceRays<<<blocks, kRenderBlock, 0, s->ctx->stream>>>(viewOf(s), rays, n, tri, t, occluded, s->integrateSlot.claimed);
+    if (s->bvh.nodeCount < kRayWalkNodes) {
+        traceRaysDirect<<<s->ctx->smCount * 8, 128, 0, s->ctx->stream>>>(viewOf(s), rays, n, tri, t, occluded);
+        CUDA_OR(cudaGetLastError(), X2_ECUDA);
+        return X2_OK;
+    }
+    const uint64_t queries = n * ((tri || t ? 1 : 0) + (occluded ? 1 : 0));
+    if (!queries) return X2_OK;
+    const uint64_t most = uint64_t(s->ctx->smCount) * s->ctx->rayBlocksPerSm, wanted = (queries + kRenderBlock - 1) / kRenderBlock;
+    unsigned long long* next = nullptr;
+    if (wanted > most) {
+        if (int rc = ensureSlot(s->integrateSlot, 1)) return rc;
+        next = s->integrateSlot.claimed;
+        cudaMemsetAsync(next, 0, sizeof(unsigned long long), s->ctx->stream);
+    }
+    traceRays<<<int(std::min(most, wanted)), kRenderBlock, 0, s->ctx->stream>>>(viewOf(s), rays, n, tri, t, occluded, next);
     CUDA_OR(cudaGetLastError(), X2_ECUDA);
     return X2_OK;
 }

@@ -424,9 +424,30 @@ __global__ void __launch_bounds__(kRenderBlock) integratePairsVolumes(SceneView 
 }
 
 // Closest hit and occlusion for n rays (8 floats each: origin, direction, near, far).
+// The ray entry one thread a ray, both walks one after the other: scenes of a few nodes, whose walks are over before
+// refilled lanes pay (kRayWalkNodes).
+__global__ void traceRaysDirect(SceneView s, const float* __restrict__ rays, unsigned long long n, uint32_t* __restrict__ tri,
+                                float* __restrict__ t, uint32_t* __restrict__ occluded) {
+    const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
+    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const float* r = rays + 8 * i;
+        const RayQ q = makeRay(s.bvh, r[0], r[1], r[2], r[3], r[4], r[5]);
+        if (tri || t) {
+            float th;
+            uint32_t leaf;
+            const uint32_t id = traceClosest<false>(s.bvh, q, r[6], r[7], th, &leaf, s.overflow, nullptr);
+            if (tri) tri[i] = id;
+            if (t) t[i] = id == ~0u ? 0.0f : th;
+        }
+        if (occluded) occluded[i] = traceAny<false>(s.bvh, q, r[6], r[7], s.overflow, nullptr) ? 1u : 0u;
+    }
+}
+
 // The ray entry: query 2 i is ray i's closest hit (when a caller wants it), 2 i + 1 its occlusion, walked a node a step by
 // persistent warps whose idle lanes take the next queries (as the wavefront's traversal kernels). One thread a ray, both
-// walks one after the other, took 0.225 ms for 262,139 scattered rays: a warp waited for its longest walk twice.
+// walks one after the other, took 0.225 ms for 262,139 scattered rays (0.111 so): a warp waited for its longest walk
+// twice. next: the fetch counter, at zero; null where the grid has a lane for every query, which then takes its own (a few
+// hundred rays: the counter's clearing alone is a twentieth of the call).
 __global__ void __launch_bounds__(kRenderBlock) traceRays(SceneView s, const float* __restrict__ rays, unsigned long long n,
                                                           uint32_t* __restrict__ tri, float* __restrict__ t, uint32_t* __restrict__ occluded,
                                                           unsigned long long* next) {
@@ -446,10 +467,12 @@ __global__ void __launch_bounds__(kRenderBlock) traceRays(SceneView s, const flo
         uint32_t lanes = __ballot_sync(full, walking);
         if (!drained && 32 - __popc(lanes) >= 8) {
             const uint32_t want = 32 - __popc(lanes);
-            unsigned long long base = 0;
-            if (lane == 0) base = atomicAdd(next, (unsigned long long)want);
-            base = __shfl_sync(full, base, 0);
-            drained = base + want >= queries;
+            unsigned long long base = (unsigned long long)blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
+            if (next) {
+                if (lane == 0) base = atomicAdd(next, (unsigned long long)want);
+                base = __shfl_sync(full, base, 0);
+            }
+            drained = !next || base + want >= queries;
             const unsigned long long q = base + __popc(~lanes & ((1u << lane) - 1u));
             if (!walking && q < queries) {
                 ray = kinds == 2 ? q >> 1 : q;
