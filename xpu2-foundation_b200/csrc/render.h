@@ -46,10 +46,10 @@ __global__ void integratePairsTextured(SceneView s, const uint32_t* pairs, unsig
                                        Counters* counters);
 __global__ void integratePairsVolumes(SceneView s, const uint32_t* pairs, unsigned long long n, double* rgba, uint32_t* status,
                                       Counters* counters);
-// The ray entry: traceRays for BVHs of at least kRayWalkNodes nodes, traceRaysDirect below. Measured at both ends, host
-// arrays in and out: the closed box (3 nodes), a million rays, 2.70 ms walked and 2.48 direct; a field of 105 k nodes 2.92
-// and 3.21 (500 rays: 0.084 and 0.123).
-constexpr uint32_t kRayWalkNodes = 64;
+// The ray entry: traceRays for BVHs of at least kRayWalkNodes nodes, traceRaysDirect below. 262,139 rays on the device,
+// walked and direct, by the BVH's nodes: 5 0.069 and 0.071 ms, 23 0.197 and 0.272, 235 0.263 and 0.452, 2,975 0.390 and
+// 0.670; a million rays of the closed box (3 nodes), host arrays in and out, 2.70 and 2.48.
+constexpr uint32_t kRayWalkNodes = 8;
 __global__ void traceRaysDirect(SceneView s, const float* rays, unsigned long long n, uint32_t* tri, float* t, uint32_t* occluded);
 __global__ void traceRays(SceneView s, const float* rays, unsigned long long n, uint32_t* tri, float* t, uint32_t* occluded,
                           unsigned long long* next);
