@@ -217,7 +217,8 @@ int x2_scene_info(x2_scene* scene, uint64_t* bvh_nodes, uint64_t* bvh_bytes, uin
                   float* build_ms);
 
 /* ---- per-sample API: integrate() (async_integrator.h:3047) for n (pixel, index) pairs ----
- * pairs: 2n uint32 (pixel, index); rgba: 4n doubles (Radiance rgb + alpha); status: n SampleStatus. */
+ * pairs: 2n uint32 (pixel, index); rgba: 4n doubles (Radiance rgb + alpha); status: n SampleStatus. A sample that its
+ * launch could not finish has status X2_ERROR and radiance zero; x2_integrate then returns X2_EDEVICE. */
 int x2_integrate(x2_scene* scene, const uint32_t* pairs, uint64_t n, double* rgba, uint32_t* status); /* waits */
 int x2_integrate_device(x2_scene* scene, const uint32_t* d_pairs, uint64_t n, double* d_rgba, uint32_t* d_status);
 

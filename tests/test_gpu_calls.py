@@ -1,0 +1,72 @@
+"""Calls beside one another and at their limits."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from oracle_lib import x2
+
+pytestmark = pytest.mark.gpu
+DEEP = 300  # beyond the wavefront's eight bits a path's depth
+
+
+def closed_room(ctx, max_depth, width=32, height=24):
+    """A closed room of one bright grey around the box's camera and light, no roulette: every path goes on to max_depth."""
+    s = x2.SyntheticScene(0)
+    d, cfg = s.desc, x2.Config.from_buffer_copy(s.config)
+    corners = np.array([[x, y, z] for x in (-6, 6) for y in (-6, 6) for z in (-6, 6)], np.float32)
+    quads = [(0, 1, 3, 2), (4, 6, 7, 5), (0, 4, 5, 1), (2, 3, 7, 6), (0, 2, 6, 4), (1, 5, 7, 3)]
+    triangles = np.array([t for a, b, c, e in quads for t in ((a, b, c), (a, c, e))], np.uint32)
+    first, material = np.array([0, 12], np.uint32), np.zeros(1, np.uint32)
+    keep = [np.ascontiguousarray(corners.reshape(-1)), np.ascontiguousarray(triangles.reshape(-1)), first, material]
+    d.vertex_count, d.triangle_count, d.mesh_count = 8, 12, 1
+    d.vertices, d.triangles = keep[0].ctypes.data_as(C.POINTER(C.c_float)), keep[1].ctypes.data_as(C.POINTER(C.c_uint32))
+    d.mesh_first, d.mesh_material = first.ctypes.data_as(C.POINTER(C.c_uint32)), material.ctypes.data_as(C.POINTER(C.c_uint32))
+    for c in range(3):
+        d.materials[0].diffuse[c] = 0.98
+    cfg.width, cfg.height, cfg.rr_threshold = width, height, 0.0
+    cfg.max_depth = cfg.max_diffuse_depth = cfg.max_glossy_depth = cfg.max_mirror_depth = max_depth
+    return s, cfg, x2.Scene(ctx, d, cfg)
+
+
+def one_thread(scene, pixels, indices):
+    """integratePairs's samples: a counting call takes that kernel."""
+    scene.count_traversal(True)
+    out = scene.integrate(pixels, indices)
+    scene.count_traversal(False)
+    return out
+
+
+def test_unfinished_samples_are_not_handed_out(ctx):
+    """Samples that the per-sample entry did not finish, in an early window of a long list or after an earlier call on the
+    same buffers: an error, or the right samples, never something else as done."""
+    import torch
+
+    s, cfg, scene = closed_room(ctx, 4)
+    n, some = (1 << 22) + 37, 100
+    pixels = np.full(n, cfg.width * cfg.height, np.uint32)  # no such pixel: an error at once
+    pixels[:some] = np.random.default_rng(2).integers(0, cfg.width * cfg.height, some, dtype=np.uint32)
+    indices = np.arange(n, dtype=np.uint32)
+    scene.integrate(pixels[:some], indices[:some])  # what an unfinished sample would find in its place
+    deep = x2.Config.from_buffer_copy(cfg)
+    deep.max_depth = deep.max_diffuse_depth = DEEP
+    scene.set_config(deep)
+    want, _ = one_thread(scene, pixels[:some], indices[:some])
+    # The device entry.
+    pairs = torch.tensor(np.stack([pixels[:some], indices[:some]], 1).astype(np.int64)).to(torch.int32).cuda()
+    rgba, status = torch.zeros((some, 4), dtype=torch.float64, device="cuda"), torch.zeros(some, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    call = x2.library().x2_integrate_device
+    assert call(scene.handle, pairs.data_ptr(), some, rgba.data_ptr(), status.data_ptr()) == x2.OK
+    ctx.synchronize()
+    done = (status == x2.DONE).cpu().numpy()
+    assert np.array_equal(rgba.cpu().numpy()[done], want[done])
+    assert (status[~torch.tensor(done)] == x2.ERROR).all()
+    # The host entry, over two windows.
+    try:
+        got, got_status = scene.integrate(pixels, indices)
+        assert np.array_equal(got[:some], want) and (got_status[:some] == x2.DONE).all()
+        assert (got_status[some:] == x2.ERROR).all()
+    except x2.X2Error as e:
+        assert e.code == x2.EDEVICE
+    scene.free()

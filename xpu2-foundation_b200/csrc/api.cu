@@ -231,7 +231,7 @@ struct x2_scene {
     float4* pairOut = nullptr;
     uint8_t* pairStatus = nullptr;
     uint32_t pairCap = 0;
-    uint32_t *pairWords = nullptr, *hostPairWords = nullptr;
+    uint32_t* pairWords = nullptr;
     float4* stepLists = nullptr;  // the plain megakernel's lists
     size_t stepThreads = 0;
     unsigned long long* auditWord = nullptr;
@@ -441,12 +441,11 @@ int ensureWave(x2_scene* s, uint32_t paths, uint32_t records) {
         m.take(s->waveCounters, kWaveCounters), m.take(s->claimed, 1), m.take(s->drainWords, 4), m.take(s->pairWords, 4);
     });
     if (ok && !s->hostWords) {
-        ok = cudaMallocHost(&s->hostWords, sizeof(uint32_t) * 12) == cudaSuccess;
+        ok = cudaMallocHost(&s->hostWords, sizeof(uint32_t) * 8) == cudaSuccess;
         if (ok) {
-            std::memset(s->hostWords, 0, sizeof(uint32_t) * 12);
+            std::memset(s->hostWords, 0, sizeof(uint32_t) * 8);
             s->hostLast = s->hostWords;
             s->hostDrain = s->hostWords + 4;
-            s->hostPairWords = s->hostWords + 8;
         }
     }
     if (!ok) {
@@ -1372,6 +1371,7 @@ int integrateWavefront(x2_scene* s, uint32_t paths, const uint32_t* pairs, uint6
     for (uint64_t first = 0; first < n; first += window) {
         const uint32_t items = uint32_t(std::min<uint64_t>(window, n - first));
         clearWave(s, paths);
+        cudaMemsetAsync(s->pairStatus, X2_SKIP, items, st);
         WaveArgs a = launchArgs(s, s->integrateSlot, paths, records, items, 0);
         a.pairs = pairs + 2 * first;
         a.out = s->pairOut;
@@ -1382,12 +1382,10 @@ int integrateWavefront(x2_scene* s, uint32_t paths, const uint32_t* pairs, uint6
         const DrainKey key = drainKey(wk, a, grids, most, items, rgba + 4 * first, status + first, nullptr);
         const int done = launchDrain(s->ctx, a, s->pairWords, most, "x2_integrate",
                                      [&] { launchIteration(wk, a, grids, st, false, &s->ctx->side); }, [&] {
-            wfPairsOut<<<(items + 255) / 256, 256, 0, st>>>(s->pairOut, s->pairStatus, items, rgba + 4 * first, status + first);
+            wfPairsOut<<<(items + 255) / 256, 256, 0, st>>>(s->pairOut, s->pairStatus, items, rgba + 4 * first, status + first,
+                                                            s->integrateSlot.counters);
         }, &s->pairGraph, &key);
         if (done) return done;
-        // A window that did not drain keeps its word until the caller waits.
-        if (first == 0 || !s->hostPairWords[2])
-            cudaMemcpyAsync(s->hostPairWords, s->pairWords, sizeof(uint32_t) * 4, cudaMemcpyDeviceToHost, st);
     }
     return X2_OK;
 }
@@ -1447,9 +1445,8 @@ int x2_integrate(x2_scene* s, const uint32_t* pairs, uint64_t n, double* rgba, u
     if (rc == X2_OK && w == X2_OK && s->integrateSlot.busy) {
         accumulate(s->total, *s->integrateSlot.hostCounters);
         s->integrateSlot.busy = false;
-        if (s->hostPairWords && s->hostPairWords[2]) {
-            s->hostPairWords[2] = 0;
-            setError("x2_integrate: the samples did not drain");
+        if (const unsigned long long left = s->integrateSlot.hostCounters->unfinished) {
+            setError("x2_integrate: %llu samples unfinished at the iteration bound", left);
             return X2_EDEVICE;
         }
     }

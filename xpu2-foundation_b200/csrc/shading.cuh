@@ -87,7 +87,8 @@ struct TexRec {
     uint32_t width, height, wrap, pad;
 };
 struct Counters {
-    unsigned long long trace, nee, bsdf, held, samples, errors, overflow, pad;
+    unsigned long long trace, nee, bsdf, held, samples, errors, overflow;
+    unsigned long long unfinished;  // the per-sample entry's samples that a window ended without (errors counts them too)
 };
 // A volume on the device (x2_volume; volume::Shader's VdbVolume fields, volume_core.h:64-111) and a dense grid.
 constexpr int kMajorantCells = 32;  // a volume's majorant grid: kMajorantCells^3 over its bounds

@@ -1365,16 +1365,21 @@ __global__ void wfFilmReduceBatch(WaveArgs a, const BatchFilm* __restrict__ film
 }
 
 __global__ void wfPairsOut(const float4* __restrict__ out, const uint8_t* __restrict__ outStatus, uint32_t n, double* __restrict__ rgba,
-                           uint32_t* __restrict__ status) {
+                           uint32_t* __restrict__ status, Counters* counters) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const float4 v = out[i];
+    const bool finished = outStatus[i] != X2_SKIP;
+    if (!finished) {
+        atomicAdd(&counters->errors, 1ull);
+        atomicAdd(&counters->unfinished, 1ull);
+    }
+    const float4 v = finished ? out[i] : make_float4(0, 0, 0, 0);
     const size_t q = 4 * size_t(i);
     rgba[q] = double(v.x);
     rgba[q + 1] = double(v.y);
     rgba[q + 2] = double(v.z);
     rgba[q + 3] = double(v.w);
-    status[i] = outStatus[i];
+    status[i] = finished ? outStatus[i] : uint32_t(X2_ERROR);
 }
 
 }  // namespace x2
