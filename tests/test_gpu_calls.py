@@ -37,6 +37,19 @@ def one_thread(scene, pixels, indices):
     return out
 
 
+@pytest.mark.parametrize("max_depth", [255, 256, DEEP])  # the deepest that the wavefront form takes, and beyond
+def test_deep_paths_equal_one_thread_a_sample(ctx, max_depth):
+    s, cfg, scene = closed_room(ctx, max_depth)
+    rng = np.random.default_rng(1)
+    pixels, indices = rng.integers(0, cfg.width * cfg.height, 200, dtype=np.uint32), np.arange(200, dtype=np.uint32)
+    rgba, status = scene.integrate(pixels, indices)
+    want, want_status = one_thread(scene, pixels, indices)
+    scene.free()
+    assert (want_status == x2.DONE).all() and (want[:, 3] == 1).all()
+    assert np.array_equal(status, want_status)
+    assert np.array_equal(rgba, want)
+
+
 def test_unfinished_samples_are_not_handed_out(ctx):
     """Samples that the per-sample entry did not finish, in an early window of a long list or after an earlier call on the
     same buffers: an error, or the right samples, never something else as done."""

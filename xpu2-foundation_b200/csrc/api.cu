@@ -1332,12 +1332,14 @@ void clearWave(x2_scene* s, uint32_t paths) {
 // sample, as integratePairs runs them, traces a vertex's up to 18 shadow rays one after another and waits for its warp's
 // longest path (60,000 samples of a field: 3.85 ms); the wavefront traces them side by side and gives each sample the same
 // radiance. integratePairs stays for what this form does not take: several BSDF samples, multiple scattering (whose
-// march would run inside shade), counting runs, the diagnostic build, lists not aligned to pairs, and path state beyond kPairBytes.
+// march would run inside shade), paths deeper than the eight bits that a slot's depths have (packDepths: past them a path
+// starts over at depth 0), counting runs, the diagnostic build, lists not aligned to pairs, and path state beyond
+// kPairBytes.
 constexpr double kPairBytes = 2e9;
 constexpr uint32_t kPairWindow = 1u << 22;
 uint32_t pairPaths(x2_scene* s, uint64_t n, const uint32_t* pairs) {
     const x2_config& c = s->config;
-    if (diagnosticKernels() || s->counting || c.bsdf_samples != 1 || (s->volumeCount && c.max_volume_depth > 1) ||
+    if (diagnosticKernels() || s->counting || c.bsdf_samples != 1 || c.max_depth > 255 || (s->volumeCount && c.max_volume_depth > 1) ||
         reinterpret_cast<uintptr_t>(pairs) % sizeof(uint2))
         return 0;
     const uint64_t records = uint64_t(c.light_count) * c.light_samples + 1;
