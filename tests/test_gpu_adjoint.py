@@ -301,3 +301,37 @@ def test_texel_gradients(field):
         print(f"texel ({x},{y}) channel {c}: adjoint {gt[texel, c]:.6g} fd {fd:.6g}")
         assert abs(fd - gt[texel, c]) <= 0.03 * abs(gt[texel, c])
     scene.set_texture(0, tex)
+
+
+def test_texture_arrays_that_are_not_the_texture_s(ctx):
+    """set_texture takes no CUDA tensor of another layout, type or size, no shorter host array, and diff.render no such
+    texture; the texels stay as they were."""
+    import torch
+    from x2.diff import render
+
+    s = x2.SyntheticScene(4)
+    cfg = s.config
+    cfg.width, cfg.height = 32, 24
+    scene = x2.Scene(ctx, s.desc, cfg)
+    texture = torch.tensor(s.texture(0), device="cuda")
+    a = torch.tensor(np.array([list(s.desc.materials[m].diffuse) for m in range(s.desc.material_count)], np.float32), device="cuda")
+    r = torch.tensor(np.array([list(s.desc.lights[i].radiance) for i in range(s.desc.light_count)], np.float32), device="cuda")
+    want = render(scene, a, r, 0, 2, texture=texture)
+    with pytest.raises(ValueError):
+        scene.set_texture(0, texture.transpose(0, 1))
+    with pytest.raises(ValueError):
+        scene.set_texture(0, texture.half())
+    with pytest.raises(ValueError):
+        scene.set_texture(0, texture[:-1].contiguous())
+    with pytest.raises(ValueError):
+        scene.set_texture(0, texture[:-1].cpu().numpy())
+    with pytest.raises(ValueError):
+        render(scene, a, r, 0, 2, texture=texture[:-1])
+    with pytest.raises(x2.X2Error):
+        scene.set_texture(1, texture)
+    assert torch.equal(render(scene, a, r, 0, 2), want)
+    strided = torch.empty((*texture.shape[:2], 4), device="cuda")[:, :, :3].copy_(texture)
+    assert torch.equal(render(scene, a, r, 0, 2, texture=strided), want)
+    scene.set_texture(0, texture.double().cpu().numpy())  # host arrays of other types are converted
+    assert torch.equal(render(scene, a, r, 0, 2), want)
+    scene.free()

@@ -353,6 +353,8 @@ class Scene:
         self._h = C.c_void_p()
         _check(library().x2_scene_load(ctx.handle, C.byref(desc) if isinstance(desc, SceneDesc) else desc, C.byref(self._h)))
         ctx._scenes.add(self)
+        d = desc if isinstance(desc, SceneDesc) else desc._obj if hasattr(desc, "_obj") else desc.contents  # a byref, a pointer
+        self._texture_floats = [3 * d.textures[k].width * d.textures[k].height for k in range(d.texture_count)]
         self.set_config(config)
 
     def set_config(self, config):
@@ -511,11 +513,20 @@ class Scene:
 
     def set_texture(self, texture, rgb):
         """x2_scene_set_texture: texture `texture`'s texels (height x width x 3 floats) set in place; a contiguous float32
-        CUDA tensor on the context's device is copied there, without a way through the host (its stream must be idle)."""
+        CUDA tensor on the context's device is copied there, without a way through the host, once its device's current
+        stream is idle."""
+        floats = self._texture_floats[texture] if 0 <= texture < len(self._texture_floats) else 0  # else: the library's error
         if getattr(rgb, "is_cuda", False):
+            import torch
+
+            if rgb.dtype != torch.float32 or not rgb.is_contiguous() or rgb.device.index != self.ctx.device or rgb.numel() < floats:
+                raise ValueError("a texture's CUDA tensor must be contiguous float32 on device %d, %d values" % (self.ctx.device, floats))
+            torch.cuda.current_stream(rgb.device).synchronize()
             _check(library().x2_scene_set_texture(self._h, texture, C.c_void_p(rgb.data_ptr())))
             return
         a = np.ascontiguousarray(rgb, np.float32)
+        if a.size < floats:
+            raise ValueError("a texture of %d values from an array of %d" % (floats, a.size))
         _check(library().x2_scene_set_texture(self._h, texture, _ptr(a)))
 
     def adjoint(self, first, count, d_dloss_dimage, d_albedo_grad, d_radiance_grad, d_roughness_grad=None, plain=False,

@@ -21,10 +21,7 @@ class Render(torch.autograd.Function):
         if texture is not None:
             # Texels that already lie on the scene's device as the library keeps them go there directly.
             here = texture.is_cuda and texture.device.index == scene.ctx.device and texture.dtype == torch.float32
-            if here:
-                texels = texture.detach().contiguous()
-                torch.cuda.current_stream(texels.device).synchronize()
-            scene.set_texture(0, texels if here else _host(texture))
+            scene.set_texture(0, texture.detach().contiguous() if here else _host(texture))
         scene.frame_begin(count)
         scene.render_frame_wavefront(first, count)
         scene.wait()
