@@ -78,3 +78,21 @@ def test_batch_rejects_bad_requests(ctx):
     with pytest.raises(x2.X2Error) as e:
         ctx.render_batch([(a, 0, 1), (b, 0, 1)])
     assert e.value.code == x2.EINVAL
+
+
+def test_undrained_batch_leaves_the_films(ctx):
+    """A batch that does not drain (paths deeper than the eight bits of the wavefront's path state go on until the
+    iteration bound) reports it and adds nothing to its films, those of the requests that did finish included."""
+    from test_gpu_calls import DEEP, closed_room
+
+    scenes = [closed_room(ctx, depth, 16, 16)[2] for depth in (4, DEEP)]
+    try:
+        ctx.render_batch([(scene, 0, 2) for scene in scenes])
+        assert all((scene.film()[1] == 2).all() for scene in scenes)
+    except x2.X2Error as e:
+        assert e.code == x2.EDEVICE
+        for scene in scenes:
+            sums, counts = scene.film()
+            assert not counts.any() and not sums.any()
+    for scene in scenes:
+        scene.free()

@@ -534,13 +534,14 @@ int ensureItems(x2_scene* s, uint64_t items) {
 }  // namespace
 
 namespace x2 {
-__global__ void addInto(double* dst, const double* src, uint32_t n) {
+// overrun (or null): a drain's overrun word; nothing is added where the drain stopped at its bound.
+__global__ void addInto(double* dst, const double* src, uint32_t n, const uint32_t* overrun) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dst[i] += src[i];
+    if (i < n && !(overrun && *overrun)) dst[i] += src[i];
 }
-__global__ void addFloatInto(double* dst, const float* src, uint64_t n) {
+__global__ void addFloatInto(double* dst, const float* src, uint64_t n, const uint32_t* overrun) {
     const uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n) dst[i] += double(src[i]);
+    if (i < n && !(overrun && *overrun)) dst[i] += double(src[i]);
 }
 
 // The scene's device view, stream and device for entry points in other translation units (noalloc.cu).
@@ -2009,10 +2010,10 @@ int x2_adjoint_plain(x2_scene* s, uint32_t first, uint32_t count, const float* d
     int rc = cudaGetLastError() == cudaSuccess ? X2_OK : X2_ECUDA;
     if (!rc) {
         // Added to the caller's arrays: albedo, roughness, radiance.
-        addInto<<<(params + 255) / 256, 256, 0, st>>>(d_albedo_grad, grads, 3 * s->materialCount);
-        if (d_roughness_grad) addInto<<<(params + 255) / 256, 256, 0, st>>>(d_roughness_grad, grads + 3 * s->materialCount, s->materialCount);
-        addInto<<<(params + 255) / 256, 256, 0, st>>>(d_radiance_grad, grads + 4 * s->materialCount, 3 * s->lightCount);
-        if (texGrads) addFloatInto<<<unsigned((texGrads + 255) / 256), 256, 0, st>>>(d_texture_grad, texGrad, texGrads);
+        addInto<<<(params + 255) / 256, 256, 0, st>>>(d_albedo_grad, grads, 3 * s->materialCount, nullptr);
+        if (d_roughness_grad) addInto<<<(params + 255) / 256, 256, 0, st>>>(d_roughness_grad, grads + 3 * s->materialCount, s->materialCount, nullptr);
+        addInto<<<(params + 255) / 256, 256, 0, st>>>(d_radiance_grad, grads + 4 * s->materialCount, 3 * s->lightCount, nullptr);
+        if (texGrads) addFloatInto<<<unsigned((texGrads + 255) / 256), 256, 0, st>>>(d_texture_grad, texGrad, texGrads, nullptr);
         rc = x2_synchronize(s->ctx, 600000);
     } else {
         setError("x2_adjoint: launch failed");
@@ -2153,15 +2154,16 @@ int x2_adjoint(x2_scene* s, uint32_t first, uint32_t count, const float* d_dloss
     const WaveKernels wk = waveKernels(s->traceBlocks, s->shadeBlocks, false, s->triUV != nullptr, s->shortStack != 0, false, false, 0,
                                        s->triOverlap != 0 && s->shortStack != 0 && s->traceBlocks < 9);
     const uint64_t maxIter = items * (uint64_t(s->config.max_depth) + 2) / paths + uint64_t(s->config.max_depth) + 64;
+    const uint32_t* const overrun = s->drainWords + 2;
     int rc = launchDrain(
         s->ctx, a, s->drainWords, uint32_t(std::min<uint64_t>(maxIter, 0xffffffffu)), "x2_adjoint",
         [&] { launchAdjointIteration(wk, adj, a, grids, s->ctx->smCount * 8, shared, st, &s->ctx->side); },
         [&] {
             wfGradRows<<<(params + 31) / 32, dim3(32, 32), 0, st>>>(rows, kRows, params, grads);
-            addInto<<<(params + 255) / 256, 256, 0, st>>>(d_albedo_grad, grads, 3 * s->materialCount);
-            if (d_roughness_grad) addInto<<<(params + 255) / 256, 256, 0, st>>>(d_roughness_grad, grads + 3 * s->materialCount, s->materialCount);
-            addInto<<<(params + 255) / 256, 256, 0, st>>>(d_radiance_grad, grads + 4 * s->materialCount, 3 * s->lightCount);
-            if (texGrads) addFloatInto<<<unsigned((texGrads + 255) / 256), 256, 0, st>>>(d_texture_grad, texGrad, texGrads);
+            addInto<<<(params + 255) / 256, 256, 0, st>>>(d_albedo_grad, grads, 3 * s->materialCount, overrun);
+            if (d_roughness_grad) addInto<<<(params + 255) / 256, 256, 0, st>>>(d_roughness_grad, grads + 3 * s->materialCount, s->materialCount, overrun);
+            addInto<<<(params + 255) / 256, 256, 0, st>>>(d_radiance_grad, grads + 4 * s->materialCount, 3 * s->lightCount, overrun);
+            if (texGrads) addFloatInto<<<unsigned((texGrads + 255) / 256), 256, 0, st>>>(d_texture_grad, texGrad, texGrads, overrun);
         });
     if (rc) return rc;
     cudaMemcpyAsync(s->hostDrain, s->drainWords, sizeof(uint32_t) * 4, cudaMemcpyDeviceToHost, st);
@@ -3001,7 +3003,7 @@ int x2_render_batch(x2_ctx* ctx, const x2_request* req, uint32_t n, x2_completio
         rc = launchDrain(
             ctx, a, s0->drainWords, uint32_t(std::min<uint64_t>(maxIter, 0xffffffffu)), "x2_render_batch",
             [&] { launchIteration(wk, a, grids, st, true, &ctx->side); },
-            [&] { wfFilmReduceBatch<<<int((64ull * (c1 - c0) + 255) / 256), 256, 0, st>>>(a, dFilms); });
+            [&] { wfFilmReduceBatch<<<int((64ull * (c1 - c0) + 255) / 256), 256, 0, st>>>(a, dFilms, s0->drainWords + 2); });
         if (rc) break;
         // The next window rewrites the host's tables: this one is waited for.
         cudaMemcpyAsync(s0->hostDrain, s0->drainWords, sizeof(uint32_t) * 4, cudaMemcpyDeviceToHost, st);

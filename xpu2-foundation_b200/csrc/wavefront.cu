@@ -1325,10 +1325,11 @@ __global__ void wfFilmReduce(WaveArgs a, uint32_t chunkCount, double* sums, doub
     atomicAdd(counts + pixel, n);
 }
 
-// A batch's films: each chunk's samples (64 x its count items from chunkItems[c]) into its request's film.
-__global__ void wfFilmReduceBatch(WaveArgs a, const BatchFilm* __restrict__ films) {
+// A batch's films: each chunk's samples (64 x its count items from chunkItems[c]) into its request's film; nothing where
+// the drain stopped at its bound (overrun).
+__global__ void wfFilmReduceBatch(WaveArgs a, const BatchFilm* __restrict__ films, const uint32_t* overrun) {
     const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= 64ull * a.chunkCount) return;
+    if (*overrun || i >= 64ull * a.chunkCount) return;
     const uint32_t chunkIndex = uint32_t(i / 64), position = uint32_t(i % 64);
     const x2_chunk chunk = a.chunks[chunkIndex];
     const uint32_t request = a.chunkRequest[chunkIndex];

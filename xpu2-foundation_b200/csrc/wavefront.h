@@ -203,7 +203,7 @@ __global__ void wfResetQueues(WaveArgs a);
 __global__ void wfDrainCheck(WaveArgs a, cudaGraphConditionalHandle loop, uint32_t* iterations, uint32_t maxIterations,
                              uint32_t* overrun);
 __global__ void wfFilmReduce(WaveArgs a, uint32_t chunkCount, double* sums, double* odd, uint32_t* counts);
-__global__ void wfFilmReduceBatch(WaveArgs a, const BatchFilm* films);
+__global__ void wfFilmReduceBatch(WaveArgs a, const BatchFilm* films, const uint32_t* overrun);
 // The per-sample entry's outputs from a launch's items: rgb and alpha as doubles, the status as a word; an item that the
 // launch left unfinished (outStatus still X2_SKIP, as it starts) as an error, counted.
 __global__ void wfPairsOut(const float4* out, const uint8_t* outStatus, uint32_t n, double* rgba, uint32_t* status, Counters* counters);
