@@ -83,3 +83,34 @@ def test_unfinished_samples_are_not_handed_out(ctx):
     except x2.X2Error as e:
         assert e.code == x2.EDEVICE
     scene.free()
+
+
+def test_integrate_without_room_for_its_outputs(ctx):
+    """The samples' outputs do not fit the device: the one-thread kernel, which needs none, takes the call."""
+    import torch
+
+    s, cfg, scene = closed_room(ctx, 4)
+    n, small = 1 << 22, 1 << 20
+    rng = np.random.default_rng(4)
+    pairs = torch.tensor(np.stack([rng.integers(0, cfg.width * cfg.height, n), np.arange(n)], 1)).to(torch.int32).cuda()
+    rgba, status = torch.zeros((n, 4), dtype=torch.float64, device="cuda"), torch.zeros(n, dtype=torch.int32, device="cuda")
+    call = x2.library().x2_integrate_device
+    torch.cuda.synchronize()
+    assert call(scene.handle, pairs.data_ptr(), small, rgba.data_ptr(), status.data_ptr()) == x2.OK
+    ctx.synchronize()
+    want = rgba[:small].clone()
+    one_thread(scene, np.zeros(1, np.uint32), np.zeros(1, np.uint32))  # that kernel's local memory is there from here on
+    rgba.zero_()
+    held = []
+    while (free := torch.cuda.mem_get_info()[0]) > 32 << 20:
+        held.append(torch.empty(max(free - (24 << 20), 2 << 20) & ~((2 << 20) - 1), dtype=torch.uint8, device="cuda"))
+    torch.cuda.synchronize()
+    try:
+        rc = call(scene.handle, pairs.data_ptr(), n, rgba.data_ptr(), status.data_ptr())
+        ctx.synchronize()
+    finally:
+        held.clear()
+        torch.cuda.empty_cache()
+    assert rc == x2.OK
+    assert (status == x2.DONE).all() and torch.equal(rgba[:small], want)
+    scene.free()

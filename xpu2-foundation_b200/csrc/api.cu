@@ -228,6 +228,7 @@ struct x2_scene {
     Counters total{};
     // the per-sample API's scratch: its counters, a window's item outputs and its drain's words
     Slot integrateSlot;
+    unsigned char* pairMemory = nullptr;
     float4* pairOut = nullptr;
     uint8_t* pairStatus = nullptr;
     uint32_t pairCap = 0;
@@ -1089,8 +1090,7 @@ int x2_scene_free(x2_scene* s) {
     for (auto& sl : s->slots) freeSlot(sl);
     freeSlot(s->integrateSlot);
     cudaFree(s->stepLists);
-    cudaFree(s->pairOut);
-    cudaFree(s->pairStatus);
+    cudaFree(s->pairMemory);
     if (s->staging) cudaFreeHost(s->staging);
     delete s;
     return X2_OK;
@@ -1358,12 +1358,10 @@ int integrateWavefront(x2_scene* s, uint32_t paths, const uint32_t* pairs, uint6
     if (rc) return rc;
     const uint32_t window = uint32_t(std::min<uint64_t>(n, kPairWindow));
     if (window > s->pairCap) {
-        cudaFree(s->pairOut);
-        cudaFree(s->pairStatus);
-        s->pairOut = nullptr;
-        s->pairStatus = nullptr;
+        cudaFree(s->pairMemory);
         s->pairCap = 0;
-        if (cudaMalloc(&s->pairOut, sizeof(float4) * window) != cudaSuccess || cudaMalloc(&s->pairStatus, window) != cudaSuccess) {
+        if (!carve(&s->pairMemory, [&](Carve& m) { m.take(s->pairOut, window), m.take(s->pairStatus, window); })) {
+            cudaGetLastError();  // the caller goes on without
             setError("device allocation failed for %u samples' outputs", window);
             return X2_ENOMEM;
         }
