@@ -221,3 +221,36 @@ def test_adaptive_arguments_refused(box):
         with pytest.raises(x2.X2Error) as e:
             call()
         assert e.value.code == x2.EINVAL
+
+
+def test_cellular_frames_around_a_rebuilt_state(ctx):
+    """Cellular frames, the adaptive state rebuilt between them at other sizes by chain steps (which keep no graph), the
+    device's free memory moved meanwhile: each frame as a scene that has done nothing else gives it."""
+    import torch
+
+    s = x2.SyntheticScene(0)
+
+    def at(width, height):
+        cfg = x2.Config.from_buffer_copy(s.config)
+        cfg.width, cfg.height = width, height
+        return cfg
+
+    a, b = at(120, 90), at(64, 200)
+    scene, fresh = x2.Scene(ctx, s.desc, a), x2.Scene(ctx, s.desc, a)
+    want_result = fresh.render_adaptive(4, 64, 0.01, True)
+    want = fresh.film(odd=True)
+    fresh.free()
+    held = []
+    for turn in range(6):
+        scene.set_config(a)
+        result = scene.render_adaptive(4, 64, 0.01, True)
+        got = scene.film(odd=True)
+        assert (result["passes"], result["samples"]) == (want_result["passes"], want_result["samples"]), turn
+        assert all(np.array_equal(g, w) for g, w in zip(got, want)), turn
+        scene.set_config(b)
+        scene.frame_begin_adaptive(1)
+        scene.render_frame_wavefront(0, 1)
+        scene.wait()
+        scene.adaptive_step(0.01, 1, 1)
+        held.append(torch.zeros(1 << (8 + turn), dtype=torch.uint8, device="cuda"))
+    scene.free()

@@ -2486,12 +2486,14 @@ int renderAdaptive(x2_scene* s, uint32_t minSamples, uint32_t maxSamples, float 
     struct AdaptiveKey {
         DrainKey drain;
         x2::AdaptiveArgs chain;
+        const uint8_t* alive;  // the cellular generations (chain.alive is set pass by pass)
         uint32_t minSamples, maxSamples, cellular;
     };
     AdaptiveKey key;
     std::memset(static_cast<void*>(&key), 0, sizeof(key));
     key.drain = drainKey(wk, a, grids, maxIter, most, s->sums, s->odd, s->counts);
     key.chain = chain;
+    key.alive = ad.alive;
     key.minSamples = minSamples;
     key.maxSamples = maxSamples;
     key.cellular = cellular ? 1 : 0;
