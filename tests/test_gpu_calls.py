@@ -114,3 +114,37 @@ def test_integrate_without_room_for_its_outputs(ctx):
     assert rc == x2.OK
     assert (status == x2.DONE).all() and torch.equal(rgba[:small], want)
     scene.free()
+
+
+@pytest.mark.parametrize("entry", ["trace_rays"])
+def test_long_lists_do_not_wait_for_other_streams(ctx, entry):
+    """A list beyond the context's kept scratch, with another stream of the program at work: the call ends first."""
+    import torch
+
+    s, cfg, scene = closed_room(ctx, 2)
+    n = 1600000  # over 64 MB at 44 bytes
+    rng = np.random.default_rng(5)
+    if entry == "integrate":
+        args = (rng.integers(0, cfg.width * cfg.height, n, dtype=np.uint32), np.arange(n, dtype=np.uint32))
+    else:
+        rays = np.zeros((n, 8), np.float32)
+        rays[:, 3:6] = rng.normal(size=(n, 3))
+        rays[:, 7] = 100.0
+        args = (rays,)
+    call = getattr(scene, entry)
+    want = call(*args)
+    few = [a[:300] for a in args]
+    call(*few)
+    other = torch.cuda.Stream()
+    with torch.cuda.stream(other):
+        torch.cuda._sleep(10)
+        other.synchronize()
+        torch.cuda._sleep(2000000000)  # about a second
+        done = torch.cuda.Event()
+        done.record()
+    got = call(*args)
+    waited = done.query()
+    other.synchronize()
+    scene.free()
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
+    assert not waited

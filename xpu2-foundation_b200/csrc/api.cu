@@ -1289,7 +1289,8 @@ DrainKey drainKey(const WaveKernels& k, const WaveArgs& a, const WaveGrids& g, u
 
 // Device memory for a host caller's arrays during one call: the context keeps one piece of at most kCallScratch bytes (a
 // scene's first call then allocates nothing), lent to one call at a time; a call that finds it lent or too small
-// allocates its own, and leaves it in place of a smaller one (dropScratch, once the call has waited).
+// allocates its own, and leaves it in place of a smaller one (dropScratch, once the call has waited). All of it in the
+// context's stream order: cudaFree would wait for every stream of the program.
 constexpr size_t kCallScratch = 64u << 20;
 unsigned char* callScratch(x2_ctx* ctx, size_t bytes) {
     {
@@ -1300,7 +1301,7 @@ unsigned char* callScratch(x2_ctx* ctx, size_t bytes) {
         }
     }
     unsigned char* p = nullptr;
-    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    if (cudaMallocAsync(&p, bytes, ctx->stream) != cudaSuccess) {
         cudaGetLastError();
         setError("device allocation failed for a call's %zu bytes", bytes);
         return nullptr;
@@ -1312,11 +1313,11 @@ void dropScratch(x2_ctx* ctx, unsigned char* p, size_t bytes) {
     if (p == ctx->scratch) {
         ctx->scratchLent = false;
     } else if (!ctx->scratchLent && bytes <= kCallScratch && bytes > ctx->scratchBytes) {
-        cudaFree(ctx->scratch);
+        if (ctx->scratch) cudaFreeAsync(ctx->scratch, ctx->stream);
         ctx->scratch = p;
         ctx->scratchBytes = bytes;
     } else {
-        cudaFree(p);
+        cudaFreeAsync(p, ctx->stream);
     }
 }
 
