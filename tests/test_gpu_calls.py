@@ -116,7 +116,7 @@ def test_integrate_without_room_for_its_outputs(ctx):
     scene.free()
 
 
-@pytest.mark.parametrize("entry", ["trace_rays"])
+@pytest.mark.parametrize("entry", ["integrate", "trace_rays"])
 def test_long_lists_do_not_wait_for_other_streams(ctx, entry):
     """A list beyond the context's kept scratch, with another stream of the program at work: the call ends first."""
     import torch

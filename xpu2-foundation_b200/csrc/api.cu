@@ -117,12 +117,29 @@ struct Slot {
 
 using namespace x2;
 
+// Graphs that no launch will use again. Destroying one that holds a conditional node waits for every stream of the
+// program, other libraries' too (a call behind a second's work elsewhere took that second), so they are put by and
+// destroyed a list at a time.
+struct RetiredGraphs {
+    static constexpr size_t kMost = 32;
+    std::vector<cudaGraphExec_t> execs;
+    void add(cudaGraphExec_t exec) {
+        if (!exec) return;
+        if (execs.size() >= kMost) destroy();
+        execs.push_back(exec);
+    }
+    void destroy() {
+        for (cudaGraphExec_t e : execs) cudaGraphExecDestroy(e);
+        execs.clear();
+    }
+};
+
 // A launch's instantiated graph and the bytes of what it was made with.
 struct KeptGraph {
     cudaGraphExec_t exec = nullptr;
     std::vector<unsigned char> key;
-    void drop() {
-        if (exec) cudaGraphExecDestroy(exec);
+    void drop(RetiredGraphs& retired) {
+        retired.add(exec);
         exec = nullptr;
         key.clear();
     }
@@ -134,6 +151,7 @@ struct x2_ctx {
     int smCount = 0;
     int renderBlocksPerSm = 0, rayBlocksPerSm = 0;
     x2::SideStreams side;  // for kernels of one iteration that run side by side
+    RetiredGraphs retired;
     std::mutex scratchMutex;
     unsigned char* scratch = nullptr;  // a host caller's arrays during x2_integrate or x2_trace_rays
     size_t scratchBytes = 0;
@@ -688,6 +706,7 @@ int x2_close(x2_ctx* ctx) {
         cudaEventDestroy(ctx->side.join[j]);
     }
     cudaEventDestroy(ctx->side.fork);
+    ctx->retired.destroy();
     cudaFree(ctx->scratch);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -1075,9 +1094,8 @@ int x2_scene_free(x2_scene* s) {
     cudaFree(s->grids);
     for (float* g : s->gridValues) cudaFree(g);
     for (float* m : s->majorants) cudaFree(m);
-    s->frameGraph.drop();
-    s->pairGraph.drop();
-    s->adaptiveGraph.drop();
+    for (KeptGraph* g : {&s->frameGraph, &s->pairGraph, &s->adaptiveGraph})
+        if (g->exec) cudaGraphExecDestroy(g->exec);
     freeWave(s);
     freeVolumeWave(s);
     cudaFree(s->out);
@@ -1259,11 +1277,11 @@ int launchDrain(x2_ctx* ctx, const WaveArgs& a, uint32_t* words, uint32_t bound,
     cudaMemsetAsync(words, 0, sizeof(uint32_t) * 4, st);
     const cudaError_t launched = cudaGraphLaunch(exec, st);
     if (kept && launched == cudaSuccess) {
-        if (kept->exec) cudaGraphExecDestroy(kept->exec);  // released once its last launch completes
+        kept->drop(ctx->retired);
         kept->exec = exec;
         kept->key.assign(reinterpret_cast<const unsigned char*>(key), reinterpret_cast<const unsigned char*>(key) + sizeof(*key));
     } else {
-        cudaGraphExecDestroy(exec);
+        ctx->retired.add(exec);
     }
     if (launched != cudaSuccess) {
         setError("%s: graph launch failed: %s", what, cudaGetErrorString(launched));
@@ -2506,7 +2524,7 @@ int renderAdaptive(x2_scene* s, uint32_t minSamples, uint32_t maxSamples, float 
     };
     const bool again = kept.exec && kept.key.size() == sizeof(key) && !std::memcmp(kept.key.data(), &key, sizeof(key));
     if (!again) {
-        kept.drop();
+        kept.drop(s->ctx->retired);
         // Built in segments: each captured onto the graph after the last segment's end nodes.
         GraphSegments g;
         g.st = st;
