@@ -117,11 +117,13 @@ def test_integrate_without_room_for_its_outputs(ctx):
 
 
 @pytest.mark.parametrize("entry", ["integrate", "trace_rays"])
-def test_long_lists_do_not_wait_for_other_streams(ctx, entry):
-    """A list beyond the context's kept scratch, with another stream of the program at work: the call ends first."""
+def test_long_lists_do_not_wait_for_other_streams(entry):
+    """A list beyond the context's kept scratch, with another stream of the program at work: the call ends first. (A context
+    of its own: one that has put by its most graphs destroys them first, which waits.)"""
     import torch
 
-    s, cfg, scene = closed_room(ctx, 2)
+    own = x2.Context(0)
+    s, cfg, scene = closed_room(own, 2)
     n = 1600000  # over 64 MB at 44 bytes
     rng = np.random.default_rng(5)
     if entry == "integrate":
@@ -145,6 +147,31 @@ def test_long_lists_do_not_wait_for_other_streams(ctx, entry):
     got = call(*args)
     waited = done.query()
     other.synchronize()
-    scene.free()
+    own.close()
     assert all(np.array_equal(a, b) for a, b in zip(got, want))
     assert not waited
+
+
+def test_scenes_share_the_context_s_memory(ctx):
+    """What per-sample calls and plain frames work in belongs to the context: more scenes hold no more of it."""
+    import torch
+
+    scenes = [x2.Scene(ctx, s.desc, s.config) for s in [x2.SyntheticScene(108) for _ in range(4)]]
+    cfg = scenes[0].config
+    pixels = np.random.default_rng(6).integers(0, cfg.width * cfg.height, 1 << 19, dtype=np.uint32)
+
+    def use(scene):
+        rgba, status = scene.integrate(pixels, np.arange(len(pixels), dtype=np.uint32))
+        scene.frame_begin(1)
+        scene.render_frame(0, 1)
+        scene.wait()
+        return rgba, scene.film()[0]
+
+    first = use(scenes[0])
+    before = torch.cuda.mem_get_info()[0]
+    for scene in scenes[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(use(scene), first))
+    after = torch.cuda.mem_get_info()[0]
+    for scene in scenes:
+        scene.free()
+    assert before - after < 64 << 20  # films, chunk lists and counters

@@ -156,6 +156,13 @@ struct x2_ctx {
     unsigned char* scratch = nullptr;  // a host caller's arrays during x2_integrate or x2_trace_rays
     size_t scratchBytes = 0;
     bool scratchLent = false;
+    // What per-sample calls and plain frames work in, whichever scene makes them (the one stream orders them), grown to the
+    // largest use and given back with the context: a sample call's path state and outputs (kPairBytes and a window's
+    // outputs at most), the plain megakernel's lists (stepLists).
+    unsigned char* pairMemory = nullptr;
+    size_t pairBytes = 0;
+    float4* stepLists = nullptr;
+    size_t stepThreads = 0;
 };
 
 // An adaptive frame's device state (adaptive.h AdaptiveArgs) and its host-side layout.
@@ -244,15 +251,9 @@ struct x2_scene {
     x2_chunk* staging = nullptr;  // pinned
     uint32_t stagingCap = 0;
     Counters total{};
-    // the per-sample API's scratch: its counters, a window's item outputs and its drain's words
+    // the per-sample API's counters and its drain's words
     Slot integrateSlot;
-    unsigned char* pairMemory = nullptr;
-    float4* pairOut = nullptr;
-    uint8_t* pairStatus = nullptr;
-    uint32_t pairCap = 0;
     uint32_t* pairWords = nullptr;
-    float4* stepLists = nullptr;  // the plain megakernel's lists
-    size_t stepThreads = 0;
     unsigned long long* auditWord = nullptr;
     TraversalStats* stats = nullptr;  // device
     bool counting = false;
@@ -438,7 +439,31 @@ void freeWave(x2_scene* s) {
     s->wavePaths = s->waveRecords = s->waveCap = 0;
 }
 
-// Path slots for `paths` paths with `records` shadow records each.
+// A launch's path slots and queues: `paths` slots with `records` shadow records each.
+void placeWave(Carve& m, WaveState& w, uint32_t*& extendQ, uint32_t*& shadowQ, uint32_t*& shadeQ, size_t paths, size_t records) {
+    const size_t P = paths, R = paths * records;
+    m.take(w.ray0, P), m.take(w.ray1, P), m.take(w.T, P), m.take(w.held, P), m.take(w.meta, P), m.take(w.branch, P), m.take(w.rad, P);
+    m.take(w.hit, P), m.take(w.state, P), m.take(w.item, P), m.take(w.ncount, P), m.take(w.sray0, R), m.take(w.sray1, R);
+    m.take(w.scontrib, R), m.take(w.svis, R), m.take(extendQ, kOctants * P), m.take(shadowQ, R), m.take(shadeQ, 3 * P);
+    m.take(w.lightJob, kLightJobWords * P), m.take(w.lightFlags, P);
+}
+
+// A scene's counters and words for its launches, on the device and pinned; false when there is no room.
+bool ensureWords(x2_scene* s) {
+    if (!s->deviceWords && !carve(&s->deviceWords, [&](Carve& m) {
+            m.take(s->waveCounters, kWaveCounters), m.take(s->claimed, 1), m.take(s->drainWords, 4), m.take(s->pairWords, 4);
+        }))
+        return false;
+    if (!s->hostWords) {
+        if (cudaMallocHost(&s->hostWords, sizeof(uint32_t) * 8) != cudaSuccess) return false;
+        std::memset(s->hostWords, 0, sizeof(uint32_t) * 8);
+        s->hostLast = s->hostWords;
+        s->hostDrain = s->hostWords + 4;
+    }
+    return true;
+}
+
+// The scene's path slots for `paths` paths with `records` shadow records each.
 // Buffers that already hold at least `paths` paths are kept (a launch indexes them by its own path count), so launches
 // of varying sizes (an adaptive frame's passes) allocate once.
 int ensureWave(x2_scene* s, uint32_t paths, uint32_t records) {
@@ -447,27 +472,7 @@ int ensureWave(x2_scene* s, uint32_t paths, uint32_t records) {
         return X2_OK;
     }
     freeWave(s);
-    WaveState& w = s->wave;
-    const size_t P = paths, R = size_t(paths) * records;
-    auto place = [&](Carve& m) {
-        m.take(w.ray0, P), m.take(w.ray1, P), m.take(w.T, P), m.take(w.held, P), m.take(w.meta, P), m.take(w.branch, P), m.take(w.rad, P);
-        m.take(w.hit, P), m.take(w.state, P), m.take(w.item, P), m.take(w.ncount, P), m.take(w.sray0, R), m.take(w.sray1, R);
-        m.take(w.scontrib, R), m.take(w.svis, R), m.take(s->extendQ, kOctants * P), m.take(s->shadowQ, R), m.take(s->shadeQ, 3 * P);
-        m.take(w.lightJob, kLightJobWords * P), m.take(w.lightFlags, P);
-    };
-    bool ok = carve(&s->waveMemory, place);
-    if (ok && !s->deviceWords) ok = carve(&s->deviceWords, [&](Carve& m) {
-        m.take(s->waveCounters, kWaveCounters), m.take(s->claimed, 1), m.take(s->drainWords, 4), m.take(s->pairWords, 4);
-    });
-    if (ok && !s->hostWords) {
-        ok = cudaMallocHost(&s->hostWords, sizeof(uint32_t) * 8) == cudaSuccess;
-        if (ok) {
-            std::memset(s->hostWords, 0, sizeof(uint32_t) * 8);
-            s->hostLast = s->hostWords;
-            s->hostDrain = s->hostWords + 4;
-        }
-    }
-    if (!ok) {
+    if (!carve(&s->waveMemory, [&](Carve& m) { placeWave(m, s->wave, s->extendQ, s->shadowQ, s->shadeQ, paths, records); }) || !ensureWords(s)) {
         cudaGetLastError();
         freeWave(s);
         setError("device allocation failed for %u wavefront paths", paths);
@@ -499,25 +504,28 @@ double volumeBytes(const x2_config& c, uint32_t records) {
 // scattering whose volume state fits kVolumeBudgetBytes (a caller may reserve any number of paths) and the device. Else
 // the march runs inside shade.
 constexpr double kVolumeBudgetBytes = 16e9;
-bool volumesApart(x2_scene* s, uint32_t paths, uint32_t records) {
+bool volumesFit(const x2_scene* s, uint32_t paths, uint32_t records) {
     const x2_config& c = s->config;
-    if (!s->volumeCount || c.max_volume_depth > 1 || c.volume_illumination_samples > 4096) return false;
-    const uint64_t tasks = volumeTasks(c);
-    if (tasks * paths > 0x7fffffffull || volumeBytes(c, records) * paths > kVolumeBudgetBytes) return false;
+    return s->volumeCount && c.max_volume_depth <= 1 && c.volume_illumination_samples <= 4096 && volumeTasks(c) * paths <= 0x7fffffffull &&
+           volumeBytes(c, records) * paths <= kVolumeBudgetBytes;
+}
+void placeVolume(Carve& m, VolumeWave& v, size_t paths, size_t records, uint64_t tasks) {
+    const size_t P = paths;
+    m.take(v.head, P), m.take(v.pass, P), m.take(v.light, P), m.take(v.parts, 2 * P * std::max<uint64_t>(tasks, 1));
+    m.take(v.crossings, x2::kMaxCrossings * P), m.take(v.checkpoints, x2::kVolumeCheckpoints * P), m.take(v.branch, records * P);
+    m.take(v.queue, P);
+}
+bool volumesApart(x2_scene* s, uint32_t paths, uint32_t records) {
+    if (!volumesFit(s, paths, records)) return false;
+    const uint64_t tasks = volumeTasks(s->config);
     if (paths <= s->volPaths && records == s->volRecords && tasks == s->volTasks) return true;
     freeVolumeWave(s);
-    x2::VolumeWave& v = s->vol;
-    const size_t P = paths;
-    if (!carve(&s->volMemory, [&](Carve& m) {
-            m.take(v.head, P), m.take(v.pass, P), m.take(v.light, P), m.take(v.parts, 2 * P * std::max<uint64_t>(tasks, 1));
-            m.take(v.crossings, x2::kMaxCrossings * P), m.take(v.checkpoints, x2::kVolumeCheckpoints * P), m.take(v.branch, records * P);
-            m.take(v.queue, P);
-        })) {
+    if (!carve(&s->volMemory, [&](Carve& m) { placeVolume(m, s->vol, paths, records, tasks); })) {
         cudaGetLastError();  // not enough memory: the form that needs none
         freeVolumeWave(s);
         return false;
     }
-    v.tasks = uint32_t(tasks);
+    s->vol.tasks = uint32_t(tasks);
     s->volPaths = paths;
     s->volRecords = records;
     s->volTasks = uint32_t(tasks);
@@ -708,6 +716,8 @@ int x2_close(x2_ctx* ctx) {
     cudaEventDestroy(ctx->side.fork);
     ctx->retired.destroy();
     cudaFree(ctx->scratch);
+    cudaFree(ctx->pairMemory);
+    cudaFree(ctx->stepLists);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
     return X2_OK;
@@ -1107,8 +1117,6 @@ int x2_scene_free(x2_scene* s) {
     cudaFree(s->counts);
     for (auto& sl : s->slots) freeSlot(sl);
     freeSlot(s->integrateSlot);
-    cudaFree(s->stepLists);
-    cudaFree(s->pairMemory);
     if (s->staging) cudaFreeHost(s->staging);
     delete s;
     return X2_OK;
@@ -1161,26 +1169,37 @@ int x2_scene_info(x2_scene* s, uint64_t* nodes, uint64_t* bvhBytes, uint64_t* tr
 }
 
 namespace {
-// A single scene's wavefront launch of `count` chunks (sl.chunks) and `items` items over `paths` path slots.
-WaveArgs launchArgs(x2_scene* s, Slot& sl, uint32_t paths, uint32_t records, unsigned long long items, uint32_t count) {
+// A sample call's path state and a window's outputs, in the context's memory.
+struct PairArrays {
+    WaveState w{};
+    uint32_t *extendQ = nullptr, *shadowQ = nullptr, *shadeQ = nullptr;
+    VolumeWave vol{};  // head null: the march runs inside shade
+    float4* out = nullptr;
+    uint8_t* status = nullptr;
+};
+
+// A single scene's wavefront launch of `count` chunks (sl.chunks) and `items` items over `paths` path slots, the scene's own
+// or a sample call's.
+WaveArgs launchArgs(x2_scene* s, Slot& sl, uint32_t paths, uint32_t records, unsigned long long items, uint32_t count,
+                    const PairArrays* pair = nullptr) {
     WaveArgs a;
     std::memset(static_cast<void*>(&a), 0, sizeof(a));  // its padding too: launches are compared by their bytes
-    if (volumesApart(s, paths, records)) {
-        a.vol = s->vol;
+    if (pair ? pair->vol.head != nullptr : volumesApart(s, paths, records)) {
+        a.vol = pair ? pair->vol : s->vol;
         a.vol.count = s->waveCounters + kWaveCounters - 1;
     }
     a.scene = viewOf(s);
-    a.w = s->wave;
+    a.w = pair ? pair->w : s->wave;
     a.paths = paths;
     a.recordsPerPath = records;
     a.chunks = sl.chunks;
     a.itemCount = items;
     a.samplesPerChunk = s->samplesPerChunk;
     a.claimed = s->claimed;
-    a.extendQ = s->extendQ;
+    a.extendQ = pair ? pair->extendQ : s->extendQ;
     a.extendCount = s->waveCounters;
     a.lastExtend = s->waveCounters + 1;
-    a.shadowQ = s->shadowQ;
+    a.shadowQ = pair ? pair->shadowQ : s->shadowQ;
     a.shadowCount = s->waveCounters + 2;
     a.shadowSlots = s->shadowOrder && !a.vol.head && a.recordsPerPath <= x2::kRecordSegments ? s->waveCounters + 8 : nullptr;
     a.extendSlots = s->extendBins ? s->waveCounters + 8 + x2::kRecordSegments : nullptr;
@@ -1188,7 +1207,7 @@ WaveArgs launchArgs(x2_scene* s, Slot& sl, uint32_t paths, uint32_t records, uns
     a.shadowNext = s->waveCounters + 4;
     // Volume scenes are shaded in the extend queue's order: its neighbouring slots hold samples of one pixel, whose
     // marches are alike; a per-lobe sort (or one by march length) scatters them and the march's lanes diverge more.
-    a.shadeQ = s->lobeQueues && !s->volumeCount ? s->shadeQ : nullptr;
+    a.shadeQ = s->lobeQueues && !s->volumeCount ? pair ? pair->shadeQ : s->shadeQ : nullptr;
     a.shadeCount = s->waveCounters + 5;
     a.adj = AdjointWave{};
     a.chunkMask = s->launchMask;
@@ -1196,8 +1215,8 @@ WaveArgs launchArgs(x2_scene* s, Slot& sl, uint32_t paths, uint32_t records, uns
     a.liveChunks = nullptr;
     a.refill = s->refill;
     a.triLimit = s->triLimit;
-    a.out = s->out;
-    a.outStatus = s->outStatus;
+    a.out = pair ? pair->out : s->out;
+    a.outStatus = pair ? pair->status : s->outStatus;
     a.counters = sl.counters;
     a.scenes = nullptr;
     a.chunkRequest = nullptr;
@@ -1208,7 +1227,7 @@ WaveArgs launchArgs(x2_scene* s, Slot& sl, uint32_t paths, uint32_t records, uns
 
 WaveKernels launchKernels(const x2_scene* s, const WaveArgs& a) {
     return waveKernels(s->traceBlocks, s->shadeBlocks, s->volumeCount != 0, s->triUV != nullptr, s->shortStack != 0, a.scene.stats != nullptr,
-                       s->shadeSplit != 0, s->wave.lightJob != nullptr ? s->lightSplit : 0u,
+                       s->shadeSplit != 0, a.w.lightJob != nullptr ? s->lightSplit : 0u,
                        s->triOverlap != 0 && s->shortStack != 0 && s->traceBlocks < 9, a.vol.head != nullptr);
 }
 
@@ -1340,10 +1359,10 @@ void dropScratch(x2_ctx* ctx, unsigned char* p, size_t bytes) {
 }
 
 // What a launch's path slots and queues must start with.
-void clearWave(x2_scene* s, uint32_t paths) {
+void clearWave(x2_scene* s, const WaveState& w, uint32_t paths) {
     cudaStream_t st = s->ctx->stream;
-    cudaMemsetAsync(s->wave.state, 0, sizeof(uint32_t) * paths, st);
-    cudaMemsetAsync(s->wave.ncount, 0, sizeof(uint32_t) * paths, st);
+    cudaMemsetAsync(w.state, 0, sizeof(uint32_t) * paths, st);
+    cudaMemsetAsync(w.ncount, 0, sizeof(uint32_t) * paths, st);
     cudaMemsetAsync(s->claimed, 0, sizeof(unsigned long long), st);
     cudaMemsetAsync(s->waveCounters, 0, sizeof(uint32_t) * kWaveCounters, st);
 }
@@ -1370,39 +1389,46 @@ uint32_t pairPaths(x2_scene* s, uint64_t n, const uint32_t* pairs) {
 }
 int integrateWavefront(x2_scene* s, uint32_t paths, const uint32_t* pairs, uint64_t n, double* rgba, uint32_t* status) {
     const uint32_t records = s->config.light_count * s->config.light_samples + 1;
-    // The last frame launch's description (x2_wavefront_info) stays its own.
-    const uint32_t framePaths = s->wavePaths;
-    const int rc = ensureWave(s, paths, records);
-    if (framePaths) s->wavePaths = framePaths;
-    if (rc) return rc;
     const uint32_t window = uint32_t(std::min<uint64_t>(n, kPairWindow));
-    if (window > s->pairCap) {
-        cudaFree(s->pairMemory);
-        s->pairCap = 0;
-        if (!carve(&s->pairMemory, [&](Carve& m) { m.take(s->pairOut, window), m.take(s->pairStatus, window); })) {
-            cudaGetLastError();  // the caller goes on without
-            setError("device allocation failed for %u samples' outputs", window);
-            return X2_ENOMEM;
-        }
-        s->pairCap = window;
+    x2_ctx* ctx = s->ctx;
+    cudaStream_t st = ctx->stream;
+    PairArrays pair;
+    const bool apart = volumesFit(s, paths, records);
+    auto place = [&](Carve& m) {
+        placeWave(m, pair.w, pair.extendQ, pair.shadowQ, pair.shadeQ, paths, records);
+        if (apart) placeVolume(m, pair.vol, paths, records, volumeTasks(s->config));
+        m.take(pair.out, window), m.take(pair.status, window);
+    };
+    Carve size;
+    place(size);
+    if (size.size > ctx->pairBytes) {
+        cudaFree(ctx->pairMemory);  // once its work is done
+        ctx->pairBytes = 0;
+        if (cudaMalloc(&ctx->pairMemory, size.size) != cudaSuccess) ctx->pairMemory = nullptr;
+        if (ctx->pairMemory) ctx->pairBytes = size.size;
     }
-    cudaStream_t st = s->ctx->stream;
-    const WaveGrids grids = waveGrids(paths, records, s->ctx->smCount, s->blocksPerSm);
+    if (!ctx->pairMemory || !ensureWords(s)) {
+        cudaGetLastError();  // the caller goes on without
+        setError("device allocation failed for %u samples' path state", window);
+        return X2_ENOMEM;
+    }
+    Carve within{ctx->pairMemory, 0};
+    place(within);
+    pair.vol.tasks = uint32_t(apart ? volumeTasks(s->config) : 0);
+    const WaveGrids grids = waveGrids(paths, records, ctx->smCount, s->blocksPerSm);
     for (uint64_t first = 0; first < n; first += window) {
         const uint32_t items = uint32_t(std::min<uint64_t>(window, n - first));
-        clearWave(s, paths);
-        cudaMemsetAsync(s->pairStatus, X2_SKIP, items, st);
-        WaveArgs a = launchArgs(s, s->integrateSlot, paths, records, items, 0);
+        clearWave(s, pair.w, paths);
+        cudaMemsetAsync(pair.status, X2_SKIP, items, st);
+        WaveArgs a = launchArgs(s, s->integrateSlot, paths, records, items, 0, &pair);
         a.pairs = pairs + 2 * first;
-        a.out = s->pairOut;
-        a.outStatus = s->pairStatus;
         const uint64_t bound = uint64_t(items) * (uint64_t(s->config.max_depth) + 2) / paths + uint64_t(s->config.max_depth) + 64;
         const WaveKernels wk = launchKernels(s, a);
         const uint32_t most = uint32_t(std::min<uint64_t>(bound, 0xffffffffu));
         const DrainKey key = drainKey(wk, a, grids, most, items, rgba + 4 * first, status + first, nullptr);
-        const int done = launchDrain(s->ctx, a, s->pairWords, most, "x2_integrate",
-                                     [&] { launchIteration(wk, a, grids, st, false, &s->ctx->side); }, [&] {
-            wfPairsOut<<<(items + 255) / 256, 256, 0, st>>>(s->pairOut, s->pairStatus, items, rgba + 4 * first, status + first,
+        const int done = launchDrain(ctx, a, s->pairWords, most, "x2_integrate",
+                                     [&] { launchIteration(wk, a, grids, st, false, &ctx->side); }, [&] {
+            wfPairsOut<<<(items + 255) / 256, 256, 0, st>>>(pair.out, pair.status, items, rgba + 4 * first, status + first,
                                                             s->integrateSlot.counters);
         }, &s->pairGraph, &key);
         if (done) return done;
@@ -1570,20 +1596,20 @@ int x2_frame_begin_adaptive(x2_scene* s, uint32_t samplesPerChunk) {
 }
 
 namespace {
-// renderSteps's lists for `threads` threads, kept with the scene (launches run one after another on the context's
-// stream), or null when the device has no room for them.
-float4* stepLists(x2_scene* s, size_t threads) {
-    if (threads <= s->stepThreads) return s->stepLists;
-    cudaFree(s->stepLists);
-    s->stepLists = nullptr;
-    s->stepThreads = 0;
-    if (cudaMalloc(&s->stepLists, sizeof(float4) * kStepListWords * threads) != cudaSuccess) {
+// renderSteps's lists for `threads` threads, kept with the context (launches run one after another on its stream), or null
+// when the device has no room for them.
+float4* stepLists(x2_ctx* ctx, size_t threads) {
+    if (threads <= ctx->stepThreads) return ctx->stepLists;
+    cudaFree(ctx->stepLists);
+    ctx->stepLists = nullptr;
+    ctx->stepThreads = 0;
+    if (cudaMalloc(&ctx->stepLists, sizeof(float4) * kStepListWords * threads) != cudaSuccess) {
         cudaGetLastError();
-        s->stepLists = nullptr;
+        ctx->stepLists = nullptr;
         return nullptr;
     }
-    s->stepThreads = threads;
-    return s->stepLists;
+    ctx->stepThreads = threads;
+    return ctx->stepLists;
 }
 }  // namespace
 
@@ -1638,7 +1664,7 @@ int x2_launch(x2_scene* s, const x2_chunk* chunks, uint32_t count) {
         uint64_t(s->config.light_count) * s->config.light_samples + s->config.bsdf_samples <= kStepRecords) {
         auto* steps = s->triUV ? renderStepsTextured<4> : renderSteps<4>;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, steps, kRenderBlock, 0);
-        a.lists = stepLists(s, size_t(s->ctx->smCount) * std::max(perSm, 1) * kRenderBlock);
+        a.lists = stepLists(s->ctx, size_t(s->ctx->smCount) * std::max(perSm, 1) * kRenderBlock);
         if (a.lists) kernel = steps;  // else no room for its lists: the kernel that needs none
     }
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, kRenderBlock, 0);
@@ -1803,7 +1829,7 @@ int x2_launch_wavefront(x2_scene* s, const x2_chunk* chunks, uint32_t count) {
     if (int rc = ensureItems(s, items)) return rc;
     cudaStream_t st = s->ctx->stream;
     CUDA_OR(cudaMemcpyAsync(sl.chunks, chunks, sizeof(x2_chunk) * count, cudaMemcpyHostToDevice, st), X2_ECUDA);
-    clearWave(s, paths);
+    clearWave(s, s->wave, paths);
     cudaMemsetAsync(sl.counters, 0, sizeof(Counters), st);
     cudaMemsetAsync(s->outStatus, X2_SKIP, items, st);
     const WaveArgs a = launchArgs(s, sl, paths, records, items, count);
