@@ -175,3 +175,22 @@ def test_scenes_share_the_context_s_memory(ctx):
     for scene in scenes:
         scene.free()
     assert before - after < 64 << 20  # films, chunk lists and counters
+
+
+def test_build_memory(ctx):
+    """The BVH build's peak in the device's pool, a triangle: no more than the 384 bytes of the build without the wide nodes'
+    cost tables."""
+    lib = C.CDLL("libcuda.so.1")
+    pool, high, zero = C.c_void_p(), C.c_uint64(), C.c_uint64(0)
+    assert lib.cuDeviceGetDefaultMemPool(C.byref(pool), ctx.device) == 0
+    s = x2.SyntheticScene(11)
+    x2.Scene(ctx, s.desc, s.config).free()
+    ctx.synchronize()
+    current = C.c_uint64()
+    assert lib.cuMemPoolGetAttribute(pool, 7, C.byref(current)) == 0
+    assert lib.cuMemPoolSetAttribute(pool, 8, C.byref(zero)) == 0  # CU_MEMPOOL_ATTR_USED_MEM_HIGH
+    x2.Scene(ctx, s.desc, s.config).free()
+    assert lib.cuMemPoolGetAttribute(pool, 8, C.byref(high)) == 0
+    each = (high.value - current.value) / s.desc.triangle_count
+    print(f"build peak: {each:.1f} bytes a triangle")
+    assert each < 385

@@ -610,6 +610,10 @@ int buildBvh(const float* dVertices, const uint32_t* dTriangles, uint32_t n, cud
         return 1;
     }
     const uint32_t bn = n > 1 ? 2 * n - 1 : 1;
+    auto release = [&](auto*& p) {
+        if (p) cudaFreeAsync(p, stream);
+        p = nullptr;
+    };
     Aabb *triBox = nullptr, *box = nullptr;
     uint64_t *keys = nullptr, *keysSorted = nullptr;
     uint32_t *values = nullptr, *order = nullptr, *left = nullptr, *right = nullptr, *parent = nullptr, *count = nullptr;
@@ -663,6 +667,9 @@ int buildBvh(const float* dVertices, const uint32_t* dTriangles, uint32_t n, cud
         restructure<<<grid, kBlock, 0, stream>>>(n, left, right, parent, box, count, cost, flags);
         CK(cudaGetLastError());
     }
+    // What the hierarchy was made from is done with: freed before the cuts' tables come, so that these do not raise the
+    // build's peak.
+    release(triBox), release(keys), release(keysSorted), release(values), release(cost), release(temp);
     CK(cudaMallocAsync(&wide, sizeof(float) * 7 * size_t(n), stream));
     CK(cudaMallocAsync(&choice, sizeof(uint32_t) * n, stream));
     CK(cudaMemsetAsync(flags, 0, sizeof(unsigned) * n, stream));
@@ -733,32 +740,11 @@ int buildBvh(const float* dVertices, const uint32_t* dTriangles, uint32_t n, cud
     nodes = nullptr;
     tris = nullptr;
 fail:
-    cudaFreeAsync(triBox, stream);
-    cudaFreeAsync(box, stream);
-    cudaFreeAsync(keys, stream);
-    cudaFreeAsync(keysSorted, stream);
-    cudaFreeAsync(values, stream);
-    cudaFreeAsync(order, stream);
-    cudaFreeAsync(left, stream);
-    cudaFreeAsync(right, stream);
-    cudaFreeAsync(parent, stream);
-    cudaFreeAsync(count, stream);
-    cudaFreeAsync(cost, stream);
-    cudaFreeAsync(wide, stream);
-    cudaFreeAsync(choice, stream);
-    cudaFreeAsync(flags, stream);
-    cudaFreeAsync(sceneBox, stream);
-    cudaFreeAsync(counters, stream);
-    cudaFreeAsync(qa, stream);
-    cudaFreeAsync(qb, stream);
-    cudaFreeAsync(temp, stream);
-    if (nodes) cudaFreeAsync(nodes, stream);
-    if (tris) cudaFreeAsync(tris, stream);
+    release(triBox), release(box), release(keys), release(keysSorted), release(values), release(order), release(left), release(right);
+    release(parent), release(count), release(cost), release(wide), release(choice), release(flags), release(sceneBox), release(counters);
+    release(qa), release(qb), release(temp), release(nodes), release(tris);
     if (!out->nodes)
-        for (TriRec*& r : out->rot) {
-            if (r) cudaFreeAsync(r, stream);
-            r = nullptr;
-        }
+        for (TriRec*& r : out->rot) release(r);
     cudaStreamSynchronize(stream);
     return out->nodes ? 0 : 1;
 }
