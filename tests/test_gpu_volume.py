@@ -185,3 +185,28 @@ def test_volume_kernels_equal_the_march_inside_shade(ctx, estimator, overlap, vo
     assert np.abs(films[0][:, :3]).sum() > 0 or width * height == 1
     for film in films[1:]:
         assert np.allclose(film, films[0], rtol=1e-12, atol=1e-12)  # the FP64 film's own summation order
+
+
+@pytest.mark.parametrize("estimator", [0, 1])
+def test_volume_kernels_without_illumination_samples(ctx, estimator):
+    """volume_illumination_samples 0: no ray takes a scattering sample (a camera ray's count is 0, and every bounce counts
+    as a scattering). The volumes in kernels of their own against the plain form's march inside the vertex."""
+    s = x2.SyntheticScene(33)
+    d, cfg = s.desc, x2.Config.from_buffer_copy(s.config)
+    cfg.width, cfg.height, cfg.volume_estimator = 64, 48, estimator
+    d.volumes[0].bound_lo[0] = 0.2  # the medium on one side: the other side's rays reach it after a bounce only
+    films = {}
+    scene = x2.Scene(ctx, d, cfg)
+    for samples in (1, 0):  # the second's path slots hold the first's parts
+        cfg.volume_illumination_samples = samples
+        scene.set_config(cfg)
+        films[samples] = []
+        for render in (scene.render_frame, scene.render_frame_wavefront):
+            scene.frame_begin(3)
+            render(0, 3)
+            scene.wait()
+            films[samples].append(scene.film()[0])
+    scene.free()
+    for plain, wave in films.values():
+        assert np.allclose(wave, plain, rtol=1e-12, atol=1e-12)
+    assert not np.allclose(films[0][0], films[1][0], rtol=1e-3)  # the samples matter here
