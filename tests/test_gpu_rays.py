@@ -50,7 +50,7 @@ def every_triangle(v, o, d, far):
 
 
 @pytest.mark.parametrize("triangles,rays", [(1, 1), (2, 31), (3, 33), (4, 500), (5, 500), (8, 129), (9, 500), (24, 500), (25, 500), (300, 4097), (1500, 2001),
-                                            (5, 90001), (1500, 90001)])
+                                            (5, 90001), (1500, 90001), (29, 500), (30, 500)])  # 4 and 5 nodes: the two kernels
 def test_rays_against_every_triangle(ctx, triangles, rays):
     scene, v = soup(ctx, triangles, 100 + triangles)
     rng = np.random.default_rng(triangles)

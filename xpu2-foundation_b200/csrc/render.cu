@@ -423,9 +423,8 @@ __global__ void __launch_bounds__(kRenderBlock) integratePairsVolumes(SceneView 
     integratePairsBody<true, true>(s, pairs, n, rgba, status, counters);
 }
 
-// Closest hit and occlusion for n rays (8 floats each: origin, direction, near, far).
-// The ray entry one thread a ray, both walks one after the other: scenes of a few nodes, whose walks are over before
-// refilled lanes pay (kRayWalkNodes).
+// The ray entry: closest hit and occlusion for n rays (8 floats each: origin, direction, near, far). One thread a ray, both
+// walks one after the other: scenes of a few nodes (kRayWalkNodes).
 __global__ void traceRaysDirect(SceneView s, const float* __restrict__ rays, unsigned long long n, uint32_t* __restrict__ tri,
                                 float* __restrict__ t, uint32_t* __restrict__ occluded) {
     const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
@@ -443,7 +442,7 @@ __global__ void traceRaysDirect(SceneView s, const float* __restrict__ rays, uns
     }
 }
 
-// The ray entry: query 2 i is ray i's closest hit (when a caller wants it), 2 i + 1 its occlusion, walked a node a step by
+// The same for larger scenes: query 2 i is ray i's closest hit (when a caller wants it), 2 i + 1 its occlusion, walked a node a step by
 // persistent warps whose idle lanes take the next queries (as the wavefront's traversal kernels). One thread a ray, both
 // walks one after the other, took 0.225 ms for 262,139 scattered rays (0.111 so): a warp waited for its longest walk
 // twice. next: the fetch counter, at zero; null where the grid has a lane for every query, which then takes its own (a few

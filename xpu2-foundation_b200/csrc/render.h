@@ -46,10 +46,13 @@ __global__ void integratePairsTextured(SceneView s, const uint32_t* pairs, unsig
                                        Counters* counters);
 __global__ void integratePairsVolumes(SceneView s, const uint32_t* pairs, unsigned long long n, double* rgba, uint32_t* status,
                                       Counters* counters);
-// The ray entry: traceRays for BVHs of at least kRayWalkNodes nodes, traceRaysDirect below. 262,139 rays on the device,
-// walked and direct, by the BVH's nodes: 5 0.069 and 0.071 ms, 23 0.197 and 0.272, 235 0.263 and 0.452, 2,975 0.390 and
-// 0.670; a million rays of the closed box (3 nodes), host arrays in and out, 2.70 and 2.48.
-constexpr uint32_t kRayWalkNodes = 8;
+// The ray entry: traceRays for BVHs of at least kRayWalkNodes nodes, traceRaysDirect below, whose few steps are over before
+// refilled lanes pay for the fetches. Device us a call for 2,000, 262,139 and a million rays, walked then direct, by the
+// BVH's nodes (random triangles, and the closed box): 1 6.3 21.5 59.7, 6.3 16.6 47.3; 2 10.4 41.2 118, 8.4 30.9 97; the box's
+// 3 16.6 61.7 177, 12.5 41.2 135; 4 12.5 57.1 160, 12.5 48.4 187; 5 12.4 61.2 178, 12.6 60.4 228; 8 14.8 84.8 265, 20.6 97.7
+// 390; 9 18.6 116 379, 20.6 117 533; 14 24.8 150 494, 39.1 194 739. At 4 nodes the direct kernel is the faster for up to some
+// hundred thousand rays, from 5 the walked one for all.
+constexpr uint32_t kRayWalkNodes = 5;
 __global__ void traceRaysDirect(SceneView s, const float* rays, unsigned long long n, uint32_t* tri, float* t, uint32_t* occluded);
 __global__ void traceRays(SceneView s, const float* rays, unsigned long long n, uint32_t* tri, float* t, uint32_t* occluded,
                           unsigned long long* next);
