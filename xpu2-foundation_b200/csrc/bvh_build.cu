@@ -316,9 +316,12 @@ __global__ void restructure(uint32_t n, uint32_t* left, uint32_t* right, uint32_
 // choice: bits 3 (j - 2) the left child's share of the best split of j = 2..8 slots, bits 21 + (i - 2) whether i = 2..7
 // slots are split (else i - 1 serve as well). Opening the largest subtree first instead left wide nodes of 7.1 triangles
 // on the 12.3M-triangle field (small subtrees got nodes of their own). A ray's triangle tests ride along with its node
-// visits (walkStepOverlap: 7 of 32 lanes test in nearly every step), so a test costs less than a visit, but not nothing:
-// on that field (extend and shadow ms of a frame, visits and tests a shadow ray) largest first 132.8, 461.3, 19.9, 5.8;
-// kWideTri 0.1 135.1, 454.2, 19.0, 6.4; 0.3 133.3, 448.9, 19.0, 5.9; 0.6 131.7, 444.0, 19.3, 5.1.
+// visits (walkStepOverlap: 7 of 32 lanes test in nearly every step), so a test costs less than a visit, but not nothing.
+// Frames of four fields, three generator seeds each (ms; the same frame's two runs within 0.1 %), largest first and
+// kWideTri 0.6: 12.3M triangles, 16 samples 202.2 203.7, 214.4 210.3, 214.0 209.3; 1.16M, 16 samples 179.5 176.8, 183.3
+// 180.5, 192.5 190.4; 771k, 64 samples 31.3 31.0, 34.0 33.3, 33.6 33.2; 191k, 128 samples 12.7 12.5, 14.3 14.3, 12.1 11.9:
+// eleven faster by up to 2.2 %, one slower by 0.7 % (the field that the bench draws). 0.1 and 0.3 are slower than 0.6 on
+// all twelve, 0.8 and 1 within 0.25 % of it.
 constexpr float kWideNode = 1.0f, kWideTri = 0.6f;
 __global__ void wideCosts(uint32_t n, const uint32_t* __restrict__ left, const uint32_t* __restrict__ right, const uint32_t* __restrict__ parent,
                           const Aabb* __restrict__ box, const uint32_t* __restrict__ count, float* c, uint32_t* choice, unsigned* flags) {
