@@ -286,9 +286,9 @@ struct x2_scene {
     uint8_t* outStatus = nullptr;
     uint64_t outCap = 0, lastItems = 0;
     uint32_t waveIterations = 0;       // of the last wavefront launch
+    KeptGraph frameGraph, pairGraph, adaptiveGraph;  // the last frame launch's, per-sample launch's and adaptive frame's graph
     // The asynchronous wavefront launch's drain: [0] its iterations, [1] a running total, [2] its overrun word
     // (device; 4 words), their host copy (pinned), the launch they belong to (0: none pending) and its bound.
-    KeptGraph frameGraph, pairGraph, adaptiveGraph;  // the last frame launch's, per-sample launch's and adaptive frame's graph
     uint32_t* drainWords = nullptr;
     uint32_t* hostDrain = nullptr;
     uint64_t drainSeq = 0;
@@ -301,18 +301,18 @@ struct x2_scene {
     const uint32_t* launchBase = nullptr;
     // the adaptive frame's state (x2_render_adaptive, x2_adaptive_step)
     AdaptiveState* adaptiveState = nullptr;
-    // the adjoint's wavefront state (x2_adjoint): vertex records, scales, counts, dL/dI shares, record auxiliaries
     x2::VolumeWave vol{};                 // a volume scene's wavefront state (its volumes in kernels of their own)
     unsigned char* volMemory = nullptr;
     uint32_t volPaths = 0, volRecords = 0, volTasks = 0;  // the paths, records and samples its buffers hold
+    // the adjoint's wavefront state (x2_adjoint): vertex records, scales, counts, dL/dI shares, record auxiliaries
     uint4* avert = nullptr;
     float4* ascale = nullptr;
     uint32_t* avcount = nullptr;
     float4* adelta = nullptr;
     uint2* aaux = nullptr;
     float4* atex = nullptr;
-    float *adjGradRows = nullptr, *adjTexGrad = nullptr;  // the gradients' rows, the texels', the FP64 sums
-    double* adjGrads = nullptr;
+    float *adjGradRows = nullptr, *adjTexGrad = nullptr;  // the gradients' rows and the texels'
+    double* adjGrads = nullptr;                           // the rows' FP64 sums
     uint32_t adjParams = 0;
     uint64_t adjTexels = 0;
     uint32_t adjPaths = 0, adjVerts = 0, adjRecords = 0;  // paths the adjoint's buffers hold; their vertices, records
@@ -1231,11 +1231,8 @@ WaveKernels launchKernels(const x2_scene* s, const WaveArgs& a) {
                        s->triOverlap != 0 && s->shortStack != 0 && s->traceBlocks < 9, a.vol.head != nullptr);
 }
 
-// A launch as one graph on the context's stream: its iterations (what iteration() enqueues) in a conditional while node,
-// each iteration's last kernel deciding whether another follows (at most `bound`; past that it raises words[2]), then what
-// tail() enqueues. words: 4 device words, cleared here.
-// A launch whose key (everything its kernels are launched with) is the last one's launches that one's graph again: building
-// and instantiating one takes the host about 0.2 ms.
+// Everything a launch's kernels are launched with, the camera and the config (its seed) within the arguments: a launch whose
+// key is the last one's launches that one's graph again.
 struct DrainKey {
     WaveKernels kernels;
     WaveArgs args;
@@ -1243,6 +1240,10 @@ struct DrainKey {
     uint32_t bound, tail;
     const void* out[3];
 };
+// A launch as one graph on the context's stream: its iterations (what iteration() enqueues) in a conditional while node,
+// each iteration's last kernel deciding whether another follows (at most `bound`; past that it raises words[2]), then what
+// tail() enqueues. words: 4 device words, cleared here. kept and key: the graph is kept for the next launch like it
+// (building and instantiating one takes the host about 0.2 ms); null: it is not.
 int launchDrain(x2_ctx* ctx, const WaveArgs& a, uint32_t* words, uint32_t bound, const char* what, const std::function<void()>& iteration,
                 const std::function<void()>& tail, KeptGraph* kept = nullptr, const DrainKey* key = nullptr) {
     cudaStream_t st = ctx->stream;
@@ -1896,8 +1897,8 @@ int x2_launch_wavefront(x2_scene* s, const x2_chunk* chunks, uint32_t count) {
         s->waveIterations = iterations;
         return X2_OK;
     }
-    // One graph, kept for the next launch like it: the launch's iterations, then the film reduce. The launch runs without the host; x2_poll / x2_wait
-    // collect it like any launch.
+    // One graph, kept for the next launch like it: the launch's iterations, then the film reduce. The launch runs without the
+    // host; x2_poll / x2_wait collect it like any launch.
     const uint32_t bound = uint32_t(std::min<uint64_t>(maxIter, 0xffffffffu));
     cudaEventRecord(sl.begin, st);
     const DrainKey key = drainKey(wk, a, grids, bound, count, s->sums, s->adaptive ? s->odd : nullptr, s->counts);

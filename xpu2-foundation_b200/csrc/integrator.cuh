@@ -133,13 +133,8 @@ __device__ __forceinline__ void cameraPending(const CameraRay& camera, Pending& 
     p0.held = V3{0, 0, 0};
 }
 
-// After a ray is traced, before its hit is shaded: the light its BSDF sample held is settled (bounce-ray reuse:
-// reached unless the ray met something short of the shadow ray's end; lightShadowKept is 0 without a clear radius),
-// then, on a camera ray, the lights the camera sees (async_integrator.h:2095-2106, :2172-2185).
-// With volumes, the volumes the ray passes on its way (async_integrator.h:2107-2118): their light, the throughput
-// through them (pv's T and volume depth change) and, for a camera ray that hits nothing, their opacity as its alpha.
-// kVolumes false compiles the volume code out (the kernels for scenes without volumes: the march's state would
-// otherwise take registers and stack from every surface vertex); a scene with volumes takes the kVolumes form.
+// What afterTrace does before a ray's volumes: the light its BSDF sample held is settled (bounce-ray reuse: reached
+// unless the ray met something short of the shadow ray's end; lightShadowKept is 0 without a clear radius).
 __device__ __forceinline__ void afterHeld(const Pending& pv, const Hit& hit, V3& radiance) {
     if (pv.heldLight != ~0u) {
         const float kept = hit.geom != ~0u && hit.t < pv.heldFar ? 0.0f : 1.0f;
@@ -158,6 +153,13 @@ __device__ __forceinline__ void afterVolumes(const SceneView& s, const Identity&
         radiance = add(radiance, Lv);
     }
 }
+// After a ray is traced, before its hit is shaded: the held light (afterHeld), then, on a camera ray, the lights the camera
+// sees (async_integrator.h:2095-2106, :2172-2185).
+// With volumes, the volumes the ray passes on its way (async_integrator.h:2107-2118): their light, the throughput
+// through them (pv's T and volume depth change) and, for a camera ray that hits nothing, their opacity as its alpha.
+// kVolumes false compiles the volume code out (the kernels for scenes without volumes: the march's state would
+// otherwise take registers and stack from every surface vertex); a scene with volumes takes the kVolumes form, or has its
+// volumes in kernels of their own (wavefront.cu), between afterHeld and afterVolumes.
 template <bool kVolumes = true>
 __device__ __forceinline__ void afterTrace(const SceneView& s, const Identity& root, Pending& pv, const Hit& hit, V3 cameraPosition,
                                            V3& radiance, float& alpha) {

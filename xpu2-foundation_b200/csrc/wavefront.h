@@ -55,7 +55,7 @@ struct AdjointWave {
     float* texGrad;      // FP32 dL/dtexel, 3 a texel over the scene's textures; null: not wanted
 };
 
-// A volume scene's rays in kernels of their own (march null: the march runs inside shade). Per path slot: the first
+// A volume scene's rays in kernels of their own (head null: the march runs inside shade). Per path slot: the first
 // march's result (VolumeHead), the ray's transmittance and what its volumes emit (and, in light.w, where the ray ends),
 // its crossings and the march's checkpoints, and the parts its scattering samples add (two a sample); per shadow record
 // the branch of its transmittance's stream (its depth waits in scontrib.w); and the slots whose rays scatter.
@@ -198,8 +198,8 @@ void launchAdjointIteration(const WaveKernels& k, const AdjointKernels& adj, con
 __global__ void wfGradRows(const float* rows, uint32_t rowCount, uint32_t params, double* grads);
 __global__ void wfResetQueues(WaveArgs a);
 // The drain loop's test, last in the body of a conditional while node: go on while the iteration extended a ray, at
-// most maxIterations times (then *overrun is set and the loop ends); the queues are reset for the next iteration. iterations[0] counts this loop's iterations,
-// iterations[1] a running total.
+// most maxIterations times (then *overrun is set and the loop ends); the queues are reset for the next iteration.
+// iterations[0] counts this loop's iterations, iterations[1] a running total.
 __global__ void wfDrainCheck(WaveArgs a, cudaGraphConditionalHandle loop, uint32_t* iterations, uint32_t maxIterations,
                              uint32_t* overrun);
 __global__ void wfFilmReduce(WaveArgs a, uint32_t chunkCount, double* sums, double* odd, uint32_t* counts);
