@@ -670,11 +670,11 @@ int buildBvh(const float* dVertices, const uint32_t* dTriangles, uint32_t n, cud
         restructure<<<grid, kBlock, 0, stream>>>(n, left, right, parent, box, count, cost, flags);
         CK(cudaGetLastError());
     }
-    // What the hierarchy was made from is done with: freed before the cuts' tables come, so that these do not raise the
-    // build's peak.
-    release(triBox), release(keys), release(keysSorted), release(values), release(cost), release(temp);
-    CK(cudaMallocAsync(&wide, sizeof(float) * 7 * size_t(n), stream));
-    CK(cudaMallocAsync(&choice, sizeof(uint32_t) * n, stream));
+    // The cuts' tables lie in memory that the build holds anyway: the costs where the leaf triangles will be written, the
+    // choices, which the collapse reads while it writes those, over the restructuring's costs.
+    static_assert(sizeof(TriRec) >= 7 * sizeof(float) && sizeof(*cost) == sizeof(*choice), "the tables fit");
+    wide = reinterpret_cast<float*>(tris);
+    choice = reinterpret_cast<uint32_t*>(cost);
     CK(cudaMemsetAsync(flags, 0, sizeof(unsigned) * n, stream));
     wideCosts<<<grid, kBlock, 0, stream>>>(n, left, right, parent, box, count, wide, choice, flags);
     CK(cudaGetLastError());
@@ -744,7 +744,7 @@ int buildBvh(const float* dVertices, const uint32_t* dTriangles, uint32_t n, cud
     tris = nullptr;
 fail:
     release(triBox), release(box), release(keys), release(keysSorted), release(values), release(order), release(left), release(right);
-    release(parent), release(count), release(cost), release(wide), release(choice), release(flags), release(sceneBox), release(counters);
+    release(parent), release(count), release(cost), release(flags), release(sceneBox), release(counters);
     release(qa), release(qb), release(temp), release(nodes), release(tris);
     if (!out->nodes)
         for (TriRec*& r : out->rot) release(r);
