@@ -500,9 +500,9 @@ double volumeBytes(const x2_config& c, uint32_t records) {
            sizeof(x2::MarchCheckpoint) * double(x2::kVolumeCheckpoints) + 32.0 * double(volumeTasks(c)) + 8.0 * records;
 }
 
-// Whether a launch of `paths` slots runs its volumes in kernels of their own, and their buffers: a volume scene with single
-// scattering whose volume state fits kVolumeBudgetBytes (a caller may reserve any number of paths) and the device. Else
-// the march runs inside shade.
+// Whether a launch of `paths` slots runs its volumes in kernels of their own: a volume scene with single scattering whose
+// volume state fits kVolumeBudgetBytes (a caller may reserve any number of paths) and, volumesApart, the device, in the
+// scene's buffers. Else the march runs inside shade.
 constexpr double kVolumeBudgetBytes = 16e9;
 bool volumesFit(const x2_scene* s, uint32_t paths, uint32_t records) {
     const x2_config& c = s->config;
