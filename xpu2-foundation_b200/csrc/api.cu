@@ -117,9 +117,10 @@ struct Slot {
 
 using namespace x2;
 
-// Graphs that no launch will use again. Destroying one that holds a conditional node waits for every stream of the
+// Graphs that no sample call will use again. Destroying one that holds a conditional node waits for every stream of the
 // program, other libraries' too (a call behind a second's work elsewhere took that second), so they are put by and
-// destroyed a list at a time.
+// destroyed a list at a time. (Frames, batches and the adjoint destroy theirs at once, behind the launch, where the 0.2 ms
+// that it takes run beside the launch's kernels.)
 struct RetiredGraphs {
     static constexpr size_t kMost = 32;
     std::vector<cudaGraphExec_t> execs;
@@ -138,8 +139,9 @@ struct RetiredGraphs {
 struct KeptGraph {
     cudaGraphExec_t exec = nullptr;
     std::vector<unsigned char> key;
-    void drop(RetiredGraphs& retired) {
-        retired.add(exec);
+    void drop(RetiredGraphs* retired = nullptr) {
+        if (retired) retired->add(exec);
+        else if (exec) cudaGraphExecDestroy(exec);  // released once its last launch completes
         exec = nullptr;
         key.clear();
     }
@@ -251,9 +253,9 @@ struct x2_scene {
     x2_chunk* staging = nullptr;  // pinned
     uint32_t stagingCap = 0;
     Counters total{};
-    // the per-sample API's counters and its drain's words
+    // the per-sample API's counters, its drain's words and its window's length
     Slot integrateSlot;
-    uint32_t* pairWords = nullptr;
+    uint32_t *pairWords = nullptr, *pairCount = nullptr;
     unsigned long long* auditWord = nullptr;
     TraversalStats* stats = nullptr;  // device
     bool counting = false;
@@ -451,7 +453,7 @@ void placeWave(Carve& m, WaveState& w, uint32_t*& extendQ, uint32_t*& shadowQ, u
 // A scene's counters and words for its launches, on the device and pinned; false when there is no room.
 bool ensureWords(x2_scene* s) {
     if (!s->deviceWords && !carve(&s->deviceWords, [&](Carve& m) {
-            m.take(s->waveCounters, kWaveCounters), m.take(s->claimed, 1), m.take(s->drainWords, 4), m.take(s->pairWords, 4);
+            m.take(s->waveCounters, kWaveCounters), m.take(s->claimed, 1), m.take(s->drainWords, 4), m.take(s->pairWords, 4), m.take(s->pairCount, 1);
         }))
         return false;
     if (!s->hostWords) {
@@ -1104,8 +1106,7 @@ int x2_scene_free(x2_scene* s) {
     cudaFree(s->grids);
     for (float* g : s->gridValues) cudaFree(g);
     for (float* m : s->majorants) cudaFree(m);
-    for (KeptGraph* g : {&s->frameGraph, &s->pairGraph, &s->adaptiveGraph})
-        if (g->exec) cudaGraphExecDestroy(g->exec);
+    for (KeptGraph* g : {&s->frameGraph, &s->pairGraph, &s->adaptiveGraph}) g->drop();
     freeWave(s);
     freeVolumeWave(s);
     cudaFree(s->out);
@@ -1169,11 +1170,12 @@ int x2_scene_info(x2_scene* s, uint64_t* nodes, uint64_t* bvhBytes, uint64_t* tr
 }
 
 namespace {
-// A sample call's path state and a window's outputs, in the context's memory.
+// A sample call's path state, a window's list and its outputs, in the context's memory.
 struct PairArrays {
     WaveState w{};
     uint32_t *extendQ = nullptr, *shadowQ = nullptr, *shadeQ = nullptr;
     VolumeWave vol{};  // head null: the march runs inside shade
+    uint2* list = nullptr;
     float4* out = nullptr;
     uint8_t* status = nullptr;
 };
@@ -1242,10 +1244,11 @@ struct DrainKey {
 };
 // A launch as one graph on the context's stream: its iterations (what iteration() enqueues) in a conditional while node,
 // each iteration's last kernel deciding whether another follows (at most `bound`; past that it raises words[2]), then what
-// tail() enqueues. words: 4 device words, cleared here. kept and key: the graph is kept for the next launch like it
-// (building and instantiating one takes the host about 0.2 ms); null: it is not.
+// tail() enqueues (null: nothing). words: 4 device words, cleared here. kept and key: the graph is kept for the next launch
+// like it (building and instantiating one takes the host about 0.2 ms); null: it is not. retired: where the kept graph that
+// this launch replaces is put by (null: it is destroyed).
 int launchDrain(x2_ctx* ctx, const WaveArgs& a, uint32_t* words, uint32_t bound, const char* what, const std::function<void()>& iteration,
-                const std::function<void()>& tail, KeptGraph* kept = nullptr, const DrainKey* key = nullptr) {
+                const std::function<void()>& tail, KeptGraph* kept = nullptr, const DrainKey* key = nullptr, RetiredGraphs* retired = nullptr) {
     cudaStream_t st = ctx->stream;
     if (kept && kept->exec && kept->key.size() == sizeof(*key) && !std::memcmp(kept->key.data(), key, sizeof(*key))) {
         cudaMemsetAsync(words, 0, sizeof(uint32_t) * 4, st);
@@ -1281,7 +1284,7 @@ int launchDrain(x2_ctx* ctx, const WaveArgs& a, uint32_t* words, uint32_t bound,
         cudaGraph_t body = nullptr;
         check(cudaStreamEndCapture(st, &body));
     }
-    if (err == cudaSuccess && check(cudaStreamBeginCaptureToGraph(st, graph, &node, nullptr, 1, cudaStreamCaptureModeThreadLocal))) {
+    if (err == cudaSuccess && tail && check(cudaStreamBeginCaptureToGraph(st, graph, &node, nullptr, 1, cudaStreamCaptureModeThreadLocal))) {
         tail();
         check(cudaGetLastError());
         cudaGraph_t out = nullptr;
@@ -1297,11 +1300,11 @@ int launchDrain(x2_ctx* ctx, const WaveArgs& a, uint32_t* words, uint32_t bound,
     cudaMemsetAsync(words, 0, sizeof(uint32_t) * 4, st);
     const cudaError_t launched = cudaGraphLaunch(exec, st);
     if (kept && launched == cudaSuccess) {
-        kept->drop(ctx->retired);
+        kept->drop(retired);
         kept->exec = exec;
         kept->key.assign(reinterpret_cast<const unsigned char*>(key), reinterpret_cast<const unsigned char*>(key) + sizeof(*key));
     } else {
-        ctx->retired.add(exec);
+        cudaGraphExecDestroy(exec);
     }
     if (launched != cudaSuccess) {
         setError("%s: graph launch failed: %s", what, cudaGetErrorString(launched));
@@ -1384,13 +1387,19 @@ uint32_t pairPaths(x2_scene* s, uint64_t n, const uint32_t* pairs) {
         return 0;
     const uint64_t records = uint64_t(c.light_count) * c.light_samples + 1;
     const double perPath = pathBytes(uint32_t(records)) + (s->volumeCount ? volumeBytes(c, uint32_t(records)) : 0.0);
-    uint64_t paths = std::min<uint64_t>(std::max<uint64_t>(n, 1024), 1u << 20);
+    uint64_t paths = 1024;
+    while (paths < n && paths < (1u << 20)) paths <<= 1;
     while (paths > 1024 && double(paths) * perPath > kPairBytes) paths >>= 1;
     return double(paths) * perPath > kPairBytes ? 0u : uint32_t(paths);
 }
+// Nothing that a window's graph is launched with is the call's own: the list is copied to a place of its own, its length
+// lies in a word, the outputs are handed out behind the graph, and paths and window are powers of two. So lists of any
+// length between two of them find the last one's graph (with the caller's arrays in it every list of another length built
+// one, and put one by).
 int integrateWavefront(x2_scene* s, uint32_t paths, const uint32_t* pairs, uint64_t n, double* rgba, uint32_t* status) {
     const uint32_t records = s->config.light_count * s->config.light_samples + 1;
-    const uint32_t window = uint32_t(std::min<uint64_t>(n, kPairWindow));
+    uint32_t window = paths;
+    while (window < n && window < kPairWindow) window <<= 1;
     x2_ctx* ctx = s->ctx;
     cudaStream_t st = ctx->stream;
     PairArrays pair;
@@ -1398,7 +1407,7 @@ int integrateWavefront(x2_scene* s, uint32_t paths, const uint32_t* pairs, uint6
     auto place = [&](Carve& m) {
         placeWave(m, pair.w, pair.extendQ, pair.shadowQ, pair.shadeQ, paths, records);
         if (apart) placeVolume(m, pair.vol, paths, records, volumeTasks(s->config));
-        m.take(pair.out, window), m.take(pair.status, window);
+        m.take(pair.list, window), m.take(pair.out, window), m.take(pair.status, window);
     };
     Carve size;
     place(size);
@@ -1417,22 +1426,26 @@ int integrateWavefront(x2_scene* s, uint32_t paths, const uint32_t* pairs, uint6
     place(within);
     pair.vol.tasks = uint32_t(apart ? volumeTasks(s->config) : 0);
     const WaveGrids grids = waveGrids(paths, records, ctx->smCount, s->blocksPerSm);
+    WaveArgs a = launchArgs(s, s->integrateSlot, paths, records, window, 0, &pair);
+    a.pairs = reinterpret_cast<const uint32_t*>(pair.list);
+    a.liveChunks = s->pairCount;
+    a.samplesPerChunk = 0;
+    a.chunkMask = nullptr;
+    a.pixelBase = nullptr;
+    const uint32_t most = uint32_t(uint64_t(window) * (uint64_t(s->config.max_depth) + 2) / paths + uint64_t(s->config.max_depth) + 64);
+    const WaveKernels wk = launchKernels(s, a);
+    const DrainKey key = drainKey(wk, a, grids, most, 0, nullptr, nullptr, nullptr);
     for (uint64_t first = 0; first < n; first += window) {
         const uint32_t items = uint32_t(std::min<uint64_t>(window, n - first));
         clearWave(s, pair.w, paths);
         cudaMemsetAsync(pair.status, X2_SKIP, items, st);
-        WaveArgs a = launchArgs(s, s->integrateSlot, paths, records, items, 0, &pair);
-        a.pairs = pairs + 2 * first;
-        const uint64_t bound = uint64_t(items) * (uint64_t(s->config.max_depth) + 2) / paths + uint64_t(s->config.max_depth) + 64;
-        const WaveKernels wk = launchKernels(s, a);
-        const uint32_t most = uint32_t(std::min<uint64_t>(bound, 0xffffffffu));
-        const DrainKey key = drainKey(wk, a, grids, most, items, rgba + 4 * first, status + first, nullptr);
-        const int done = launchDrain(ctx, a, s->pairWords, most, "x2_integrate",
-                                     [&] { launchIteration(wk, a, grids, st, false, &ctx->side); }, [&] {
-            wfPairsOut<<<(items + 255) / 256, 256, 0, st>>>(pair.out, pair.status, items, rgba + 4 * first, status + first,
-                                                            s->integrateSlot.counters);
-        }, &s->pairGraph, &key);
-        if (done) return done;
+        cudaMemcpyAsync(pair.list, pairs + 2 * first, sizeof(uint2) * items, cudaMemcpyDeviceToDevice, st);
+        cudaMemcpyAsync(s->pairCount, &items, sizeof(items), cudaMemcpyHostToDevice, st);
+        if (int rc = launchDrain(ctx, a, s->pairWords, most, "x2_integrate",
+                                 [&] { launchIteration(wk, a, grids, st, false, &ctx->side); }, nullptr, &s->pairGraph, &key, &ctx->retired))
+            return rc;
+        wfPairsOut<<<(items + 255) / 256, 256, 0, st>>>(pair.out, pair.status, items, rgba + 4 * first, status + first,
+                                                        s->integrateSlot.counters);
     }
     return X2_OK;
 }
@@ -2551,7 +2564,7 @@ int renderAdaptive(x2_scene* s, uint32_t minSamples, uint32_t maxSamples, float 
     };
     const bool again = kept.exec && kept.key.size() == sizeof(key) && !std::memcmp(kept.key.data(), &key, sizeof(key));
     if (!again) {
-        kept.drop(s->ctx->retired);
+        kept.drop();
         // Built in segments: each captured onto the graph after the last segment's end nodes.
         GraphSegments g;
         g.st = st;

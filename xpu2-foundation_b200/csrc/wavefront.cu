@@ -183,7 +183,8 @@ __device__ __forceinline__ void logicBody(const WaveArgs& a) {
     extern __shared__ float partial[];  // the adjoint's block partials
     const Layout at{a.adj.materials, a.adj.lights};
     if (kAdjoint) partialsBegin(partial, at);
-    const unsigned long long itemCount = a.liveChunks ? (unsigned long long)(*a.liveChunks) * 64ull * a.samplesPerChunk : a.itemCount;
+    const unsigned long long itemCount =
+        a.liveChunks ? (unsigned long long)(*a.liveChunks) * (a.pairs ? 1ull : 64ull * a.samplesPerChunk) : a.itemCount;
     for (uint32_t base = blockIdx.x * blockDim.x; base < a.paths; base += gridDim.x * blockDim.x) {
         const uint32_t p = base + threadIdx.x;
         uint32_t st = p < a.paths ? w.state[p] : kTrace + 100;  // out of range: no work, no claim

@@ -106,7 +106,8 @@ struct WaveArgs {
     const uint64_t* chunkMask;
     const uint32_t* pixelBase;
     // A launch queued before its chunks are known (an adaptive frame's pass): its chunk count in device memory, read
-    // when the launch runs; its items are that count x 64 x samplesPerChunk (null: itemCount and the count given).
+    // when the launch runs; its items are that count x 64 x samplesPerChunk (null: itemCount and the count given). The
+    // per-sample entry: its list's length, the items themselves.
     const uint32_t* liveChunks;
     uint32_t refill;       // a warp fetches new rays once this many of its lanes are idle (1..32)
     uint32_t triLimit;     // triangle tests a lane makes a traversal step
