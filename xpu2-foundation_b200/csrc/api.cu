@@ -1402,7 +1402,8 @@ uint32_t pairPaths(x2_scene* s, uint64_t n, const uint32_t* pairs) {
 // Nothing that a window's graph is launched with is the call's own: the list is copied to a place of its own, its length
 // lies in a word, the outputs are handed out behind the graph, and paths and window are rounded up (pairClass). So lists of
 // about the last one's length find its graph (with the caller's arrays in it every list of another length built one, and
-// put one by: 50,000 to 50,199 samples of the closed box 1.09 ms a call instead of 0.82). kind: where pairs lies; a host list is one window at most.
+// put one by: 50,000 to 50,199 samples of the closed box 1.09 ms a call instead of 0.82). kind: where pairs lies; a host
+// list is one window at most.
 int integrateWavefront(x2_scene* s, uint32_t paths, const uint32_t* pairs, cudaMemcpyKind kind, uint64_t n, double* rgba, uint32_t* status) {
     const uint32_t records = s->config.light_count * s->config.light_samples + 1;
     const uint32_t window = n <= paths ? paths : uint32_t(std::min<uint64_t>(pairClass(n), kPairWindow));
