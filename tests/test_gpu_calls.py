@@ -247,3 +247,18 @@ def test_one_scene_every_call_in_turn(ctx):
         for g, w in zip(got, want):
             assert np.array_equal(g, w) if exact else np.allclose(g, w, rtol=1e-12, atol=1e-12), k
     scene.free()
+
+
+def test_sample_lists_that_share_a_launch(ctx):
+    """Lists of lengths about the steps that a launch's slots are rounded to, longer and shorter ones in turn: each list's own
+    samples, whatever the last one left in its place."""
+    s = x2.SyntheticScene(0)
+    scene = x2.Scene(ctx, s.desc, s.config)
+    rng = np.random.default_rng(8)
+    lengths = [2048, 2000, 2047, 1, 1024, 1023, 1025, 1152, 1153, 2049, 2176, 2177, 2100, 2048, 5, 36864, 36865, 34000, 36864]
+    lists = [(rng.integers(0, s.config.width * s.config.height, n, dtype=np.uint32), rng.integers(0, 1 << 16, n, dtype=np.uint32)) for n in lengths]
+    got = [scene.integrate(*each) for each in lists]
+    want, want_status = one_thread(scene, np.concatenate([p for p, _ in lists]), np.concatenate([i for _, i in lists]))
+    scene.free()
+    assert np.array_equal(np.concatenate([r for r, _ in got]), want)
+    assert np.array_equal(np.concatenate([t for _, t in got]), want_status)
